@@ -115,6 +115,11 @@ int ctx_fail(mdet_ctx* ctx, int code, const char* fmt, ...);
 int ctx_cuda(mdet_ctx* ctx, cudaError_t e, const char* what);
 int ctx_check_launch(mdet_ctx* ctx, const char* what);
 
+// Tensor map over a row-major [rows][cols] array of eb-byte elements (2: BF16,
+// 4: FP32), box {box_k elements, box_rows rows}; rows past the array read zeros.
+int tensor_map_2d(mdet_ctx* ctx, CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint32_t box_k,
+                  uint32_t box_rows, CUtensorMapSwizzle sw, int eb);
+
 #define MDET_TRY(call)                     \
     do {                                   \
         int _rc = (call);                  \

@@ -634,35 +634,11 @@ __global__ void __launch_bounds__(Shape<BM, BN, NST, EB>::kThreads, Shape<BM, BN
 
 // ---------------------------------------------------------------- host --
 
-PFN_cuTensorMapEncodeTiled_v12000 get_encode(mdet_ctx* ctx) {
-    if (!ctx->encode_tiled) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
-                cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            return nullptr;
-        ctx->encode_tiled = fn;
-    }
-    return (PFN_cuTensorMapEncodeTiled_v12000)ctx->encode_tiled;
-}
-
 // Tensor map over [rows][144] elements of eb bytes (2: BF16, 4: FP32 holding
 // TF32 values), box {box_k elements, box_rows rows}.
 int make_map(mdet_ctx* ctx, CUtensorMap* map, const void* base, uint64_t rows, uint32_t box_k, uint32_t box_rows,
              CUtensorMapSwizzle sw, int eb) {
-    auto enc = get_encode(ctx);
-    if (!enc) return ctx_fail(ctx, MDET_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-    cuuint64_t dims[2] = {MDET_KPAD, rows};
-    cuuint64_t strides[1] = {(cuuint64_t)MDET_KPAD * eb};
-    cuuint32_t box[2] = {box_k, box_rows};
-    cuuint32_t es[2] = {1, 1};
-    CUresult r = enc(map, eb == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                     (void*)base, dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return ctx_fail(ctx, MDET_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-    return MDET_OK;
+    return tensor_map_2d(ctx, map, base, MDET_KPAD, rows, box_k, box_rows, sw, eb);
 }
 
 template <int BM, int BN, int NST, int EB>
@@ -740,4 +716,33 @@ int filter_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, con
     }
     return launch_tc<128, 256, 2, 2>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
                                      row_tbl, tbl_stride, rowoff);
+}
+
+static PFN_cuTensorMapEncodeTiled_v12000 get_encode(mdet_ctx* ctx) {
+    if (!ctx->encode_tiled) {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            return nullptr;
+        ctx->encode_tiled = fn;
+    }
+    return (PFN_cuTensorMapEncodeTiled_v12000)ctx->encode_tiled;
+}
+
+int tensor_map_2d(mdet_ctx* ctx, CUtensorMap* map, const void* base, uint64_t cols, uint64_t rows, uint32_t box_k,
+                  uint32_t box_rows, CUtensorMapSwizzle sw, int eb) {
+    auto enc = get_encode(ctx);
+    if (!enc) return ctx_fail(ctx, MDET_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+    cuuint64_t dims[2] = {cols, rows};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * eb};
+    cuuint32_t box[2] = {box_k, box_rows};
+    cuuint32_t es[2] = {1, 1};
+    CUresult r = enc(map, eb == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                     (void*)base, dims, strides, box, es,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return ctx_fail(ctx, MDET_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return MDET_OK;
 }

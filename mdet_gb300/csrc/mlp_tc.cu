@@ -23,8 +23,8 @@
 // each epilogue multiplying by GELU' of the saved pre-activation and writing
 // dZ in FP32 (bias gradients) and transposed BF16.  Weight gradients
 // (k_mlp_dw_tc): dW = dZ^T H with K = the batch's rows, split over CTAs, the
-// A and B tiles staged from the transposed arrays, partial sums added into
-// the FP32 gradient.  Numerics: BF16 GEMM operands, FP32 accumulation.  All
+// A and B tiles brought by TMA from the transposed arrays, partial sums added
+// into the FP32 gradient.  Numerics: BF16 GEMM operands, FP32 accumulation.  All
 // waits are bounded.
 #include <cuda_bf16.h>
 
@@ -52,9 +52,6 @@ constexpr uint32_t kImgBytes = kW1Bytes + kW2Bytes + kW3Bytes + kW3tBytes + kW2t
 // the backward kernel's operands take 96 KB; 120 KB keeps it at one CTA per
 // SM, so that its 512 TMEM columns are never contended
 constexpr uint32_t kSmemBwd = 120 * 1024;
-// weight gradients: an A chunk (128 x 64) and a B chunk (up to 256 x 64);
-// 100 KB allows two CTAs per SM, whose 256 TMEM columns each fit together
-constexpr uint32_t kSmemDw = 100 * 1024;
 constexpr uint32_t kTmemCols = 512;                  // layer outputs at columns 0, 256, 384
 constexpr uint32_t kLayoutSW128 = 2;
 
@@ -474,23 +471,62 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_bwd_tc(const float* __restr
     ch.finish(kTmemCols);
 }
 
-// Weight gradient dW[m][c] += sum_k A[m][k] B[c][k] for m < M, c < nout:
-// A = dZ^T ([M][ld] BF16), B = H^T ([nb][ld] BF16, rows nb .. nn - 1 read as
-// zeros), over this CTA's K range [k0, k0 + kspan) of the ld rows; a 128-row
-// block of dW per blockIdx.x (M = 64 fills the block's lower half, the rest
-// zeros), nn (a multiple of 16, <= 256) accumulator columns.
-__global__ void __launch_bounds__(kThreads, 1) k_mlp_dw_tc(const __nv_bfloat16* __restrict__ A, uint32_t M,
-                                                            const __nv_bfloat16* __restrict__ B, uint32_t nb,
-                                                            uint32_t nn, uint32_t nout, uint64_t ld, uint64_t kspan,
-                                                            float* __restrict__ dW, int* flag) {
+// Weight gradients dW[m][c] += sum_k A[m][k] B[c][k], A = dZ^T ([M][ld]
+// BF16), B = H^T ([nb][ld] BF16): the three layers in one launch.  A CTA
+// takes one 128-row block of one dW (blockIdx.x: dW3, dW2, the two halves of
+// dW1) over a span of K chunks (64 rows of the batch each, blockIdx.y).
+//
+// The work is small (2.5 GFLOP and 32 MB from L2 at 16,384 rows), so what
+// bounds a CTA is the latency of its chunks: they come by TMA into a
+// four-stage ring (one thread issues the copies, another the MMAs), all of a
+// short span in flight at once, and the spans are as many as keep one CTA on
+// every SM.  Partial sums go into the FP32 gradient four columns at a time
+// (red.v4).  16,384 rows: 317 us for the three launches whose threads
+// staged 512-row spans synchronously, 15.4 us so.
+constexpr int kDwStages = 4;
+constexpr uint32_t kDwStageBytes = kChunkA + 256 * 128;
+constexpr uint32_t kSmemDw = kDwStages * kDwStageBytes + 1024;
+
+struct DwMaps {
+    CUtensorMap a[3], b[3];
+};
+struct DwJob {
+    uint32_t M, nn, nout;  // rows of dW, accumulator columns (a multiple of 16), columns of dW
+    float* out;
+};
+struct DwArgs {
+    DwJob job[3];
+    uint32_t chunks, span;  // K chunks in all and per CTA
+    int* flag;
+};
+struct __align__(8) DwCtl {
+    uint64_t full[kDwStages], empty[kDwStages], done;
+    uint32_t tmem_base;
+};
+
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
+}
+
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+__global__ void __launch_bounds__(kThreads, 1) k_mlp_dw_tc(const __grid_constant__ DwMaps maps, DwArgs p) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ MlpCtl ctl;
+    __shared__ DwCtl ctl;
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    unsigned char* sA = smem;                 // 128 rows x 64 K
-    unsigned char* sB = smem + kChunkA;       // nn rows x 64 K
     const uint32_t t = threadIdx.x, warp = t >> 5;
     if (t == 0) {
-        mbar_init(&ctl.mma_done, 1);
+        for (int s = 0; s < kDwStages; ++s) {
+            mbar_init(&ctl.full[s], 1);
+            mbar_init(&ctl.empty[s], 1);
+        }
+        mbar_init(&ctl.done, 1);
         mbar_fence_init();
     }
     if (warp == 0) {
@@ -503,57 +539,48 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_dw_tc(const __nv_bfloat16* 
     __syncthreads();
     fence_after();
     const uint32_t tmem = ctl.tmem_base;
-    const uint32_t m0 = blockIdx.x * kRows;
-    const uint64_t k0 = blockIdx.y * kspan, k1 = min(ld, k0 + kspan);
-    const uint32_t sa = smem_u32(sA), sb = smem_u32(sB);
-    uint32_t ph = 0;
-    bool ok = true, any = false;
-    for (uint64_t kc = k0; kc < k1; kc += 64) {
-        // stage the K chunk [kc, kc + 64) of A's 128 rows and B's nn rows
-        for (uint32_t gi = t; gi < (kRows + nn) * 8; gi += kThreads) {
-            const uint32_t row = gi >> 3, kg = (gi & 7) * 8;
-            uint4 u = make_uint4(0, 0, 0, 0);
-            if (row < kRows) {
-                if (m0 + row < M && kc + kg < k1)
-                    u = *reinterpret_cast<const uint4*>(A + (uint64_t)(m0 + row) * ld + kc + kg);
-                *reinterpret_cast<uint4*>(sA + swz(kRows, row, kg)) = u;
-            } else {
-                const uint32_t c = row - kRows;
-                if (c < nb && kc + kg < k1) u = *reinterpret_cast<const uint4*>(B + (uint64_t)c * ld + kc + kg);
-                *reinterpret_cast<uint4*>(sB + swz(nn, c, kg)) = u;
-            }
+    const uint32_t which = blockIdx.x < 2 ? blockIdx.x : 2, m0 = blockIdx.x == 3 ? kRows : 0;
+    const DwJob job = p.job[which];
+    const uint32_t c0 = blockIdx.y * p.span, c1 = min(p.chunks, c0 + p.span);
+    if (t == 0) {
+        const uint32_t bytes = kChunkA + job.nn * 128;
+        for (uint32_t c = c0; c < c1; ++c) {
+            const uint32_t s = (c - c0) % kDwStages, round = (c - c0) / kDwStages;
+            if (!mbar_wait(&ctl.empty[s], (round & 1) ^ 1, p.flag)) break;
+            unsigned char* st = smem + s * kDwStageBytes;
+            mbar_arrive_tx(&ctl.full[s], bytes);
+            tma_load_2d(st, &maps.a[which], (int)(c * 64), (int)m0, &ctl.full[s]);
+            tma_load_2d(st + kChunkA, &maps.b[which], (int)(c * 64), 0, &ctl.full[s]);
         }
-        fence_proxy_async_smem();
-        fence_before();
-        __syncthreads();
-        fence_after();
-        if (t == 0) {
-            for (int s = 0; s < 4; ++s)
-                mma_bf16(tmem, desc_sw128(sa + s * 32), desc_sw128(sb + s * 32), idesc(nn), (any || s > 0) ? 1u : 0u);
-            mma_commit(&ctl.mma_done);
-        }
-        any = true;
-        const bool w = mbar_wait(&ctl.mma_done, ph, flag);
-        ph ^= 1;
-        fence_after();
-        if (__syncthreads_or(!w)) {
-            ok = false;
-            break;
+    } else if (t == 32) {
+        const uint32_t base = smem_u32(smem), id = idesc(job.nn);
+        for (uint32_t c = c0; c < c1; ++c) {
+            const uint32_t s = (c - c0) % kDwStages, round = (c - c0) / kDwStages;
+            if (!mbar_wait(&ctl.full[s], round & 1, p.flag)) break;
+            fence_after();
+            const uint32_t sa = base + s * kDwStageBytes, sb = sa + kChunkA;
+            for (int k = 0; k < 4; ++k)
+                mma_bf16(tmem, desc_sw128(sa + k * 32), desc_sw128(sb + k * 32), id, (c > c0 || k > 0) ? 1u : 0u);
+            mma_commit(&ctl.empty[s]);
+            if (c + 1 == c1) mma_commit(&ctl.done);
         }
     }
-    if (ok && any) {
+    __syncwarp();
+    // every thread waits for the last MMA, also to keep the ring alive
+    const bool ok = c0 < c1 && mbar_wait(&ctl.done, 0, p.flag);
+    fence_after();
+    if (__syncthreads_and(ok)) {
         const uint32_t tmem_row = tmem + ((warp * 32) << 16);
         const uint32_t m = m0 + t;
+        float* row = job.out + (uint64_t)m * job.nout;
 #pragma unroll 1
-        for (uint32_t q = 0; q * 32 < nn; ++q) {
+        for (uint32_t q = 0; q * 32 < job.nout; ++q) {
             float v[32];
             tmem_ld32(tmem_row + 32 * q, v);
-            if (m < M)
+            if (m < job.M)
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const uint32_t c = 32 * q + j;
-                    if (c < nout) atomicAdd(dW + (uint64_t)m * nout + c, v[j]);
-                }
+                for (int j = 0; j < 32; j += 4)
+                    if (32 * q + j < job.nout) red_add4(row + 32 * q + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
         }
     }
     fence_before();
@@ -563,13 +590,46 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_dw_tc(const __nv_bfloat16* 
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
-__global__ void k_colsum_tc(const float* __restrict__ d, uint64_t rows, int cols, float* __restrict__ g) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    const uint64_t r0 = blockIdx.y * 256ull, r1 = min(rows, r0 + 256);
-    float s = 0.f;
-    for (uint64_t r = r0; r < r1; ++r) s += d[r * cols + c];
-    atomicAdd(&g[c], s);
+// Bias gradients: column sums of the three FP32 output gradients, 64 rows of
+// the batch per block -- a thread sums four columns over half of them, the
+// block's halves meet in shared memory and go out with red.v4.  (16,384
+// rows: 50 us for three launches of one thread per column over 256 rows,
+// a chain of dependent loads; 11 us so.)
+constexpr int kBiasCols4 = (MLP_OUT + MLP_H2 + MLP_H1) / 4;  // 112 groups of four columns
+constexpr int kBiasRows = 64;
+__global__ void __launch_bounds__(2 * kBiasCols4) k_bias_grad(const float* __restrict__ d3,
+                                                              const float* __restrict__ d2,
+                                                              const float* __restrict__ d1, uint64_t rows,
+                                                              float* __restrict__ g) {
+    __shared__ float4 half[kBiasCols4];
+    const uint32_t c = threadIdx.x % kBiasCols4, part = threadIdx.x / kBiasCols4;
+    const float* src;
+    uint32_t ld;
+    float* dst;
+    if (c < MLP_OUT / 4) {
+        src = d3 + 4 * c, ld = MLP_OUT, dst = g + MLP_B3 + 4 * c;
+    } else if (c < (MLP_OUT + MLP_H2) / 4) {
+        src = d2 + 4 * (c - MLP_OUT / 4), ld = MLP_H2, dst = g + MLP_B2 + 4 * (c - MLP_OUT / 4);
+    } else {
+        src = d1 + 4 * (c - (MLP_OUT + MLP_H2) / 4), ld = MLP_H1, dst = g + MLP_B1 + 4 * (c - (MLP_OUT + MLP_H2) / 4);
+    }
+    const uint64_t r0 = blockIdx.x * (uint64_t)kBiasRows + part * (kBiasRows / 2);
+    const uint64_t r1 = min(rows, r0 + kBiasRows / 2);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (uint64_t r = r0; r < r1; ++r) {
+        const float4 x = *reinterpret_cast<const float4*>(src + r * ld);
+        s.x += x.x;
+        s.y += x.y;
+        s.z += x.z;
+        s.w += x.w;
+    }
+    if (part) half[c] = s;
+    __syncthreads();
+    if (!part) {
+        const float4 h = half[c];
+        red_add4(dst, s.x + h.x, s.y + h.y, s.z + h.z, s.w + h.w);
+    }
 }
 
 int weight_images(mdet_ctx* ctx, const float* P, unsigned char** img) {
@@ -658,39 +718,37 @@ int mlp_backward_tc(mdet_ctx* ctx, const float* P, const MlpTcActs& a, uint64_t 
     MDET_TRY(set_attrs(ctx));
     const unsigned char* img = (const unsigned char*)ctx_scratch(ctx, "mlptc.wimg", kImgBytes);  // from the forward
     MDET_CUDA(ctx, cudaMemsetAsync(grad, 0, MLP_NTRAIN * 4, s));
-    MDET_CUDA(ctx, cudaMemsetAsync(a.d3, 0, ld * MLP_OUT * 4, s));
+    if (ld > rows)  // the loss writes the real rows
+        MDET_CUDA(ctx, cudaMemsetAsync(a.d3 + rows * MLP_OUT, 0, (ld - rows) * MLP_OUT * 4, s));
     MDET_TRY(mlp_pair_loss(ctx, a.z3, np, labels, m_pos, m_neg, a.d3, loss_sum));
     const uint64_t tiles = ld / kRows;
     const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)ctx->num_sms);
     k_mlp_bwd_tc<<<grid, kThreads, kSmemBwd, s>>>(a.d3, rows, ld, a.z1, a.z2, img, a.d2, a.d1, a.d3T, a.d2T, a.d1T,
                                                    ctx->d_flag);
     MDET_LAUNCHED(ctx, "k_mlp_bwd_tc");
-    // weight gradients: K = the ld rows in spans of 512 rows per CTA
-    const uint64_t kspan = 512;
-    const unsigned ks = (unsigned)((ld + kspan - 1) / kspan);
-    struct Dw {
+    // weight gradients: the K chunks in as many spans as give every SM one CTA
+    struct Src {
         const __nv_bfloat16* A;
-        uint32_t M;
         const __nv_bfloat16* B;
-        uint32_t nb, nn, nout;
-        float* out;
-    } dws[3] = {
-        {a.d3T, MLP_OUT, a.h2T, MLP_H2, MLP_H2, MLP_H2, grad + MLP_W3},
-        {a.d2T, MLP_H2, a.h1T, MLP_H1, MLP_H1, MLP_H1, grad + MLP_W2},
-        {a.d1T, MLP_H1, a.xT, 64 * kKc1, 144, MLP_IN, grad + MLP_W1},  // K = 136 padded to 144 columns
-    };
-    for (const Dw& d : dws) {
-        dim3 g((d.M + kRows - 1) / kRows, ks);
-        k_mlp_dw_tc<<<g, kThreads, kSmemDw, s>>>(d.A, d.M, d.B, d.nb, d.nn, d.nout, ld, kspan, d.out, ctx->d_flag);
-        MDET_LAUNCHED(ctx, "k_mlp_dw_tc");
+        uint32_t nb;
+    } src[3] = {{a.d3T, a.h2T, MLP_H2}, {a.d2T, a.h1T, MLP_H1}, {a.d1T, a.xT, 64 * kKc1}};
+    DwArgs p;
+    p.job[0] = {MLP_OUT, MLP_H2, MLP_H2, grad + MLP_W3};
+    p.job[1] = {MLP_H2, MLP_H1, MLP_H1, grad + MLP_W2};
+    p.job[2] = {MLP_H1, 144, MLP_IN, grad + MLP_W1};  // 136 columns, padded to 144
+    DwMaps maps;
+    for (int k = 0; k < 3; ++k) {
+        MDET_TRY(tensor_map_2d(ctx, &maps.a[k], src[k].A, ld, p.job[k].M, 64, kRows, CU_TENSOR_MAP_SWIZZLE_128B, 2));
+        MDET_TRY(tensor_map_2d(ctx, &maps.b[k], src[k].B, ld, src[k].nb, 64, p.job[k].nn, CU_TENSOR_MAP_SWIZZLE_128B,
+                               2));
     }
-    // bias gradients: column sums of the FP32 output gradients
-    const dim3 cg(1, (unsigned)((rows + 255) / 256));
-    k_colsum_tc<<<cg, MLP_OUT, 0, s>>>(a.d3, rows, MLP_OUT, grad + MLP_B3);
-    MDET_LAUNCHED(ctx, "k_colsum_tc");
-    k_colsum_tc<<<cg, MLP_H2, 0, s>>>(a.d2, rows, MLP_H2, grad + MLP_B2);
-    MDET_LAUNCHED(ctx, "k_colsum_tc");
-    k_colsum_tc<<<cg, MLP_H1, 0, s>>>(a.d1, rows, MLP_H1, grad + MLP_B1);
-    MDET_LAUNCHED(ctx, "k_colsum_tc");
+    constexpr uint32_t kBlocks = 4;  // 128-row blocks of the three gradients
+    p.chunks = (uint32_t)(ld / 64);
+    p.span = std::max<uint32_t>(1, (p.chunks * kBlocks + ctx->num_sms - 1) / ctx->num_sms);
+    p.flag = ctx->d_flag;
+    k_mlp_dw_tc<<<dim3(kBlocks, (p.chunks + p.span - 1) / p.span), kThreads, kSmemDw, s>>>(maps, p);
+    MDET_LAUNCHED(ctx, "k_mlp_dw_tc");
+    k_bias_grad<<<(unsigned)((rows + kBiasRows - 1) / kBiasRows), 2 * kBiasCols4, 0, s>>>(a.d3, a.d2, a.d1, rows, grad);
+    MDET_LAUNCHED(ctx, "k_bias_grad");
     return MDET_OK;
 }
