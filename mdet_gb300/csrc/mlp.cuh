@@ -50,13 +50,14 @@ int mlp_embed(mdet_ctx* ctx, const float* params, const float* tnf, uint64_t n, 
 int mlp_embed_tc(mdet_ctx* ctx, const float* params, const float* tnf, uint64_t n, float* z, const uint32_t* idx);
 
 // Training on the tensor cores (mlp_tc.cu): rows padded to ld (a multiple of
-// 128); FP32 pre-activations and output gradients row-major, BF16 GEMM
-// operands of the weight gradients feature-major ([features][ld]).
+// 128); the embedding and its gradient row-major, the FP32 pre-activations
+// and the BF16 GEMM operands of the weight gradients feature-major
+// ([features][ld]).
 #include <cuda_bf16.h>
 struct MlpTcActs {
     uint64_t ld;
-    float *z1, *z2, *z3;  // [ld][256], [ld][128], [ld][64] (z3: the embedding)
-    float *d3, *d2, *d1;  // dL/dz3, dL/dz2, dL/dz1
+    float *z1, *z2;                 // [256][ld], [128][ld]
+    float *z3, *d3;                 // [ld][64]: the embedding and dL/dz3
     __nv_bfloat16 *xT, *h1T, *h2T;  // layer inputs: [192][ld], [256][ld], [128][ld]
     __nv_bfloat16 *d3T, *d2T, *d1T; // output gradients: [64][ld], [128][ld], [256][ld]
 };

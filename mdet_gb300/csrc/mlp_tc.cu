@@ -10,18 +10,18 @@
 // granule g of row r stored at g ^ (r mod 8)).  The weights are laid out in
 // that image once per call (k_mlp_wimage) and copied into shared memory with
 // one bulk copy per layer; the input rows are centred, scaled and rounded to
-// BF16 by the CTA's threads as they are staged.  Each thread owns one TMEM
-// lane (a row of the tile): a layer's epilogue reads its row of the
+// BF16 by the CTA's threads as they are staged.  Four threads share a TMEM
+// lane (a row of the tile): a layer's epilogue reads their parts of the row's
 // accumulator (tcgen05.ld), adds the bias, applies GELU, rounds to BF16 and
 // writes the row into the next layer's A operand; the last layer's row goes to
 // global memory in FP32.  For training the forward pass also keeps the
-// pre-activations (FP32) and the BF16 layer inputs transposed (feature-major),
-// the operands of the weight gradients.
+// pre-activations (FP32) and the BF16 layer inputs, feature-major (the latter
+// are the operands of the weight gradients).
 //
 // Backward (k_mlp_bwd_tc): per 128-row tile, dH2 = dZ3 W3 and dH1 = dZ2 W2 as
 // the same fused two-layer scheme (B operands: the transposed weight images),
-// each epilogue multiplying by GELU' of the saved pre-activation and writing
-// dZ in FP32 (bias gradients) and transposed BF16.  Weight gradients
+// each epilogue multiplying by GELU' of the saved pre-activation, adding dZ's
+// FP32 column sums into the bias gradients and writing it in transposed BF16.  Weight gradients
 // (k_mlp_dw_tc): dW = dZ^T H with K = the batch's rows, split over CTAs, the
 // A and B tiles brought by TMA from the transposed arrays, partial sums added
 // into the FP32 gradient.  Numerics: BF16 GEMM operands, FP32 accumulation.  All
@@ -35,7 +35,12 @@
 namespace {
 
 constexpr int kRows = 128;                 // rows per tile = TMEM lanes
-constexpr int kThreads = 128;
+constexpr int kThreads = 128;              // weight gradients: one thread per TMEM lane
+// The layer chains run kSplit threads per row: the epilogues (GELU, BF16,
+// the kept arrays) are what bounds a tile, and one CTA of 128 threads left
+// three quarters of an SM's warps unused.
+constexpr int kSplit = 4;
+constexpr int kChainThreads = kRows * kSplit;
 constexpr uint32_t kChunkA = kRows * 128;  // one 64-element K chunk of a 128-row operand
 // K chunks (64 elements) of each layer's input; 136 is padded to 192
 constexpr int kKc1 = 3, kKc2 = MLP_H1 / 64, kKc3 = MLP_H2 / 64;
@@ -161,8 +166,8 @@ struct __align__(8) MlpCtl {
     uint32_t tmem_base;
 };
 
-// The per-CTA machinery of a fused layer chain: 128 threads, one TMEM lane
-// each, an A operand (act) written by the threads and a B operand (wsm)
+// The per-CTA machinery of a fused layer chain: kSplit threads per TMEM lane
+// (tile row), an A operand (act) written by the threads and a B operand (wsm)
 // bulk-copied from a weight image.
 struct Chain {
     MlpCtl* ctl;
@@ -242,9 +247,10 @@ struct Chain {
     }
 };
 
-// Outputs the training pass keeps (null in inference): FP32 pre-activations
-// [rows][256] and [rows][128]; BF16 layer inputs transposed, [192][ld],
-// [256][ld] and [128][ld] (ld = the padded row count).
+// Outputs the training pass keeps (null in inference), all feature-major so
+// that a warp's 32 rows are one run (ld = the padded row count): FP32
+// pre-activations [256][ld] and [128][ld]; BF16 layer inputs [192][ld],
+// [256][ld] and [128][ld].
 struct FwdKeep {
     float* z1;
     float* z2;
@@ -254,23 +260,24 @@ struct FwdKeep {
     uint64_t ld;
 };
 
-// A hidden layer's epilogue for this thread's row r (global row g, kept when
-// g < n): columns [col0, col0 + 32 * NQ) of the accumulator, + bias, GELU,
-// BF16 into the next A operand; the training pass also keeps z and h^T.
+// A hidden layer's epilogue for this thread's part of row r (global row g,
+// kept when g < n): its share of the columns [col0, col0 + 32 * NQ) of the
+// accumulator, + bias, GELU, BF16 into the next A operand; the training pass
+// also keeps z^T and h^T.
 template <int NQ>
 __device__ __forceinline__ void epi_hidden(uint32_t tmem_row, uint32_t col0, const float* __restrict__ bias,
-                                           unsigned char* act, uint32_t r, float* zkeep, __nv_bfloat16* hT,
-                                           uint64_t ld, uint64_t g, bool keep) {
+                                           unsigned char* act, uint32_t r, uint32_t part, float* zkeep,
+                                           __nv_bfloat16* hT, uint64_t ld, uint64_t g, bool keep) {
+    static_assert(NQ % kSplit == 0, "whole groups of 32 columns per thread");
 #pragma unroll 1
-    for (int q = 0; q < NQ; ++q) {
+    for (int q = part * (NQ / kSplit); q < (int)(part + 1) * (NQ / kSplit); ++q) {
         float v[32];
         tmem_ld32(tmem_row + col0 + 32 * q, v);
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] += __ldg(bias + 32 * q + j);
         if (zkeep && keep) {
-            float4* zd = reinterpret_cast<float4*>(zkeep + g * (NQ * 32) + 32 * q);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) zd[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            for (int j = 0; j < 32; ++j) zkeep[(uint64_t)(32 * q + j) * ld + g] = v[j];
         }
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = gelu(v[j]);
@@ -292,7 +299,7 @@ __device__ __forceinline__ void epi_hidden(uint32_t tmem_row, uint32_t col0, con
 
 // Forward pass over n rows (row i is tnf row idx[i], or i without idx): the
 // embedding into z (FP32 [n][64]); with keep, the training outputs too.
-__global__ void __launch_bounds__(kThreads, 1) k_mlp_fwd_tc(const float* __restrict__ tnf,
+__global__ void __launch_bounds__(kChainThreads, 1) k_mlp_fwd_tc(const float* __restrict__ tnf,
                                                              const uint32_t* __restrict__ idx, uint64_t n,
                                                              const float* __restrict__ P,
                                                              const unsigned char* __restrict__ wimg,
@@ -302,10 +309,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fwd_tc(const float* __restr
     __shared__ float mu[MLP_IN];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t t = threadIdx.x, warp = t >> 5;
-    for (uint32_t k = t; k < MLP_IN; k += kThreads) mu[k] = P[MLP_MU + k];
+    const uint32_t row = t % kRows, part = t / kRows;  // warps w, w + 4, ... share a TMEM lane quarter
+    for (uint32_t k = t; k < MLP_IN; k += kChainThreads) mu[k] = P[MLP_MU + k];
     Chain ch;
     ch.init(&ctl, smem, kActBytes, kTmemCols, flag);
-    const uint32_t tmem_row = ch.tmem + ((warp * 32) << 16);
+    const uint32_t tmem_row = ch.tmem + (((warp & 3) * 32) << 16);
     const float scale = P[MLP_SCALE];
     const uint64_t tiles = (n + kRows - 1) / kRows;
     const bool train = keep.xT != nullptr;
@@ -314,7 +322,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fwd_tc(const float* __restr
         const uint64_t r0 = tile * kRows;
         // stage the tile's rows: centred, scaled, BF16, K padded to 192
         // (granule g: row g % 128, K columns 8 * (g / 128) .. + 7)
-        for (uint32_t gi = t; gi < kRows * kKc1 * 8; gi += kThreads) {
+#pragma unroll 2
+        for (uint32_t gi = t; gi < kRows * kKc1 * 8; gi += kChainThreads) {
             const uint32_t r = gi % kRows, k = (gi / kRows) * 8;
             float e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (r0 + r < n && k < MLP_IN) {
@@ -340,16 +349,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fwd_tc(const float* __restr
 #pragma unroll
                 for (int j = 0; j < 8; ++j) keep.xT[(uint64_t)(k + j) * keep.ld + r0 + r] = bf(e[j]);
         }
-        const uint64_t g = r0 + t;
+        const uint64_t g = r0 + row;
         const bool valid = g < n;
         if (!ch.layer(kW1Bytes, wimg, kKc1, MLP_H1, 0, MLP_H1)) break;
-        epi_hidden<MLP_H1 / 32>(tmem_row, 0, P + MLP_B1, ch.act, t, keep.z1, keep.h1T, keep.ld, g, valid);
+        epi_hidden<MLP_H1 / 32>(tmem_row, 0, P + MLP_B1, ch.act, row, part, keep.z1, keep.h1T, keep.ld, g,
+                                     valid);
         if (!ch.layer(kW2Bytes, wimg + kW1Bytes, kKc2, MLP_H2, 256, MLP_H2)) break;
-        epi_hidden<MLP_H2 / 32>(tmem_row, 256, P + MLP_B2, ch.act, t, keep.z2, keep.h2T, keep.ld, g, valid);
+        epi_hidden<MLP_H2 / 32>(tmem_row, 256, P + MLP_B2, ch.act, row, part, keep.z2, keep.h2T, keep.ld, g,
+                                     valid);
         if (!ch.layer(kW3Bytes, wimg + kW1Bytes + kW2Bytes, kKc3, MLP_OUT, 384, MLP_OUT)) break;
         // the embedding: + b3, FP32 to global
-#pragma unroll
-        for (int q = 0; q < MLP_OUT / 32; ++q) {
+        if (part < MLP_OUT / 32) {
+            const int q = part;
             float v[32];
             tmem_ld32(tmem_row + 384 + 32 * q, v);
             if (valid) {
@@ -370,32 +381,38 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_fwd_tc(const float* __restr
     ch.finish(kTmemCols);
 }
 
-// A backward layer's epilogue for this thread's row: columns [col0, col0 +
-// 32 * NQ) of dH, times GELU' of the saved pre-activation zs (FP32 row) ->
-// dZ: FP32 into dout (bias gradients), BF16 transposed into dT (weight
-// gradients), and BF16 into the next A operand when act is non-null.  Rows
-// at or past n give zeros.
+// Adds the 32 columns of v over the warp's 32 rows into g[0..31]: a
+// reduce-scatter (31 shuffles), after which lane j holds column j.
+__device__ __forceinline__ void add_columns(float (&v)[32], float* __restrict__ g) {
+    const uint32_t lane = lane_id();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    atomicAdd(g + lane, v[0]);
+}
+
+// A backward layer's epilogue for this thread's part of row r: its share of
+// the columns [col0, col0 + 32 * NQ) of dH, times GELU' of the saved
+// pre-activation zs (feature-major FP32) -> dZ: its column sums in FP32 into
+// the bias gradient db, BF16 transposed into dT (weight gradients), and BF16
+// into the next A operand when act is non-null.  Rows at or past n give zeros.
 template <int NQ>
-__device__ __forceinline__ void epi_back(uint32_t tmem_row, uint32_t col0, const float* zs, float* dout,
-                                         __nv_bfloat16* dT, uint64_t ld, unsigned char* act, uint32_t r, uint64_t g,
-                                         bool valid) {
+__device__ __forceinline__ void epi_back(uint32_t tmem_row, uint32_t col0, const float* zs, float* db,
+                                         __nv_bfloat16* dT, uint64_t ld, unsigned char* act, uint32_t r,
+                                         uint32_t part, uint64_t g, bool valid) {
 #pragma unroll 1
-    for (int q = 0; q < NQ; ++q) {
+    for (int q = part * (NQ / kSplit); q < (int)(part + 1) * (NQ / kSplit); ++q) {
         float v[32];
         tmem_ld32(tmem_row + col0 + 32 * q, v);
         if (valid) {
-            const float4* zr = reinterpret_cast<const float4*>(zs + g * (NQ * 32) + 32 * q);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float4 zz = zr[j];
-                v[4 * j] *= gelu_grad(zz.x);
-                v[4 * j + 1] *= gelu_grad(zz.y);
-                v[4 * j + 2] *= gelu_grad(zz.z);
-                v[4 * j + 3] *= gelu_grad(zz.w);
-            }
-            float4* dd = reinterpret_cast<float4*>(dout + g * (NQ * 32) + 32 * q);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) dd[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            for (int j = 0; j < 32; ++j) v[j] *= gelu_grad(zs[(uint64_t)(32 * q + j) * ld + g]);
         } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = 0.f;
@@ -413,33 +430,43 @@ __device__ __forceinline__ void epi_back(uint32_t tmem_row, uint32_t col0, const
                 *reinterpret_cast<uint4*>(act + swz(kRows, r, (uint32_t)(32 * q + 8 * c8))) = u;
             }
         }
+        add_columns(v, db + 32 * q);
     }
 }
 
 // Backward of the two upper layers over ld rows (n of them real): from
-// dZ3 (FP32 [ld][64]) to dZ2 and dZ1 (FP32, and BF16 transposed), dZ3^T too.
-__global__ void __launch_bounds__(kThreads, 1) k_mlp_bwd_tc(const float* __restrict__ d3, uint64_t n, uint64_t ld,
-                                                             const float* __restrict__ z1,
-                                                             const float* __restrict__ z2,
-                                                             const unsigned char* __restrict__ wimg,
-                                                             float* __restrict__ d2, float* __restrict__ d1,
-                                                             __nv_bfloat16* __restrict__ d3T,
-                                                             __nv_bfloat16* __restrict__ d2T,
-                                                             __nv_bfloat16* __restrict__ d1T, int* flag) {
+// dZ3 (FP32 [ld][64]) to dZ2 and dZ1 (BF16 transposed, dZ3^T too) and the
+// three bias gradients (FP32 column sums added into grad).
+//
+// 16,384 rows (one tile per SM), forward and backward: 39.6 and 37.4 us with
+// 128 threads a tile, row-major FP32 arrays (every store of a warp on 32
+// lines) and a separate pass for the bias gradients (11 us); 25.6 and 22.8 us
+// so.
+__global__ void __launch_bounds__(kChainThreads, 1) k_mlp_bwd_tc(const float* __restrict__ d3, uint64_t n, uint64_t ld,
+                                                                 const float* __restrict__ z1,
+                                                                 const float* __restrict__ z2,
+                                                                 const unsigned char* __restrict__ wimg,
+                                                                 float* __restrict__ grad,
+                                                                 __nv_bfloat16* __restrict__ d3T,
+                                                                 __nv_bfloat16* __restrict__ d2T,
+                                                                 __nv_bfloat16* __restrict__ d1T, int* flag) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ MlpCtl ctl;
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const uint32_t t = threadIdx.x, warp = t >> 5;
+    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const uint32_t row = t % kRows, part = t / kRows;
     Chain ch;
     ch.init(&ctl, smem, kRows * 2 * 128, kTmemCols, flag);  // A: up to 128 K (dZ2)
-    const uint32_t tmem_row = ch.tmem + ((warp * 32) << 16);
+    const uint32_t tmem_row = ch.tmem + (((warp & 3) * 32) << 16);
     const unsigned char* w3t = wimg + kW1Bytes + kW2Bytes + kW3Bytes;
     const unsigned char* w2t = w3t + kW3tBytes;
     const uint64_t tiles = (ld + kRows - 1) / kRows;
     for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint64_t r0 = tile * kRows;
-        // stage dZ3 as BF16 (K = 64), and dZ3^T
-        for (uint32_t gi = t; gi < kRows * 8; gi += kThreads) {
+        // stage dZ3 as BF16 (K = 64), and dZ3^T; a warp's 32 rows share a
+        // granule of eight columns, whose sums go into the bias gradient
+#pragma unroll 2
+        for (uint32_t gi = t; gi < kRows * 8; gi += kChainThreads) {
             const uint32_t r = gi % kRows, k = (gi / kRows) * 8;
             float e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (r0 + r < n) {
@@ -455,15 +482,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_bwd_tc(const float* __restr
             *reinterpret_cast<uint4*>(ch.act + swz(kRows, r, k)) = u;
 #pragma unroll
             for (int j = 0; j < 8; ++j) d3T[(uint64_t)(k + j) * ld + r0 + r] = bf(e[j]);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {  // lane l then holds column l % 8 of its quarter-warp's rows
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int i = 0; i < o; ++i) {
+                    const float keep = up ? e[i + o] : e[i], send = up ? e[i] : e[i + o];
+                    e[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            e[0] += __shfl_xor_sync(0xffffffffu, e[0], 8);
+            e[0] += __shfl_xor_sync(0xffffffffu, e[0], 16);
+            if (lane < 8) atomicAdd(grad + MLP_B3 + k + lane, e[0]);
         }
-        const uint64_t g = r0 + t;
+        const uint64_t g = r0 + row;
         const bool valid = g < n;
         // dH2 = dZ3 W3 (N = 128, K = 64)
         if (!ch.layer(kW3tBytes, w3t, 1, MLP_H2, 0, MLP_H2)) break;
-        epi_back<MLP_H2 / 32>(tmem_row, 0, z2, d2, d2T, ld, ch.act, t, g, valid);
+        epi_back<MLP_H2 / 32>(tmem_row, 0, z2, grad + MLP_B2, d2T, ld, ch.act, row, part, g, valid);
         // dH1 = dZ2 W2 (N = 256, K = 128)
         if (!ch.layer(kW2tBytes, w2t, 2, MLP_H1, 256, MLP_H1)) break;
-        epi_back<MLP_H1 / 32>(tmem_row, 256, z1, d1, d1T, ld, nullptr, t, g, valid);
+        epi_back<MLP_H1 / 32>(tmem_row, 256, z1, grad + MLP_B1, d1T, ld, nullptr, row, part, g, valid);
         fence_before();
         __syncthreads();
         fence_after();
@@ -590,48 +629,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_dw_tc(const __grid_constant
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
-// Bias gradients: column sums of the three FP32 output gradients, 64 rows of
-// the batch per block -- a thread sums four columns over half of them, the
-// block's halves meet in shared memory and go out with red.v4.  (16,384
-// rows: 50 us for three launches of one thread per column over 256 rows,
-// a chain of dependent loads; 11 us so.)
-constexpr int kBiasCols4 = (MLP_OUT + MLP_H2 + MLP_H1) / 4;  // 112 groups of four columns
-constexpr int kBiasRows = 64;
-__global__ void __launch_bounds__(2 * kBiasCols4) k_bias_grad(const float* __restrict__ d3,
-                                                              const float* __restrict__ d2,
-                                                              const float* __restrict__ d1, uint64_t rows,
-                                                              float* __restrict__ g) {
-    __shared__ float4 half[kBiasCols4];
-    const uint32_t c = threadIdx.x % kBiasCols4, part = threadIdx.x / kBiasCols4;
-    const float* src;
-    uint32_t ld;
-    float* dst;
-    if (c < MLP_OUT / 4) {
-        src = d3 + 4 * c, ld = MLP_OUT, dst = g + MLP_B3 + 4 * c;
-    } else if (c < (MLP_OUT + MLP_H2) / 4) {
-        src = d2 + 4 * (c - MLP_OUT / 4), ld = MLP_H2, dst = g + MLP_B2 + 4 * (c - MLP_OUT / 4);
-    } else {
-        src = d1 + 4 * (c - (MLP_OUT + MLP_H2) / 4), ld = MLP_H1, dst = g + MLP_B1 + 4 * (c - (MLP_OUT + MLP_H2) / 4);
-    }
-    const uint64_t r0 = blockIdx.x * (uint64_t)kBiasRows + part * (kBiasRows / 2);
-    const uint64_t r1 = min(rows, r0 + kBiasRows / 2);
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (uint64_t r = r0; r < r1; ++r) {
-        const float4 x = *reinterpret_cast<const float4*>(src + r * ld);
-        s.x += x.x;
-        s.y += x.y;
-        s.z += x.z;
-        s.w += x.w;
-    }
-    if (part) half[c] = s;
-    __syncthreads();
-    if (!part) {
-        const float4 h = half[c];
-        red_add4(dst, s.x + h.x, s.y + h.y, s.z + h.z, s.w + h.w);
-    }
-}
-
 int weight_images(mdet_ctx* ctx, const float* P, unsigned char** img) {
     *img = (unsigned char*)ctx_scratch(ctx, "mlptc.wimg", kImgBytes);
     if (!*img) return MDET_ERR_NOMEM;
@@ -657,7 +654,7 @@ int fwd_launch(mdet_ctx* ctx, const float* P, const unsigned char* img, const fl
     const uint64_t tiles = (n + kRows - 1) / kRows;
     const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)ctx->num_sms);
     ctx_timer_begin(ctx, "k_mlp_fwd_tc");
-    k_mlp_fwd_tc<<<grid, kThreads, kSmem, ctx->stream>>>(tnf, idx, n, P, img, z, keep, ctx->d_flag);
+    k_mlp_fwd_tc<<<grid, kChainThreads, kSmem, ctx->stream>>>(tnf, idx, n, P, img, z, keep, ctx->d_flag);
     MDET_LAUNCHED(ctx, "k_mlp_fwd_tc");
     ctx_timer_end(ctx, "k_mlp_fwd_tc");
     return MDET_OK;
@@ -687,15 +684,13 @@ int mlp_tc_alloc(mdet_ctx* ctx, const char* tag, uint64_t rows, MlpTcActs* a) {
     a->z2 = f(".z2", MLP_H2);
     a->z3 = f(".z3", MLP_OUT);
     a->d3 = f(".d3", MLP_OUT);
-    a->d2 = f(".d2", MLP_H2);
-    a->d1 = f(".d1", MLP_H1);
     a->xT = h(".xT", 64 * kKc1);
     a->h1T = h(".h1T", MLP_H1);
     a->h2T = h(".h2T", MLP_H2);
     a->d3T = h(".d3T", MLP_OUT);
     a->d2T = h(".d2T", MLP_H2);
     a->d1T = h(".d1T", MLP_H1);
-    return (a->z1 && a->z2 && a->z3 && a->d3 && a->d2 && a->d1 && a->xT && a->h1T && a->h2T && a->d3T && a->d2T &&
+    return (a->z1 && a->z2 && a->z3 && a->d3 && a->xT && a->h1T && a->h2T && a->d3T && a->d2T &&
             a->d1T)
                ? MDET_OK
                : MDET_ERR_NOMEM;
@@ -723,8 +718,8 @@ int mlp_backward_tc(mdet_ctx* ctx, const float* P, const MlpTcActs& a, uint64_t 
     MDET_TRY(mlp_pair_loss(ctx, a.z3, np, labels, m_pos, m_neg, a.d3, loss_sum));
     const uint64_t tiles = ld / kRows;
     const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)ctx->num_sms);
-    k_mlp_bwd_tc<<<grid, kThreads, kSmemBwd, s>>>(a.d3, rows, ld, a.z1, a.z2, img, a.d2, a.d1, a.d3T, a.d2T, a.d1T,
-                                                   ctx->d_flag);
+    k_mlp_bwd_tc<<<grid, kChainThreads, kSmemBwd, s>>>(a.d3, rows, ld, a.z1, a.z2, img, grad, a.d3T, a.d2T, a.d1T,
+                                                       ctx->d_flag);
     MDET_LAUNCHED(ctx, "k_mlp_bwd_tc");
     // weight gradients: the K chunks in as many spans as give every SM one CTA
     struct Src {
@@ -748,7 +743,5 @@ int mlp_backward_tc(mdet_ctx* ctx, const float* P, const MlpTcActs& a, uint64_t 
     p.flag = ctx->d_flag;
     k_mlp_dw_tc<<<dim3(kBlocks, (p.chunks + p.span - 1) / p.span), kThreads, kSmemDw, s>>>(maps, p);
     MDET_LAUNCHED(ctx, "k_mlp_dw_tc");
-    k_bias_grad<<<(unsigned)((rows + kBiasRows - 1) / kBiasRows), 2 * kBiasCols4, 0, s>>>(a.d3, a.d2, a.d1, rows, grad);
-    MDET_LAUNCHED(ctx, "k_bias_grad");
     return MDET_OK;
 }
