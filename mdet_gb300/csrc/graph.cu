@@ -325,7 +325,7 @@ int gather_rows_bf16(mdet_ctx* ctx, const GraphPrep& g, const uint32_t* row_map,
 
 int graph_candidates(mdet_ctx* ctx, const GraphPrep& g, double cutoff, int mode, uint2** cand, uint64_t* ncand) {
     DstarTable tbl;
-    MDET_TRY(build_dstar_table(ctx, g.ls, g.n, logit(cutoff), &tbl));
+    MDET_TRY(build_dstar_table(ctx, g.ls, g.n, logit(cutoff), &tbl, g.lrange));
     unsigned long long nc = 0;
     MDET_TRY(run_filter(ctx, mode, g, false, nullptr, nullptr, nullptr, 0, nullptr, nullptr, tbl, "g", cand, &nc));
     *ncand = nc;
@@ -341,7 +341,7 @@ int graph_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n
     MDET_TRY(abd_gate(ctx, g));
     const double L = logit(cutoff);
     DstarTable tbl;
-    MDET_TRY(build_dstar_table(ctx, g.ls, n, L, &tbl));
+    MDET_TRY(build_dstar_table(ctx, g.ls, n, L, &tbl, g.lrange));
     tm.mark();
     uint2* cand = nullptr;
     unsigned long long ncand = 0;
@@ -406,7 +406,7 @@ int graph_shard_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint
     const uint32_t s1 = (uint32_t)std::min<uint64_t>(n, blocks * (shard + 1) / nshards * 256);
     const double L = logit(cutoff);
     DstarTable tbl;
-    MDET_TRY(build_dstar_table(ctx, g.ls, n, L, &tbl));
+    MDET_TRY(build_dstar_table(ctx, g.ls, n, L, &tbl, g.lrange));
     tm.mark();
     uint2* cand = nullptr;
     unsigned long long ncand = 0;
@@ -461,7 +461,7 @@ int validate_graph_args(mdet_ctx* ctx, uint64_t n, double cutoff, uint32_t max_e
 
 // --- max-probability sample on a prepared contig set ---
 int maxprob_core(mdet_ctx* ctx, const GraphPrep& g, const uint64_t* d_contigs, uint64_t m, int mode,
-                 double floor_prob, double* d_out, double* lrange = nullptr) {
+                 double floor_prob, double* d_out) {
     cudaStream_t s = ctx->stream;
     if (m == 0) return MDET_OK;
     uint32_t* keys = (uint32_t*)ctx_scratch(ctx, "mp.keys", m * 4);
@@ -488,7 +488,7 @@ int maxprob_core(mdet_ctx* ctx, const GraphPrep& g, const uint64_t* d_contigs, u
     MDET_LAUNCHED(ctx, "k_sample_gather");
     const double L = floor_prob > 0 ? logit(floor_prob) : -INFINITY;
     DstarTable tbl;
-    MDET_TRY(build_dstar_table(ctx, g.ls, g.n, L, &tbl, true, lrange));
+    MDET_TRY(build_dstar_table(ctx, g.ls, g.n, L, &tbl, g.lrange));
     uint2* cand = nullptr;
     unsigned long long ncand = 0;
     if (mode != MDET_MODE_PLAIN) {
@@ -753,7 +753,6 @@ int mdet_tnf_ptnf_search_dev(mdet_ctx* ctx, const float* d_tnf, const double* d_
     // first floor of a pass: just below the previous pass's cutoff, on a
     // 0.005 grid so that passes share a d* table
     double next_floor = 0.9;
-    double lrange[2] = {NAN, NAN};  // log-size range of the sorted rows, found once
     auto sample = [&](bool full, double* p_out) -> int {
         uint64_t m = full ? n : std::min<uint64_t>(n, 2500);
         // random_unique (cuda/Cuda2.cu:500-511): a partial Fisher-Yates
@@ -800,7 +799,7 @@ int mdet_tnf_ptnf_search_dev(mdet_ctx* ctx, const float* d_tnf, const double* d_
         const double f1 = full ? floor_prob : std::max(floor_prob, next_floor);
         auto maxima = [&](const uint64_t* ids, uint64_t k, double floor, double* out) -> int {
             MDET_CUDA(ctx, cudaMemcpyAsync(d_idx, ids, k * 8, cudaMemcpyHostToDevice, s));
-            MDET_TRY(maxprob_core(ctx, g, d_idx, k, mode, floor, d_mx, lrange));
+            MDET_TRY(maxprob_core(ctx, g, d_idx, k, mode, floor, d_mx));
             MDET_CUDA(ctx, cudaMemcpyAsync(out, d_mx, k * 8, cudaMemcpyDeviceToHost, s));
             MDET_CUDA(ctx, cudaStreamSynchronize(s));
             return MDET_OK;

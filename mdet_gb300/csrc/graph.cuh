@@ -113,7 +113,8 @@ struct GraphPrep {
     float* nsq;                      // ||x~||^2 per sorted row (inf for padding rows)
     BlockMeta* meta;                 // per 128-row block (rounding of the rows held)
     BlockMeta* meta32;               // per 128-row block (no rounding term)
-    float* mu;                       // column means [136]
+    float* mu;                       // column means [136] (of every set)
+    double lrange[2];                // log-size range of a preparation in size order
     const uint8_t* low = nullptr;    // abundance gate: sorted position has no depth above 1 (null: no gate)
 };
 
@@ -133,20 +134,30 @@ inline int tc_kind(int mode) {
 // to make (kTcNone, kTcBf16, kTcTf32; a bool true means kTcBf16).
 int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, int tck, GraphPrep* out,
                 const uint32_t* order = nullptr);
-// Arrays of a prepared set of `rows` positions (a multiple of 256) in
-// scratch named after tag; prep_into fills positions [base, base + npad) of
-// them with one contig set (perm/inv values are base + local indices).
-int prep_alloc(mdet_ctx* ctx, const char* tag, uint64_t rows, int tck, GraphPrep* g);
-int prep_into(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, int tck, const GraphPrep& g,
-              uint64_t base, const uint32_t* order = nullptr);
-// sorted: d_ls_sorted is ascending (else its range is found by a scan).
-// range: optional host copy of the log-size range {min, max}; when given with
-// range[0] not NaN it is used as is, else it is found (one device round trip)
-// and stored there for the next call over the same sizes.
-int build_dstar_table(mdet_ctx* ctx, const double* d_ls_sorted, uint64_t n, double logit_cut, DstarTable* out,
-                      bool sorted = true, double* range = nullptr);
-// A table over a given log-size range written to st (MDET_TBL_LEVELS x TBL x TBL floats).
-int build_dstar_table_at(mdet_ctx* ctx, double lmin, double lmax, double logit_cut, float* st, DstarTable* out);
+// One contig set of a preparation: n contigs whose prepared rows start at
+// `base` (a multiple of 256).
+struct PrepSeg {
+    const float* tnf;
+    const double* ls;
+    uint32_t n, base;
+};
+// One set (`one`), or `count` of them laid end to end: segs, and the set of
+// every 256-row block, on the device.
+struct PrepSet {
+    uint32_t count;
+    PrepSeg one;
+    const PrepSeg* segs;
+    const uint32_t* blk_seg;
+};
+// Arrays of `rows` prepared positions (a multiple of 256) of `sets` contig sets
+// in scratch named after tag; prep_set fills them (perm/inv values are a set's
+// base + its local indices), without a host synchronisation.
+int prep_alloc(mdet_ctx* ctx, const char* tag, uint64_t rows, int tck, uint32_t sets, GraphPrep* g);
+int prep_set(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, const GraphPrep& g);
+// range: the log sizes' range {min, max} on the host (GraphPrep::lrange); null:
+// it is found by a scan of d_ls (one device round trip).
+int build_dstar_table(mdet_ctx* ctx, const double* d_ls, uint64_t n, double logit_cut, DstarTable* out,
+                      const double* range = nullptr);
 // The same over the union of `count` device ranges (lo, hi pairs; entries
 // with lo > hi are empty): no host synchronisation, grid left in *grid.
 int grid_from_ranges(mdet_ctx* ctx, const double* ranges, uint32_t count, TableGrid* grid);

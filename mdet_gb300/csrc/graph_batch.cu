@@ -151,6 +151,7 @@ struct Dev {
     uint8_t* rtbl;
     BlkCut* bcut;
     BatchOut* bo;
+    PrepSeg* segs;
     int* status;
     float* tbl;
     TableGrid* grid;
@@ -172,16 +173,18 @@ int upload_sides(mdet_ctx* ctx, const mdet_assembly* as, const Layout& L, Dev& d
     d.j1 = (uint32_t*)ctx_scratch(ctx, "bt.j1", (uint64_t)L.nrt * 4);
     d.off = (unsigned long long*)ctx_scratch(ctx, "bt.off", ((uint64_t)L.nrt + 1) * 8);
     d.bo = (BatchOut*)ctx_scratch(ctx, "bt.bo", count * sizeof(BatchOut));
+    d.segs = (PrepSeg*)ctx_scratch(ctx, "bt.segs", count * sizeof(PrepSeg));
     d.status = (int*)ctx_scratch(ctx, "bt.status", count * 4);
     d.tbl = (float*)ctx_scratch(ctx, "bt.tbl", L.tab_of.size() * MDET_TBL_FLOATS * 4);
     d.grid = (TableGrid*)ctx_scratch(ctx, "bt.grid", sizeof(TableGrid));
     if (!d.R || !d.n || !d.range || !d.outs || !d.rtbl || !d.bcut || !d.bK || !d.bA || !d.j0 || !d.j1 || !d.off ||
-        !d.bo || !d.status || !d.tbl || !d.grid)
+        !d.bo || !d.segs || !d.status || !d.tbl || !d.grid)
         return MDET_ERR_NOMEM;
     std::vector<uint8_t> row_tbl(L.nrt, 0);
     std::vector<BlkCut> bcut(L.nblk256);
     std::vector<uint32_t> bK(L.nblk256, 1), bA(L.nblk256, 0);
     std::vector<BatchOut> bo(count);
+    std::vector<PrepSeg> segs(count);
     for (uint32_t k = 0; k < count; ++k) {
         bo[k].from = as[k].d_from;
         bo[k].to = as[k].d_to;
@@ -190,6 +193,7 @@ int upload_sides(mdet_ctx* ctx, const mdet_assembly* as, const Layout& L, Dev& d
         bo[k].R = L.R[k];
         bo[k].n = L.nn[k];
         bo[k].pad[0] = bo[k].pad[1] = 0;
+        segs[k] = PrepSeg{as[k].d_tnf, as[k].d_log_size, L.nn[k], L.R[k]};
         const uint32_t npad = (L.nn[k] + 255) / 256 * 256;
         if (!npad) continue;
         const double Lc = logit(as[k].cutoff);
@@ -213,6 +217,7 @@ int upload_sides(mdet_ctx* ctx, const mdet_assembly* as, const Layout& L, Dev& d
     MDET_CUDA(ctx, cudaMemcpyAsync(d.bK, bK.data(), L.nblk256 * 4, cudaMemcpyHostToDevice, s));
     MDET_CUDA(ctx, cudaMemcpyAsync(d.bA, bA.data(), L.nblk256 * 4, cudaMemcpyHostToDevice, s));
     MDET_CUDA(ctx, cudaMemcpyAsync(d.bo, bo.data(), count * sizeof(BatchOut), cudaMemcpyHostToDevice, s));
+    MDET_CUDA(ctx, cudaMemcpyAsync(d.segs, segs.data(), count * sizeof(PrepSeg), cudaMemcpyHostToDevice, s));
     // the host vectors die here: wait for the copies
     MDET_CUDA(ctx, cudaStreamSynchronize(s));
     return MDET_OK;
@@ -247,13 +252,11 @@ int build_list(mdet_ctx* ctx, const Layout& L, Dev& d, int w, uint64_t* nlist) {
 }
 
 // Preparation and d* tables of every assembly; no host synchronisation.
-int prep_and_tables(mdet_ctx* ctx, const mdet_assembly* as, const Layout& L, bool bf16, Dev& d, GraphPrep& g,
-                    DstarTable* tbl) {
-    MDET_TRY(prep_alloc(ctx, "bt", L.N, bf16, &g));
+int prep_and_tables(mdet_ctx* ctx, const Layout& L, bool bf16, Dev& d, GraphPrep& g, DstarTable* tbl) {
+    MDET_TRY(prep_alloc(ctx, "bt", L.N, bf16, L.count, &g));
     g.n = (uint32_t)L.N;
     g.npad = (uint32_t)L.N;
-    for (uint32_t k = 0; k < L.count; ++k)
-        if (L.nn[k]) MDET_TRY(prep_into(ctx, as[k].d_tnf, as[k].d_log_size, L.nn[k], bf16, g, L.R[k]));
+    MDET_TRY(prep_set(ctx, PrepSet{L.count, PrepSeg{}, d.segs, d.bA}, L.N, bf16, g));
     k_batch_ends<<<(L.count + 127) / 128, 128, 0, ctx->stream>>>(g.ls, nullptr, d.R, d.n, L.count, d.range, d.outs);
     MDET_LAUNCHED(ctx, "k_batch_ends");
     MDET_TRY(grid_from_ranges(ctx, d.range, L.count, d.grid));
@@ -283,7 +286,7 @@ int device_pass(mdet_ctx* ctx, const mdet_assembly* as, const Layout& L, int mod
                 unsigned long long cap) {
     GraphPrep g;
     DstarTable tbl;
-    MDET_TRY(prep_and_tables(ctx, as, L, mode == MDET_MODE_BF16, d, g, &tbl));
+    MDET_TRY(prep_and_tables(ctx, L, mode == MDET_MODE_BF16, d, g, &tbl));
     uint2* cand = nullptr;
     unsigned long long ncap = 0, *ncand_dev = nullptr, *ne_dev = nullptr;
     MDET_TRY(run_filter(ctx, mode, g, false, nullptr, nullptr, nullptr, 0, nullptr, nullptr, tbl, "bt", &cand, &ncap,
@@ -490,7 +493,7 @@ extern "C" int mdet_tnf_graph_batched(mdet_ctx* ctx, mdet_assembly* as, uint32_t
             MDET_TRY(upload_sides(ctx, as, L, d));
             GraphPrep g;
             DstarTable tbl;
-            MDET_TRY(prep_and_tables(ctx, as, L, bf16, d, g, &tbl));
+            MDET_TRY(prep_and_tables(ctx, L, bf16, d, g, &tbl));
             // one filter launch over every assembly's tiles, one exact stage, one selection
             uint64_t nlist = 0;
             uint2* cand = nullptr;

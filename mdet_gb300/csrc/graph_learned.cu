@@ -453,7 +453,7 @@ int graph_learned(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_
     MDET_TRY(abd_gate(ctx, g));
     const double L = logit(cutoff);
     DstarTable tbl;
-    MDET_TRY(build_dstar_table(ctx, g.ls, n, L, &tbl, false));
+    MDET_TRY(build_dstar_table(ctx, g.ls, n, L, &tbl));
     tm.mark();
 
     // block statistics in embedding space

@@ -9,6 +9,13 @@
 // FP64 model parts used by the exact stage, the centred BF16 rows with their
 // norms and rounding errors for the tensor-core filter, per-block metadata,
 // and the d* table.
+//
+// Every kernel works on a set of one or more contig sets ("segments") laid
+// end to end, each from a 256-row boundary on, so a batch of assemblies is
+// prepared by the same few launches as one: k_scan (one pass over the rows
+// as they come: column means, and for a single set a content hash and the
+// log-size range), the sort, k_rows (gather, model parts, reduced-precision
+// rows), k_meta.
 #include <cub/cub.cuh>
 
 #include <string>
@@ -25,12 +32,141 @@ __device__ __forceinline__ unsigned long long dkey(double v) {
     return (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
 }
 
-__global__ void k_keys(const double* __restrict__ ls, uint64_t n, unsigned long long* __restrict__ keys,
-                       uint32_t* __restrict__ vals) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    keys[i] = dkey(ls[i]);
+// The segment of prepared row `pos`: its index and itself.
+__device__ __forceinline__ uint32_t seg_of(const PrepSet& v, uint64_t pos, PrepSeg& seg) {
+    const uint32_t k = v.segs ? v.blk_seg[pos >> 8] : 0u;
+    seg = v.segs ? v.segs[k] : v.one;
+    return k;
+}
+
+// Four consecutive floats at p; rows are 544 bytes, so a row array is 16-byte
+// aligned in every row or in none.
+__device__ __forceinline__ float4 load4(const float* __restrict__ p, bool aligned) {
+    if (aligned) return __ldg(reinterpret_cast<const float4*>(p));
+    return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+
+// Sort keys and values: the value is the prepared-row index of the contig
+// before the sort (segment base + original index).  Padding rows (present
+// when several segments are sorted together) sort last in their segment.
+__global__ void k_keys(PrepSet v, uint64_t rows, unsigned long long* __restrict__ keys, uint32_t* __restrict__ vals) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i >= rows) return;
+    PrepSeg seg;
+    seg_of(v, i, seg);
+    const uint64_t r = i - seg.base;
+    keys[i] = r < seg.n ? dkey(seg.ls[r]) : ~0ull;
     vals[i] = (uint32_t)i;
+}
+
+// The segment index of every value, the key of the second (stable) sort.
+__global__ void k_seg_keys(PrepSet v, uint64_t rows, const uint32_t* __restrict__ vals, uint32_t* __restrict__ keys) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i < rows) keys[i] = v.blk_seg[vals[i] >> 8];
+}
+
+constexpr int kCols4 = MDET_NTNF / 4;  // 34
+constexpr int kScanGroups = 8;
+constexpr int kScanThreads = (kCols4 * kScanGroups + 31) / 32 * 32;  // whole warps
+
+// What k_scan finds over a single set: a hash of the contents, and the
+// smallest (complemented, so that zeros start both) and largest size key.
+struct ScanStat {
+    unsigned long long hash, min_inv, max;
+    unsigned long long pad;
+};
+
+// One pass over the rows in their original order, rpb rows per block, thread
+// (row group, float4 column): column sums, and with stat the content hash --
+// per 16 bytes one 64 x 64 -> 128-bit product of the words, each offset by
+// its position, folded and added up -- and the log sizes' range.  The sums
+// run in float-float (250,000 contigs: 163 us for the FP64 adds of a separate
+// pass and 79 us for a separate hash; 62 us here, 136 MB); the last block of a
+// segment turns them into means.  rpb is 256, the size of a segment's blocks,
+// or 64 up to 65,536 rows, where 256 would leave SMs without a block (1,500
+// contigs: 22 us with 256, 10 us with 64).
+__global__ void __launch_bounds__(kScanThreads) k_scan(PrepSet v, uint32_t rpb, double* __restrict__ sums,
+                                                       uint32_t* __restrict__ done, float* __restrict__ mu,
+                                                       ScanStat* __restrict__ stat) {
+    __shared__ ff part[kScanGroups][MDET_NTNF];
+    __shared__ bool last;
+    PrepSeg seg;
+    const uint64_t pos0 = (uint64_t)blockIdx.x * rpb;
+    const uint32_t k = seg_of(v, pos0, seg);
+    const uint32_t r0 = (uint32_t)(pos0 - seg.base);
+    if (r0 >= seg.n) return;  // block-uniform
+    const uint32_t rows = min(rpb, seg.n - r0);
+    const uint32_t t = threadIdx.x, c = t % kCols4, grp = t / kCols4;
+    const bool al = ((uintptr_t)seg.tnf & 15) == 0;
+    const float* src = seg.tnf + (uint64_t)r0 * MDET_NTNF + 4 * c;
+    ff acc[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j] = ff_make(0.f, 0.f);
+    unsigned long long h = 0;
+#pragma unroll 4
+    for (uint32_t r = grp; r < (grp < kScanGroups ? rows : 0u); r += kScanGroups) {
+        const float4 x = load4(src + (uint64_t)r * MDET_NTNF, al);
+        if (sums) {
+            const float e[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const ff s2 = two_sum(acc[j].hi, e[j]);
+                acc[j].hi = s2.hi;
+                acc[j].lo = __fadd_rn(acc[j].lo, s2.lo);
+            }
+        }
+        if (stat) {
+            const unsigned long long pos = ((uint64_t)(r0 + r) * kCols4 + c + 1) * 0x9E3779B97F4A7C15ull;
+            const unsigned long long a =
+                ((unsigned long long)__float_as_uint(x.y) << 32 | __float_as_uint(x.x)) + pos;
+            const unsigned long long b =
+                ((unsigned long long)__float_as_uint(x.w) << 32 | __float_as_uint(x.z)) ^ (pos + 0xBF58476D1CE4E5B9ull);
+            h += (a * b) ^ __umul64hi(a, b) ^ (a + (b << 1));
+        }
+    }
+    if (stat) {
+        unsigned long long lo = 0, hi = 0;
+        if (t < rows) {
+            const double s = seg.ls[r0 + t];
+            unsigned long long z = (unsigned long long)__double_as_longlong(s) +
+                                   (unsigned long long)(r0 + t + 1) * 0x94D049BB133111EBull;
+            z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+            h += z ^ (z >> 31);
+            hi = dkey(s);
+            lo = ~hi;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            h += __shfl_xor_sync(0xffffffffu, h, o);
+            const unsigned long long l2 = __shfl_xor_sync(0xffffffffu, lo, o);
+            const unsigned long long h2 = __shfl_xor_sync(0xffffffffu, hi, o);
+            lo = lo > l2 ? lo : l2;
+            hi = hi > h2 ? hi : h2;
+        }
+        if ((t & 31) == 0) {
+            atomicAdd(&stat->hash, h);
+            if (hi | lo) {
+                atomicMax(&stat->min_inv, lo);
+                atomicMax(&stat->max, hi);
+            }
+        }
+    }
+    if (!sums) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (grp < kScanGroups) part[grp][4 * c + j] = acc[j];
+    __syncthreads();
+    if (t < MDET_NTNF) {
+        ff a = part[0][t];
+        for (int q = 1; q < kScanGroups; ++q) a = ff_add(a, part[q][t]);
+        atomicAdd(&sums[(uint64_t)k * MDET_NTNF + t], ff_to_double(a));
+    }
+    __threadfence();
+    __syncthreads();
+    if (t == 0) last = atomicAdd(&done[k], 1u) + 1 == (seg.n + rpb - 1) / rpb;
+    __syncthreads();
+    if (last && t < MDET_NTNF)
+        mu[(uint64_t)k * MDET_NTNF + t] = (float)(__ldcg(&sums[(uint64_t)k * MDET_NTNF + t]) / (double)seg.n);
 }
 
 __device__ __forceinline__ double poly(const double* c, int deg, double v) {
@@ -39,279 +175,366 @@ __device__ __forceinline__ double poly(const double* c, int deg, double v) {
     return r;
 }
 
-// Warp per position s of [0, npad) of one contig set placed at row `base`
-// of the prepared arrays (all pointers here already offset by base): perm
-// arrives with local original indices and leaves with base + local; inv is
-// the full array.  Padding positions map to themselves.  The row is copied
-// by the whole warp; the nine FP64 polynomials of the model parts run on
-// nine lanes side by side (FP64 is a narrow unit here, so one long serial
-// chain per row would bound the kernel).
-__global__ void k_gather(const float* __restrict__ tnf, const double* __restrict__ ls, uint32_t* __restrict__ perm,
-                         uint64_t n, uint64_t npad, uint32_t base, uint32_t* __restrict__ inv,
-                         float* __restrict__ x32, double* __restrict__ ls_s, PartsFF* __restrict__ parts,
-                         ModelSplit ms) {
-    const uint64_t s = blockIdx.x * (uint64_t)(blockDim.x / 32) + (threadIdx.x >> 5);
-    const uint32_t lane = threadIdx.x & 31;
-    if (s >= npad) return;
-    if (s >= n) {
-        if (lane == 0) {
-            perm[s] = base + (uint32_t)s;
-            inv[base + s] = base + (uint32_t)s;
-        }
-        return;
-    }
-    uint32_t o = 0;
-    if (lane == 0) o = perm[s];
-    o = __shfl_sync(0xffffffffu, o, 0);  // read by lane 0 before lane 0 rewrites it below
-    const float* src = tnf + (uint64_t)o * MDET_NTNF;
-    float* dst = x32 + s * MDET_NTNF;
-    for (int k = lane; k < MDET_NTNF; k += 32) dst[k] = src[k];
-    const double v = ls[o];
-    if (lane == 0) {
-        perm[s] = base + o;
-        inv[base + o] = base + (uint32_t)s;
-        ls_s[s] = v;
-    }
-    // lanes 0-3: f[m] = F_m(v) (degree 7); lanes 4-7: g[m] = G_m(v) without
-    // its constant (degree 6); lane 8: the log size itself
-    ff* out = reinterpret_cast<ff*>(parts + s);  // f[0..3], g[0..3], ls
-    if (lane < 4) {
-        out[lane] = ff_from_double(poly(ms.F[lane], 7, v));
-    } else if (lane < 8) {
-        const int m = lane - 4;
-        double r = ms.G[m][6];
-        for (int k = 5; k >= 1; --k) r = fma(r, v, ms.G[m][k]);
-        out[lane] = ff_from_double(r * v);
-    } else if (lane == 8) {
-        out[8] = ff_from_double(v);
-    } else if (lane == 9) {
-        parts[s].pad[0] = 0.f;
-        parts[s].pad[1] = 0.f;
-    }
-}
-
-__global__ void k_colsum(const float* __restrict__ x32, uint64_t n, double* __restrict__ sums) {
-    // block: 136 threads (one per column), rows strided over the grid
-    int k = threadIdx.x;
-    if (k >= MDET_NTNF) return;
-    double acc = 0;
-    for (uint64_t s = blockIdx.x; s < n; s += gridDim.x) acc += x32[s * MDET_NTNF + k];
-    atomicAdd(&sums[k], acc);
-}
-
-__global__ void k_mean(const double* __restrict__ sums, uint64_t n, float* __restrict__ mu) {
-    int k = threadIdx.x;
-    if (k < MDET_NTNF) mu[k] = (float)(sums[k] / (double)n);
-}
-
-// Warp per sorted row: centred BF16 copies in both GEMM roles, the squared
-// norm of the rounded row, and its exact distance to the unrounded centred
-// row.  Columns 136/137 fold the column term of ||a||^2+||b||^2-2a.b into the
-// GEMM: the A role carries 1, 1 and the B role -hi, -lo of ||b~||^2/2 (a
-// two-term BF16 split), so a.b' = a.b - ||b~||^2/2 comes out of TMEM.
-__global__ void k_bf16(const float* __restrict__ x32, const float* __restrict__ mu, uint64_t n, uint64_t npad,
-                       uint16_t* __restrict__ xa, uint16_t* __restrict__ xb, float* __restrict__ nsq,
-                       float* __restrict__ err, float* __restrict__ nrm) {
-    uint64_t s = blockIdx.x * (uint64_t)(blockDim.x / 32) + (threadIdx.x >> 5);
-    uint32_t lane = threadIdx.x & 31;
-    if (s >= npad) return;
-    uint16_t* rowa = xa + s * MDET_KPAD;
-    uint16_t* rowb = xb + s * MDET_KPAD;
-    const uint16_t one = 0x3F80;      // bf16 1.0
-    const uint16_t neg_inf = 0xFF80;  // bf16 -inf
-    if (s >= n) {
-        for (int k = lane; k < MDET_KPAD; k += 32) {
-            rowa[k] = (k == MDET_NTNF || k == MDET_NTNF + 1) ? one : 0;
-            rowb[k] = (k == MDET_NTNF) ? neg_inf : 0;
-        }
-        if (lane == 0) {
-            nsq[s] = __int_as_float(0x7f800000);
-            err[s] = 0.f;
-            nrm[s] = 0.f;
-        }
-        return;
-    }
-    // FP32 throughout (FP64 is a narrow unit here).  hv^2 is exact in FP32
-    // (8-bit significands), so a float-float accumulator gives ||x~||^2
-    // exactly to ~2^-44; the rounding error d = hv - (a - mu) is exact per
-    // entry up to one FP32 rounding (TwoSum of a - mu; v - hv is exact by
-    // Sterbenz), and its sum of squares is inflated before the square root
-    // is rounded up, so err stays an upper bound of ||x~ - x||.
-    float e2 = 0.f;
-    ff q = ff_make(0.f, 0.f);
-    for (int k = lane; k < MDET_NTNF; k += 32) {
-        const float a = x32[s * MDET_NTNF + k];
-        const ff v = two_sum(a, -mu[k]);  // v.hi + v.lo == a - mu exactly
-        const __nv_bfloat16 h = __float2bfloat16_rn(v.hi);
-        const uint16_t b = *reinterpret_cast<const uint16_t*>(&h);
-        const float hv = __bfloat162float(h);
-        const float d = __fadd_rn(__fsub_rn(v.hi, hv), v.lo);
-        e2 = __fmaf_rn(d, d, e2);
-        q = ff_add_f(q, __fmul_rn(hv, hv));
-        rowa[k] = b;
-        rowb[k] = b;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        e2 += __shfl_xor_sync(0xffffffffu, e2, o);
-        ff t;
-        t.hi = __shfl_xor_sync(0xffffffffu, q.hi, o);
-        t.lo = __shfl_xor_sync(0xffffffffu, q.lo, o);
-        q = ff_add(q, t);
-    }
-    const float half = 0.5f * q.hi;
-    const __nv_bfloat16 hi = __float2bfloat16_rn(half);
-    const __nv_bfloat16 lo = __float2bfloat16_rn(half - __bfloat162float(hi));
-    const uint16_t nhi = *reinterpret_cast<const uint16_t*>(&hi) ^ 0x8000u;
-    const uint16_t nlo = *reinterpret_cast<const uint16_t*>(&lo) ^ 0x8000u;
-    for (int k = MDET_NTNF + lane; k < MDET_KPAD; k += 32) {
-        rowa[k] = (k < MDET_NTNF + 2) ? one : 0;
-        rowb[k] = k == MDET_NTNF ? nhi : (k == MDET_NTNF + 1 ? nlo : 0);
-    }
-    if (lane == 0) {
-        nsq[s] = q.hi;
-        err[s] = __fsqrt_ru(__fmul_ru(e2, 1.001f));
-        nrm[s] = __fsqrt_ru(__fadd_ru(q.hi, q.lo));
-    }
-}
-
-// TF32 form of k_bf16: the same rows rounded to TF32 (round to nearest,
-// ties away; low 13 bits zero, so the tensor cores read them unchanged) in
-// FP32 containers.  hv^2 is exact in FP32 (11-bit significands); the column
-// term -||x~||^2/2 rides in columns 136/137 as a two-term TF32 split.
+// round to nearest, ties away, low 13 bits zero: the tensor cores read such
+// FP32 containers unchanged
 __device__ __forceinline__ float to_tf32(float x) {
     uint32_t r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
     return __uint_as_float(r);
 }
 
-__global__ void k_tf32(const float* __restrict__ x32, const float* __restrict__ mu, uint64_t n, uint64_t npad,
-                       float* __restrict__ ta, float* __restrict__ tb, float* __restrict__ nsq,
-                       float* __restrict__ err, float* __restrict__ nrm) {
-    uint64_t s = blockIdx.x * (uint64_t)(blockDim.x / 32) + (threadIdx.x >> 5);
-    uint32_t lane = threadIdx.x & 31;
-    if (s >= npad) return;
-    float* rowa = ta + s * MDET_KPAD;
-    float* rowb = tb + s * MDET_KPAD;
-    if (s >= n) {
-        for (int k = lane; k < MDET_KPAD; k += 32) {
-            rowa[k] = (k == MDET_NTNF || k == MDET_NTNF + 1) ? 1.f : 0.f;
-            rowb[k] = (k == MDET_NTNF) ? __int_as_float(0xff800000) : 0.f;
-        }
-        if (lane == 0) {
-            nsq[s] = __int_as_float(0x7f800000);
-            err[s] = 0.f;
-            nrm[s] = 0.f;
-        }
-        return;
-    }
-    float e2 = 0.f;
-    ff q = ff_make(0.f, 0.f);
-    for (int k = lane; k < MDET_NTNF; k += 32) {
-        const float a = x32[s * MDET_NTNF + k];
-        const ff v = two_sum(a, -mu[k]);  // v.hi + v.lo == a - mu exactly
-        const float hv = to_tf32(v.hi);
-        const float d = __fadd_rn(__fsub_rn(v.hi, hv), v.lo);
-        e2 = __fmaf_rn(d, d, e2);
-        q = ff_add_f(q, __fmul_rn(hv, hv));
-        rowa[k] = hv;
-        rowb[k] = hv;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        e2 += __shfl_xor_sync(0xffffffffu, e2, o);
-        ff t;
-        t.hi = __shfl_xor_sync(0xffffffffu, q.hi, o);
-        t.lo = __shfl_xor_sync(0xffffffffu, q.lo, o);
-        q = ff_add(q, t);
-    }
-    const float half = 0.5f * q.hi;
-    const float hi = to_tf32(half);
-    const float lo = to_tf32(__fsub_rn(half, hi));
-    for (int k = MDET_NTNF + lane; k < MDET_KPAD; k += 32) {
-        rowa[k] = (k < MDET_NTNF + 2) ? 1.f : 0.f;
-        rowb[k] = k == MDET_NTNF ? -hi : (k == MDET_NTNF + 1 ? -lo : 0.f);
-    }
-    if (lane == 0) {
-        nsq[s] = q.hi;
-        err[s] = __fsqrt_ru(__fmul_ru(e2, 1.001f));
-        nrm[s] = __fsqrt_ru(__fadd_ru(q.hi, q.lo));
+// The prepared arrays as k_rows writes them.
+struct RowsOut {
+    uint32_t* perm;  // in: sorted position -> pre-sort row (padding of a single set is filled in)
+    uint32_t* inv;
+    float* x32;
+    double* ls;
+    PartsFF* parts;
+    uint16_t *xa, *xb;
+    float *ta, *tb;
+    float *nsq, *err, *nrm;
+    const float* mu;
+};
+
+__device__ __forceinline__ uint32_t bf16_bits(float v) {
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    return *reinterpret_cast<const uint16_t*>(&h);
+}
+
+// Four columns (4q ..) of a reduced-precision row in one of its roles.
+template <int TCK>
+__device__ __forceinline__ void store4(uint16_t* bf, float* tf, uint64_t row, uint32_t q, const float (&e)[4]) {
+    if constexpr (TCK == kTcBf16) {
+        uint2 u;
+        u.x = bf16_bits(e[0]) | bf16_bits(e[1]) << 16;
+        u.y = bf16_bits(e[2]) | bf16_bits(e[3]) << 16;
+        *reinterpret_cast<uint2*>(bf + row * MDET_KPAD + 4 * q) = u;
+    } else if constexpr (TCK == kTcTf32) {
+        *reinterpret_cast<float4*>(tf + row * MDET_KPAD + 4 * q) = make_float4(e[0], e[1], e[2], e[3]);
     }
 }
 
-__global__ void k_meta(const double* __restrict__ ls_s, const float* __restrict__ err, const float* __restrict__ nrm,
-                       uint64_t n, uint64_t nblk, BlockMeta* __restrict__ meta, BlockMeta* __restrict__ meta32) {
-    uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+// Blocks [0, pblocks): the model parts, thread per sorted position -- FP64 is
+// a narrow unit here (about two lanes a clock), so its work is spread over
+// whole warps with eight independent polynomials a thread.  (250,000 contigs:
+// 381 us for a gather with nine lanes of each row's warp on one polynomial
+// each, 117 us for the reduced-precision rows in a pass of their own; 136 us
+// for both here, 436 MB.)
+//
+// The other blocks: warp per sorted position, four columns a lane.  The
+// FP32 row is copied; with TCK the centred reduced-precision copies in both
+// GEMM roles, the squared norm of the rounded row and its exact distance to
+// the unrounded centred row follow from the registers.  Columns 136/137 fold
+// the column term of ||a||^2+||b||^2-2a.b into the GEMM: the A role carries
+// 1, 1 and the B role -hi, -lo of ||b~||^2/2 (a two-term split in the row's
+// own precision), so a.b' = a.b - ||b~||^2/2 comes out of TMEM.
+template <int TCK>
+__global__ void __launch_bounds__(256) k_rows(PrepSet v, uint64_t rows, uint32_t pblocks, RowsOut out, ModelSplit ms) {
+    if (blockIdx.x < pblocks) {
+        const uint64_t s = blockIdx.x * 256ull + threadIdx.x;
+        if (s >= rows) return;
+        PrepSeg seg;
+        seg_of(v, s, seg);
+        if (s - seg.base >= seg.n) return;
+        const double x = seg.ls[out.perm[s] - seg.base];
+        out.ls[s] = x;
+        PartsFF p;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            p.f[m] = ff_from_double(poly(ms.F[m], 7, x));
+            double r = ms.G[m][6];  // G_m without its constant
+#pragma unroll
+            for (int k = 5; k >= 1; --k) r = fma(r, x, ms.G[m][k]);
+            p.g[m] = ff_from_double(r * x);
+        }
+        p.ls = ff_from_double(x);
+        p.pad[0] = p.pad[1] = 0.f;
+        out.parts[s] = p;
+        return;
+    }
+    const uint64_t s = (blockIdx.x - pblocks) * 8ull + (threadIdx.x >> 5);
+    const uint32_t lane = threadIdx.x & 31;
+    if (s >= rows) return;
+    PrepSeg seg;
+    const uint32_t k = seg_of(v, s, seg);
+    const float inf = __int_as_float(0x7f800000);
+    if (s - seg.base >= seg.n) {  // padding: neutral rows that no pair passes with
+        if (lane == 0) {
+            out.perm[s] = (uint32_t)s;
+            out.inv[s] = (uint32_t)s;
+        }
+        if constexpr (TCK != kTcNone) {
+            for (uint32_t q = lane; q < MDET_KPAD / 4; q += 32) {
+                const bool tail = q == MDET_NTNF / 4;
+                const float ea[4] = {tail ? 1.f : 0.f, tail ? 1.f : 0.f, 0.f, 0.f};
+                const float eb[4] = {tail ? -inf : 0.f, 0.f, 0.f, 0.f};
+                store4<TCK>(out.xa, out.ta, s, q, ea);
+                store4<TCK>(out.xb, out.tb, s, q, eb);
+            }
+            if (lane == 0) {
+                out.nsq[s] = inf;
+                out.err[s] = 0.f;
+                out.nrm[s] = 0.f;
+            }
+        }
+        return;
+    }
+    const uint32_t o = out.perm[s];
+    if (lane == 0) out.inv[o] = (uint32_t)s;
+    const float* src = seg.tnf + (uint64_t)(o - seg.base) * MDET_NTNF;
+    const bool al = ((uintptr_t)seg.tnf & 15) == 0;
+    // FP32 throughout.  hv^2 is exact in FP32 (8- or 11-bit significands), so
+    // a float-float accumulator gives ||x~||^2 exactly to ~2^-44; the rounding
+    // error d = hv - (a - mu) is exact per entry up to one FP32 rounding
+    // (TwoSum of a - mu; v - hv is exact by Sterbenz), and its sum of squares
+    // is inflated before the square root is rounded up, so err stays an upper
+    // bound of ||x~ - x||.
+    float e2 = 0.f;
+    ff q2 = ff_make(0.f, 0.f);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const uint32_t q = lane + 32 * half;
+        if (q < kCols4) {
+            const float4 x = load4(src + 4 * q, al);
+            *reinterpret_cast<float4*>(out.x32 + s * MDET_NTNF + 4 * q) = x;
+            if constexpr (TCK != kTcNone) {
+                const float4 m = __ldg(reinterpret_cast<const float4*>(out.mu + (uint64_t)k * MDET_NTNF + 4 * q));
+                const float a[4] = {x.x, x.y, x.z, x.w}, mm[4] = {m.x, m.y, m.z, m.w};
+                float e[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const ff c = two_sum(a[j], -mm[j]);  // c.hi + c.lo == a - mu exactly
+                    e[j] = TCK == kTcBf16 ? __bfloat162float(__float2bfloat16_rn(c.hi)) : to_tf32(c.hi);
+                    const float d = __fadd_rn(__fsub_rn(c.hi, e[j]), c.lo);
+                    e2 = __fmaf_rn(d, d, e2);
+                    q2 = ff_add_f(q2, __fmul_rn(e[j], e[j]));
+                }
+                store4<TCK>(out.xa, out.ta, s, q, e);
+                store4<TCK>(out.xb, out.tb, s, q, e);
+            }
+        }
+    }
+    if constexpr (TCK != kTcNone) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            e2 += __shfl_xor_sync(0xffffffffu, e2, d);
+            ff t;
+            t.hi = __shfl_xor_sync(0xffffffffu, q2.hi, d);
+            t.lo = __shfl_xor_sync(0xffffffffu, q2.lo, d);
+            q2 = ff_add(q2, t);
+        }
+        const float half = 0.5f * q2.hi;
+        const float hi = TCK == kTcBf16 ? __bfloat162float(__float2bfloat16_rn(half)) : to_tf32(half);
+        const float rest = __fsub_rn(half, hi);
+        const float lo = TCK == kTcBf16 ? __bfloat162float(__float2bfloat16_rn(rest)) : to_tf32(rest);
+        if (lane < 2) {  // columns 136 .. 139 and 140 .. 143
+            const float ea[4] = {lane ? 0.f : 1.f, lane ? 0.f : 1.f, 0.f, 0.f};
+            const float eb[4] = {lane ? 0.f : -hi, lane ? 0.f : -lo, 0.f, 0.f};
+            store4<TCK>(out.xa, out.ta, s, kCols4 + lane, ea);
+            store4<TCK>(out.xb, out.tb, s, kCols4 + lane, eb);
+        }
+        if (lane == 0) {
+            out.nsq[s] = q2.hi;
+            out.err[s] = __fsqrt_ru(__fmul_ru(e2, 1.001f));
+            out.nrm[s] = __fsqrt_ru(__fadd_ru(q2.hi, q2.lo));
+        }
+    }
+}
+
+// Metadata of every 128-row block, a warp per block (a thread per block walked
+// its rows one dependent load after another: 24 us at 1,500 contigs and 39 us
+// at 250,000, 4.3 and 6.7 us so).
+__global__ void k_meta(PrepSet v, uint64_t nblk, const double* __restrict__ ls_s, const float* __restrict__ err,
+                       const float* __restrict__ nrm, BlockMeta* __restrict__ meta, BlockMeta* __restrict__ meta32) {
+    const uint64_t b = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31;
     if (b >= nblk) return;
-    uint64_t s0 = b * MDET_BLK, s1 = min(n, s0 + MDET_BLK);
+    PrepSeg seg;
+    seg_of(v, b * MDET_BLK, seg);
+    const uint64_t s0 = b * MDET_BLK, end = (uint64_t)seg.base + seg.n;
     BlockMeta m;
-    if (s0 >= n) {
-        m.lo = m.hi = (float)ls_s[n - 1];
-        m.emax = m.nmax = 0.f;
+    m.emax = m.nmax = 0.f;
+    if (s0 >= end) {
+        m.lo = m.hi = (float)ls_s[end - 1];
     } else {
-        // true range (the rows need not be in size order)
-        double lo = ls_s[s0], hi = ls_s[s0];
-        for (uint64_t s = s0 + 1; s < s1; ++s) {
+        // true range (the rows need not be in size order); NaN is the identity of fmin/fmax
+        const uint64_t s1 = min(end, s0 + MDET_BLK);
+        double lo = __longlong_as_double(0x7ff8000000000000ll), hi = lo;
+        float e = 0.f, nm = 0.f;
+        for (uint64_t s = s0 + lane; s < s1; s += 32) {
             lo = fmin(lo, ls_s[s]);
             hi = fmax(hi, ls_s[s]);
-        }
-        m.lo = __double2float_rd(lo);
-        m.hi = __double2float_ru(hi);
-        float e = 0.f, nm = 0.f;
-        if (err)
-            for (uint64_t s = s0; s < s1; ++s) {
+            if (err) {
                 e = fmaxf(e, err[s]);
                 nm = fmaxf(nm, nrm[s]);
             }
+        }
+#pragma unroll
+        for (int d = 16; d; d >>= 1) {
+            lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+            hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+            e = fmaxf(e, __shfl_xor_sync(0xffffffffu, e, d));
+            nm = fmaxf(nm, __shfl_xor_sync(0xffffffffu, nm, d));
+        }
+        m.lo = __double2float_rd(lo);
+        m.hi = __double2float_ru(hi);
         m.emax = e;
         m.nmax = nm;
     }
+    if (lane) return;
     if (meta) meta[b] = m;
-    BlockMeta m32 = m;
-    m32.emax = 0.f;
-    m32.nmax = 0.f;
-    meta32[b] = m32;
+    m.emax = 0.f;
+    m.nmax = 0.f;
+    meta32[b] = m;
 }
 
 // ---- d* table ----
 
-__device__ double dev_dstar(double x, double y, double L, const ModelSplit& ms) {
-    const double ln9 = 2.1972245773362196;
-    double t = x * y, c[4];
-    for (int m = 0; m < 4; ++m) {
-        double g[7] = {0, ms.G[m][1], ms.G[m][2], ms.G[m][3], ms.G[m][4], ms.G[m][5], ms.G[m][6]};
-        double h[6] = {0, ms.H[m][1], ms.H[m][2], ms.H[m][3], ms.H[m][4], ms.H[m][5]};
-        c[m] = poly(ms.F[m], 7, x) + poly(g, 6, y) + poly(h, 5, t);
+constexpr int kPts = 4 * MDET_TBL + 1;
+
+// F_m and G_m at the table's 1,025 grid points: axis[m][p], axis[4 + m][p].
+// The grid comes from device memory when `grid` is given.
+__global__ void k_dstar_axis(const TableGrid* __restrict__ grid, double lmin, double h, ModelSplit ms,
+                             double* __restrict__ axis) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= kPts) return;
+    if (grid) {
+        lmin = grid->lmin;
+        h = grid->h;
     }
+    const double x = lmin + p * (h / 4);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        axis[m * kPts + p] = poly(ms.F[m], 7, x);
+        const double g[7] = {0, ms.G[m][1], ms.G[m][2], ms.G[m][3], ms.G[m][4], ms.G[m][5], ms.G[m][6]};
+        axis[(4 + m) * kPts + p] = poly(g, 6, x);
+    }
+}
+
+// d* at log sizes x <= y with F(x) and G(y) given (+inf where the model is
+// not decreasing in d).
+__device__ __forceinline__ double dstar_at(double x, double y, const double (&F)[4], const double (&G)[4], double L,
+                                           const ModelSplit& ms) {
+    const double ln9 = 2.1972245773362196, t = x * y;
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
-    if (!(c[1] > 0)) return inf;
-    if (L >= ln9) return (-L - c[0]) / c[1];
-    if (!(c[3] > 0)) return inf;
-    double d1 = (-ln9 - c[0]) / c[1];
-    double d2 = (-L - c[2]) / c[3];
+    auto coef = [&](int m) {
+        const double h[6] = {0, ms.H[m][1], ms.H[m][2], ms.H[m][3], ms.H[m][4], ms.H[m][5]};
+        return F[m] + G[m] + poly(h, 5, t);
+    };
+    const double c1 = coef(1);
+    if (!(c1 > 0)) return inf;
+    const double c0 = coef(0);
+    if (L >= ln9) return (-L - c0) / c1;
+    const double c3 = coef(3);
+    if (!(c3 > 0)) return inf;
+    const double d1 = (-ln9 - c0) / c1;
+    const double d2 = (-L - coef(2)) / c3;
     return d1 > d2 ? d1 : d2;
 }
 
-constexpr int kPts = 4 * MDET_TBL + 1;
-
-__global__ void k_dstar_points(double lmin, double h, double L, ModelSplit ms, float* __restrict__ pts) {
-    int a = blockIdx.y, b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= kPts) return;
-    int lo = min(a, b), hi = max(a, b);
-    double x = lmin + lo * (h / 4), y = lmin + hi * (h / 4);
-    double d = dev_dstar(x, y, L, ms);
-    pts[a * kPts + b] = __double2float_ru(d);
+// Block per cell row a: the 5 x 5 points of every cell (a, b), b >= a (the
+// points are symmetric, so cell (b, a) is the same), then the cell's bound
+// with its slack.  The one-variable polynomials come from k_dstar_axis, so a
+// point costs the x * y terms and the divisions.
+__global__ void __launch_bounds__(MDET_TBL) k_dstar_cells(const TableGrid* __restrict__ grid, double lmin, double h,
+                                                          double L, ModelSplit ms, const double* __restrict__ axis,
+                                                          float* __restrict__ st0) {
+    __shared__ float pts[5][kPts + 3];
+    const int a = blockIdx.x, b = threadIdx.x;
+    if (grid) {
+        lmin = grid->lmin;
+        h = grid->h;
+    }
+    // point (4a + i, q), q from 4a + i up
+    for (int i = 0; i < 5; ++i) {
+        const int pa = 4 * a + i;
+        double F[4], G[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) F[m] = axis[m * kPts + pa];
+        for (int q = pa + b; q < kPts; q += MDET_TBL) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) G[m] = axis[(4 + m) * kPts + q];
+            pts[i][q] = __double2float_ru(dstar_at(lmin + pa * (h / 4), lmin + q * (h / 4), F, G, L, ms));
+        }
+    }
+    __syncthreads();
+    if (b < a) return;
+    float mx = -__int_as_float(0x7f800000), mn = __int_as_float(0x7f800000);
+    for (int i = 0; i <= 4; ++i)
+        for (int j = 0; j <= 4; ++j) {
+            const int pa = 4 * a + i, pb = 4 * b + j;
+            const float v = pa <= pb ? pts[i][pb] : pts[pb - 4 * a][pa];
+            mx = fmaxf(mx, v);
+            mn = fminf(mn, v);
+        }
+    float T = mx + 0.5f * (mx - mn) + 1e-6f + 1e-5f * fabsf(mx);
+    if (isinf(mx) || isnan(mx)) T = __int_as_float(0x7f800000);
+    st0[a * MDET_TBL + b] = T;
+    st0[b * MDET_TBL + a] = T;
 }
 
-// the same points on a grid held in device memory
-__global__ void k_dstar_points_dev(const TableGrid* __restrict__ grid, double L, ModelSplit ms, float* __restrict__ pts) {
-    int a = blockIdx.y, b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= kPts) return;
-    int lo = min(a, b), hi = max(a, b);
-    const double lmin = grid->lmin, h = grid->h;
-    double x = lmin + lo * (h / 4), y = lmin + hi * (h / 4);
-    double d = dev_dstar(x, y, L, ms);
-    pts[a * kPts + b] = __double2float_ru(d);
+// Suffix maximum along x (the min-size axis): cell (a, b) then bounds every
+// cell (a', b) with a' >= a, so a box [x0, x1] x [y0, y1] is bounded by row
+// x0 alone.  d* falls as the smaller contig grows, so this costs little.
+// A warp per column (eight cells a lane, then a scan over the lanes), eight
+// columns per block.
+__global__ void __launch_bounds__(256) k_suffix_x(float* __restrict__ st0) {
+    __shared__ float t[MDET_TBL][9];
+    const int c0 = blockIdx.x * 8;
+    for (int i = threadIdx.x; i < MDET_TBL * 8; i += 256) t[i >> 3][i & 7] = st0[(i >> 3) * MDET_TBL + c0 + (i & 7)];
+    __syncthreads();
+    const int col = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float v[8], m = -__int_as_float(0x7f800000);
+#pragma unroll
+    for (int i = 7; i >= 0; --i) {
+        m = fmaxf(m, t[8 * lane + i][col]);
+        v[i] = m;
+    }
+    float after = m;  // inclusive suffix maximum over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float u = __shfl_down_sync(0xffffffffu, after, o);
+        if (lane + o < 32) after = fmaxf(after, u);
+    }
+    const float next = __shfl_down_sync(0xffffffffu, after, 1);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[8 * lane + i][col] = lane < 31 ? fmaxf(v[i], next) : v[i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < MDET_TBL * 8; i += 256) st0[(i >> 3) * MDET_TBL + c0 + (i & 7)] = t[i >> 3][i & 7];
+}
+
+// The sparse table's upper levels, block per row.
+__global__ void __launch_bounds__(MDET_TBL) k_sparse(float* __restrict__ st) {
+    __shared__ float lev[2][MDET_TBL];
+    const int a = blockIdx.x, b = threadIdx.x;
+    lev[0][b] = st[a * MDET_TBL + b];
+    __syncthreads();
+    for (int k = 1; k < MDET_TBL_LEVELS; ++k) {
+        const float* prev = lev[(k - 1) & 1];
+        const float m = fmaxf(prev[b], prev[min(b + (1 << (k - 1)), MDET_TBL - 1)]);
+        lev[k & 1][b] = m;
+        st[(size_t)k * MDET_TBL * MDET_TBL + a * MDET_TBL + b] = m;
+        __syncthreads();
+    }
+}
+
+// Builds a table into st: the grid is (lmin, h), or *grid on the device.
+// Four launches, 78 us (eleven, 300 us, in the first form: 204 us for the
+// points, each with all eight polynomials, and 58 us for the suffix maxima of
+// one thread per column).
+int launch_table(mdet_ctx* ctx, const TableGrid* grid, double lmin, double h, double logit_cut, float* st) {
+    cudaStream_t s = ctx->stream;
+    double* axis = (double*)ctx_scratch(ctx, "tbl.axis", (size_t)8 * kPts * 8);
+    if (!axis) return MDET_ERR_NOMEM;
+    k_dstar_axis<<<(kPts + 63) / 64, 64, 0, s>>>(grid, lmin, h, model_split(), axis);
+    MDET_LAUNCHED(ctx, "k_dstar_axis");
+    k_dstar_cells<<<MDET_TBL, MDET_TBL, 0, s>>>(grid, lmin, h, logit_cut, model_split(), axis, st);
+    MDET_LAUNCHED(ctx, "k_dstar_cells");
+    k_suffix_x<<<MDET_TBL / 8, 256, 0, s>>>(st);
+    MDET_LAUNCHED(ctx, "k_suffix_x");
+    k_sparse<<<MDET_TBL, MDET_TBL, 0, s>>>(st);
+    MDET_LAUNCHED(ctx, "k_sparse");
+    return MDET_OK;
 }
 
 // union of (lo, hi) ranges -> table grid (one thread)
@@ -333,49 +556,8 @@ __global__ void k_grid_from_ranges(const double* __restrict__ r, uint32_t count,
     g->inv_hf = (float)(1.0 / h);
 }
 
-__global__ void k_dstar_cells(const float* __restrict__ pts, float* __restrict__ st0) {
-    int a = blockIdx.x, b = threadIdx.x;
-    float mx = -__int_as_float(0x7f800000), mn = __int_as_float(0x7f800000);
-    for (int i = 0; i <= 4; ++i)
-        for (int j = 0; j <= 4; ++j) {
-            float v = pts[(4 * a + i) * kPts + (4 * b + j)];
-            mx = fmaxf(mx, v);
-            mn = fminf(mn, v);
-        }
-    float T = mx + 0.5f * (mx - mn) + 1e-6f + 1e-5f * fabsf(mx);
-    if (isinf(mx) || isnan(mx)) T = __int_as_float(0x7f800000);
-    st0[a * MDET_TBL + b] = T;
-}
-
-// Suffix maximum along x (the min-size axis): cell (a, b) then bounds every
-// cell (a', b) with a' >= a, so a box [x0, x1] x [y0, y1] is bounded by row
-// x0 alone.  d* falls as the smaller contig grows, so this costs little.
-__global__ void k_suffix_x(float* __restrict__ st0) {
-    const int b = threadIdx.x;
-    float m = st0[(MDET_TBL - 1) * MDET_TBL + b];
-    for (int a = MDET_TBL - 2; a >= 0; --a) {
-        m = fmaxf(m, st0[a * MDET_TBL + b]);
-        st0[a * MDET_TBL + b] = m;
-    }
-}
-
-__global__ void k_sparse(float* __restrict__ st, int k) {
-    int a = blockIdx.x, b = threadIdx.x;
-    const float* prev = st + (size_t)(k - 1) * MDET_TBL * MDET_TBL;
-    float* cur = st + (size_t)k * MDET_TBL * MDET_TBL;
-    int b2 = min(b + (1 << (k - 1)), MDET_TBL - 1);
-    cur[a * MDET_TBL + b] = fmaxf(prev[a * MDET_TBL + b], prev[a * MDET_TBL + b2]);
-}
-
-// Range of the log sizes: the end points when sorted, else a one-block scan.
-__global__ void k_minmax(const double* __restrict__ ls_s, uint64_t n, int sorted, double* __restrict__ out) {
-    if (sorted) {
-        if (threadIdx.x == 0) {
-            out[0] = ls_s[0];
-            out[1] = ls_s[n - 1];
-        }
-        return;
-    }
+// Range of the log sizes: a one-block scan.
+__global__ void k_minmax(const double* __restrict__ ls_s, uint64_t n, double* __restrict__ out) {
     __shared__ double smin[32], smax[32];
     double lo = INFINITY, hi = -INFINITY;
     for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -423,7 +605,15 @@ ModelH model_h() {
     return h;
 }
 
-int prep_alloc(mdet_ctx* ctx, const char* tag, uint64_t rows, int tck, GraphPrep* g) {
+// The double whose order-preserving key is k.
+static double size_of_key(unsigned long long k) {
+    const unsigned long long b = (k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k;
+    double v;
+    memcpy(&v, &b, 8);
+    return v;
+}
+
+int prep_alloc(mdet_ctx* ctx, const char* tag, uint64_t rows, int tck, uint32_t sets, GraphPrep* g) {
     const std::string t(tag);
     const uint64_t nblk = rows / MDET_BLK;
     g->perm = (uint32_t*)ctx_scratch(ctx, (t + ".perm").c_str(), rows * 4);
@@ -432,7 +622,7 @@ int prep_alloc(mdet_ctx* ctx, const char* tag, uint64_t rows, int tck, GraphPrep
     g->ls = (double*)ctx_scratch(ctx, (t + ".ls").c_str(), rows * 8);
     g->parts = (PartsFF*)ctx_scratch(ctx, (t + ".parts").c_str(), rows * sizeof(PartsFF));
     g->meta32 = (BlockMeta*)ctx_scratch(ctx, (t + ".meta32").c_str(), nblk * sizeof(BlockMeta));
-    g->mu = (float*)ctx_scratch(ctx, (t + ".mu").c_str(), MDET_NTNF * 4);
+    g->mu = (float*)ctx_scratch(ctx, (t + ".mu").c_str(), (uint64_t)sets * MDET_NTNF * 4);
     g->xa = g->xb = nullptr;
     g->ta = g->tb = nullptr;
     g->tck = tck;
@@ -456,79 +646,94 @@ int prep_alloc(mdet_ctx* ctx, const char* tag, uint64_t rows, int tck, GraphPrep
     return MDET_OK;
 }
 
-int prep_into(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, int tck, const GraphPrep& g,
-              uint64_t base, const uint32_t* order) {
+// Zeroed accumulators of k_scan in one buffer: the statistics, the column
+// sums and finished-block counts per segment.
+struct ScanBuf {
+    ScanStat* stat;
+    double* sums;
+    uint32_t* done;
+};
+
+static int scan_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, bool stat, float* mu, ScanBuf* out) {
+    const uint64_t nsum = (uint64_t)set.count * MDET_NTNF;
+    const size_t bytes = sizeof(ScanStat) + nsum * 8 + set.count * 4ull;
+    unsigned char* p = (unsigned char*)ctx_scratch(ctx, "pre.scan", bytes);
+    if (!p) return MDET_ERR_NOMEM;
+    out->stat = (ScanStat*)p;
+    out->sums = (double*)(p + sizeof(ScanStat));
+    out->done = (uint32_t*)(out->sums + nsum);
+    MDET_CUDA(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
+    const uint32_t rpb = rows <= 65536 ? 64 : 256;
+    k_scan<<<(unsigned)(rows / rpb), kScanThreads, 0, ctx->stream>>>(
+        set, rpb, tck != kTcNone ? out->sums : nullptr, out->done, mu, stat ? out->stat : nullptr);
+    MDET_LAUNCHED(ctx, "k_scan");
+    return MDET_OK;
+}
+
+// Everything after the scan: the order, the rows, the metadata.
+static int prep_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, const GraphPrep& g,
+                     const uint32_t* order) {
     cudaStream_t s = ctx->stream;
-    const uint64_t npad = (n + 255) / 256 * 256;
-    const uint64_t nblk = npad / MDET_BLK;
-    unsigned long long* keys = (unsigned long long*)ctx_scratch(ctx, "pre.keys", n * 8);
-    unsigned long long* keys2 = (unsigned long long*)ctx_scratch(ctx, "pre.keys2", n * 8);
-    uint32_t* vals = (uint32_t*)ctx_scratch(ctx, "pre.vals", n * 4);
-    double* sums = (double*)ctx_scratch(ctx, "pre.sums", MDET_NTNF * 8);
-    if (!keys || !keys2 || !vals || !sums) return MDET_ERR_NOMEM;
-    uint32_t* perm = g.perm + base;
-    float* x32 = g.x32 + base * MDET_NTNF;
-    double* ls = g.ls + base;
-    PartsFF* parts = g.parts + base;
-    const unsigned blocks = (unsigned)((n + 255) / 256);
+    const uint64_t nblk = rows / MDET_BLK;
+    // one set: its n contigs are sorted; several: every row, padding included
+    const uint64_t ns = set.segs ? rows : set.one.n;
     if (order) {
         // caller's order (original index per position)
-        MDET_CUDA(ctx, cudaMemcpyAsync(perm, order, n * 4, cudaMemcpyDeviceToDevice, s));
+        MDET_CUDA(ctx, cudaMemcpyAsync(g.perm, order, ns * 4, cudaMemcpyDeviceToDevice, s));
     } else {
-        k_keys<<<blocks, 256, 0, s>>>(d_ls, n, keys, vals);
+        unsigned long long* keys = (unsigned long long*)ctx_scratch(ctx, "pre.keys", ns * 8);
+        unsigned long long* keys2 = (unsigned long long*)ctx_scratch(ctx, "pre.keys2", ns * 8);
+        uint32_t* vals = (uint32_t*)ctx_scratch(ctx, "pre.vals", ns * 4);
+        if (!keys || !keys2 || !vals) return MDET_ERR_NOMEM;
+        const unsigned blocks = (unsigned)((ns + 255) / 256);
+        k_keys<<<blocks, 256, 0, s>>>(set, ns, keys, vals);
         MDET_LAUNCHED(ctx, "k_keys");
-        size_t tmpb = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, tmpb, keys, keys2, vals, perm, (int)n, 0, 64, s);
-        void* tmp = ctx_scratch(ctx, "pre.cubtmp", tmpb);
+        // several sets: by size, then (stable) by set -- two sorts over all
+        // rows cost less than one per set
+        uint32_t* vals2 = set.segs ? (uint32_t*)ctx_scratch(ctx, "pre.vals2", ns * 4) : g.perm;
+        if (!vals2) return MDET_ERR_NOMEM;
+        size_t t1 = 0, t2 = 0;
+        cub::DeviceRadixSort::SortPairs(nullptr, t1, keys, keys2, vals, vals2, (int)ns, 0, 64, s);
+        int bits = 1;
+        uint32_t *k32 = (uint32_t*)keys, *k32b = (uint32_t*)keys2;
+        if (set.segs) {
+            while (bits < 32 && (set.count - 1) >> bits) ++bits;
+            cub::DeviceRadixSort::SortPairs(nullptr, t2, k32, k32b, vals2, g.perm, (int)ns, 0, bits, s);
+        }
+        size_t tb = t1 > t2 ? t1 : t2;
+        void* tmp = ctx_scratch(ctx, "pre.cubtmp", tb);
         if (!tmp) return MDET_ERR_NOMEM;
-        MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tmpb, keys, keys2, vals, perm, (int)n, 0, 64, s));
-    }
-    k_gather<<<(unsigned)((npad + 7) / 8), 256, 0, s>>>(d_tnf, d_ls, perm, n, npad, (uint32_t)base, g.inv, x32, ls,
-                                                       parts, model_split());
-    MDET_LAUNCHED(ctx, "k_gather");
-    float* err = nullptr;
-    float* nrm = nullptr;
-    if (tck != kTcNone) {
-        err = (float*)ctx_scratch(ctx, "pre.err", npad * 4);
-        nrm = (float*)ctx_scratch(ctx, "pre.nrm", npad * 4);
-        if (!err || !nrm) return MDET_ERR_NOMEM;
-        MDET_CUDA(ctx, cudaMemsetAsync(sums, 0, MDET_NTNF * 8, s));
-        k_colsum<<<std::min<uint64_t>(1024, n), MDET_NTNF, 0, s>>>(x32, n, sums);
-        MDET_LAUNCHED(ctx, "k_colsum");
-        k_mean<<<1, MDET_NTNF, 0, s>>>(sums, n, g.mu);
-        MDET_LAUNCHED(ctx, "k_mean");
-        if (tck == kTcTf32) {
-            k_tf32<<<(unsigned)((npad + 7) / 8), 256, 0, s>>>(x32, g.mu, n, npad, g.ta + base * MDET_KPAD,
-                                                             g.tb + base * MDET_KPAD, g.nsq + base, err, nrm);
-            MDET_LAUNCHED(ctx, "k_tf32");
-        } else {
-            k_bf16<<<(unsigned)((npad + 7) / 8), 256, 0, s>>>(x32, g.mu, n, npad, g.xa + base * MDET_KPAD,
-                                                             g.xb + base * MDET_KPAD, g.nsq + base, err, nrm);
-            MDET_LAUNCHED(ctx, "k_bf16");
+        MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, t1, keys, keys2, vals, vals2, (int)ns, 0, 64, s));
+        if (set.segs) {
+            k_seg_keys<<<blocks, 256, 0, s>>>(set, ns, vals2, k32);
+            MDET_LAUNCHED(ctx, "k_seg_keys");
+            MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, t2, k32, k32b, vals2, g.perm, (int)ns, 0, bits, s));
         }
     }
-    k_meta<<<(unsigned)((nblk + 127) / 128), 128, 0, s>>>(ls, err, nrm, n, nblk,
-                                                         tck != kTcNone ? g.meta + base / MDET_BLK : nullptr,
-                                                         g.meta32 + base / MDET_BLK);
+    RowsOut out{g.perm, g.inv, g.x32, g.ls, g.parts, g.xa, g.xb, g.ta, g.tb, g.nsq, nullptr, nullptr, g.mu};
+    if (tck != kTcNone) {
+        out.err = (float*)ctx_scratch(ctx, "pre.err", rows * 4);
+        out.nrm = (float*)ctx_scratch(ctx, "pre.nrm", rows * 4);
+        if (!out.err || !out.nrm) return MDET_ERR_NOMEM;
+    }
+    const unsigned pblocks = (unsigned)(rows / 256), grid = pblocks + (unsigned)(rows / 8);
+    if (tck == kTcBf16)
+        k_rows<kTcBf16><<<grid, 256, 0, s>>>(set, rows, pblocks, out, model_split());
+    else if (tck == kTcTf32)
+        k_rows<kTcTf32><<<grid, 256, 0, s>>>(set, rows, pblocks, out, model_split());
+    else
+        k_rows<kTcNone><<<grid, 256, 0, s>>>(set, rows, pblocks, out, model_split());
+    MDET_LAUNCHED(ctx, "k_rows");
+    k_meta<<<(unsigned)((nblk * 32 + 255) / 256), 256, 0, s>>>(set, nblk, g.ls, out.err, out.nrm,
+                                                             tck != kTcNone ? g.meta : nullptr, g.meta32);
     MDET_LAUNCHED(ctx, "k_meta");
     return MDET_OK;
 }
 
-// A 64-bit hash of the prepared inputs' contents (sum over the words of a
-// splitmix64 finaliser of word and position), to recognise unchanged inputs.
-__global__ void k_content_hash(const uint32_t* __restrict__ a, uint64_t na, const uint32_t* __restrict__ b,
-                               uint64_t nb, unsigned long long* __restrict__ out) {
-    unsigned long long h = 0;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < na + nb; i += stride) {
-        unsigned long long z = (unsigned long long)(i < na ? a[i] : b[i - na]) + (i + 1) * 0x9E3779B97F4A7C15ull;
-        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-        h += z ^ (z >> 31);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out, h);
+int prep_set(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, const GraphPrep& g) {
+    ScanBuf sb;
+    MDET_TRY(scan_rows(ctx, set, rows, tck, false, g.mu, &sb));
+    return prep_rows(ctx, set, rows, tck, g, nullptr);
 }
 
 // Rows sorted by size (or in the caller's order).  A preparation of the very
@@ -538,65 +743,40 @@ int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t 
                 const uint32_t* order) {
     g->n = (uint32_t)n;
     g->npad = (uint32_t)((n + 255) / 256 * 256);
-    MDET_TRY(prep_alloc(ctx, "pre", g->npad, tck, g));
+    MDET_TRY(prep_alloc(ctx, "pre", g->npad, tck, 1, g));
+    const PrepSet set{1, PrepSeg{d_tnf, d_ls, (uint32_t)n, 0}, nullptr, nullptr};
     auto& c = ctx->prep_cache;
+    ScanBuf sb;
     if (order) {
         c.valid = false;
-        return prep_into(ctx, d_tnf, d_ls, n, tck, *g, 0, order);
+        MDET_TRY(scan_rows(ctx, set, g->npad, tck, false, g->mu, &sb));
+        return prep_rows(ctx, set, g->npad, tck, *g, order);
     }
-    unsigned long long* dh = (unsigned long long*)ctx_scratch(ctx, "pre.hash", 8);
-    if (!dh) return MDET_ERR_NOMEM;
-    cudaStream_t s = ctx->stream;
-    unsigned long long h = 0;
-    MDET_CUDA(ctx, cudaMemsetAsync(dh, 0, 8, s));
-    k_content_hash<<<ctx->num_sms * 8, 256, 0, s>>>((const uint32_t*)d_tnf, n * MDET_NTNF, (const uint32_t*)d_ls,
-                                                    n * 2, dh);
-    MDET_LAUNCHED(ctx, "k_content_hash");
-    MDET_CUDA(ctx, cudaMemcpyAsync(&h, dh, 8, cudaMemcpyDeviceToHost, s));
-    MDET_CUDA(ctx, cudaStreamSynchronize(s));
+    // the scan writes the means, so a preparation it confirms keeps equal ones
+    MDET_TRY(scan_rows(ctx, set, g->npad, tck, true, g->mu, &sb));
+    ScanStat st;
+    MDET_CUDA(ctx, cudaMemcpyAsync(&st, sb.stat, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
+    MDET_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    g->lrange[0] = size_of_key(~st.min_inv);
+    g->lrange[1] = size_of_key(st.max);
     // a preparation with other reduced-precision rows (or none) is remade:
     // nsq and the block metadata describe the rows last made
     if (c.valid && c.tnf == d_tnf && c.ls == d_ls && c.n == n && (c.tck == tck || tck == kTcNone) &&
-        c.hash == h && c.x32 == g->x32 && (tck == kTcNone || (c.xa == g->xa && c.ta == g->ta)) &&
+        c.hash == st.hash && c.x32 == g->x32 && (tck == kTcNone || (c.xa == g->xa && c.ta == g->ta)) &&
         c.gen == ctx->scratch_gen)
         return MDET_OK;
     c.valid = false;
-    MDET_TRY(prep_into(ctx, d_tnf, d_ls, n, tck, *g, 0, nullptr));
+    MDET_TRY(prep_rows(ctx, set, g->npad, tck, *g, nullptr));
     c.valid = true;
     c.tnf = d_tnf;
     c.ls = d_ls;
     c.n = n;
     c.tck = tck;
-    c.hash = h;
+    c.hash = st.hash;
     c.x32 = g->x32;
     c.xa = g->xa;
     c.ta = g->ta;
     c.gen = ctx->scratch_gen;
-    return MDET_OK;
-}
-
-int build_dstar_table_at(mdet_ctx* ctx, double lmin, double lmax, double logit_cut, float* st, DstarTable* out) {
-    cudaStream_t s = ctx->stream;
-    out->dyn = nullptr;
-    float* pts = (float*)ctx_scratch(ctx, "tbl.pts", (size_t)kPts * kPts * 4);
-    if (!pts) return MDET_ERR_NOMEM;
-    double h = (lmax - lmin) / MDET_TBL;
-    if (!(h > 1e-7)) h = 1e-7;
-    lmin -= 1e-9;
-    dim3 grid((kPts + 127) / 128, kPts);
-    k_dstar_points<<<grid, 128, 0, s>>>(lmin, h, logit_cut, model_split(), pts);
-    MDET_LAUNCHED(ctx, "k_dstar_points");
-    k_dstar_cells<<<MDET_TBL, MDET_TBL, 0, s>>>(pts, st);
-    MDET_LAUNCHED(ctx, "k_dstar_cells");
-    k_suffix_x<<<1, MDET_TBL, 0, s>>>(st);
-    MDET_LAUNCHED(ctx, "k_suffix_x");
-    for (int k = 1; k < MDET_TBL_LEVELS; ++k) {
-        k_sparse<<<MDET_TBL, MDET_TBL, 0, s>>>(st, k);
-        MDET_LAUNCHED(ctx, "k_sparse");
-    }
-    out->st = st;
-    out->lmin = (float)lmin;
-    out->inv_h = (float)(1.0 / h);
     return MDET_OK;
 }
 
@@ -607,20 +787,7 @@ int grid_from_ranges(mdet_ctx* ctx, const double* ranges, uint32_t count, TableG
 }
 
 int build_dstar_table_dev(mdet_ctx* ctx, const TableGrid* grid, double logit_cut, float* st, DstarTable* out) {
-    cudaStream_t s = ctx->stream;
-    float* pts = (float*)ctx_scratch(ctx, "tbl.pts", (size_t)kPts * kPts * 4);
-    if (!pts) return MDET_ERR_NOMEM;
-    dim3 g((kPts + 127) / 128, kPts);
-    k_dstar_points_dev<<<g, 128, 0, s>>>(grid, logit_cut, model_split(), pts);
-    MDET_LAUNCHED(ctx, "k_dstar_points");
-    k_dstar_cells<<<MDET_TBL, MDET_TBL, 0, s>>>(pts, st);
-    MDET_LAUNCHED(ctx, "k_dstar_cells");
-    k_suffix_x<<<1, MDET_TBL, 0, s>>>(st);
-    MDET_LAUNCHED(ctx, "k_suffix_x");
-    for (int k = 1; k < MDET_TBL_LEVELS; ++k) {
-        k_sparse<<<MDET_TBL, MDET_TBL, 0, s>>>(st, k);
-        MDET_LAUNCHED(ctx, "k_sparse");
-    }
+    MDET_TRY(launch_table(ctx, grid, 0, 0, logit_cut, st));
     out->st = st;
     out->lmin = 0.f;
     out->inv_h = 0.f;
@@ -628,12 +795,12 @@ int build_dstar_table_dev(mdet_ctx* ctx, const TableGrid* grid, double logit_cut
     return MDET_OK;
 }
 
-int build_dstar_table(mdet_ctx* ctx, const double* d_ls_sorted, uint64_t n, double logit_cut, DstarTable* out,
-                      bool sorted, double* range) {
+int build_dstar_table(mdet_ctx* ctx, const double* d_ls, uint64_t n, double logit_cut, DstarTable* out,
+                      const double* range) {
     out->dyn = nullptr;
     cudaStream_t s = ctx->stream;
     double lmin, lmax;
-    if (range && !std::isnan(range[0])) {
+    if (range) {
         lmin = range[0];
         lmax = range[1];
     } else {
@@ -641,16 +808,12 @@ int build_dstar_table(mdet_ctx* ctx, const double* d_ls_sorted, uint64_t n, doub
         double* mm = (double*)ctx_scratch(ctx, "tbl.mm", 16);
         if (!mm) return MDET_ERR_NOMEM;
         double r[2];
-        k_minmax<<<1, sorted ? 32 : 1024, 0, s>>>(d_ls_sorted, n, sorted ? 1 : 0, mm);
+        k_minmax<<<1, 1024, 0, s>>>(d_ls, n, mm);
         MDET_LAUNCHED(ctx, "k_minmax");
         MDET_CUDA(ctx, cudaMemcpyAsync(r, mm, 16, cudaMemcpyDeviceToHost, s));
         MDET_CUDA(ctx, cudaStreamSynchronize(s));
         lmin = r[0];
         lmax = r[1];
-        if (range) {
-            range[0] = lmin;
-            range[1] = lmax;
-        }
     }
     double h = (lmax - lmin) / MDET_TBL;
     if (!(h > 1e-7)) h = 1e-7;
@@ -672,20 +835,8 @@ int build_dstar_table(mdet_ctx* ctx, const double* d_ls_sorted, uint64_t n, doub
     out->lmin = (float)(lmin - 1e-9);
     out->inv_h = (float)(1.0 / h);
     if (hit) return MDET_OK;
-    float* pts = (float*)ctx_scratch(ctx, "tbl.pts", (size_t)kPts * kPts * 4);
-    if (!pts) return MDET_ERR_NOMEM;
     t.valid = false;
-    dim3 grid((kPts + 127) / 128, kPts);
-    k_dstar_points<<<grid, 128, 0, s>>>(lmin - 1e-9, h, logit_cut, model_split(), pts);
-    MDET_LAUNCHED(ctx, "k_dstar_points");
-    k_dstar_cells<<<MDET_TBL, MDET_TBL, 0, s>>>(pts, st);
-    MDET_LAUNCHED(ctx, "k_dstar_cells");
-    k_suffix_x<<<1, MDET_TBL, 0, s>>>(st);
-    MDET_LAUNCHED(ctx, "k_suffix_x");
-    for (int k = 1; k < MDET_TBL_LEVELS; ++k) {
-        k_sparse<<<MDET_TBL, MDET_TBL, 0, s>>>(st, k);
-        MDET_LAUNCHED(ctx, "k_sparse");
-    }
+    MDET_TRY(launch_table(ctx, nullptr, lmin - 1e-9, h, logit_cut, st));
     t.valid = true;
     t.L = logit_cut;
     t.lmin = lmin;
