@@ -268,11 +268,12 @@ typedef struct {
 
 int mdet_tnf_graph_batched(mdet_ctx* ctx, mdet_assembly* assemblies, uint32_t count, int mode,
                            mdet_graph_stats* stats);
-/* CUDA-graph recording of batched calls (on by default): after a batch has
- * run once, its whole device work -- preparation, d* tables, filter, exact
- * stage, selection, output -- is recorded as one CUDA graph with every count
- * kept on the device; a later call with the same sizes, cutoffs, max_edges,
- * buffers and capacities (the data may differ) replays it with one launch.
+/* CUDA-graph recording of batched calls (on by default): when a batch comes
+ * back -- the same sizes, cutoffs, max_edges, buffers and capacities as the
+ * batch before it (the data may differ) -- its whole device work --
+ * preparation, d* tables, filter, exact stage, selection, output -- is recorded
+ * as one CUDA graph with every count kept on the device, and that call and
+ * later ones replay it with one launch.
  * A replay whose candidates outgrow the recording falls back to the sized
  * path.  The recording is dropped when any scratch buffer of the context is
  * reallocated.  mdet_ctx_graph_replays counts replays. */

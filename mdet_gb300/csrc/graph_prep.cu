@@ -537,15 +537,20 @@ int launch_table(mdet_ctx* ctx, const TableGrid* grid, double lmin, double h, do
     return MDET_OK;
 }
 
-// union of (lo, hi) ranges -> table grid (one thread)
+// union of (lo, hi) ranges -> table grid (one warp)
 __global__ void k_grid_from_ranges(const double* __restrict__ r, uint32_t count, TableGrid* __restrict__ g) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     double lo = INFINITY, hi = -INFINITY;
-    for (uint32_t k = 0; k < count; ++k)
+    for (uint32_t k = threadIdx.x; k < count; k += 32)
         if (r[2 * k] <= r[2 * k + 1]) {
             lo = fmin(lo, r[2 * k]);
             hi = fmax(hi, r[2 * k + 1]);
         }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (threadIdx.x) return;
     if (!(lo <= hi)) lo = hi = 0;
     double h = (hi - lo) / MDET_TBL;
     if (!(h > 1e-7)) h = 1e-7;
