@@ -11,15 +11,20 @@
 // before that drop minus its newlines.  A name line that reaches the end of
 // the buffer without a newline is not a record.
 //
-// Pass 1 (k_fa_starts) reads every byte once in 16-byte loads; a thread that
-// sees a '>' settles whether it is the first of its line from its own 16 bytes
-// or, when the line began in an earlier chunk, by walking back to the line's
-// previous '\n' or '>'.  Starts are appended with an atomic (they are rare:
-// one per record) and sorted.  Pass 2 (k_fa_records) gives each record a warp:
-// it finds the name line's newline and first space with ballots over 32-byte
-// windows, then counts the newlines of the sequence view with 16-byte loads
-// (the view's bytes are read once more).  A scan of the size-class flags
-// places the records with size >= min_contig in file order.
+// Pass 1 (k_fa_scan) reads every byte once in 16-byte loads, a warp per 2 KB,
+// and leaves the number of newlines of every 64 bytes in a byte array (1/64 of
+// the file).  A thread that sees a '>' settles whether it is the
+// first of its line from its own 16 bytes or, when the line began in an
+// earlier chunk, by walking back to the line's previous '\n' or '>'.  A block
+// takes a contiguous range of the file and leaves its starts in order, so one
+// small launch (k_fa_compact) joins them; a file with more records in a range
+// than a block's queue holds is scanned again with the starts appended as
+// they come, and sorted.  Pass 2
+// (k_fa_records) gives each record a warp: it finds the name line's newline and
+// first space with ballots over 32-byte windows, and the view's newlines are
+// the byte array's sum over its whole 64-byte blocks and a count over the bytes
+// at its two ends, so the sequence is not read again.  A scan of the
+// size-class flags places the records with size >= min_contig in file order.
 #include <cstring>
 
 #include <cub/cub.cuh>
@@ -47,58 +52,169 @@ __device__ bool line_has_no_gt_before(const unsigned char* __restrict__ b, uint6
     return true;
 }
 
-// The '>' bytes of one 16-byte chunk at base: appends the record starts.
-__device__ __forceinline__ void chunk_starts(const unsigned char* __restrict__ b, uint64_t base, const uint4& q,
-                                             uint64_t* __restrict__ starts, uint64_t cap,
-                                             unsigned long long* __restrict__ count) {
-    const uint32_t any = __vcmpeq4(q.x, 0x3E3E3E3Eu) | __vcmpeq4(q.y, 0x3E3E3E3Eu) | __vcmpeq4(q.z, 0x3E3E3E3Eu) |
-                         __vcmpeq4(q.w, 0x3E3E3E3Eu);
-    if (!any) return;
-    // state carried left to right through the chunk: 1 = a line start (no '>'
-    // since the last '\n'), 0 = a '>' already on this line, 2 = not known yet
-    // (the line began before this chunk)
-    int state = 2;
-    for (int j = 0; j < 16; ++j) {
-        const unsigned char ch = byte_of(q, j);
-        if (ch == '\n') {
-            state = 1;
-        } else if (ch == '>') {
-            if (state == 2) state = line_has_no_gt_before(b, base) ? 1 : 0;
-            if (state == 1) {
-                const unsigned long long pos = atomicAdd(count, 1ull);
-                if (pos < cap) starts[pos] = base + j;
-            }
-            state = 0;
+constexpr uint32_t kBlk = 64;  // bytes per newline count
+
+// 0x80 in every byte of w that equals '\n'
+__device__ __forceinline__ uint32_t newline_bits(uint32_t w) {
+    const uint32_t z = w ^ 0x0A0A0A0Au;
+    return ~(((z & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | z | 0x7F7F7F7Fu);
+}
+
+// 0x80 in every byte of w that equals '>'
+__device__ __forceinline__ uint32_t gt_bits(uint32_t w) {
+    const uint32_t z = w ^ 0x3E3E3E3Eu;
+    return ~(((z & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | z | 0x7F7F7F7Fu);
+}
+
+// not 0 when a byte of w is '>'
+__device__ __forceinline__ uint32_t has_gt(uint32_t w) {
+    const uint32_t z = w ^ 0x3E3E3E3Eu;
+    return (z - 0x01010101u) & ~z & 0x80808080u;
+}
+
+// the byte flags (0x80) of four words as 16 bits
+__device__ __forceinline__ uint32_t flags16(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    auto four = [](uint32_t m) { return ((m >> 7) * 0x01020408u) >> 24; };  // byte k -> bit k
+    return four(a) | four(b) << 4 | four(c) << 8 | four(d) << 12;
+}
+
+// Record starts found by a block, in shared memory until the block ends: an
+// atomic on the file's one counter per record start was what the scan waited
+// for at 4 KB a record.
+constexpr uint32_t kQueue = 1536;
+struct StartQueue {
+    uint64_t pos[kQueue];
+    uint32_t n;
+};
+
+// The '>' bytes of one 16-byte chunk at base: queues the record starts, or
+// (sq null) appends them.
+__device__ __noinline__ void chunk_starts(const unsigned char* __restrict__ b, uint64_t base, uint4 q,
+                                          StartQueue* sq, uint64_t* __restrict__ starts, uint64_t cap,
+                                          unsigned long long* __restrict__ count) {
+    uint32_t gt = flags16(gt_bits(q.x), gt_bits(q.y), gt_bits(q.z), gt_bits(q.w));
+    const uint32_t nl = flags16(newline_bits(q.x), newline_bits(q.y), newline_bits(q.z), newline_bits(q.w));
+    const uint32_t all = gt | nl;
+    while (gt) {
+        const uint32_t j = __ffs(gt) - 1;
+        gt &= gt - 1;
+        const uint32_t before = all & ((1u << j) - 1u);  // the last of these decides
+        const bool first = before ? (nl >> (31 - __clz(before))) & 1u : line_has_no_gt_before(b, base);
+        if (!first) continue;
+        if (sq) {
+            const uint32_t slot = atomicAdd(&sq->n, 1u);
+            if (slot < kQueue) sq->pos[slot] = base + j;
+        } else {
+            const unsigned long long pos = atomicAdd(count, 1ull);
+            if (pos < cap) starts[pos] = base + j;
         }
     }
 }
 
-// Four chunks per thread and round, their loads issued together.
-__global__ void k_fa_starts(const unsigned char* __restrict__ b, uint64_t nbytes, uint64_t* __restrict__ starts,
-                            uint64_t cap, unsigned long long* __restrict__ count) {
-    const uint64_t nfull = nbytes / 16;
-    const uint64_t G = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint4* b4 = reinterpret_cast<const uint4*>(b);
-    for (uint64_t c = t; c < nfull; c += 4 * G) {
+// The newlines of one 16-byte chunk (0 .. 16) and whether it has a '>'.
+__device__ __forceinline__ uint32_t chunk_newlines(const uint4& q, uint32_t& gt) {
+    gt = has_gt(q.x) | has_gt(q.y) | has_gt(q.z) | has_gt(q.w);
+    const uint32_t acc = (newline_bits(q.x) >> 7) + (newline_bits(q.y) >> 7) + (newline_bits(q.z) >> 7) +
+                         (newline_bits(q.w) >> 7);
+    return __dp4a(acc, 0x01010101u, 0u);
+}
+
+// A warp per 2 KB: lane l takes the 16-byte chunks l, l + 32, l + 64 and
+// l + 96, all four loads in flight.  The four chunk counts ride in one word's
+// bytes, so two shuffle-adds make the sums of all 32 64-byte blocks, a byte per
+// lane to write.
+//
+// kAppend false: the block's starts go to found[blockIdx.x * kQueue ..] in
+// order and their number (which may exceed the queue) to nfound[blockIdx.x].
+// (0.93 GB, 220,000 records: 465 us with a global atomic per start, 179 us so.)
+template <bool kAppend>
+__global__ void __launch_bounds__(256) k_fa_scan(const unsigned char* __restrict__ b, uint64_t nbytes,
+                                                 uint8_t* __restrict__ nlc, uint64_t* __restrict__ found,
+                                                 uint32_t* __restrict__ nfound, uint64_t cap,
+                                                 unsigned long long* __restrict__ count) {
+    __shared__ StartQueue queue;
+    StartQueue* sq = kAppend ? nullptr : &queue;
+    if (threadIdx.x == 0) queue.n = 0;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t ntile = nbytes / 2048;
+    const uint64_t t0 = ntile * blockIdx.x / gridDim.x, t1 = ntile * (blockIdx.x + 1) / gridDim.x;
+    for (uint64_t tile = t0 + (threadIdx.x >> 5); tile < t1; tile += blockDim.x >> 5) {
+        const uint4* p = reinterpret_cast<const uint4*>(b + tile * 2048) + lane;
         uint4 q[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) q[u] = c + u * G < nfull ? __ldg(b4 + c + u * G) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < 4; ++u) q[u] = __ldg(p + 32 * u);
+        uint32_t sum = 0, gt[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (c + u * G < nfull) chunk_starts(b, (c + u * G) * 16, q[u], starts, cap, count);
+        for (int u = 0; u < 4; ++u) sum |= chunk_newlines(q[u], gt[u]) << (8 * u);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        nlc[tile * 32 + 8 * (lane & 3) + (lane >> 2)] = (uint8_t)(sum >> (8 * (lane & 3)));
+        if (gt[0] | gt[1] | gt[2] | gt[3]) {
+#pragma unroll 1
+            for (int u = 0; u < 4; ++u) {
+                const uint4 c = u == 0 ? q[0] : u == 1 ? q[1] : u == 2 ? q[2] : q[3];
+                if (u == 0 ? gt[0] : u == 1 ? gt[1] : u == 2 ? gt[2] : gt[3])
+                    chunk_starts(b, tile * 2048 + 16 * lane + 512 * u, c, sq, found, cap, count);
+            }
+        }
     }
-    if (t == 0 && nbytes % 16) {  // the ragged last chunk
-        const uint64_t base = nfull * 16;
-        uint32_t w[4] = {0, 0, 0, 0};
-        for (uint64_t j = 0; base + j < nbytes; ++j) w[j >> 2] |= (uint32_t)b[base + j] << (8 * (j & 3));
-        chunk_starts(b, base, make_uint4(w[0], w[1], w[2], w[3]), starts, cap, count);
+    // the rest of the file, less than 2 KB: a lane per 64-byte block (the
+    // newlines of a ragged last block are counted by its record)
+    const uint64_t g = ntile * 32 + lane;
+    if (blockIdx.x + 1 == gridDim.x && threadIdx.x < 32 && g * kBlk < nbytes) {
+        uint32_t nl = 0;
+        for (uint64_t base = g * kBlk; base < g * kBlk + kBlk && base < nbytes; base += 16) {
+            uint32_t w[4] = {0, 0, 0, 0};
+            for (uint64_t j = 0; j < 16 && base + j < nbytes; ++j) w[j >> 2] |= (uint32_t)b[base + j] << (8 * (j & 3));
+            const uint4 c = make_uint4(w[0], w[1], w[2], w[3]);
+            uint32_t gt;
+            nl += chunk_newlines(c, gt);
+            if (gt) chunk_starts(b, base, c, sq, found, cap, count);
+        }
+        if ((g + 1) * kBlk <= nbytes) nlc[g] = (uint8_t)nl;
+    }
+    if (kAppend) return;
+    __syncthreads();
+    const uint32_t n = queue.n;
+    if (threadIdx.x == 0) {
+        nfound[blockIdx.x] = n;
+        if (n) atomicAdd(count, (unsigned long long)n);
+        if (n > kQueue) atomicMax(count + 1, (unsigned long long)n);
+    }
+    if (n > kQueue) return;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {  // its place is how many lie before it
+        const uint64_t v = queue.pos[i];
+        uint32_t at = 0;
+        for (uint32_t k = 0; k < n; ++k) at += queue.pos[k] < v;
+        found[(uint64_t)blockIdx.x * kQueue + at] = v;
     }
 }
 
+// Joins the blocks' starts: block k's go after those of blocks 0 .. k - 1.
+__global__ void __launch_bounds__(256) k_fa_compact(const uint64_t* __restrict__ found,
+                                                    const uint32_t* __restrict__ nfound,
+                                                    uint64_t* __restrict__ starts) {
+    __shared__ uint32_t part[8];
+    uint32_t before = 0;
+    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) before += nfound[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = before;
+    __syncthreads();
+    uint64_t at = 0;
+    for (int w = 0; w < 8; ++w) at += part[w];
+    const uint32_t n = nfound[blockIdx.x];
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) starts[at + i] = found[(uint64_t)blockIdx.x * kQueue + i];
+}
+
+// (0.93 GB, 220,000 records: k_fa_records 661 us while it read the whole views
+// and counted its records with one global atomic each, 96 us so; the sort of
+// the starts took 48 us, k_fa_compact takes 6.)
 struct RecArgs {
     const unsigned char* b;
     uint64_t nbytes;
+    const uint8_t* nlc;  // newlines of every whole 64-byte block
     const uint64_t* starts;
     uint64_t nr;
     uint64_t min_contig;
@@ -114,11 +230,15 @@ struct RecArgs {
 
 // A warp per record.
 __global__ void k_fa_records(RecArgs p) {
+    __shared__ unsigned int tally[2];  // the block's valid and small records
+    if (threadIdx.x < 2) tally[threadIdx.x] = 0;
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
     for (uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; r < p.nr; r += nw) {
         const uint64_t g = p.starts[r];
         const uint64_t nx = r + 1 < p.nr ? p.starts[r + 1] : p.nbytes;
+        const unsigned char last = p.b[nx - 1];  // nx > g: in flight beside the name line
         // name line: its newline h and the first space before it
         uint64_t h = kNone, sp = kNone;
         for (uint64_t q0 = g + 1; q0 < nx; q0 += 32) {
@@ -138,43 +258,40 @@ __global__ void k_fa_records(RecArgs p) {
             continue;
         }
         const uint64_t s0 = h + 1, s1 = nx;
-        // newlines of the view [s0, s1): ragged head and tail by bytes, the
-        // aligned middle by 16-byte loads
-        uint64_t a0 = (s0 + 15) & ~15ull, a1 = s1 & ~15ull;
-        if (a0 > s1) a0 = s1;
-        if (a1 < a0) a1 = a0;
+        // newlines of the view [s0, s1): the bytes before its first whole
+        // block and after its last, and the blocks' counts, four per load
+        const uint64_t B0 = (s0 + kBlk - 1) / kBlk, B1 = s1 / kBlk;
+        const uint64_t h1 = B0 < B1 ? B0 * kBlk : s1, t0 = B0 < B1 ? B1 * kBlk : s1;
         uint32_t nl = 0;
-        if (s0 + lane < a0) nl += p.b[s0 + lane] == '\n';
-        if (a1 + lane < s1) nl += p.b[a1 + lane] == '\n';
-        // four 16-byte loads per lane in flight
-        for (uint64_t c = a0 + 16 * (uint64_t)lane; c < a1; c += 4 * 16 * 32) {
-            uint4 q[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint64_t cu = c + (uint64_t)u * 16 * 32;
-                q[u] = cu < a1 ? __ldg(reinterpret_cast<const uint4*>(p.b + cu)) : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                nl += (__popc(__vcmpeq4(q[u].x, 0x0A0A0A0Au)) + __popc(__vcmpeq4(q[u].y, 0x0A0A0A0Au)) +
-                       __popc(__vcmpeq4(q[u].z, 0x0A0A0A0Au)) + __popc(__vcmpeq4(q[u].w, 0x0A0A0A0Au))) >>
-                      3;
+        for (uint64_t q = s0 + lane; q < h1; q += 32) nl += p.b[q] == '\n';
+        for (uint64_t q = t0 + lane; q < s1; q += 32) nl += p.b[q] == '\n';
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(p.nlc);
+        for (uint64_t w = B0 / 4 + lane; B0 < B1 && w < (B1 + 3) / 4; w += 32) {
+            uint32_t v = words[w];
+            if (4 * w < B0) v &= ~0u << (8 * (uint32_t)(B0 - 4 * w));
+            if (4 * w + 4 > B1) v &= ~0u >> (8 * (uint32_t)(4 * w + 4 - B1));
+            nl = __dp4a(v, 0x01010101u, nl);
         }
 #pragma unroll
         for (int d = 16; d; d >>= 1) nl += __shfl_xor_sync(0xffffffffu, nl, d);
         if (lane == 0) {
             uint64_t view = s1 - s0;
             const uint64_t sz = view - nl;
-            if (view > 0 && p.b[s1 - 1] == '\n') --view;
+            if (view > 0 && last == '\n') --view;
             p.off[r] = s0;
             p.len[r] = view;
             p.size[r] = sz;
             p.name_off[r] = g + 1;
             p.name_len[r] = (uint32_t)((sp != kNone ? sp : h) - (g + 1));
             p.large[r] = sz >= p.min_contig ? 1u : 0u;
-            atomicAdd(p.n_valid, 1ull);
-            if (sz < p.min_contig && sz >= 1000) atomicAdd(p.n_small, 1ull);
+            atomicAdd(&tally[0], 1u);
+            if (sz < p.min_contig && sz >= 1000) atomicAdd(&tally[1], 1u);
         }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && tally[0]) {
+        atomicAdd(p.n_valid, (unsigned long long)tally[0]);
+        if (tally[1]) atomicAdd(p.n_small, (unsigned long long)tally[1]);
     }
 }
 
@@ -223,31 +340,28 @@ int index_core(mdet_ctx* ctx, const char* d_bytes, uint64_t nbytes, uint64_t min
     const unsigned char* b = (const unsigned char*)d_bytes;
     unsigned long long* cnt = (unsigned long long*)ctx_scratch(ctx, "fa.cnt", 3 * 8);
     if (!cnt) return MDET_ERR_NOMEM;
-    // pass 1: record starts (sized by a guess, redone once at the exact count)
-    uint64_t cap = nbytes / 2048 + 4096;
-    DevBuf& sb = ctx->bufs["fa.starts"];
-    if (sb.cap / 8 > cap) cap = sb.cap / 8;
+    uint8_t* nlc = (uint8_t*)ctx_scratch(ctx, "fa.nlc", nbytes / kBlk + 4);
+    const unsigned sgrid = grid_for(ctx, nbytes / kBlk, 256);
+    uint64_t* found = (uint64_t*)ctx_scratch(ctx, "fa.found", (uint64_t)sgrid * kQueue * 8);
+    uint32_t* nfound = (uint32_t*)ctx_scratch(ctx, "fa.nfound", sgrid * 4ull);
+    if (!nlc || !found || !nfound) return MDET_ERR_NOMEM;
+    // pass 1: record starts, queued per block
     unsigned long long h_cnt[3] = {0, 0, 0};
-    uint64_t* starts = nullptr;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        starts = (uint64_t*)ctx_scratch(ctx, "fa.starts", cap * 8);
-        if (!starts) return MDET_ERR_NOMEM;
-        cap = ctx->bufs["fa.starts"].cap / 8;
-        MDET_CUDA(ctx, cudaMemsetAsync(cnt, 0, 3 * 8, s));
-        ctx_timer_begin(ctx, "k_fa_starts");
-        k_fa_starts<<<grid_for(ctx, (nbytes / 16 + 3) / 4, 256), 256, 0, s>>>(b, nbytes, starts, cap, cnt);
-        ctx_timer_end(ctx, "k_fa_starts");
-        MDET_LAUNCHED(ctx, "k_fa_starts");
-        MDET_CUDA(ctx, cudaMemcpyAsync(h_cnt, cnt, 8, cudaMemcpyDeviceToHost, s));
-        MDET_CUDA(ctx, cudaStreamSynchronize(s));
-        if (h_cnt[0] <= cap) break;
-        cap = h_cnt[0];
-    }
+    MDET_CUDA(ctx, cudaMemsetAsync(cnt, 0, 3 * 8, s));
+    ctx_timer_begin(ctx, "k_fa_scan");
+    k_fa_scan<false><<<sgrid, 256, 0, s>>>(b, nbytes, nlc, found, nfound, 0, cnt);
+    ctx_timer_end(ctx, "k_fa_scan");
+    MDET_LAUNCHED(ctx, "k_fa_scan");
+    MDET_CUDA(ctx, cudaMemcpyAsync(h_cnt, cnt, 16, cudaMemcpyDeviceToHost, s));
+    MDET_CUDA(ctx, cudaStreamSynchronize(s));
+    const bool queued = h_cnt[1] == 0;
     const uint64_t nr = h_cnt[0];
     if (nr >= (1ull << 31)) return ctx_fail(ctx, MDET_ERR_INVALID, "too many FASTA records (%llu)", (unsigned long long)nr);
     st->n_records = st->n_large = st->n_small = 0;
     if (nr == 0) return MDET_OK;
     uint64_t* sorted = (uint64_t*)ctx_scratch(ctx, "fa.sorted", nr * 8);
+    uint64_t* starts = queued ? nullptr : (uint64_t*)ctx_scratch(ctx, "fa.starts", nr * 8);
+    if (!queued && !starts) return MDET_ERR_NOMEM;
     uint64_t* r_off = (uint64_t*)ctx_scratch(ctx, "fa.off", nr * 8);
     uint64_t* r_len = (uint64_t*)ctx_scratch(ctx, "fa.len", nr * 8);
     uint64_t* r_size = (uint64_t*)ctx_scratch(ctx, "fa.size", nr * 8);
@@ -256,16 +370,24 @@ int index_core(mdet_ctx* ctx, const char* d_bytes, uint64_t nbytes, uint64_t min
     uint32_t* large = (uint32_t*)ctx_scratch(ctx, "fa.large", (nr + 1) * 4);
     uint32_t* dst = (uint32_t*)ctx_scratch(ctx, "fa.dst", (nr + 1) * 4);
     if (!sorted || !r_off || !r_len || !r_size || !r_noff || !r_nlen || !large || !dst) return MDET_ERR_NOMEM;
+    size_t t1 = 0, t2 = 0;
     int bits = 1;
     while (bits < 64 && (nbytes >> bits)) ++bits;
-    size_t t1 = 0, t2 = 0;
-    MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(nullptr, t1, starts, sorted, (int)nr, 0, bits, s));
+    if (!queued) MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(nullptr, t1, starts, sorted, (int)nr, 0, bits, s));
     MDET_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, t2, large, dst, (int)nr + 1, s));
     void* tmp = ctx_scratch(ctx, "fa.cubtmp", t1 > t2 ? t1 : t2);
     if (!tmp) return MDET_ERR_NOMEM;
-    MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, t1, starts, sorted, (int)nr, 0, bits, s));
+    MDET_CUDA(ctx, cudaMemsetAsync(cnt, 0, 3 * 8, s));
+    if (queued) {
+        k_fa_compact<<<sgrid, 256, 0, s>>>(found, nfound, sorted);
+        MDET_LAUNCHED(ctx, "k_fa_compact");
+    } else {
+        k_fa_scan<true><<<sgrid, 256, 0, s>>>(b, nbytes, nlc, starts, nullptr, nr, cnt);
+        MDET_LAUNCHED(ctx, "k_fa_scan");
+        MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, t1, starts, sorted, (int)nr, 0, bits, s));
+    }
 
-    RecArgs ra{b, nbytes, sorted, nr, min_contig, r_off, r_len, r_size, r_noff, r_nlen, large, cnt + 1, cnt + 2};
+    RecArgs ra{b, nbytes, nlc, sorted, nr, min_contig, r_off, r_len, r_size, r_noff, r_nlen, large, cnt + 1, cnt + 2};
     ctx_timer_begin(ctx, "k_fa_records");
     k_fa_records<<<grid_for(ctx, nr * 32, 256), 256, 0, s>>>(ra);
     ctx_timer_end(ctx, "k_fa_records");
