@@ -44,6 +44,7 @@ struct mdet_ctx {
     uint32_t launches = 0;     // kernels launched by the current call
     void* encode_tiled = nullptr;  // cuTensorMapEncodeTiled entry point
     bool count_scratch_dirty = false;
+    int count_grid = 0;  // blocks of the counting kernel (0: not asked yet)
     uint64_t total_launches = 0;
     // keys of the d* tables held in scratch "tbl.st0".."tbl.st3" (least
     // recently used one is rebuilt on a miss)

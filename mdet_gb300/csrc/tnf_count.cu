@@ -8,8 +8,8 @@
 // exact integers; TNF = float(c / sqrt(sum float(c*c))).
 //
 // GB300 layout: the sequence bytes sit in HBM exactly as the FASTA reader
-// left them (newlines included).  Work is cut into pieces of <= 64 KB of
-// one contig; each warp takes pieces from a global counter, and each lane
+// left them (newlines included).  Work is cut into pieces of 2 to 64 KB of
+// one contig (by the size of the whole); each warp takes pieces from a global counter, and each lane
 // walks a contiguous 1/32 of the piece with its own rolling state
 // (16-byte loads, the next one in flight), warmed up on the bytes just
 // before its run, so no lane depends on another while it counts.  The
@@ -32,7 +32,9 @@
 namespace {
 
 constexpr int kWarps = 8;
-constexpr uint64_t kPiece = 65536;  // bytes per piece
+constexpr uint64_t kPiece = 65536;  // most bytes per piece
+constexpr uint64_t kMinPiece = 2048;
+constexpr uint64_t kPlanContigs = 8192;  // most contigs of the one-block plan
 constexpr uint32_t kPoison = 0xFF00u;
 
 struct FoldTables {
@@ -46,7 +48,7 @@ struct FoldTables {
 // piece total, which the host compares with its limits before the uint32 scan
 // of npieces is used.  status must be zero on entry.
 __global__ void k_piece_counts(const uint64_t* __restrict__ off, const uint64_t* __restrict__ len, uint64_t n,
-                               uint64_t nbytes, uint32_t* __restrict__ npieces,
+                               uint64_t nbytes, uint64_t piece, uint32_t* __restrict__ npieces,
                                unsigned long long* __restrict__ status) {
     uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     uint64_t np = 0, bad = 0;
@@ -56,7 +58,7 @@ __global__ void k_piece_counts(const uint64_t* __restrict__ off, const uint64_t*
             bad = 1;
             np = 1;
         } else {
-            np = L == 0 ? 1 : L / kPiece + (L % kPiece != 0);  // <= 2^48: no overflow
+            np = L == 0 ? 1 : L / piece + (L % piece != 0);  // <= 2^53: no overflow
         }
         npieces[i] = (uint32_t)min(np, (uint64_t)0xFFFFFFFFu);
     }
@@ -77,6 +79,63 @@ __global__ void k_piece_map(const uint32_t* __restrict__ npieces, const uint32_t
     if (i >= n) return;
     uint32_t s = start[i], np = npieces[i];
     for (uint32_t k = 0; k < np; ++k) piece_contig[s + k] = (uint32_t)i;
+}
+
+// The plan of a small set in one block: pieces per contig, their starts and the
+// piece -> contig map, with the checks of k_piece_counts.  plan[0] receives
+// the pieces to count: 0 when a view is bad or the map (cap entries) is too
+// small, so that the counting kernel can be queued without a host check.
+__global__ void __launch_bounds__(1024) k_piece_plan(const uint64_t* __restrict__ off, const uint64_t* __restrict__ len,
+                                                     uint32_t n, uint64_t nbytes, uint64_t piece, uint64_t cap,
+                                                     uint32_t* __restrict__ npieces, uint32_t* __restrict__ start,
+                                                     uint32_t* __restrict__ pmap, uint32_t* __restrict__ plan,
+                                                     unsigned long long* __restrict__ status) {
+    __shared__ unsigned long long wsum[32];
+    __shared__ unsigned int nbad;
+    const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (t == 0) nbad = 0;
+    __syncthreads();
+    const uint32_t per = (n + 1023) / 1024, i0 = min(n, t * per), i1 = min(n, i0 + per);
+    unsigned long long mine = 0;
+    uint32_t bad = 0;
+    for (uint32_t i = i0; i < i1; ++i) {
+        const uint64_t L = len[i], o = off[i];
+        uint64_t np = 1;
+        if (o > nbytes || L > nbytes - o)
+            ++bad;
+        else if (L)
+            np = L / piece + (L % piece != 0);
+        npieces[i] = (uint32_t)min(np, (uint64_t)0xFFFFFFFFu);
+        mine += np;
+    }
+    if (bad) atomicAdd(&nbad, bad);
+    unsigned long long inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    unsigned long long before = 0, total = 0;
+    for (uint32_t k = 0; k < 32; ++k) {
+        if (k < w) before += wsum[k];
+        total += wsum[k];
+    }
+    const bool ok = nbad == 0 && total <= cap;
+    if (t == 0) {
+        plan[0] = ok ? (uint32_t)total : 0u;
+        status[0] = total;
+        status[1] = nbad;
+    }
+    if (!ok) return;  // block-uniform
+    uint32_t at = (uint32_t)(before + inc - mine);
+    for (uint32_t i = i0; i < i1; ++i) {
+        start[i] = at;
+        const uint32_t np = npieces[i];
+        for (uint32_t k = 0; k < np; ++k) pmap[at + k] = i;
+        at += np;
+    }
 }
 
 __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v) {
@@ -165,7 +224,7 @@ __device__ __forceinline__ void clip_chunk(uint4& v, uint64_t q, uint64_t a, uin
     }
 }
 
-// Warp per piece (<= 64 KB of one contig, taken from a global counter);
+// Warp per piece (at most `piece` bytes of one contig, taken from a global counter);
 // lane l walks its 1/32 of the piece in order with its own rolling state,
 // warmed up on the bytes just before its run, and counts each window that
 // ends in its run into the warp's shared histogram of raw 8-bit codes.  No
@@ -175,7 +234,8 @@ __global__ void __launch_bounds__(kWarps * 32) k_count(const unsigned char* __re
                                                       const uint64_t* __restrict__ len, uint64_t n,
                                                       const uint32_t* __restrict__ piece_start,
                                                       const uint32_t* __restrict__ npieces,
-                                                      const uint32_t* __restrict__ piece_contig, uint32_t total,
+                                                      const uint32_t* __restrict__ piece_contig, uint64_t piece,
+                                                      const uint32_t* __restrict__ plan, uint32_t total,
                                                       uint32_t* __restrict__ work, uint32_t* __restrict__ acc,
                                                       uint32_t* __restrict__ done, uint32_t* __restrict__ counts,
                                                       float* __restrict__ tnf, FoldTables tabs, int* flag) {
@@ -190,6 +250,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_count(const unsigned char* __re
         lut[c] = (uint16_t)(c == '\n' ? 0x8000u : (((c >> 1) & 3u) | (valid ? 0u : 0x300u)));
     }
     __syncthreads();
+    if (plan) total = plan[0];  // planned on the device
 
     while (true) {
         // the next piece (lane 0) and the abort flag (lane 1) load side by side
@@ -203,8 +264,8 @@ __global__ void __launch_bounds__(kWarps * 32) k_count(const unsigned char* __re
         const uint64_t c = piece_contig[p];
         const uint32_t k = p - piece_start[c];
         const uint64_t s0 = off[c], L = len[c];
-        const uint64_t p0 = s0 + (uint64_t)k * kPiece;
-        const uint64_t p1 = min(s0 + L, p0 + kPiece);
+        const uint64_t p0 = s0 + (uint64_t)k * piece;
+        const uint64_t p1 = min(s0 + L, p0 + piece);
 
         for (int i = lane; i < 257; i += 32) hist[i] = 0;
         __syncwarp();
@@ -321,32 +382,51 @@ static size_t count_cub_bytes(uint64_t n, cudaStream_t s) {
 // Phase 1 of a count: pieces per contig and the view check (status), piece
 // starts; the caller reads status back and checks it before phase 2.
 static cudaError_t count_phase1(const CountScratch& S, const uint64_t* d_off, const uint64_t* d_len, uint64_t n,
-                                uint64_t nbytes, cudaStream_t s) {
+                                uint64_t nbytes, uint64_t piece, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(S.status, 0, 16, s);
     if (e != cudaSuccess) return e;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    k_piece_counts<<<blocks, 256, 0, s>>>(d_off, d_len, n, nbytes, S.npieces, S.status);
+    k_piece_counts<<<blocks, 256, 0, s>>>(d_off, d_len, n, nbytes, piece, S.npieces, S.status);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     size_t tb = S.cub_bytes;
     return cub::DeviceScan::ExclusiveSum(S.cub_tmp, tb, S.npieces, S.start, (int)n, s);
 }
 
+// The counting kernel over `total` pieces, or (plan) as many as plan[0] says.
+static cudaError_t count_launch(const CountScratch& S, const unsigned char* d_bytes, const uint64_t* d_off,
+                                const uint64_t* d_len, uint64_t n, uint64_t piece, const uint32_t* plan,
+                                uint32_t total, uint32_t* d_counts, float* d_tnf, int* flag, int grid,
+                                cudaStream_t s) {
+    FoldTables tabs;
+    const TnTables& t = tn_tables();
+    memcpy(tabs.fw, t.col_fw, MDET_NTNF);
+    memcpy(tabs.rc, t.col_rc, MDET_NTNF);
+    k_count<<<grid, kWarps * 32, 0, s>>>(d_bytes, d_off, d_len, n, S.start, S.npieces, S.pmap, piece, plan, total,
+                                         S.work, S.acc, S.done, d_counts, d_tnf, tabs, flag);
+    return cudaGetLastError();
+}
+
 // Phase 2: piece map and the counting kernel.
 static cudaError_t count_phase2(const CountScratch& S, const unsigned char* d_bytes, const uint64_t* d_off,
-                                const uint64_t* d_len, uint64_t n, uint32_t total, uint32_t* d_counts, float* d_tnf,
-                                int* flag, int grid, cudaStream_t s) {
+                                const uint64_t* d_len, uint64_t n, uint64_t piece, uint32_t total,
+                                uint32_t* d_counts, float* d_tnf, int* flag, int grid, cudaStream_t s) {
     const unsigned blocks = (unsigned)((n + 255) / 256);
     k_piece_map<<<blocks, 256, 0, s>>>(S.npieces, S.start, n, S.pmap);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(S.work, 0, 4, s)) != cudaSuccess) return e;
-    FoldTables tabs;
-    const TnTables& t = tn_tables();
-    memcpy(tabs.fw, t.col_fw, MDET_NTNF);
-    memcpy(tabs.rc, t.col_rc, MDET_NTNF);
-    k_count<<<grid, kWarps * 32, 0, s>>>(d_bytes, d_off, d_len, n, S.start, S.npieces, S.pmap, total, S.work, S.acc,
-                                         S.done, d_counts, d_tnf, tabs, flag);
-    return cudaGetLastError();
+    return count_launch(S, d_bytes, d_off, d_len, n, piece, nullptr, total, d_counts, d_tnf, flag, grid, s);
+}
+
+// Bytes per piece: 64 KB (a warp's fixed work per piece, the fold of its
+// histogram, is then under 1 %), halved while the buffer would give the
+// chip's warps less than two pieces each: a lane walks its share of a piece
+// alone, at about 35 ns a byte, so a small set is as slow as one piece.  (300
+// contigs, 2.5 MB: k_count 72 us with 64 KB, 20 us with 2 KB.)
+static uint64_t piece_bytes(uint64_t nbytes, int grid) {
+    uint64_t p = kPiece;
+    while (p > kMinPiece && nbytes / p < 2ull * grid * kWarps) p >>= 1;
+    return p;
 }
 
 static int k_count_grid(int num_sms) {
@@ -355,8 +435,16 @@ static int k_count_grid(int num_sms) {
     return num_sms * (per_sm < 1 ? 1 : per_sm);
 }
 
+static int k_count_grid(mdet_ctx* ctx) {
+    if (!ctx->count_grid) ctx->count_grid = k_count_grid(ctx->num_sms);
+    return ctx->count_grid;
+}
+
+// flag: receives the device error flag when the call has read it (it had to
+// wait for the device anyway), and stays -1 otherwise.
 static int count_impl(mdet_ctx* ctx, const char* d_bytes, uint64_t nbytes, const uint64_t* d_off,
-                      const uint64_t* d_len, uint64_t n, uint32_t* d_counts, float* d_tnf) {
+                      const uint64_t* d_len, uint64_t n, uint32_t* d_counts, float* d_tnf, int* flag) {
+    *flag = -1;
     if (n == 0) return MDET_OK;
     if (n >= 0xFFFFFFFFull) return ctx_fail(ctx, MDET_ERR_INVALID, "too many contigs (%llu)", (unsigned long long)n);
     ctx->prep_cache.valid = false;  // new TNF rows: no preparation carries over past a count
@@ -381,30 +469,70 @@ static int count_impl(mdet_ctx* ctx, const char* d_bytes, uint64_t nbytes, const
     S.cub_bytes = count_cub_bytes(n, s);
     S.cub_tmp = ctx_scratch(ctx, "cnt.cubtmp", S.cub_bytes);
     if (!S.cub_tmp) return MDET_ERR_NOMEM;
-    MDET_CUDA(ctx, count_phase1(S, d_off, d_len, n, nbytes, s));
+    const int grid = k_count_grid(ctx);
+    uint64_t piece = piece_bytes(nbytes, grid);
+    unsigned long long st[2] = {0, 0};
+    // A small set is planned by one block and counted without a host check in
+    // between; views that overlap may need more pieces than the buffer's
+    // bytes do, in which case the general path below counts them.
+    const uint64_t cap = n + 2 * (nbytes / piece) + 64;
+    if (n <= kPlanContigs && cap < 0xFFFFFFFFull) {
+        S.pmap = (uint32_t*)ctx_scratch(ctx, "cnt.pmap", cap * 4);
+        if (!S.pmap) return MDET_ERR_NOMEM;
+        unsigned long long* h = (unsigned long long*)ctx_pinned(ctx, 64);
+        if (!h) return MDET_ERR_NOMEM;
+        uint32_t* plan = S.work + 6;
+        ctx_timer_begin(ctx, "k_count");
+        MDET_CUDA(ctx, cudaMemsetAsync(S.work, 0, 32, s));
+        k_piece_plan<<<1, 1024, 0, s>>>(d_off, d_len, (uint32_t)n, nbytes, piece, cap, S.npieces, S.start, S.pmap, plan,
+                                        S.status);
+        MDET_LAUNCHED(ctx, "k_piece_plan");
+        MDET_CUDA(ctx, count_launch(S, (const unsigned char*)d_bytes, d_off, d_len, n, piece, plan, 0, d_counts, d_tnf,
+                                    ctx->d_flag, grid, s));
+        ctx_timer_end(ctx, "k_count");
+        MDET_LAUNCHED(ctx, "k_count");
+        MDET_CUDA(ctx, cudaMemcpyAsync(h, S.status, 16, cudaMemcpyDeviceToHost, s));
+        MDET_CUDA(ctx, cudaMemcpyAsync(h + 2, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+        MDET_CUDA(ctx, cudaStreamSynchronize(s));
+        if (h[1]) return ctx_fail(ctx, MDET_ERR_INVALID, "%llu contig view(s) lie outside the byte buffer", h[1]);
+        if (h[0] <= cap) {
+            *flag = *(int*)(h + 2);
+            return MDET_OK;
+        }
+    }
+    MDET_CUDA(ctx, count_phase1(S, d_off, d_len, n, nbytes, piece, s));
     MDET_LAUNCHED(ctx, "k_piece_counts");
     // exact piece total in 64 bits (contig views may overlap, so it is not
     // bounded by nbytes) and the number of views outside the buffer
-    unsigned long long st[2] = {0, 0};
     MDET_CUDA(ctx, cudaMemcpyAsync(st, S.status, 16, cudaMemcpyDeviceToHost, s));
     MDET_CUDA(ctx, cudaStreamSynchronize(s));
+    if (st[0] > 0xFFFFFFFFull && piece < kPiece && !st[1]) {  // too many for the map: the largest pieces
+        piece = kPiece;
+        MDET_CUDA(ctx, count_phase1(S, d_off, d_len, n, nbytes, piece, s));
+        MDET_LAUNCHED(ctx, "k_piece_counts");
+        MDET_CUDA(ctx, cudaMemcpyAsync(st, S.status, 16, cudaMemcpyDeviceToHost, s));
+        MDET_CUDA(ctx, cudaStreamSynchronize(s));
+    }
     if (st[1]) return ctx_fail(ctx, MDET_ERR_INVALID, "%llu contig view(s) lie outside the byte buffer", st[1]);
     if (st[0] > 0xFFFFFFFFull)
         return ctx_fail(ctx, MDET_ERR_CAPACITY, "%llu 64-KB pieces of sequence (views overlap too much)", st[0]);
     S.pmap = (uint32_t*)ctx_scratch(ctx, "cnt.pmap", (size_t)st[0] * 4);
     if (!S.pmap) return MDET_ERR_NOMEM;
     ctx_timer_begin(ctx, "k_count");
-    MDET_CUDA(ctx, count_phase2(S, (const unsigned char*)d_bytes, d_off, d_len, n, (uint32_t)st[0], d_counts, d_tnf,
-                                ctx->d_flag, k_count_grid(ctx->num_sms), s));
+    MDET_CUDA(ctx, count_phase2(S, (const unsigned char*)d_bytes, d_off, d_len, n, piece, (uint32_t)st[0], d_counts,
+                                d_tnf, ctx->d_flag, grid, s));
     ctx_timer_end(ctx, "k_count");
     MDET_LAUNCHED(ctx, "k_count");
     return MDET_OK;
 }
 
-static int check_flag(mdet_ctx* ctx) {
-    int h = 0;
-    MDET_CUDA(ctx, cudaMemcpyAsync(&h, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    MDET_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+// known: the flag as count_impl read it, or -1 to read it here.
+static int check_flag(mdet_ctx* ctx, int known = -1) {
+    int h = known;
+    if (known < 0) {
+        MDET_CUDA(ctx, cudaMemcpyAsync(&h, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        MDET_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    }
     if (h) {
         cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream);
         ctx->count_scratch_dirty = true;
@@ -422,12 +550,13 @@ int mdet_tnf_count_dev(mdet_ctx* ctx, const char* d_bytes, uint64_t nbytes, cons
         return ctx_fail(ctx, MDET_ERR_INVALID, "null pointer");
     MDET_CUDA(ctx, cudaSetDevice(ctx->device));
     ctx->launches = 0;
-    int rc = count_impl(ctx, d_bytes, nbytes, d_off, d_len, n, d_counts, d_tnf);
+    int flag = -1;
+    int rc = count_impl(ctx, d_bytes, nbytes, d_off, d_len, n, d_counts, d_tnf, &flag);
     if (rc != MDET_OK) {
         ctx->count_scratch_dirty = true;
         return rc;
     }
-    return check_flag(ctx);
+    return check_flag(ctx, flag);
 }
 
 // Chunked host-buffer path of mdet_tnf_count (file-order views, see there).
@@ -466,10 +595,11 @@ static int count_chunked(mdet_ctx* ctx, const char* bytes, uint64_t nbytes, cons
     }
     for (size_t k = 0; k < K && rc == MDET_OK; ++k) {
         const uint64_t c0 = cs[k], nk = cs[k + 1] - cs[k];
+        int flag = -1;
         rc = ctx_cuda(ctx, cudaStreamWaitEvent(s, landed[k], 0), "cudaStreamWaitEvent");
         if (rc == MDET_OK && nk)
             rc = count_impl(ctx, d_bytes, nbytes, d_off + c0, d_len + c0, nk, d_counts + c0 * MDET_NTNF,
-                            d_tnf + c0 * MDET_NTNF);
+                            d_tnf + c0 * MDET_NTNF, &flag);
         if (rc == MDET_OK) rc = ctx_cuda(ctx, cudaEventRecord(counted[k], s), "cudaEventRecord");
         if (rc == MDET_OK) rc = ctx_cuda(ctx, cudaStreamWaitEvent(ctx->io_out, counted[k], 0), "cudaStreamWaitEvent");
         if (rc == MDET_OK && nk && counts)
@@ -525,7 +655,8 @@ int mdet_tnf_count(mdet_ctx* ctx, const char* bytes, uint64_t nbytes, const uint
     if (ordered) return count_chunked(ctx, bytes, nbytes, off, len, n, counts, tnf, d_bytes, d_off, d_len, d_counts,
                                       d_tnf);
     MDET_CUDA(ctx, cudaMemcpyAsync(d_bytes, bytes, nbytes, cudaMemcpyHostToDevice, s));
-    int rc = count_impl(ctx, d_bytes, nbytes, d_off, d_len, n, d_counts, d_tnf);
+    int flag = -1;  // the rows are copied out before the flag is looked at
+    int rc = count_impl(ctx, d_bytes, nbytes, d_off, d_len, n, d_counts, d_tnf, &flag);
     if (rc != MDET_OK) {
         ctx->count_scratch_dirty = true;
         return rc;
@@ -565,7 +696,8 @@ int mdet_tnf_count_fasta(mdet_ctx* ctx, const char* bytes, uint64_t nbytes, uint
     uint32_t* d_counts = (uint32_t*)ctx_scratch(ctx, "io.counts", n * MDET_NTNF * 4);
     float* d_tnf = (float*)ctx_scratch(ctx, "io.tnf", n * MDET_NTNF * 4);
     if (!d_counts || !d_tnf) return MDET_ERR_NOMEM;
-    int rc = count_impl(ctx, d_bytes, nbytes, d_off, d_len, n, d_counts, d_tnf);
+    int flag = -1;  // the rows are copied out before the flag is looked at
+    int rc = count_impl(ctx, d_bytes, nbytes, d_off, d_len, n, d_counts, d_tnf, &flag);
     if (rc != MDET_OK) {
         ctx->count_scratch_dirty = true;
         return rc;
@@ -677,7 +809,7 @@ extern "C" int mdet_tnf_count_noalloc(const char* d_bytes, uint64_t nbytes, cons
         cudaMemsetAsync(S.acc, 0, (size_t)n * MDET_NTNF * 4, s) != cudaSuccess ||
         cudaMemsetAsync(S.work, 0, 64 * 4, s) != cudaSuccess)
         return fail(MDET_ERR_CUDA);
-    if (count_phase1(S, d_off, d_len, n, nbytes, s) != cudaSuccess) return fail(MDET_ERR_CUDA);
+    if (count_phase1(S, d_off, d_len, n, nbytes, kPiece, s) != cudaSuccess) return fail(MDET_ERR_CUDA);
     // the 64-bit piece total and the count of views outside [0, nbytes),
     // checked before k_piece_map writes piece entries into the array
     unsigned long long st[2] = {0, 0};
@@ -686,7 +818,7 @@ extern "C" int mdet_tnf_count_noalloc(const char* d_bytes, uint64_t nbytes, cons
         return fail(MDET_ERR_CUDA);
     if (st[1]) return MDET_ERR_INVALID;
     if (st[0] > MDET_NOALLOC_MAX_PIECES) return MDET_ERR_CAPACITY;
-    if (count_phase2(S, (const unsigned char*)d_bytes, d_off, d_len, n, (uint32_t)st[0], d_counts, d_tnf, flag,
+    if (count_phase2(S, (const unsigned char*)d_bytes, d_off, d_len, n, kPiece, (uint32_t)st[0], d_counts, d_tnf, flag,
                      d.grid, s) != cudaSuccess)
         return fail(MDET_ERR_CUDA);
     int h_flag = 0;
