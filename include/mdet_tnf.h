@@ -410,7 +410,7 @@ typedef struct {
     uint64_t binned_bases, leftover_bases, small_bases;
     int leftovers_accepted, small_accepted; /* the 10 % and 15 % gates */
     uint64_t pairs_tested;        /* (contig, scored bin) pairs */
-    uint64_t pairs_exact;         /* of those, the ones the FP32 prefilter left to the exact FP64 test */
+    uint64_t pairs_exact;         /* of those, the ones the FP32 prefilter on ten members did not reject */
     uint64_t pairs_undecided;     /* of those, tests within the error bound of a bin's estimated mean */
     uint64_t bins_exact;          /* bins whose exact mean was computed (degenerate rows, undecided tests) */
 } mdet_recruit_stats;

@@ -20,8 +20,9 @@
 // mean taken once (k_corr_rows); a correlation is then one cross sum.  The
 // bins' means are first estimated in FP32 with a proven error bound; an FP32
 // prefilter drops the (contig, bin) pairs the reference's first-ten test
-// provably rejects; the rest get the reference's test in FP64, term by term
-// in member order.  A test whose value lands within the bound of its bin's
+// provably rejects; the rest are decided by FP32 means where those are
+// further from the bin's mean than their own bounds (k_recruit_est), and the
+// few others get the reference's test in FP64, term by term in member order.  A test whose value lands within the bound of its bin's
 // estimate is decided again with a finer estimate (the FP64 terms in a fixed
 // tree) and at last with the bin's exact mean (the reference's terms in the
 // reference's order), so every decision is the reference's.  The unit is
@@ -146,6 +147,10 @@ __device__ __forceinline__ float corr32(const float* __restrict__ x, const float
 // (1.02 m + 20.5) u of the reference's.  A pair whose FP32 mean is below the
 // bin's threshold less delta = 4 (m + 32) u is one the reference's
 // first-ten test rejects.
+//
+// A contig's mean over a whole bin of cs members, from FP32 terms added in
+// FP32 runs of eight, the runs in FP64 (per-lane sums and a fixed tree), has
+// the error of a bin's mean below with T = cs.
 //
 // A bin's mean, estimated from FP32 terms added in FP32 runs of eight, the
 // runs in FP64 (per-thread sums and a fixed tree), is within
@@ -469,7 +474,73 @@ __global__ void __launch_bounds__(256) k_recruit_filter(const float* __restrict_
     }
 }
 
-// The reference's two-step test for the pairs the prefilter kept: a warp
+// The reference's two-step test by FP32 estimates, for the pairs the
+// prefilter kept: a warp per (contig, bin), the lanes on consecutive members
+// (column-major rows).  The first-ten mean is within d10 of the reference's
+// and the whole mean within mean_eps(cs terms), so a value further than that
+// from [lo, hi) decides as the reference's does; a pair that neither mean
+// decides, or with a row the bounds do not cover, goes to the list `rest` for
+// k_recruit_exact.  (150,000 contigs and 20,000 small ones, 333 bins: the
+// FP64 test of all kept pairs took 1,135 us, 450 ordered adds a pair on the
+// narrow FP64 unit; this takes 137 us and leaves no pair.)
+__global__ void __launch_bounds__(256) k_recruit_est(const float* __restrict__ xw, const float* __restrict__ gf,
+                                                     uint32_t nabd, const uint32_t* __restrict__ left, uint64_t nl,
+                                                     uint64_t n, const uint64_t* __restrict__ off,
+                                                     const double* __restrict__ lo, const double* __restrict__ hi,
+                                                     double d10, double scale, const uint2* __restrict__ pass,
+                                                     const unsigned long long* __restrict__ npass, uint64_t cap,
+                                                     uint32_t* __restrict__ qcount, uint32_t* __restrict__ qbin,
+                                                     uint2* __restrict__ rest, unsigned long long* __restrict__ nrest) {
+    const uint32_t m = nabd - 1;
+    const uint64_t warps = (gridDim.x * (uint64_t)blockDim.x) >> 5, np = min((uint64_t)*npass, cap);
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint64_t p = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; p < np; p += warps) {
+        const uint2 pr = pass[p];
+        const uint64_t cand = pr.x;
+        const uint32_t b = pr.y;
+        const float* y = xw + (cand < nl ? (uint64_t)left[cand] : n + (cand - nl)) * nabd;
+        const uint64_t o = off[b], cs = off[b + 1] - o;
+        const float* g = gf + o * nabd;
+        const double l = lo[b], h = hi[b];
+        bool covered = y[m] <= 1.0f / kMinDev;
+        // a lane's terms, in FP32 runs of eight; lane l < 10 starts with member l
+        double pd = 0.0;
+        float pf = 0.f, ten = 0.f;
+        uint32_t run = 0;
+        for (uint64_t i = lane; i < cs; i += 32) {
+            covered = covered && g[m * cs + i] <= 1.0f / kMinDev;
+            const float t = corr32_col(y, g + i, cs, m);
+            if (i < kMinCS) ten = t;
+            pf += t;
+            if (++run == 8) {
+                pd += (double)pf;
+                pf = 0.f;
+                run = 0;
+            }
+        }
+        pd += (double)pf;
+        for (int d = 16; d > 0; d >>= 1) {
+            ten += __shfl_xor_sync(0xffffffffu, ten, d);
+            pd += __shfl_xor_sync(0xffffffffu, pd, d);
+        }
+        covered = __all_sync(0xffffffffu, covered);
+        if (lane) continue;
+        const double v = (double)(ten / (float)kMinCS), c = pd / (double)cs, e = mean_eps(m, cs, true, scale);
+        // NaN compares false everywhere: left to the exact test
+        if (covered && v + d10 < l) continue;  // the reference's early stop on the first ten members
+        if (covered && v - d10 >= h) {
+            if (c + e < l) continue;
+            if (c - e >= h) {
+                atomicAdd(&qcount[cand], 1u);
+                qbin[cand] = b;
+                continue;
+            }
+        }
+        rest[atomicAdd(nrest, 1ull)] = pr;
+    }
+}
+
+// The reference's two-step test for the pairs k_recruit_est left: a warp
 // per (contig, bin); the lanes compute FP64 member correlations side by
 // side and every lane adds them in member order (the first ten, the early
 // stop, the rest, the division), as the reference's.  The two comparisons
@@ -608,6 +679,36 @@ extern "C" int mdet_recruit(mdet_ctx* ctx, const float* abd, const float* small_
         return ctx_fail(ctx, MDET_ERR_INVALID, "%u depth columns (1..%u supported)", nabd, kMaxSamples);
     if (n >= 0xFFFFFFFFull || n_small >= 0xFFFFFFFFull || n + n_small >= 0xFFFFFFFFull)
         return ctx_fail(ctx, MDET_ERR_INVALID, "too many contigs");
+    cudaStream_t s = ctx->stream;
+    const uint64_t rows = n + n_small;
+    float *d_abd = nullptr, *d_sabd = nullptr, *d_xf = nullptr, *d_xw = nullptr;
+    double* d_d64 = nullptr;
+    // the depth rows on the device, ranked, with their deviations
+    auto rank_rows = [&]() -> int {
+        d_abd = (float*)ctx_scratch(ctx, "rc.abd", n * nabd * 4);
+        d_sabd = (float*)ctx_scratch(ctx, "rc.sabd", std::max<uint64_t>(n_small, 1) * nabd * 4);
+        d_d64 = (double*)ctx_scratch(ctx, "rc.d64", rows * nabd * 8);
+        d_xf = (float*)ctx_scratch(ctx, "rc.xf", rows * nabd * 4);
+        d_xw = (float*)ctx_scratch(ctx, "rc.xw", rows * nabd * 4);
+        if (!d_abd || !d_sabd || !d_d64 || !d_xf || !d_xw) return MDET_ERR_NOMEM;
+        ctx_timer_begin(ctx, "k_rank_rows");
+        auto set = [&](const float* src, float* d, uint64_t k, uint64_t row0) -> int {
+            if (!k) return MDET_OK;
+            MDET_CUDA(ctx, cudaMemcpyAsync(d, src, k * nabd * 4, cudaMemcpyHostToDevice, s));
+            k_rank_rows<<<(unsigned)((k + 127) / 128), 128, 0, s>>>(d, k, nabd);
+            MDET_LAUNCHED(ctx, "k_rank_rows");
+            k_corr_rows<<<(unsigned)((k + 127) / 128), 128, 0, s>>>(d, k, nabd, row0, d_d64, d_xf, d_xw);
+            MDET_LAUNCHED(ctx, "k_corr_rows");
+            return MDET_OK;
+        };
+        MDET_TRY(set(abd, d_abd, n, 0));
+        MDET_TRY(set(small_abd, d_sabd, n_small, n));
+        ctx_timer_end(ctx, "k_rank_rows");
+        return MDET_OK;
+    };
+    // with small contigs there is something to test whatever the bins are: the
+    // device ranks the rows while the host groups the labels
+    if (n_small) MDET_TRY(rank_rows());
     // bins by label in ascending label order, members ascending (the
     // reference's std::map of vectors); dissolve those under min_cls_size
     std::vector<int64_t> glabel;
@@ -648,13 +749,8 @@ extern "C" int mdet_recruit(mdet_ctx* ctx, const float* abd, const float* small_
         st->binned_bases = binned;
     }
     if (nl == 0 && n_small == 0) return MDET_OK;
-    cudaStream_t s = ctx->stream;
-    const uint64_t rows = n + n_small, ncand = nl + n_small;
-    float* d_abd = (float*)ctx_scratch(ctx, "rc.abd", n * nabd * 4);
-    float* d_sabd = (float*)ctx_scratch(ctx, "rc.sabd", std::max<uint64_t>(n_small, 1) * nabd * 4);
-    double* d_d64 = (double*)ctx_scratch(ctx, "rc.d64", rows * nabd * 8);
-    float* d_xf = (float*)ctx_scratch(ctx, "rc.xf", rows * nabd * 4);
-    float* d_xw = (float*)ctx_scratch(ctx, "rc.xw", rows * nabd * 4);
+    if (!n_small) MDET_TRY(rank_rows());
+    const uint64_t ncand = nl + n_small;
     uint64_t* d_off = (uint64_t*)ctx_scratch(ctx, "rc.off", (nb + 1) * 8);
     uint32_t* d_mem = (uint32_t*)ctx_scratch(ctx, "rc.mem", std::max<size_t>(bmem.size(), 1) * 4);
     uint32_t* d_left = (uint32_t*)ctx_scratch(ctx, "rc.left", std::max<uint64_t>(nl, 1) * 4);
@@ -662,29 +758,15 @@ extern "C" int mdet_recruit(mdet_ctx* ctx, const float* abd, const float* small_
     float* d_thr = (float*)ctx_scratch(ctx, "rc.thr", std::max<uint32_t>(nb, 1) * 4);
     uint32_t* d_qc = (uint32_t*)ctx_scratch(ctx, "rc.qc", std::max<uint64_t>(ncand, 1) * 4);
     uint32_t* d_qb = (uint32_t*)ctx_scratch(ctx, "rc.qb", std::max<uint64_t>(ncand, 1) * 4);
-    unsigned long long* d_np = (unsigned long long*)ctx_scratch(ctx, "rc.npass", 8);
-    if (!d_abd || !d_sabd || !d_d64 || !d_xf || !d_xw || !d_off || !d_mem || !d_left || !d_bc || !d_thr || !d_qc ||
+    unsigned long long* d_np = (unsigned long long*)ctx_scratch(ctx, "rc.npass", 16);
+    if (!d_off || !d_mem || !d_left || !d_bc || !d_thr || !d_qc ||
         !d_qb || !d_np)
         return MDET_ERR_NOMEM;
-    MDET_CUDA(ctx, cudaMemcpyAsync(d_abd, abd, n * nabd * 4, cudaMemcpyHostToDevice, s));
-    if (n_small) MDET_CUDA(ctx, cudaMemcpyAsync(d_sabd, small_abd, n_small * nabd * 4, cudaMemcpyHostToDevice, s));
     MDET_CUDA(ctx, cudaMemcpyAsync(d_off, boff.data(), (nb + 1) * 8, cudaMemcpyHostToDevice, s));
     if (!bmem.empty()) MDET_CUDA(ctx, cudaMemcpyAsync(d_mem, bmem.data(), bmem.size() * 4, cudaMemcpyHostToDevice, s));
     if (nl) MDET_CUDA(ctx, cudaMemcpyAsync(d_left, leftovers.data(), nl * 4, cudaMemcpyHostToDevice, s));
     MDET_CUDA(ctx, cudaMemsetAsync(d_qc, 0, std::max<uint64_t>(ncand, 1) * 4, s));
-    ctx_timer_begin(ctx, "k_rank_rows");
-    k_rank_rows<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(d_abd, n, nabd);
-    MDET_LAUNCHED(ctx, "k_rank_rows");
-    k_corr_rows<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(d_abd, n, nabd, 0, d_d64, d_xf, d_xw);
-    MDET_LAUNCHED(ctx, "k_corr_rows");
-    if (n_small) {
-        k_rank_rows<<<(unsigned)((n_small + 127) / 128), 128, 0, s>>>(d_sabd, n_small, nabd);
-        MDET_LAUNCHED(ctx, "k_rank_rows");
-        k_corr_rows<<<(unsigned)((n_small + 127) / 128), 128, 0, s>>>(d_sabd, n_small, nabd, n, d_d64, d_xf, d_xw);
-        MDET_LAUNCHED(ctx, "k_corr_rows");
-    }
-    ctx_timer_end(ctx, "k_rank_rows");
-    uint64_t npass = 0;
+    uint64_t npass = 0, nrest = 0;
     if (nb) {
         double* d_est = (double*)ctx_scratch(ctx, "rc.est", nb * 8);
         double* d_est2 = (double*)ctx_scratch(ctx, "rc.est2", nb * 8);
@@ -795,8 +877,10 @@ extern "C" int mdet_recruit(mdet_ctx* ctx, const float* abd, const float* small_
         ctx_timer_begin(ctx, "k_recruit_filter");
         for (int pass_no = 0; pass_no < 2; ++pass_no) {
             uint2* d_pass = (uint2*)ctx_scratch(ctx, "rc.pass", cap * 8);
-            if (!d_pass) return MDET_ERR_NOMEM;
-            MDET_CUDA(ctx, cudaMemsetAsync(d_np, 0, 8, s));
+            uint2* d_rest = (uint2*)ctx_scratch(ctx, "rc.rest", cap * 8);
+            if (!d_pass || !d_rest) return MDET_ERR_NOMEM;
+            MDET_CUDA(ctx, cudaMemsetAsync(d_np, 0, 16, s));
+            if (pass_no) MDET_CUDA(ctx, cudaMemsetAsync(d_qc, 0, ncand * 4, s));
             const uint32_t m = nabd - 1;
             if (m <= 16)
                 k_recruit_filter<16><<<grid, 256, 0, s>>>(d_xf, d_xw, nabd, d_left, nl, n, ncand, d_off, d_mem, nb,
@@ -808,23 +892,29 @@ extern "C" int mdet_recruit(mdet_ctx* ctx, const float* abd, const float* small_
                 k_recruit_filter<0><<<grid, 256, 0, s>>>(d_xf, d_xw, nabd, d_left, nl, n, ncand, d_off, d_mem, nb,
                                                          chunk, d_thr, d_pass, cap, d_np);
             MDET_LAUNCHED(ctx, "k_recruit_filter");
-            MDET_CUDA(ctx, cudaMemcpyAsync(&npass, d_np, 8, cudaMemcpyDeviceToHost, s));
+            k_recruit_est<<<(unsigned)ctx->num_sms * 8, 256, 0, s>>>(
+                d_xw, d_gf, nabd, d_left, nl, n, d_off, d_lo, d_hi, delta * eps_scale, eps_scale, d_pass, d_np, cap,
+                d_qc, d_qb, d_rest, d_np + 1);
+            MDET_LAUNCHED(ctx, "k_recruit_est");
+            uint64_t h_np[2];
+            MDET_CUDA(ctx, cudaMemcpyAsync(h_np, d_np, 16, cudaMemcpyDeviceToHost, s));
             MDET_CUDA(ctx, cudaStreamSynchronize(s));
+            npass = h_np[0];
+            nrest = h_np[1];
             if (npass <= cap) break;
             cap = npass;  // the list overflowed: once more with room for all of it
         }
         ctx_timer_end(ctx, "k_recruit_filter");
         if (npass > cap) return ctx_fail(ctx, MDET_ERR_INTERNAL, "prefilter list overflow");
         uint64_t undecided = 0;
-        if (npass) {
+        if (nrest) {
             // the tests; those within eps of a bin's estimate again with the
             // bin's next estimate, and at last with its exact mean
-            uint2* d_list[2] = {(uint2*)ctx_scratch(ctx, "rc.pass", cap * 8), nullptr};
-            uint2* d_amb[2] = {(uint2*)ctx_scratch(ctx, "rc.amb", npass * 8),
-                               (uint2*)ctx_scratch(ctx, "rc.amb2", npass * 8)};
-            if (!d_list[0] || !d_amb[0] || !d_amb[1]) return MDET_ERR_NOMEM;
-            const uint2* cur = d_list[0];
-            uint64_t ncur = npass;
+            const uint2* cur = (const uint2*)ctx_scratch(ctx, "rc.rest", cap * 8);
+            uint2* d_amb[2] = {(uint2*)ctx_scratch(ctx, "rc.amb", nrest * 8),
+                               (uint2*)ctx_scratch(ctx, "rc.amb2", nrest * 8)};
+            if (!cur || !d_amb[0] || !d_amb[1]) return MDET_ERR_NOMEM;
+            uint64_t ncur = nrest;
             ctx_timer_begin(ctx, "k_recruit");
             for (uint8_t round = 0; ncur; ++round) {
                 uint2* next = d_amb[round & 1];
