@@ -18,10 +18,12 @@
 // Contigs that share no edge do not read each other, so the sweep runs level
 // by level over the order's dependency graph (level = 1 + the deepest level
 // among the contig's neighbours earlier in the order, found by Kahn peeling):
-// one block per contig of a level, the levels in turn -- the same result as
-// the sequential sweep.  A block sorts its contig's (neighbour label, edge
+// the contigs of a level side by side, the levels in turn -- the same result
+// as the sequential sweep.  The peeling and all sweeps of a run are one
+// cooperative launch each, with a bounded grid barrier between levels.  A
+// block sorts its contig's (neighbour label, edge
 // position) keys (bitonic sort in shared memory, or in a global slice for
-// contigs with more than 2,048 edges), folds each label's log(1 - score) in
+// contigs with more than 1,024 edges), folds each label's log(1 - score) in
 // edge order (the reference's summation order), evaluates the CDF
 // (lp_math.h, bit-identical to the host checker) and breaks exact ties by the
 // reference map's iteration order (lp_umap.h); contigs with at most 32 edges
@@ -48,9 +50,13 @@ int check_flag(mdet_ctx* ctx);
 
 namespace {
 
-constexpr uint32_t kSmallCap = 2048;  // incident edges a block sorts in shared memory
+constexpr uint32_t kSmallCap = 1024;  // incident edges a group sorts in shared memory (four areas per SM)
 constexpr uint32_t kWarpCap = 32;     // incident edges a warp sorts in registers
-constexpr int kThreads = 256;
+constexpr int kThreads = 256;         // threads that evaluate one block contig
+// The cooperative kernels run one block of 32 warps per SM, four groups of
+// kThreads: a grid barrier takes 1.4 us over 152 blocks, 2.6 us over 608.
+constexpr int kCoopThreads = 1024;
+constexpr int kGroups = kCoopThreads / kThreads;
 constexpr uint32_t kProbeLimit = 1u << 16;
 
 // flags
@@ -94,15 +100,21 @@ struct LpArgs {
     const uint32_t* slot_of;
 };
 
+// What a block's contigs did in a sweep, added to the counters once per
+// sweep: one address taking an atomic per changed contig was what the
+// first sweeps waited for.
+struct Tally {
+    unsigned int moved, entries;
+};
+
 // true when (v, lab) was not in the table
-__device__ bool visit(const LpArgs& P, uint32_t v, uint32_t lab) {
+__device__ bool visit(const LpArgs& P, uint32_t v, uint32_t lab, Tally& T) {
     const unsigned long long key = (((unsigned long long)v << 32) | lab) + 1ull;
     unsigned long long h = mix64(key) & P.vt_mask;
     for (uint32_t it = 0; it < kProbeLimit; ++it) {
         const unsigned long long old = atomicCAS(P.vt + h, 0ull, key);
         if (old == 0ull) {
-            const unsigned long long cnt = atomicAdd(P.counters + 1, 1ull) + 1;
-            if (cnt * 4 > (P.vt_mask + 1) * 3) atomicOr(P.counters + 2, kErrTable);
+            atomicAdd(&T.entries, 1u);
             return true;
         }
         if (old == key) return false;
@@ -112,19 +124,63 @@ __device__ bool visit(const LpArgs& P, uint32_t v, uint32_t lab) {
     return false;
 }
 
-// One sweep step for the contigs of one level: block per contig.
-__global__ void __launch_bounds__(kThreads) k_lp_level(LpArgs P, const uint32_t* __restrict__ nodes) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double red_v[kThreads / 32];
-    __shared__ uint32_t red_c[kThreads / 32];
-    __shared__ double s_vmax;
-    __shared__ uint32_t s_ties, s_best, s_changed;
-    const uint32_t v = nodes[blockIdx.x];
+// A barrier over all blocks of a cooperative launch: every block adds one to
+// *bar, whose target grows by the grid's size each time.  The wait is bounded;
+// a block whose wait runs out raises the context's flag, and every block's
+// loops end at their next barrier.  False then.
+__device__ bool grid_barrier(unsigned int* bar, unsigned int& target, int* flag) {
+    __shared__ bool ok;
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        bool good = true;
+        const long long t0 = clock64();
+        for (uint32_t poll = 1; (int)(*(volatile unsigned int*)bar - target) < 0; ++poll) {
+            if (poll & 255u) continue;  // the flag and the clock now and then
+            const bool late = (unsigned long long)(clock64() - t0) > MDET_SPIN_CYCLES;
+            if (late) atomicOr(flag, MDET_FLAG_TIMEOUT);
+            if (late || *(volatile int*)flag) {
+                good = false;
+                break;
+            }
+        }
+        __threadfence();
+        ok = good;
+    }
+    __syncthreads();
+    const bool r = ok;
+    __syncthreads();
+    return r;
+}
+
+// Barrier of the kThreads threads of this thread's group.
+__device__ __forceinline__ void group_sync() {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / kThreads), "n"(kThreads) : "memory");
+}
+
+// Shared variables of one contig's evaluation by a group.
+struct BlockWs {
+    double red_v[kThreads / 32];
+    uint32_t red_c[kThreads / 32];
+    double vmax;
+    uint32_t ties, best, changed;
+};
+
+// One contig's sweep step by a group of kThreads threads.  Labels and flags change while
+// the sweep kernel runs, so they are read past the L1 cache.
+__device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, BlockWs& B, Tally& T) {
+    double* red_v = B.red_v;
+    uint32_t* red_c = B.red_c;
+    double& s_vmax = B.vmax;
+    uint32_t &s_ties = B.ties, &s_best = B.best, &s_changed = B.changed;
     const uint32_t s = P.inc_off[v];
     const uint32_t d = P.inc_off[v + 1] - s;
     // no neighbour changed since the last evaluation: the same label wins
     // and the update is a no-op
-    if (d == 0 || !P.dirty[v]) return;
+    if (d == 0 || !__ldcg(P.dirty + v)) return;
+    group_sync();  // the group's previous contig is done with the shared arrays
     const uint32_t N = pow2_at_least(d);
     unsigned char* base = smem;
     if (N > kSmallCap) {
@@ -142,20 +198,20 @@ __global__ void __launch_bounds__(kThreads) k_lp_level(LpArgs P, const uint32_t*
     uint32_t* ins = reinterpret_cast<uint32_t*>(base + (size_t)N * 28);
     int32_t* nxt = reinterpret_cast<int32_t*>(base + (size_t)N * 32);
     int32_t* bb = reinterpret_cast<int32_t*>(base + (size_t)N * 36);
-    const uint32_t t = threadIdx.x;
+    const uint32_t t = threadIdx.x % kThreads;
 
     // (neighbour label, edge position) keys and the edges' log(1 - score)
     for (uint32_t j = t; j < N; j += kThreads) {
         if (j < d) {
             const uint32_t o = P.oth[s + j];
-            sk[j] = ((unsigned long long)P.mem[o] << 32) | j;
+            sk[j] = ((unsigned long long)__ldcg(P.mem + o) << 32) | j;
             w[j] = P.ilw[s + j];
         } else {
             sk[j] = ~0ull;
         }
         fidx[j] = -1;
     }
-    __syncthreads();
+    group_sync();
     // bitonic sort, ascending
     for (uint32_t k = 2; k <= N; k <<= 1) {
         for (uint32_t jj = k >> 1; jj > 0; jj >>= 1) {
@@ -170,7 +226,7 @@ __global__ void __launch_bounds__(kThreads) k_lp_level(LpArgs P, const uint32_t*
                     }
                 }
             }
-            __syncthreads();
+            group_sync();
         }
     }
     // each label's run: the Fisher-combined CDF of its edges, folded in edge
@@ -195,31 +251,31 @@ __global__ void __launch_bounds__(kThreads) k_lp_level(LpArgs P, const uint32_t*
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
     if ((t & 31) == 0) red_v[t >> 5] = vmax;
-    __syncthreads();
+    group_sync();
     if (t == 0) {
         double m = red_v[0];
         for (int i = 1; i < kThreads / 32; ++i) m = fmax(m, red_v[i]);
         s_vmax = m;
     }
-    __syncthreads();
+    group_sync();
     const double top = s_vmax;
     uint32_t ties = 0;
     for (uint32_t p = t; p < d; p += kThreads) ties += val[p] == top;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ties += __shfl_xor_sync(0xffffffffu, ties, o);
     if ((t & 31) == 0) red_c[t >> 5] = ties;
-    __syncthreads();
+    group_sync();
     if (t == 0) {
         uint32_t nt = 0;
         for (int i = 0; i < kThreads / 32; ++i) nt += red_c[i];
         s_ties = nt;
     }
-    __syncthreads();
+    group_sync();
     if (s_ties == 1) {
         for (uint32_t p = t; p < d; p += kThreads)
             if (val[p] == top) s_best = (uint32_t)(sk[p] >> 32);
     }
-    __syncthreads();
+    group_sync();
     if (t == 0) {
         P.dirty[v] = 0;
         if (s_ties > 1) {
@@ -241,16 +297,16 @@ __global__ void __launch_bounds__(kThreads) k_lp_level(LpArgs P, const uint32_t*
         }
         const uint32_t b = s_best;
         s_changed = 0;
-        if (P.mem[v] != b && !P.stuck[v]) {
+        if (__ldcg(P.mem + v) != b && !__ldcg(P.stuck + v)) {
             P.mem[v] = b;
             s_changed = 1;
-            if (visit(P, v, b))
-                atomicAdd(P.counters, 1ull);
+            if (visit(P, v, b, T))
+                atomicAdd(&T.moved, 1u);
             else
                 P.stuck[v] = 1;
         }
     }
-    __syncthreads();
+    group_sync();
     if (s_changed)
         for (uint32_t j = t; j < d; j += kThreads) {
             P.dirty[P.oth[s + j]] = 1;
@@ -259,7 +315,7 @@ __global__ void __launch_bounds__(kThreads) k_lp_level(LpArgs P, const uint32_t*
 
 // The same step for contigs with at most 32 edges: a warp per contig, the
 // keys sorted in registers (bitonic over lanes), a lane per edge.
-constexpr int kWarpsPerBlock = kThreads / 32;
+constexpr int kWarpsPerBlock = kCoopThreads / 32;
 struct WarpWs {
     unsigned long long sk[32];
     double w[32];
@@ -270,29 +326,46 @@ struct WarpWs {
     int32_t bb[64];  // lpu::buckets_for(32) = 59
 };
 
-__global__ void __launch_bounds__(kThreads) k_lp_level_warp(LpArgs P, const uint32_t* __restrict__ nodes,
-                                                            uint32_t count) {
-    __shared__ WarpWs ws_all[kWarpsPerBlock];
-    const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t idx = blockIdx.x * kWarpsPerBlock + wid;
-    if (idx >= count) return;
-    WarpWs& W = ws_all[wid];
-    const uint32_t v = nodes[idx];
-    const uint32_t s = P.inc_off[v];
-    const uint32_t d = P.inc_off[v + 1] - s;
-    if (d == 0 || !P.dirty[v]) return;  // as in the block form
+// What of a warp contig does not change while the sweeps run, a lane per edge.
+struct WarpNode {
+    uint32_t v, d, o;  // contig, edges, the lane's other contig
+    double w;          // the lane's log(1 - score)
+};
+
+__device__ __forceinline__ WarpNode lp_load(const LpArgs& P, const uint32_t* __restrict__ list, uint32_t i,
+                                            uint32_t count) {
+    WarpNode N{0, 0, 0, 0.0};
+    if (i >= count) return N;
+    const uint32_t lane = threadIdx.x & 31;
+    N.v = list[i];
+    const uint32_t s = P.inc_off[N.v];
+    N.d = P.inc_off[N.v + 1] - s;
+    if (lane < N.d) {
+        N.o = P.oth[s + lane];
+        N.w = P.ilw[s + lane];
+    }
+    return N;
+}
+
+__device__ void lp_node_warp(const LpArgs& P, const WarpNode& N, WarpWs& W, Tally& T) {
+    const uint32_t lane = threadIdx.x & 31, v = N.v, d = N.d, o = N.o;
+    if (d == 0) return;
+    // all that changes between sweeps, loaded side by side: only this warp
+    // writes its contig's label and frozen flag
+    const uint32_t other = lane < d ? __ldcg(P.mem + o) : 0u;
+    const uint32_t mine = __ldcg(P.mem + v);
+    const uint8_t frozen = __ldcg(P.stuck + v);
+    if (!__ldcg(P.dirty + v)) return;  // as in the block form
+    __syncwarp();
     unsigned long long key = ~0ull;
-    uint32_t o = 0;
     if (lane < d) {
-        o = P.oth[s + lane];
-        key = ((unsigned long long)P.mem[o] << 32) | lane;
-        W.w[lane] = P.ilw[s + lane];
+        key = ((unsigned long long)other << 32) | lane;
+        W.w[lane] = N.w;
     }
     W.fidx[lane] = -1;
-    // bitonic sort over the lanes, ascending
-#pragma unroll
-    for (uint32_t k = 2; k <= 32; k <<= 1) {
-#pragma unroll
+    // bitonic sort over the lanes, ascending, as far as the edges reach (the
+    // lanes past them hold the largest key)
+    for (uint32_t k = 2; k < 2 * d; k <<= 1) {
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
             const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, j);
             const bool lower = (lane & j) == 0, up = (lane & k) == 0;
@@ -304,7 +377,13 @@ __global__ void __launch_bounds__(kThreads) k_lp_level_warp(LpArgs P, const uint
     const uint32_t lab = (uint32_t)(key >> 32);
     const uint32_t prev = __shfl_up_sync(0xffffffffu, lab, 1);
     double val = -1.0;
-    if (lane < d && (lane == 0 || prev != lab)) {
+    const bool head = lane < d && (lane == 0 || prev != lab);
+    // with one label among the neighbours its CDF decides nothing
+    const bool one = __popc(__ballot_sync(0xffffffffu, head)) == 1;
+    if (head && one) {
+        val = 0.0;
+        W.fidx[(uint32_t)key] = (int32_t)lane;
+    } else if (head) {
         double sum = 0.0;
         uint32_t q = lane;
         do {
@@ -339,11 +418,11 @@ __global__ void __launch_bounds__(kThreads) k_lp_level_warp(LpArgs P, const uint
             while (q >= 0 && W.val[W.fidx[q]] != top) q = W.nxt[q];
             best = W.ins[q >= 0 ? q : 0];
         }
-        if (P.mem[v] != best && !P.stuck[v]) {
+        if (mine != best && !frozen) {
             P.mem[v] = best;
             changed = 1;
-            if (visit(P, v, best))
-                atomicAdd(P.counters, 1ull);
+            if (visit(P, v, best, T))
+                atomicAdd(&T.moved, 1u);
             else
                 P.stuck[v] = 1;
         }
@@ -365,67 +444,190 @@ struct LevelInfo {
     unsigned int count, maxdeg, nbig, nsmall, maxall, off, soff, pad;
 };
 
+// Contig w joins the next level.  The lanes that enqueue together share one
+// atomic per counter.
 __device__ __forceinline__ void lp_enqueue(uint32_t w, uint32_t deg, uint32_t* next, uint32_t* next_small,
                                            LevelInfo* info, uint32_t* slot_of) {
-    atomicMax(&info->maxall, deg);
+    const uint32_t lane = threadIdx.x & 31, all = __activemask();
+    const uint32_t most = __reduce_max_sync(all, deg);
+    const uint32_t small = __ballot_sync(all, deg <= kWarpCap), big = all & ~small;
+    if (lane == __ffs(all) - 1) atomicMax(&info->maxall, most);
     if (deg <= kWarpCap) {
-        next_small[atomicAdd(&info->nsmall, 1u)] = w;
+        uint32_t at = 0;
+        if (lane == __ffs(small) - 1) at = atomicAdd(&info->nsmall, (unsigned)__popc(small));
+        at = __shfl_sync(small, at, __ffs(small) - 1);
+        next_small[at + __popc(small & ((1u << lane) - 1u))] = w;
         return;
     }
-    next[atomicAdd(&info->count, 1u)] = w;
-    atomicMax(&info->maxdeg, deg);
+    uint32_t at = 0;
+    if (lane == __ffs(big) - 1) {
+        at = atomicAdd(&info->count, (unsigned)__popc(big));
+        atomicMax(&info->maxdeg, most);
+    }
+    at = __shfl_sync(big, at, __ffs(big) - 1);
+    next[at + __popc(big & ((1u << lane) - 1u))] = w;
     if (pow2_at_least(deg) > kSmallCap) slot_of[w] = atomicAdd(&info->nbig, 1u);
 }
 
-// earlier neighbours of each contig of the order (warp per contig); those
-// with none form level 0
-__global__ void __launch_bounds__(256) k_lp_pred(const uint32_t* __restrict__ order, uint32_t norder,
-                                                 const uint32_t* __restrict__ pos_of,
-                                                 const uint32_t* __restrict__ inc_off,
-                                                 const uint32_t* __restrict__ oth, uint32_t* __restrict__ pred,
-                                                 uint32_t* __restrict__ level0, uint32_t* __restrict__ level0_small,
-                                                 LevelInfo* info, uint32_t* __restrict__ slot_of) {
-    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (wid >= norder) return;
-    const uint32_t u = order[wid], pu = wid;
-    const uint32_t s = inc_off[u], d = inc_off[u + 1] - s;
-    uint32_t c = 0;
-    for (uint32_t j = lane; j < d; j += 32) c += pos_of[oth[s + j]] < pu;
+struct LevelArgs {
+    const uint32_t* order;
+    uint32_t norder;
+    const uint32_t* pos_of;
+    const uint32_t* inc_off;
+    const uint32_t* oth;
+    const uint32_t* deg;
+    uint32_t* pred;
+    uint32_t *lvl, *lvls;  // block and warp contigs, level after level
+    LevelInfo* info;
+    uint32_t lcap;         // entries of info
+    uint32_t* slot_of;
+    LevelInfo* sum;        // over all levels: count = contigs levelled, nsmall = levels, the maxima
+    unsigned int* bar;
+    int* flag;
+};
+
+// The dependency levels of the order, one cooperative launch: the earlier
+// neighbours of each contig are counted (those with none form level 0), then
+// Kahn steps until a level is empty, a grid barrier after each -- eight lanes
+// per contig, and a contig whose last earlier neighbour is in level L joins
+// level L + 1.  (60,000 contigs, 10 runs: 176 launches of 6.1 us, queued
+// sixteen at a time past the last level, became 10 of these.)
+__global__ void __launch_bounds__(kCoopThreads) k_lp_levels(LevelArgs A) {
+    // groups of eight lanes: most contigs have few edges, and the chain of
+    // dependent loads wants as many contigs in flight as there are lanes for
+    const uint32_t sub = threadIdx.x & 7, ng = gridDim.x * (blockDim.x >> 3);
+    const uint32_t g0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const uint32_t gmask = 0xFFu << (threadIdx.x & 24);
+    unsigned int target = 0;
+    for (uint32_t pu = g0; pu < A.norder; pu += ng) {
+        const uint32_t u = A.order[pu];
+        const uint32_t s = A.inc_off[u], d = A.inc_off[u + 1] - s;
+        uint32_t c = 0;
+        for (uint32_t j = sub; j < d; j += 8) c += A.pos_of[A.oth[s + j]] < pu;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if (lane == 0) {
-        pred[u] = c;
-        if (c == 0) lp_enqueue(u, d, level0, level0_small, info, slot_of);
+        for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(gmask, c, o);
+        if (sub == 0) {
+            A.pred[u] = c;
+            if (c == 0) lp_enqueue(u, d, A.lvl, A.lvls, A.info, A.slot_of);
+        }
+    }
+    uint32_t off = 0, soff = 0, done = 0, L = 0, maxdeg = 0, maxall = 0, maxbig = 0;
+    for (;; ++L) {
+        if (!grid_barrier(A.bar, target, A.flag)) return;
+        if (L + 1 >= A.lcap) break;
+        const uint32_t count = __ldcg(&A.info[L].count), nsmall = __ldcg(&A.info[L].nsmall);
+        if (count + nsmall == 0) break;
+        maxdeg = max(maxdeg, __ldcg(&A.info[L].maxdeg));
+        maxall = max(maxall, __ldcg(&A.info[L].maxall));
+        maxbig = max(maxbig, __ldcg(&A.info[L].nbig));
+        done += count + nsmall;
+        const uint32_t noff = off + count, nsoff = soff + nsmall;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            A.info[L].off = off;
+            A.info[L].soff = soff;
+        }
+        for (uint32_t wid = g0; wid < count + nsmall; wid += ng) {
+            const uint32_t u = wid < count ? __ldcg(A.lvl + off + wid) : __ldcg(A.lvls + soff + wid - count);
+            const uint32_t pu = A.pos_of[u];
+            const uint32_t s = A.inc_off[u], d = A.inc_off[u + 1] - s;
+            for (uint32_t j = sub; j < d; j += 8) {
+                const uint32_t o = A.oth[s + j], dego = A.deg[o];
+                if (A.pos_of[o] > pu && atomicSub(A.pred + o, 1u) == 1u)
+                    lp_enqueue(o, dego, A.lvl + noff, A.lvls + nsoff, A.info + L + 1, A.slot_of);
+            }
+        }
+        off = noff;
+        soff = nsoff;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        LevelInfo r{};
+        r.count = done;
+        r.nsmall = L;
+        r.maxdeg = maxdeg;
+        r.maxall = maxall;
+        r.nbig = maxbig;
+        *A.sum = r;
     }
 }
 
-// One Kahn step for level L (its size and place read from info[L], so steps
-// can be queued without the host): contigs whose last earlier neighbour is
-// in this level join level L + 1.  A warp per contig, grid-stride.
-__global__ void __launch_bounds__(256) k_lp_kahn(uint32_t L, const uint32_t* __restrict__ pos_of,
-                                                 const uint32_t* __restrict__ inc_off,
-                                                 const uint32_t* __restrict__ oth, uint32_t* __restrict__ pred,
-                                                 uint32_t* __restrict__ lvl, uint32_t* __restrict__ lvls,
-                                                 LevelInfo* info, uint32_t* __restrict__ slot_of) {
-    const LevelInfo cur = info[L];
-    const uint32_t total = cur.count + cur.nsmall;
-    const uint32_t noff = cur.off + cur.count, nsoff = cur.soff + cur.nsmall;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        info[L + 1].off = noff;
-        info[L + 1].soff = nsoff;
-    }
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t nw = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; wid < total; wid += nw) {
-        const uint32_t u = wid < cur.count ? lvl[cur.off + wid] : lvls[cur.soff + wid - cur.count];
-        const uint32_t pu = pos_of[u];
-        const uint32_t s = inc_off[u], d = inc_off[u + 1] - s;
-        for (uint32_t j = lane; j < d; j += 32) {
-            const uint32_t o = oth[s + j];
-            if (pos_of[o] > pu && atomicSub(pred + o, 1u) == 1u)
-                lp_enqueue(o, inc_off[o + 1] - inc_off[o], lvl + noff, lvls + nsoff, info + L + 1, slot_of);
+// One propagation call's sweeps in one cooperative launch: per sweep, level
+// after level with a grid barrier in between; a level's contigs are never
+// neighbours of one another (a contig's level exceeds its earlier
+// neighbours'), so its block contigs and warp contigs run side by side.  All
+// blocks read the sweep's count of moved contigs after its last barrier and
+// take the same decision to go on.  out[0]: sweeps run.
+//
+// What bounds it is the chain of one contig's evaluation (gathers at half a
+// microsecond a hop, the sort, the CDF's serial series, the visited table's
+// atomic) once per level, which is why all that is fixed is loaded before
+// the barrier and the rest side by side.
+__global__ void __launch_bounds__(kCoopThreads) k_lp_sweeps(LpArgs P, const uint32_t* __restrict__ lvl,
+                                                        const uint32_t* __restrict__ lvls,
+                                                        const LevelInfo* __restrict__ info, uint32_t nlevels,
+                                                        uint32_t group_bytes, unsigned int* bar, int* flag,
+                                                        unsigned long long* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ WarpWs ws_all[kWarpsPerBlock];
+    __shared__ BlockWs bws[kGroups];
+    __shared__ unsigned long long s_cnt[2];
+    const uint32_t grp = threadIdx.x / kThreads;
+    __shared__ Tally T;
+    WarpWs& W = ws_all[threadIdx.x >> 5];
+    if (threadIdx.x == 0) T.moved = T.entries = 0;
+    // warps count from the last block, which has block contigs last
+    const uint32_t nw = gridDim.x * kWarpsPerBlock;
+    const uint32_t w0 = (gridDim.x - 1 - blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
+    unsigned int target = 0;
+    unsigned long long before = 0, low = INT_MAX, attempt = 0, sweeps = 0;
+    __syncthreads();
+    WarpNode next = lp_load(P, lvls + info[0].soff, w0, info[0].nsmall);
+    while (true) {
+        for (uint32_t L = 0; L < nlevels; ++L) {
+            const uint32_t off = info[L].off, soff = info[L].soff, count = info[L].count, nsmall = info[L].nsmall;
+            for (uint32_t i = grp * gridDim.x + blockIdx.x; i < count; i += kGroups * gridDim.x)
+                lp_node_block(P, lvl[off + i], smem + grp * group_bytes, bws[grp], T);
+            for (uint32_t i = w0; i < nsmall; i += nw) {
+                const WarpNode cur = next;
+                next = lp_load(P, lvls + soff, i + nw, nsmall);
+                lp_node_warp(P, cur, W, T);
+            }
+            // the next level's first contig, in flight across the barrier
+            const uint32_t Ln = L + 1 < nlevels ? L + 1 : 0;
+            next = lp_load(P, lvls + info[Ln].soff, w0, info[Ln].nsmall);
+            if (L + 1 == nlevels) {
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    if (T.moved) atomicAdd(P.counters, (unsigned long long)T.moved);
+                    if (T.entries) atomicAdd(P.counters + 1, (unsigned long long)T.entries);
+                    T.moved = T.entries = 0;
+                }
+            }
+            if (!grid_barrier(bar, target, flag)) return;
         }
+        ++sweeps;
+        if (threadIdx.x == 0) {
+            s_cnt[0] = __ldcg(P.counters);
+            // a table filled beyond three quarters ends the call (a sweep adds at
+            // most an eighth)
+            s_cnt[1] = __ldcg(P.counters + 2) |
+                       (__ldcg(P.counters + 1) * 4 > (P.vt_mask + 1) * 3 ? kErrTable : 0ull);
+        }
+        __syncthreads();
+        const unsigned long long moved = s_cnt[0] - before, err = s_cnt[1];
+        before = s_cnt[0];
+        // every block has read the counters before any goes on to change them
+        if (!grid_barrier(bar, target, flag)) return;
+        if (err && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(P.counters + 2, err);
+        if (err) break;
+        if (moved < low) {
+            low = moved;
+            attempt = 0;
+        } else if (++attempt >= 10) {
+            break;
+        }
+        if (moved == 0) break;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = sweeps;
 }
 
 // ---- the traversal ----------------------------------------------------------
@@ -631,39 +833,14 @@ struct LpState {
     uint64_t recip_n = 0;
 };
 
-// A CUDA graph recorded from a body of stream work (owned; freed on scope exit).
-struct SweepGraph {
-    cudaGraphExec_t exec = nullptr;
-    uint64_t launches = 0;  // kernels in the graph
-    SweepGraph() = default;
-    SweepGraph(const SweepGraph&) = delete;
-    SweepGraph& operator=(const SweepGraph&) = delete;
-    ~SweepGraph() {
-        if (exec) cudaGraphExecDestroy(exec);
-    }
-    template <class Body>
-    int record(mdet_ctx* ctx, Body body) {
-        if (!ctx->cap_stream)
-            MDET_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
-        if (!ctx->cap_stream2)
-            MDET_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream2, cudaStreamNonBlocking));
-        if (!ctx->cap_fork) MDET_CUDA(ctx, cudaEventCreateWithFlags(&ctx->cap_fork, cudaEventDisableTiming));
-        if (!ctx->cap_join) MDET_CUDA(ctx, cudaEventCreateWithFlags(&ctx->cap_join, cudaEventDisableTiming));
-        const cudaStream_t cs = ctx->cap_stream;
-        MDET_CUDA(ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-        const uint64_t l0 = ctx->launches;
-        body(cs);
-        launches = ctx->launches - l0;
-        ctx->launches = l0;  // counted per replay
-        const cudaError_t le = cudaGetLastError();  // a launch that failed to enqueue
-        cudaGraph_t graph = nullptr;
-        const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
-        int rc = ctx_cuda(ctx, le != cudaSuccess ? le : ce, "sweep capture");
-        if (rc == MDET_OK) rc = ctx_cuda(ctx, cudaGraphInstantiate(&exec, graph, 0), "sweep graph instantiate");
-        if (graph) cudaGraphDestroy(graph);
-        return rc;
-    }
-};
+// Cooperative launch of one block per SM.
+template <class K>
+int launch_grid(mdet_ctx* ctx, K kernel, size_t smem, const char* what, void** args) {
+    MDET_CUDA(ctx, cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)ctx->num_sms), dim3(kCoopThreads),
+                                               args, smem, ctx->stream));
+    MDET_LAUNCHED(ctx, what);
+    return MDET_OK;
+}
 
 // One propagation call over the traversal graph (m2 edges) and order.
 int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
@@ -692,10 +869,12 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
     MDET_LAUNCHED(ctx, "k_lp_inc_keys");
     {
         size_t tb = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, ikey, ikey2, ival, inc, (int)(2 * m), 0, 32, s);
+        int bits = 1;  // keys are contigs, below n
+        while (bits < 32 && (n - 1) >> bits) ++bits;
+        cub::DeviceRadixSort::SortPairs(nullptr, tb, ikey, ikey2, ival, inc, (int)(2 * m), 0, bits, s);
         void* tmp = ctx_scratch(ctx, "lp.sorttmp", tb);
         if (!tmp) return MDET_ERR_NOMEM;
-        MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, ikey, ikey2, ival, inc, (int)(2 * m), 0, 32, s));
+        MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, ikey, ikey2, ival, inc, (int)(2 * m), 0, bits, s));
         tb = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, tb, deg, inc_off, (int)(n + 1), s);
         tmp = ctx_scratch(ctx, "lp.scantmp", tb);
@@ -709,50 +888,30 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
     MDET_CUDA(ctx, cudaMemsetAsync(pos_of, 0xFF, n * 4, s));
     k_lp_pos<<<grid_for(no), 256, 0, s>>>(S.order, (uint32_t)no, pos_of);
     MDET_LAUNCHED(ctx, "k_lp_pos");
-    // levels: Kahn steps queued sixteen at a time, their table read back once
-    // per batch
-    const uint64_t lcap = no + 18;
-    LevelInfo* info = (LevelInfo*)ctx_scratch(ctx, "lp.info", lcap * sizeof(LevelInfo));
+    const uint64_t lcap = no + 2;
+    LevelInfo* info = (LevelInfo*)ctx_scratch(ctx, "lp.info", (lcap + 2) * sizeof(LevelInfo));
     if (!info) return MDET_ERR_NOMEM;
-    MDET_CUDA(ctx, cudaMemsetAsync(info, 0, lcap * sizeof(LevelInfo), s));
-    k_lp_pred<<<grid_for(no * 32), 256, 0, s>>>(S.order, (uint32_t)no, pos_of, inc_off, oth, pred, lvl, lvls, info,
-                                                 slot_of);
-    MDET_LAUNCHED(ctx, "k_lp_pred");
-    std::vector<uint64_t> loff{0}, soff{0};
-    std::vector<LevelInfo> linfo;
-    uint64_t done = 0;
-    uint32_t maxdeg = 0, maxall = 0, maxbig = 0;
-    const unsigned kgrid = (unsigned)ctx->num_sms * 8;
-    std::vector<LevelInfo> batch(17);
-    for (uint32_t L0 = 0; done < no && L0 + 17 <= lcap;) {
-        for (uint32_t L = L0; L < L0 + 16; ++L) {
-            k_lp_kahn<<<kgrid, 256, 0, s>>>(L, pos_of, inc_off, oth, pred, lvl, lvls, info, slot_of);
-            MDET_LAUNCHED(ctx, "k_lp_kahn");
-        }
-        MDET_CUDA(ctx, cudaMemcpyAsync(batch.data(), info + L0, 17 * sizeof(LevelInfo), cudaMemcpyDeviceToHost, s));
-        MDET_CUDA(ctx, cudaStreamSynchronize(s));
-        bool ended = false;
-        for (int k = 0; k < 16; ++k) {
-            const LevelInfo& h = batch[k];
-            if (h.count + h.nsmall == 0) {
-                ended = true;
-                break;
-            }
-            linfo.push_back(h);
-            maxdeg = std::max(maxdeg, h.maxdeg);
-            maxall = std::max(maxall, h.maxall);
-            maxbig = std::max(maxbig, h.nbig);
-            loff.push_back(h.off + h.count);
-            soff.push_back(h.soff + h.nsmall);
-            done += h.count + h.nsmall;
-        }
-        if (ended || done >= no) break;
-        L0 += 16;
+    MDET_CUDA(ctx, cudaMemsetAsync(info, 0, (lcap + 2) * sizeof(LevelInfo), s));
+    unsigned int* bar = (unsigned int*)(info + lcap + 1);  // barrier counters: levels, sweeps
+    LevelInfo* dsum = info + lcap;
+    {
+        LevelArgs A{S.order, (uint32_t)no, pos_of, inc_off, oth, deg, pred, lvl, lvls, info, (uint32_t)lcap, slot_of, dsum,
+                    bar, ctx->d_flag};
+        void* args[] = {&A};
+        MDET_TRY(launch_grid(ctx, k_lp_levels, 0, "k_lp_levels", args));
     }
+    LevelInfo* hsum = (LevelInfo*)ctx_pinned(ctx, 128);
+    if (!hsum) return MDET_ERR_NOMEM;
+    MDET_CUDA(ctx, cudaMemcpyAsync(hsum, dsum, sizeof(LevelInfo), cudaMemcpyDeviceToHost, s));
+    MDET_CUDA(ctx, cudaStreamSynchronize(s));
+    const uint64_t done = hsum->count;
+    const uint32_t nlevels = hsum->nsmall, maxall = hsum->maxall, maxbig = hsum->nbig;
+    uint32_t maxdeg = hsum->maxdeg;
     ctx_timer_end(ctx, "lp_levels");
+    MDET_TRY(done == no ? MDET_OK : check_flag(ctx));  // a barrier that ran out says so
     if (done != no) return ctx_fail(ctx, MDET_ERR_INTERNAL, "label propagation: %llu of %llu contigs levelled",
                                     (unsigned long long)done, (unsigned long long)no);
-    st->levels_max = std::max<uint64_t>(st->levels_max, linfo.size());
+    st->levels_max = std::max<uint64_t>(st->levels_max, nlevels);
     st->degree_max = std::max<uint64_t>(st->degree_max, maxall);
     maxdeg = std::max(maxdeg, kWarpCap);
     // the CDF's log-factorials up to the largest label count
@@ -781,8 +940,11 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
         big_ws = (unsigned char*)ctx_scratch(ctx, "lp.bigws", big_stride * maxbig);
         if (!big_ws) return MDET_ERR_NOMEM;
     }
-    const size_t small_max = ws_bytes(kSmallCap);
-    MDET_CUDA(ctx, cudaFuncSetAttribute(k_lp_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_max));
+    // a group's work area in shared memory
+    const size_t dyn =
+        maxdeg > kWarpCap ? (ws_bytes(std::min<uint32_t>(pow2_at_least(maxdeg), kSmallCap)) + 15) / 16 * 16 : 0;
+    MDET_CUDA(ctx, cudaFuncSetAttribute(k_lp_sweeps, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)(kGroups * dyn)));
     // visited table: sized for the order, doubled (and the call re-run from
     // its starting labels) when a call overfills it
     uint64_t vt_cap = 1u << 20;
@@ -805,67 +967,32 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
         MDET_CUDA(ctx, cudaMemsetAsync(S.cnt, 0, 4 * 8, s));
         LpArgs P{inc_off,  oth,   ilw,       S.mem,   S.stuck,    S.dirty,          vt,
                  vt_cap - 1, logfact, S.recip, (uint32_t)S.recip_n, S.cnt, big_ws, big_stride, maxbig, slot_of};
-        uint64_t low = INT_MAX, attempt = 0, sweeps = 0;
-        unsigned long long* hc = (unsigned long long*)ctx_pinned(ctx, 32);
+        unsigned long long* hc = (unsigned long long*)ctx_pinned(ctx, 128);
         if (!hc) return MDET_ERR_NOMEM;
-        bool overfull = false;
-        // one sweep -- the moved counter cleared, a launch or two per level,
-        // the counters copied back -- recorded once as a CUDA graph on the
-        // context's capture stream and replayed on its stream for every sweep.
-        // A level's contigs are never neighbours of one another (a contig's
-        // level exceeds its earlier neighbours'), so its warp-per-contig and
-        // block-per-contig launches are independent branches of the graph,
-        // joined before the next level.
-        SweepGraph sg;
-        MDET_TRY(sg.record(ctx, [&](cudaStream_t cs) {
-            const cudaStream_t cs2 = ctx->cap_stream2;
-            cudaMemsetAsync(S.cnt, 0, 8, cs);
-            for (size_t L = 0; L < linfo.size(); ++L) {
-                const bool both = linfo[L].nsmall && linfo[L].count;
-                if (both) {
-                    cudaEventRecord(ctx->cap_fork, cs);
-                    cudaStreamWaitEvent(cs2, ctx->cap_fork, 0);
-                }
-                if (linfo[L].nsmall) {
-                    k_lp_level_warp<<<(linfo[L].nsmall + kWarpsPerBlock - 1) / kWarpsPerBlock, kThreads, 0, cs>>>(
-                        P, lvls + soff[L], linfo[L].nsmall);
-                    ctx->launches++;
-                }
-                if (linfo[L].count) {
-                    const uint32_t cap = std::min<uint32_t>(pow2_at_least(linfo[L].maxdeg), kSmallCap);
-                    k_lp_level<<<linfo[L].count, kThreads, ws_bytes(cap), both ? cs2 : cs>>>(P, lvl + loff[L]);
-                    ctx->launches++;
-                }
-                if (both) {
-                    cudaEventRecord(ctx->cap_join, cs2);
-                    cudaStreamWaitEvent(cs, ctx->cap_join, 0);
-                }
-            }
-            cudaMemcpyAsync(hc, S.cnt, 32, cudaMemcpyDeviceToHost, cs);
-        }));
-        while (true) {
-            ctx_timer_begin(ctx, "lp_sweep");
-            MDET_CUDA(ctx, cudaGraphLaunch(sg.exec, s));
-            ctx->launches += sg.launches;
-            ctx->total_launches += sg.launches;
-            ctx_timer_end(ctx, "lp_sweep");
-            MDET_CUDA(ctx, cudaStreamSynchronize(s));
-            ++sweeps;
-            if (hc[2] & (kErrSlots | kErrScore))
-                return ctx_fail(ctx, MDET_ERR_INTERNAL, "label propagation: flags %llu", hc[2]);
-            if (hc[2] & kErrTable) {
-                overfull = true;
-                break;
-            }
-            const uint64_t moved = hc[0];
-            if (moved < low) {
-                low = moved;
-                attempt = 0;
-            } else if (++attempt >= 10) {
-                break;
-            }
-            if (moved == 0) break;
+        ctx_timer_begin(ctx, "lp_sweep");
+        unsigned int* sbar = bar + 1 + attempt_table;
+        unsigned long long* dsweeps = S.cnt + 4;
+        MDET_CUDA(ctx, cudaMemsetAsync(dsweeps, 0, 8, s));
+        {
+            const uint32_t *a_lvl = lvl, *a_lvls = lvls;
+            const LevelInfo* a_info = info;
+            uint32_t a_n = nlevels;
+            int* a_flag = ctx->d_flag;
+            uint32_t a_bytes = (uint32_t)dyn;
+            void* args[] = {&P, &a_lvl, &a_lvls, &a_info, &a_n, &a_bytes, &sbar, &a_flag, &dsweeps};
+            MDET_TRY(launch_grid(ctx, k_lp_sweeps, kGroups * dyn, "k_lp_sweeps", args));
         }
+        ctx_timer_end(ctx, "lp_sweep");
+        MDET_CUDA(ctx, cudaMemcpyAsync(hc, S.cnt, 40, cudaMemcpyDeviceToHost, s));
+        MDET_CUDA(ctx, cudaStreamSynchronize(s));
+        const uint64_t sweeps = hc[4];
+        if (sweeps == 0) {  // a barrier's wait ran out
+            MDET_TRY(check_flag(ctx));
+            return ctx_fail(ctx, MDET_ERR_INTERNAL, "label propagation: no sweep");
+        }
+        if (hc[2] & (kErrSlots | kErrScore))
+            return ctx_fail(ctx, MDET_ERR_INTERNAL, "label propagation: flags %llu", hc[2]);
+        const bool overfull = (hc[2] & kErrTable) != 0;
         if (!overfull) {
             st->sweeps += sweeps;
             st->ties += hc[3];
@@ -912,7 +1039,13 @@ int lp_impl(mdet_ctx* ctx, const uint64_t* d_from, const uint64_t* d_to, const d
     S.ea = (uint32_t*)ctx_scratch(ctx, "lp.ea", ne1 * 4);
     S.eb = (uint32_t*)ctx_scratch(ctx, "lp.eb", ne1 * 4);
     S.lw = (double*)ctx_scratch(ctx, "lp.lw", ne1 * 8);
-    const uint64_t kChunk = std::min<uint64_t>(ne1, 1ull << 22);  // edges traversed per pass
+    // edges traversed per pass: a stretch starts with about as many as n
+    // contigs need and takes four times as many each time it goes on (the first
+    // stretches end within the first edges; passes of 4M edges from the start
+    // took 1.0 of 6.5 ms at 60,000 contigs and 2.9M edges)
+    const uint64_t kChunk = std::min<uint64_t>(ne1, 1ull << 22);
+    uint64_t chunk0 = 1ull << 16;
+    while (chunk0 < n / 4 && chunk0 < kChunk) chunk0 <<= 1;
     uint8_t* slot = (uint8_t*)ctx_scratch(ctx, "lp.slot", 2 * kChunk);
     uint32_t* ssel = (uint32_t*)ctx_scratch(ctx, "lp.ssel", 2 * kChunk * 4);
     uint32_t* sel = (uint32_t*)ctx_scratch(ctx, "lp.sel", kChunk * 4);
@@ -975,8 +1108,9 @@ int lp_impl(mdet_ctx* ctx, const uint64_t* d_from, const uint64_t* d_to, const d
         uint64_t i_run = kNone;
         bool at_last = false, ended = false;
         // the stretch from pos, a chunk at a time, until the run position
-        for (uint64_t p0 = pos;;) {
-            const uint64_t p1 = std::min(ne, p0 + kChunk);
+        uint64_t chunk = chunk0;
+        for (uint64_t p0 = pos;; chunk = std::min(4 * chunk, kChunk)) {
+            const uint64_t p1 = std::min(ne, p0 + std::min(chunk, kChunk));
             unsigned long long h2[2] = {kNone, kNone};
             MDET_CUDA(ctx, cudaMemcpyAsync(S.cnt, h2, 16, cudaMemcpyHostToDevice, s));
             k_lp_seg<<<std::min<unsigned>(grid_for(p1 - p0), 8 * ctx->num_sms), 256, 0, s>>>(S.sa, S.sb, S.ss, p0,

@@ -30,8 +30,12 @@
 
 #if defined(__CUDACC__)
 #define LP_HD __host__ __device__ __forceinline__
+// The series' coefficients are constants only once their loops are unrolled;
+// left rolled, every step divides in FP64.
+#define LP_UNROLL _Pragma("unroll")
 #else
 #define LP_HD inline
+#define LP_UNROLL
 #endif
 
 namespace lpm {
@@ -222,6 +226,7 @@ LP_HD F2 log(double x) {
     const F2 s2 = mul(s, s);
     // atanh series: s (1 + s^2/3 + s^4/5 + ... + s^22/23), |s| <= 0.172
     F2 q = from_double(1.0 / 23.0);
+    LP_UNROLL
     for (int k = 10; k >= 1; --k) q = add(mul(q, s2), from_double(1.0 / (2 * k + 1)));
     q = add(mul(q, s2), make(1.0f, 0.0f));
     const F2 t = mul(s, q);
@@ -238,6 +243,7 @@ LP_HD F2 exp(F2 x) {
     // Taylor series to degree 14 (truncation < 1e-17 for |r| <= 0.35)
     F2 p = from_double(1.0 / 87178291200.0);  // 1/14!
     double f = 87178291200.0;
+    LP_UNROLL
     for (int n = 13; n >= 1; --n) {
         f = f / (n + 1);
         p = add(mul(p, r), from_double(1.0 / f));
@@ -275,25 +281,28 @@ LP_HD double chi2_cdf(double dof, double x, const F2* logfact, const F2* recip =
     if (yd == INFINITY) return 1.0;
     const F2 y = from_double(yd);
     const F2 ly = lpf::log(yd);
-    if (yd < (double)c) {
-        const F2 lp = add(add(mul_f(ly, (float)c), neg(y)), neg(logfact[c]));
-        F2 t = make(1.0f, 0.0f), v = make(1.0f, 0.0f);
+    // both forms start from pois(cc; y) -- written once, so that lanes of a
+    // warp on different sides share its logarithm and exponential
+    const bool low = yd < (double)c;
+    const uint32_t cc = low ? c : c - 1;
+    const F2 lp = add(add(mul_f(ly, (float)cc), neg(y)), neg(logfact[cc]));
+    F2 t = make(1.0f, 0.0f), v = make(1.0f, 0.0f);
+    if (low) {
         for (uint32_t k = 1; k < 1000000u; ++k) {
             t = mul(mul(t, y), inv(c + k, recip, nrecip));
             v = add(v, t);
             if (t.hi < v.hi * 1e-17f) break;
         }
-        return to_double(mul(lpf::exp(lp), v));
+    } else {
+        const F2 iy = lpf::recip(y);
+        for (uint32_t i = c - 1; i >= 1; --i) {
+            t = mul(mul_f(t, (float)i), iy);
+            v = add(v, t);
+            if (t.hi < v.hi * 1e-17f) break;
+        }
     }
-    const F2 lq = add(add(mul_f(ly, (float)(c - 1)), neg(y)), neg(logfact[c - 1]));
-    const F2 iy = lpf::recip(y);
-    F2 u = make(1.0f, 0.0f), w = make(1.0f, 0.0f);
-    for (uint32_t i = c - 1; i >= 1; --i) {
-        u = mul(mul_f(u, (float)i), iy);
-        w = add(w, u);
-        if (u.hi < w.hi * 1e-17f) break;
-    }
-    return to_double(add(make(1.0f, 0.0f), neg(mul(lpf::exp(lq), w))));
+    const F2 p = mul(lpf::exp(lp), v);
+    return to_double(low ? p : add(make(1.0f, 0.0f), neg(p)));
 }
 
 }  // namespace lpf
