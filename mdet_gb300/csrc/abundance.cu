@@ -28,32 +28,43 @@
 
 namespace {
 
-// erfc in float-float from this project's own table (erfc_table.cuh,
-// generated by gen_erfc_table.py): degree-13 interpolants on 26 pieces of
-// [0, 6.5], absolute error ~5e-16 before the float-float evaluation; 0
-// beyond 6.5 (erfc < 4e-20 there); erfc(-z) = 2 - erfc(z).  The FP32 pipes
-// run this far faster than the FP64 pipe runs the double erfc.  Kept out of
-// line: the score kernel calls it from eight places, and eight inlined
-// copies stall the kernel on instruction fetch.
-__device__ __noinline__ ff erfc_ff(ff z) {
-    const bool neg = z.hi < 0.f;
-    if (neg) z = ff_neg(z);
-    ff r;
-    if (!(z.hi < 6.5f)) {
-        r = ff_make(0.f, 0.f);  // NaN arguments land here too
-        if (z.hi != z.hi) return z;
-    } else {
-        const int p = min((int)(z.hi * 4.f), MDET_ERFC_PIECES - 1);
-        // u = (z - centre) * 8, exact scaling of an exact difference
-        ff u = ff_add_f(z, -((float)p + 0.5f) * 0.25f);
-        u.hi *= 8.f;
-        u.lo *= 8.f;
-        const float(*c)[2] = kErfcTable[p];
-        r = ff_make(__ldg(&c[MDET_ERFC_DEG][0]), __ldg(&c[MDET_ERFC_DEG][1]));
+// erfc(z), z >= 0, in float-float from this project's own table
+// (erfc_table.cuh, generated by gen_erfc_table.py): degree-13 interpolants on
+// 26 pieces of [0, 6.5], absolute error ~5e-16 before the float-float
+// evaluation; 0 beyond 6.5 (erfc < 4e-20 there).  The FP32 pipes run this far
+// faster than the FP64 pipe runs the double erfc.  The terms from degree 8 up
+// run in FP32: they sum to less than 7e-10, so rounding them costs 4e-17, a
+// tenth of the table's own error; degrees 7 to 2 (below 8e-3) take the shorter
+// float-float sum, whose error is 2^-47 of its operands.  Kept out of line:
+// the score kernel calls it from several places, and inlined copies stall the
+// kernel on instruction fetch.
+__device__ __noinline__ ff erfc_pos(ff z) {
+    if (!(z.hi < 6.5f)) return z.hi != z.hi ? z : ff_make(0.f, 0.f);  // NaN stays
+    const int p = min((int)(z.hi * 4.f), MDET_ERFC_PIECES - 1);
+    // u = (z - centre) * 8, exact scaling of an exact difference
+    ff u = ff_add_f(z, -((float)p + 0.5f) * 0.25f);
+    u.hi *= 8.f;
+    u.lo *= 8.f;
+    const float(*c)[2] = kErfcTable[p];
+    float h = __ldg(&c[MDET_ERFC_DEG][0]);
 #pragma unroll
-        for (int j = MDET_ERFC_DEG - 1; j >= 0; --j)
-            r = ff_add(ff_mul(r, u), ff_make(__ldg(&c[j][0]), __ldg(&c[j][1])));
+    for (int j = MDET_ERFC_DEG - 1; j >= 8; --j) h = __fmaf_rn(h, u.hi, __ldg(&c[j][0]));
+    ff r = ff_make(h, 0.f);
+#pragma unroll
+    for (int j = 7; j >= 2; --j) {
+        const ff m = ff_mul(r, u);
+        const ff t = two_sum(m.hi, __ldg(&c[j][0]));
+        r = quick_two_sum(t.hi, __fadd_rn(t.lo, __fadd_rn(m.lo, __ldg(&c[j][1]))));
     }
+#pragma unroll
+    for (int j = 1; j >= 0; --j) r = ff_add(ff_mul(r, u), ff_make(__ldg(&c[j][0]), __ldg(&c[j][1])));
+    return r;
+}
+
+// erfc(-z) = 2 - erfc(z)
+__device__ __forceinline__ ff erfc_ff(ff z) {
+    const bool neg = z.hi < 0.f;
+    const ff r = erfc_pos(neg ? ff_neg(z) : z);
     return neg ? ff_add_f(ff_neg(r), 2.f) : r;
 }
 
@@ -75,21 +86,29 @@ __device__ __forceinline__ double normal_cdf_ff(double mean, ff isd, double x) {
 // What the scoring needs of one contig's depths, formed once when the depths
 // are set (everything here depends on one contig alone, so per edge it would
 // be formed again for every edge the contig is in):
-//   vv[i]   = s * s, s = sqrt(max(var[i], 1)) (the variance the crossing
-//             points use) and isd[i] = cdf_scale(s), per sample;
-//   dev[i]  = the deviation of depth i + 1 from the running mean of depths
-//             0..i, i < nabd - 1, and dev[nabd - 1] = sqrt of the running
-//             sum of squared deviations times i / (i + 1): the one-row steps
-//             of cal_abd_corr, in its order.  The edge's correlation is then
-//             (sum (dev1[i] * dev2[i]) * ratio[i]) / (sx1 * sx2): the
-//             reference's operations on the reference's values.
+//   vv[i]   = s * s, s = sqrt(max(var[i], 1)) (the variance the FP64 crossing
+//             points use);
 //   ratio[i] = (i + 1) / (i + 2.0), as the reference forms it;
-//   m3[i]   = the clamped mean max(abd[i], 1e-6) as three floats whose sum is
-//             exactly that double (hi, mid, low), vf[i] = vv[i] in
-//             float-float: the inputs of the float-float crossing points.
+//   rec[i]  = everything the float-float path reads of sample i, side by
+//             side (AbdRec): the clamped mean max(abd[i], 1e-6) as three
+//             floats whose sum is exactly that double, cdf_scale(s), vv[i] and
+//             its logarithm in float-float, and the deviation of depth i from
+//             the running mean of depths 0 .. i - 1 (FP64);
+//   sx      = sqrt of the running sum of squared deviations times i / (i + 1):
+//             with the deviations, the one-row steps of cal_abd_corr, in its
+//             order.  The edge's correlation is then (sum (dev1[i] * dev2[i]) *
+//             ratio[i]) / (sx1 * sx2): the reference's operations on the
+//             reference's values.
+struct __align__(16) AbdRec {
+    float m[3], isd_hi;
+    float isd_lo, v_hi, v_lo, lv_hi;
+    float lv_lo, pad;
+    double dev;
+};
+
 __global__ void k_abd_prep(const double* __restrict__ abd, const double* __restrict__ var, uint64_t n, uint32_t nabd,
-                           double* __restrict__ vv, float2* __restrict__ isd, double* __restrict__ dev,
-                           double* __restrict__ ratio, float4* __restrict__ m3, float2* __restrict__ vf) {
+                           double* __restrict__ vv, double* __restrict__ ratio, AbdRec* __restrict__ rec,
+                           double* __restrict__ sx) {
     const uint64_t t0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (t0 + 1 < nabd) ratio[t0] = (t0 + 1) / (t0 + 2.0);
     for (uint64_t r = t0; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
@@ -99,29 +118,36 @@ __global__ void k_abd_prep(const double* __restrict__ abd, const double* __restr
         for (uint32_t i = 0; i < nabd; ++i) {
             const double u = w[i];
             const double sd = sqrt(u < 1 ? 1. : u);
+            AbdRec q;
             vv[r * nabd + i] = sd * sd;
-            const ff f = cdf_scale(sd);
-            isd[r * nabd + i] = make_float2(f.hi, f.lo);
-            const ff fv = ff_from_double(sd * sd);
-            vf[r * nabd + i] = make_float2(fv.hi, fv.lo);
+            const ff f = cdf_scale(sd), fv = ff_from_double(sd * sd), fl = ff_from_double(log(sd * sd));
+            q.isd_hi = f.hi;
+            q.isd_lo = f.lo;
+            q.v_hi = fv.hi;
+            q.v_lo = fv.lo;
+            q.lv_hi = fl.hi;
+            q.lv_lo = fl.lo;
             const double x = a[i];
             // the clamped mean as three floats that sum to it exactly
             const double mc = x < 1e-6 ? 1e-6 : x;
-            const float mh = __double2float_rn(mc);
-            const double r1 = mc - (double)mh;
-            const float ml = __double2float_rn(r1);
-            m3[r * nabd + i] = make_float4(mh, ml, __double2float_rn(r1 - (double)ml), 0.f);
+            q.m[0] = __double2float_rn(mc);
+            const double r1 = mc - (double)q.m[0];
+            q.m[1] = __double2float_rn(r1);
+            q.m[2] = __double2float_rn(r1 - (double)q.m[1]);
+            q.pad = 0.f;
+            q.dev = 0.;
             if (i == 0) {
                 mx = x;
             } else {
-                const double q = i / (i + 1.0);
+                const double t = i / (i + 1.0);
                 const double dx = x - mx;
-                sxx += dx * dx * q;
+                sxx += dx * dx * t;
                 mx += dx / (i + 1.0);
-                dev[r * nabd + i - 1] = dx;
+                q.dev = dx;
             }
+            rec[r * nabd + i] = q;
         }
-        dev[r * nabd + nabd - 1] = sqrt(sxx);
+        sx[r] = sqrt(sxx);
     }
 }
 
@@ -171,21 +197,52 @@ __device__ __noinline__ double abd_dist2(double m1, double v1, ff f1, double m2,
     return fabs(normal_cdf_ff(ma, fa, k2) - normal_cdf_ff(ma, fa, k1) + normal_cdf_ff(mb, fb, k1) - normal_cdf_ff(mb, fb, k2));
 }
 
-// k - m in float-float, m given exactly as three floats: error ~2^-48 of
-// the result.
-__device__ __forceinline__ ff ff_sub_m3(ff k, float4 m) {
-    ff s = two_sum(k.hi, -m.x);
+// One contig's sample as the float-float path reads it.
+struct Rec {
+    float m0, m1, m2;  // the clamped mean, exactly
+    ff isd, v, lv;
+    double dev;
+};
+__device__ __forceinline__ Rec load_rec(const AbdRec* __restrict__ p) {
+    const float4* q = reinterpret_cast<const float4*>(p);
+    const float4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+    Rec r;
+    r.m0 = a.x, r.m1 = a.y, r.m2 = a.z;
+    r.isd = ff_make(a.w, b.x);
+    r.v = ff_make(b.y, b.z);
+    r.lv = ff_make(b.w, c.x);
+    r.dev = __hiloint2double(__float_as_int(c.w), __float_as_int(c.z));
+    return r;
+}
+
+// The mean of r (three floats, each the rounding of what the ones before leave)
+// against another double in that form: the first floats that differ decide.
+__device__ __forceinline__ bool mean_gt(const Rec& r, float3 c) {
+    return r.m0 > c.x || (r.m0 == c.x && (r.m1 > c.y || (r.m1 == c.y && r.m2 > c.z)));
+}
+__device__ __forceinline__ bool same_mean(const Rec& a, const Rec& b) {
+    return a.m0 == b.m0 && a.m1 == b.m1 && a.m2 == b.m2;
+}
+
+// k - mean in float-float: error ~2^-48 of the result.
+__device__ __forceinline__ ff ff_sub_mean(ff k, const Rec& r) {
+    ff s = two_sum(k.hi, -r.m0);
     s = ff_add_f(s, k.lo);
-    s = ff_add_f(s, -m.y);
-    return ff_add_f(s, -m.z);
+    s = ff_add_f(s, -r.m1);
+    return ff_add_f(s, -r.m2);
 }
 
-// twice the normal CDF at k (erfc of the scaled difference), in double
-__device__ __forceinline__ double cdf2_at(ff k, float4 m, ff isd) {
-    return ff_to_double(erfc_ff(ff_neg(ff_mul(ff_sub_m3(k, m), isd))));
+// Twice the normal CDF at k is n + t, n = 0 or 2 and t the tail the table
+// gives: t keeps its relative accuracy where the CDF is near 1.
+__device__ __forceinline__ ff cdf2_tail(ff k, const Rec& r, float& n) {
+    const ff z = ff_mul(ff_sub_mean(k, r), r.isd);
+    const bool up = z.hi >= 0.f;
+    const ff e = erfc_pos(up ? z : ff_neg(z));
+    n = up ? 2.f : 0.f;
+    return up ? ff_neg(e) : e;
 }
 
-// cal_abd_dist2 with the crossing points in float-float.  At the crossing
+// 1 - cal_abd_dist2 with the crossing points in float-float.  At the crossing
 // points the two densities are equal, so the overlap is stationary in k1
 // and k2: an error e in either moves it by O((e / sd)^2).  Where the
 // variances differ by at least 1e-3 of the larger one, the crossing points'
@@ -193,49 +250,51 @@ __device__ __forceinline__ double cdf2_at(ff k, float4 m, ff isd) {
 // ~1e-9 sd of the true points (the reference's FP64 points are nearer
 // still), so the overlap agrees with the reference's to ~1e-18 -- far inside
 // the CDFs' own error.  The CDF arguments are formed from the three-float
-// means to float-float accuracy, and the four CDF values are combined in
-// FP64 in the reference's order, as in the FP64 path: the combination needs
-// FP64, since for far-apart distributions 1 - d is small and must keep its
-// relative accuracy.  Returns -1 where the FP64 path decides instead: closer
-// variances, values out of the float-float range, crossing points that do
-// not separate.
-__device__ __forceinline__ double abd_dist2_ff(float4 mm1, float4 mm2, ff vf1, ff vf2, ff f1, ff f2) {
+// means to float-float accuracy.  Each doubled CDF value is its integer part
+// and a tail; the integers cancel exactly, to d = |n + t| / 2 with n = 0 or
+// +-2, so 1 - d is |t| / 2 where d is near 1 and keeps the tails' relative
+// accuracy without FP64 (three FP64 sums of the four converted values cost
+// half of the kernel on this part's narrow FP64 unit).  Returns hi = -1 where
+// the FP64 path decides instead: closer variances, values out of the
+// float-float range, crossing points that do not separate.
+__device__ __forceinline__ ff abd_sim_ff(const Rec& a, const Rec& b) {
+    const ff none = ff_make(-1.f, 0.f);
     // in FP32: variances (>= 1) this far apart also pass the reference's own
     // |v2 - v1| >= 1e-4 test, and their order is that of the FP64 values
-    if (!(fabsf(vf1.hi - vf2.hi) >= 1e-3f * fmaxf(vf1.hi, vf2.hi))) return -1.;
-    const ff q = ff_mul(vf2, ff_recip(vf1));
-    if (!(q.hi > 1e-30f && q.hi < 1e30f && vf1.hi < 1e15f && vf2.hi < 1e15f && mm1.x < 1e15f && mm2.x < 1e15f))
-        return -1.;
-    const ff m1 = ff_make(mm1.x, mm1.y), m2 = ff_make(mm2.x, mm2.y);
-    const ff L = ff_log(q);  // 2 log(sqrt(v2 / v1))
+    if (!(fabsf(a.v.hi - b.v.hi) >= 1e-3f * fmaxf(a.v.hi, b.v.hi))) return none;
+    if (!(a.v.hi < 1e15f && b.v.hi < 1e15f && a.m0 < 1e15f && b.m0 < 1e15f)) return none;
+    const ff m1 = ff_make(a.m0, a.m1), m2 = ff_make(b.m0, b.m1);
+    const ff L = ff_add(b.lv, ff_neg(a.lv));  // 2 log(sqrt(v2 / v1))
     const ff dm = ff_add(m1, ff_neg(m2));
-    const ff dv = ff_add(vf1, ff_neg(vf2));
+    const ff dv = ff_add(a.v, ff_neg(b.v));
     // t = sqrt(v1 v2 ((m1 - m2)^2 - 2 (v1 - v2) log(sqrt(v2 / v1))))
     const ff A = ff_add(ff_mul(dm, dm), ff_neg(ff_mul(dv, L)));
-    const ff t = ff_sqrt(ff_mul(ff_mul(vf1, vf2), A));
-    const ff c = ff_add(ff_mul(m1, vf2), ff_neg(ff_mul(m2, vf1)));  // m1 v2 - m2 v1
+    const ff t = ff_sqrt(ff_mul(ff_mul(a.v, b.v), A));
+    const ff c = ff_add(ff_mul(m1, b.v), ff_neg(ff_mul(m2, a.v)));  // m1 v2 - m2 v1
     const ff idv = ff_recip(dv);
     ff k1 = ff_mul(ff_add(t, ff_neg(c)), idv);  // (t - m1 v2 + m2 v1) / (v1 - v2)
     ff k2 = ff_mul(ff_add(t, c), ff_neg(idv));  // (t + m1 v2 - m2 v1) / (v2 - v1)
     if (!(fabsf(k1.hi) < 1e30f && fabsf(k2.hi) < 1e30f &&
           fabsf(k1.hi - k2.hi) > 0x1p-30f * (fabsf(k1.hi) + fabsf(k2.hi))))
-        return -1.;
+        return none;
     if (ff_gt(k1, k2)) {
         const ff x = k1;
         k1 = k2;
         k2 = x;
     }
-    float4 ma = mm1, mb = mm2;
-    ff fa = f1, fb = f2;
-    if (vf1.hi > vf2.hi) {
-        ma = mm2;
-        fa = f2;
-        mb = mm1;
-        fb = f1;
+    // the doubled overlap of the narrower distribution minus that of the wider
+    // one is n + tl, up to its sign, which the absolute value drops
+    float n2a, n1a, n1b, n2b;
+    const ff t2a = cdf2_tail(k2, a, n2a), t1a = cdf2_tail(k1, a, n1a);
+    const ff t1b = cdf2_tail(k1, b, n1b), t2b = cdf2_tail(k2, b, n2b);
+    const float n = (n2a - n1a) + (n1b - n2b);
+    ff tl = ff_add(ff_add(t2a, ff_neg(t1a)), ff_add(t1b, ff_neg(t2b)));
+    if (n != 0.f) {  // d = (2 + (n > 0 ? tl : -tl)) / 2
+        const float h = n > 0.f ? -0.5f : 0.5f;
+        return ff_make(tl.hi * h, tl.lo * h);
     }
-    // the reference's sum of the four halved values, halved once at the end
-    // (scaling by 1/2 commutes with every rounding here)
-    return fabs(cdf2_at(k2, ma, fa) - cdf2_at(k1, ma, fa) + cdf2_at(k1, mb, fb) - cdf2_at(k2, mb, fb)) * 0.5;
+    if (tl.hi < 0.f) tl = ff_neg(tl);
+    return ff_add_f(ff_make(-0.5f * tl.hi, -0.5f * tl.lo), 1.f);
 }
 
 struct ScoreArgs {
@@ -244,13 +303,13 @@ struct ScoreArgs {
     uint64_t ne, n;
     const double* abd;
     const double* vv;     // per contig and sample (k_abd_prep)
-    const float2* isd;
-    const float4* m3;
-    const float2* vf;
-    const double* dev;
+    const AbdRec* rec;
+    const double* sx;     // per contig
     const double* ratio;
     uint32_t nabd;
     double min_cv;
+    float3 cv3;      // min_cv as three floats
+    bool cv_clamped; // min_cv >= 1e-6: the clamped means compare with it as the depths do
     bool corr;
     double* raw;     // mean abundance similarity per edge
     uint32_t* nnz;   // samples where either depth exceeds min_cv
@@ -259,7 +318,21 @@ struct ScoreArgs {
     unsigned long long* bad;  // edges with an index out of range or no covered sample
 };
 
-// One thread per edge: r1 = to[e], r2 = from[e] (the reference's order).
+// cal_abd_dist of one sample by the FP64 path: its similarity 1 - d.
+__device__ __noinline__ double abd_sim64(const ScoreArgs& p, uint64_t i1, uint64_t i2, ff f1, ff f2) {
+    const double x = p.abd[i1], y = p.abd[i2];
+    const double m1 = x < 1e-6 ? 1e-6 : x, m2 = y < 1e-6 ? 1e-6 : y;
+    double d = 0.;
+    if (m1 != m2) d = abd_dist2(m1, p.vv[i1], f1, m2, p.vv[i2], f2);
+    d = d < 1e-6 ? 1e-6 : d;  // std::min(std::max(d, 1e-6), 1 - 1e-6), NaN kept
+    d = (1. - 1e-6) < d ? 1. - 1e-6 : d;
+    return 1. - d;
+}
+
+// One thread per edge: r1 = to[e], r2 = from[e] (the reference's order).  The
+// FP64 left is the correlation's cross sum and the sum of the similarities.
+// (3.8M edges, 10 samples: 3,358 us with the similarities combined and compared
+// in FP64, a logarithm per pair and all 14 table terms in float-float.)
 __global__ void k_abd_score(ScoreArgs p) {
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < p.ne;
          e += (uint64_t)gridDim.x * blockDim.x) {
@@ -272,43 +345,41 @@ __global__ void k_abd_score(ScoreArgs p) {
             if (p.corr) p.cor[e] = 0.;
             continue;
         }
-        const double* a1 = p.abd + r1 * p.nabd;
-        const double* a2 = p.abd + r2 * p.nabd;
-        const double* q1 = p.vv + r1 * p.nabd;
-        const double* q2 = p.vv + r2 * p.nabd;
-        const float2* f1 = p.isd + r1 * p.nabd;
-        const float2* f2 = p.isd + r2 * p.nabd;
-        const double* d1 = p.dev + r1 * p.nabd;
-        const double* d2 = p.dev + r2 * p.nabd;
+        const AbdRec* q1 = p.rec + r1 * p.nabd;
+        const AbdRec* q2 = p.rec + r2 * p.nabd;
         double sum = 0.;
         uint32_t k = 0;
         // the cross sum of the Pearson correlation (cal_abd_corr), from the
         // rows' own deviations
         double sxy = 0.;
+        // 1 - min(max(d, 1e-6), 1 - 1e-6) at its ends, as FP64 forms them
+        const ff lo = ff_make(0x1.0c6f7ap-20f, 0x1.7p-49f), hi = ff_make(0x1.ffffdep-1f, 0x1.c842fap-27f);
         for (uint32_t i = 0; i < p.nabd; ++i) {
-            const double x = a1[i], y = a2[i];
+            const Rec a = load_rec(q1 + i), b = load_rec(q2 + i);
             // cal_abd_dist for sample i
-            if (x > p.min_cv || y > p.min_cv) {
-                double d = 0.;
-                const double m1 = x < 1e-6 ? 1e-6 : x, m2 = y < 1e-6 ? 1e-6 : y;
-                if (m1 != m2) {
-                    const float2 g1 = f1[i], g2 = f2[i];
-                    const float2 w1 = p.vf[r1 * p.nabd + i], w2 = p.vf[r2 * p.nabd + i];
-                    d = abd_dist2_ff(p.m3[r1 * p.nabd + i], p.m3[r2 * p.nabd + i], ff_make(w1.x, w1.y),
-                                     ff_make(w2.x, w2.y), ff_make(g1.x, g1.y), ff_make(g2.x, g2.y));
-                    if (d < 0.) d = abd_dist2(m1, q1[i], ff_make(g1.x, g1.y), m2, q2[i], ff_make(g2.x, g2.y));
+            bool covered;
+            if (p.cv_clamped)
+                covered = mean_gt(a, p.cv3) || mean_gt(b, p.cv3);
+            else
+                covered = p.abd[r1 * p.nabd + i] > p.min_cv || p.abd[r2 * p.nabd + i] > p.min_cv;
+            if (covered) {
+                ff s = hi;
+                if (!same_mean(a, b)) s = abd_sim_ff(a, b);
+                if (s.hi >= 0.f) {
+                    if (ff_gt(lo, s)) s = lo;
+                    if (ff_gt(s, hi)) s = hi;
+                    sum += ff_to_double(s);
+                } else {
+                    sum += abd_sim64(p, r1 * p.nabd + i, r2 * p.nabd + i, a.isd, b.isd);
                 }
-                d = d < 1e-6 ? 1e-6 : d;  // std::min(std::max(d, 1e-6), 1 - 1e-6), NaN kept
-                d = (1. - 1e-6) < d ? 1. - 1e-6 : d;
-                sum += 1. - d;
                 ++k;
             }
-            if (i > 0) sxy += d1[i - 1] * d2[i - 1] * __ldg(p.ratio + i - 1);
+            if (i > 0) sxy += a.dev * b.dev * __ldg(p.ratio + i - 1);
         }
         if (k == 0) atomicAdd(p.bad, 1ull);
         p.raw[e] = sum / (double)k;
         p.nnz[e] = k;
-        if (p.corr) p.cor[e] = sxy / (d1[p.nabd - 1] * d2[p.nabd - 1]);
+        if (p.corr) p.cor[e] = sxy / (__ldg(p.sx + r1) * __ldg(p.sx + r2));
     }
 }
 
@@ -413,13 +484,15 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     p.n = ctx->abd_n;
     p.abd = (const double*)ctx->bufs["abd.m"].p;
     p.vv = (const double*)ctx->bufs["abd.vv"].p;
-    p.isd = (const float2*)ctx->bufs["abd.isd"].p;
-    p.dev = (const double*)ctx->bufs["abd.dev"].p;
+    p.rec = (const AbdRec*)ctx->bufs["abd.rec"].p;
+    p.sx = (const double*)ctx->bufs["abd.sx"].p;
     p.ratio = (const double*)ctx->bufs["abd.ratio"].p;
-    p.m3 = (const float4*)ctx->bufs["abd.m3"].p;
-    p.vf = (const float2*)ctx->bufs["abd.vf"].p;
     p.nabd = ctx->abd_nabd;
     p.min_cv = min_cv;
+    p.cv_clamped = min_cv >= 1e-6 && min_cv < 1e30;
+    p.cv3.x = (float)min_cv;
+    p.cv3.y = (float)(min_cv - (double)p.cv3.x);
+    p.cv3.z = (float)(min_cv - (double)p.cv3.x - (double)p.cv3.y);
     p.corr = corr;
     p.raw = raw;
     p.nnz = nnz;
@@ -487,18 +560,16 @@ int mdet_ctx_set_abundance(mdet_ctx* ctx, const double* abd, const double* abd_v
     double* dv = (double*)ctx_scratch(ctx, "abd.v", n * nabd * 8);
     uint8_t* low = (uint8_t*)ctx_scratch(ctx, "abd.low", n);
     double* vv = (double*)ctx_scratch(ctx, "abd.vv", n * nabd * 8);
-    float2* isd = (float2*)ctx_scratch(ctx, "abd.isd", n * nabd * 8);
-    double* dev = (double*)ctx_scratch(ctx, "abd.dev", n * nabd * 8);
+    AbdRec* rec = (AbdRec*)ctx_scratch(ctx, "abd.rec", n * nabd * sizeof(AbdRec));
+    double* sx = (double*)ctx_scratch(ctx, "abd.sx", n * 8);
     double* ratio = (double*)ctx_scratch(ctx, "abd.ratio", nabd * 8);
-    float4* m3 = (float4*)ctx_scratch(ctx, "abd.m3", n * nabd * 16);
-    float2* vf = (float2*)ctx_scratch(ctx, "abd.vf", n * nabd * 8);
-    if (!dm || !dv || !low || !vv || !isd || !dev || !ratio || !m3 || !vf) return MDET_ERR_NOMEM;
+    if (!dm || !dv || !low || !vv || !rec || !sx || !ratio) return MDET_ERR_NOMEM;
     MDET_CUDA(ctx, cudaMemcpyAsync(dm, abd, n * nabd * 8, cudaMemcpyHostToDevice, s));
     MDET_CUDA(ctx, cudaMemcpyAsync(dv, abd_var, n * nabd * 8, cudaMemcpyHostToDevice, s));
     k_abd_low<<<grid_for(ctx, n, 256), 256, 0, s>>>(dm, n, nabd, low);
     MDET_LAUNCHED(ctx, "k_abd_low");
     k_abd_prep<<<std::max<unsigned>(grid_for(ctx, n, 256), (nabd + 255) / 256), 256, 0, s>>>(dm, dv, n, nabd, vv,
-                                                                                            isd, dev, ratio, m3, vf);
+                                                                                            ratio, rec, sx);
     MDET_LAUNCHED(ctx, "k_abd_prep");
     MDET_CUDA(ctx, cudaStreamSynchronize(s));
     ctx->abd_n = n;
