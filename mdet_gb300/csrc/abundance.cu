@@ -37,34 +37,51 @@ namespace {
 // tenth of the table's own error; degrees 7 to 2 (below 8e-3) take the shorter
 // float-float sum, whose error is 2^-47 of its operands.  Kept out of line:
 // the score kernel calls it from several places, and inlined copies stall the
-// kernel on instruction fetch.
-__device__ __noinline__ ff erfc_pos(ff z) {
+// kernel on instruction fetch.  tab: the table in shared memory
+// (load_erfc_table) -- the lanes sit on different pieces, and rows kErfcRow
+// words apart put 16 of the 26 pieces on banks of their own, where reads of
+// the table in global memory filled 60 % of the L1's wavefronts.
+constexpr int kErfcRow = 2 * (MDET_ERFC_DEG + 2);
+constexpr int kErfcWords = MDET_ERFC_PIECES * kErfcRow;
+__device__ __forceinline__ void load_erfc_table(float* tab) {
+    for (int i = threadIdx.x; i < MDET_ERFC_PIECES * (MDET_ERFC_DEG + 1); i += blockDim.x) {
+        const int p = i / (MDET_ERFC_DEG + 1), j = i % (MDET_ERFC_DEG + 1);
+        tab[p * kErfcRow + 2 * j] = kErfcTable[p][j][0];
+        tab[p * kErfcRow + 2 * j + 1] = kErfcTable[p][j][1];
+    }
+    __syncthreads();
+}
+__device__ __noinline__ ff erfc_pos(ff z, const float* tab) {
     if (!(z.hi < 6.5f)) return z.hi != z.hi ? z : ff_make(0.f, 0.f);  // NaN stays
     const int p = min((int)(z.hi * 4.f), MDET_ERFC_PIECES - 1);
     // u = (z - centre) * 8, exact scaling of an exact difference
     ff u = ff_add_f(z, -((float)p + 0.5f) * 0.25f);
     u.hi *= 8.f;
     u.lo *= 8.f;
-    const float(*c)[2] = kErfcTable[p];
-    float h = __ldg(&c[MDET_ERFC_DEG][0]);
+    const float2* c = reinterpret_cast<const float2*>(tab + p * kErfcRow);
+    float h = c[MDET_ERFC_DEG].x;
 #pragma unroll
-    for (int j = MDET_ERFC_DEG - 1; j >= 8; --j) h = __fmaf_rn(h, u.hi, __ldg(&c[j][0]));
+    for (int j = MDET_ERFC_DEG - 1; j >= 8; --j) h = __fmaf_rn(h, u.hi, c[j].x);
     ff r = ff_make(h, 0.f);
 #pragma unroll
     for (int j = 7; j >= 2; --j) {
         const ff m = ff_mul(r, u);
-        const ff t = two_sum(m.hi, __ldg(&c[j][0]));
-        r = quick_two_sum(t.hi, __fadd_rn(t.lo, __fadd_rn(m.lo, __ldg(&c[j][1]))));
+        const float2 k = c[j];
+        const ff t = two_sum(m.hi, k.x);
+        r = quick_two_sum(t.hi, __fadd_rn(t.lo, __fadd_rn(m.lo, k.y)));
     }
 #pragma unroll
-    for (int j = 1; j >= 0; --j) r = ff_add(ff_mul(r, u), ff_make(__ldg(&c[j][0]), __ldg(&c[j][1])));
+    for (int j = 1; j >= 0; --j) {
+        const float2 k = c[j];
+        r = ff_add(ff_mul(r, u), ff_make(k.x, k.y));
+    }
     return r;
 }
 
 // erfc(-z) = 2 - erfc(z)
-__device__ __forceinline__ ff erfc_ff(ff z) {
+__device__ __forceinline__ ff erfc_ff(ff z, const float* tab) {
     const bool neg = z.hi < 0.f;
-    const ff r = erfc_pos(neg ? ff_neg(z) : z);
+    const ff r = erfc_pos(neg ? ff_neg(z) : z, tab);
     return neg ? ff_add_f(ff_neg(r), 2.f) : r;
 }
 
@@ -77,10 +94,10 @@ __device__ __forceinline__ ff cdf_scale(double sd) {
 // Boost's normal CDF, erfc(-(x - mean) / (sd * sqrt(2))) / 2 (the function
 // the reference calls), with x - mean formed in FP64 as the reference forms
 // it and the rest in float-float (isd = cdf_scale(sd)); returned in double.
-__device__ __forceinline__ double normal_cdf_ff(double mean, ff isd, double x) {
+__device__ __forceinline__ double normal_cdf_ff(double mean, ff isd, double x, const float* tab) {
     const ff diff = ff_from_double(x - mean);
     const ff z = ff_mul(diff, isd);
-    return ff_to_double(erfc_ff(ff_neg(z))) * 0.5;
+    return ff_to_double(erfc_ff(ff_neg(z), tab)) * 0.5;
 }
 
 // What the scoring needs of one contig's depths, formed once when the depths
@@ -171,7 +188,7 @@ __global__ void k_low_sorted(const uint32_t* __restrict__ perm, const uint8_t* _
 // crossing points, whose numerator cancels when the variances are close, in
 // FP64 in the reference's order; the four CDF values in float-float.  Used
 // where abd_dist2_ff declines.
-__device__ __noinline__ double abd_dist2(double m1, double v1, ff f1, double m2, double v2, ff f2) {
+__device__ __noinline__ double abd_dist2(double m1, double v1, ff f1, double m2, double v2, ff f2, const float* tab) {
     double k1, k2;
     if (fabs(v2 - v1) < 1e-4) {
         k1 = k2 = (m1 + m2) / 2;
@@ -193,8 +210,9 @@ __device__ __noinline__ double abd_dist2(double m1, double v1, ff f1, double m2,
         mb = m1;
         fb = f1;
     }
-    if (k1 == k2) return fabs(normal_cdf_ff(ma, fa, k1) - normal_cdf_ff(mb, fb, k1));
-    return fabs(normal_cdf_ff(ma, fa, k2) - normal_cdf_ff(ma, fa, k1) + normal_cdf_ff(mb, fb, k1) - normal_cdf_ff(mb, fb, k2));
+    if (k1 == k2) return fabs(normal_cdf_ff(ma, fa, k1, tab) - normal_cdf_ff(mb, fb, k1, tab));
+    return fabs(normal_cdf_ff(ma, fa, k2, tab) - normal_cdf_ff(ma, fa, k1, tab) + normal_cdf_ff(mb, fb, k1, tab) -
+                normal_cdf_ff(mb, fb, k2, tab));
 }
 
 // One contig's sample as the float-float path reads it.
@@ -234,12 +252,22 @@ __device__ __forceinline__ ff ff_sub_mean(ff k, const Rec& r) {
 
 // Twice the normal CDF at k is n + t, n = 0 or 2 and t the tail the table
 // gives: t keeps its relative accuracy where the CDF is near 1.
-__device__ __forceinline__ ff cdf2_tail(ff k, const Rec& r, float& n) {
+__device__ __forceinline__ ff cdf2_tail(ff k, const Rec& r, float& n, const float* tab) {
     const ff z = ff_mul(ff_sub_mean(k, r), r.isd);
     const bool up = z.hi >= 0.f;
-    const ff e = erfc_pos(up ? z : ff_neg(z));
+    const ff e = erfc_pos(up ? z : ff_neg(z), tab);
     n = up ? 2.f : 0.f;
     return up ? ff_neg(e) : e;
+}
+
+// 1 - |n + tl| / 2, n = 0 or +-2
+__device__ __forceinline__ ff sim_of_parts(float n, ff tl) {
+    if (n != 0.f) {  // |n + tl| = 2 + (n > 0 ? tl : -tl)
+        const float h = n > 0.f ? -0.5f : 0.5f;
+        return ff_make(tl.hi * h, tl.lo * h);
+    }
+    if (tl.hi < 0.f) tl = ff_neg(tl);
+    return ff_add_f(ff_make(-0.5f * tl.hi, -0.5f * tl.lo), 1.f);
 }
 
 // 1 - cal_abd_dist2 with the crossing points in float-float.  At the crossing
@@ -257,13 +285,23 @@ __device__ __forceinline__ ff cdf2_tail(ff k, const Rec& r, float& n) {
 // half of the kernel on this part's narrow FP64 unit).  Returns hi = -1 where
 // the FP64 path decides instead: closer variances, values out of the
 // float-float range, crossing points that do not separate.
-__device__ __forceinline__ ff abd_sim_ff(const Rec& a, const Rec& b) {
+__device__ __forceinline__ ff abd_sim_ff(const Rec& a, const Rec& b, const float* tab) {
     const ff none = ff_make(-1.f, 0.f);
+    if (!(a.v.hi < 1e15f && b.v.hi < 1e15f && a.m0 < 1e15f && b.m0 < 1e15f)) return none;
+    const ff m1 = ff_make(a.m0, a.m1), m2 = ff_make(b.m0, b.m1);
+    // Equal variances (a depth's variance below 1 counts as 1): one crossing
+    // point, half way, where the overlap is stationary too.
+    if (a.v.hi == b.v.hi && a.v.lo == b.v.lo) {
+        ff k = ff_add(m1, m2);
+        k.hi *= 0.5f;
+        k.lo *= 0.5f;
+        float na, nb;
+        const ff ta = cdf2_tail(k, a, na, tab), tb = cdf2_tail(k, b, nb, tab);
+        return sim_of_parts(na - nb, ff_add(ta, ff_neg(tb)));
+    }
     // in FP32: variances (>= 1) this far apart also pass the reference's own
     // |v2 - v1| >= 1e-4 test, and their order is that of the FP64 values
     if (!(fabsf(a.v.hi - b.v.hi) >= 1e-3f * fmaxf(a.v.hi, b.v.hi))) return none;
-    if (!(a.v.hi < 1e15f && b.v.hi < 1e15f && a.m0 < 1e15f && b.m0 < 1e15f)) return none;
-    const ff m1 = ff_make(a.m0, a.m1), m2 = ff_make(b.m0, b.m1);
     const ff L = ff_add(b.lv, ff_neg(a.lv));  // 2 log(sqrt(v2 / v1))
     const ff dm = ff_add(m1, ff_neg(m2));
     const ff dv = ff_add(a.v, ff_neg(b.v));
@@ -285,16 +323,9 @@ __device__ __forceinline__ ff abd_sim_ff(const Rec& a, const Rec& b) {
     // the doubled overlap of the narrower distribution minus that of the wider
     // one is n + tl, up to its sign, which the absolute value drops
     float n2a, n1a, n1b, n2b;
-    const ff t2a = cdf2_tail(k2, a, n2a), t1a = cdf2_tail(k1, a, n1a);
-    const ff t1b = cdf2_tail(k1, b, n1b), t2b = cdf2_tail(k2, b, n2b);
-    const float n = (n2a - n1a) + (n1b - n2b);
-    ff tl = ff_add(ff_add(t2a, ff_neg(t1a)), ff_add(t1b, ff_neg(t2b)));
-    if (n != 0.f) {  // d = (2 + (n > 0 ? tl : -tl)) / 2
-        const float h = n > 0.f ? -0.5f : 0.5f;
-        return ff_make(tl.hi * h, tl.lo * h);
-    }
-    if (tl.hi < 0.f) tl = ff_neg(tl);
-    return ff_add_f(ff_make(-0.5f * tl.hi, -0.5f * tl.lo), 1.f);
+    const ff t2a = cdf2_tail(k2, a, n2a, tab), t1a = cdf2_tail(k1, a, n1a, tab);
+    const ff t1b = cdf2_tail(k1, b, n1b, tab), t2b = cdf2_tail(k2, b, n2b, tab);
+    return sim_of_parts((n2a - n1a) + (n1b - n2b), ff_add(ff_add(t2a, ff_neg(t1a)), ff_add(t1b, ff_neg(t2b))));
 }
 
 struct ScoreArgs {
@@ -319,11 +350,12 @@ struct ScoreArgs {
 };
 
 // cal_abd_dist of one sample by the FP64 path: its similarity 1 - d.
-__device__ __noinline__ double abd_sim64(const ScoreArgs& p, uint64_t i1, uint64_t i2, ff f1, ff f2) {
+__device__ __noinline__ double abd_sim64(const ScoreArgs& p, uint64_t i1, uint64_t i2, ff f1, ff f2,
+                                         const float* tab) {
     const double x = p.abd[i1], y = p.abd[i2];
     const double m1 = x < 1e-6 ? 1e-6 : x, m2 = y < 1e-6 ? 1e-6 : y;
     double d = 0.;
-    if (m1 != m2) d = abd_dist2(m1, p.vv[i1], f1, m2, p.vv[i2], f2);
+    if (m1 != m2) d = abd_dist2(m1, p.vv[i1], f1, m2, p.vv[i2], f2, tab);
     d = d < 1e-6 ? 1e-6 : d;  // std::min(std::max(d, 1e-6), 1 - 1e-6), NaN kept
     d = (1. - 1e-6) < d ? 1. - 1e-6 : d;
     return 1. - d;
@@ -332,8 +364,11 @@ __device__ __noinline__ double abd_sim64(const ScoreArgs& p, uint64_t i1, uint64
 // One thread per edge: r1 = to[e], r2 = from[e] (the reference's order).  The
 // FP64 left is the correlation's cross sum and the sum of the similarities.
 // (3.8M edges, 10 samples: 3,358 us with the similarities combined and compared
-// in FP64, a logarithm per pair and all 14 table terms in float-float.)
+// in FP64, a logarithm per pair and all 14 table terms in float-float; 1,931 us
+// so, issue slots 79 % used.)
 __global__ void k_abd_score(ScoreArgs p) {
+    __shared__ __align__(16) float tab[kErfcWords];
+    load_erfc_table(tab);
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < p.ne;
          e += (uint64_t)gridDim.x * blockDim.x) {
         p.idx[e] = (uint32_t)e;
@@ -364,13 +399,13 @@ __global__ void k_abd_score(ScoreArgs p) {
                 covered = p.abd[r1 * p.nabd + i] > p.min_cv || p.abd[r2 * p.nabd + i] > p.min_cv;
             if (covered) {
                 ff s = hi;
-                if (!same_mean(a, b)) s = abd_sim_ff(a, b);
+                if (!same_mean(a, b)) s = abd_sim_ff(a, b, tab);
                 if (s.hi >= 0.f) {
                     if (ff_gt(lo, s)) s = lo;
                     if (ff_gt(s, hi)) s = hi;
                     sum += ff_to_double(s);
                 } else {
-                    sum += abd_sim64(p, r1 * p.nabd + i, r2 * p.nabd + i, a.isd, b.isd);
+                    sum += abd_sim64(p, r1 * p.nabd + i, r2 * p.nabd + i, a.isd, b.isd, tab);
                 }
                 ++k;
             }
@@ -383,11 +418,125 @@ __global__ void k_abd_score(ScoreArgs p) {
     }
 }
 
-// Sorted position p starts its run of equal keys: p, else 0 (a max-scan then
-// gives every position the start of its run).
-__global__ void k_run_heads(const double* __restrict__ keys, uint64_t ne, uint32_t* __restrict__ head) {
+// ---- ranks by 32-bit sorts -------------------------------------------------
+// A radix sort of FP64 keys with indices takes eight passes over 12 bytes an
+// edge.  The values of one call span a narrow range, so the sorts run on the
+// top 32 bits of the keys' offsets from their minimum (four passes over 8
+// bytes); the few runs of equal 32-bit keys are put in order by their full
+// keys afterwards (k_fix_runs).  Runs longer than kFixRun whose full keys
+// differ -- values crowded within 2^-32 of the range -- raise a flag, and the call
+// sorts the full keys instead.  (3.8M edges: 1,093 us for the three full sorts
+// and their ranks, 898 us so.)
+constexpr uint32_t kFixRun = 48;
+
+struct KeyRange {
+    unsigned long long min_inv, max;  // of the order keys; min complemented, so that zeros start both
+};
+
+// The order of the radix sort: negative values reversed, -0 as 0.
+__device__ __forceinline__ unsigned long long order_key(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v == 0. ? 0. : v);
+    return (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
+}
+
+struct RankArrays {  // blockIdx.y: which
+    const double* v[3];
+    uint32_t* key[3];
+};
+
+__global__ void __launch_bounds__(256) k_key_range(RankArrays A, uint64_t ne, KeyRange* __restrict__ r) {
+    const double* v = A.v[blockIdx.y];
+    unsigned long long lo = 0, hi = 0;
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < ne; e += (uint64_t)gridDim.x * blockDim.x) {
+        const unsigned long long k = order_key(v[e]);
+        lo = lo > ~k ? lo : ~k;
+        hi = hi > k ? hi : k;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long l2 = __shfl_xor_sync(0xffffffffu, lo, o), h2 = __shfl_xor_sync(0xffffffffu, hi, o);
+        lo = lo > l2 ? lo : l2;
+        hi = hi > h2 ? hi : h2;
+    }
+    __shared__ unsigned long long part[2][8];
+    if ((threadIdx.x & 31) == 0) {
+        part[0][threadIdx.x >> 5] = lo;
+        part[1][threadIdx.x >> 5] = hi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            lo = lo > part[0][w] ? lo : part[0][w];
+            hi = hi > part[1][w] ? hi : part[1][w];
+        }
+        if (lo | hi) {
+            atomicMax(&r[blockIdx.y].min_inv, lo);
+            atomicMax(&r[blockIdx.y].max, hi);
+        }
+    }
+}
+
+__global__ void k_key32(RankArrays A, uint64_t ne, const KeyRange* __restrict__ r) {
+    const double* v = A.v[blockIdx.y];
+    const unsigned long long lo = ~r[blockIdx.y].min_inv, span = r[blockIdx.y].max - lo;
+    const int sh = max(0, 32 - __clzll((long long)span));
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < ne; e += (uint64_t)gridDim.x * blockDim.x)
+        A.key[blockIdx.y][e] = (uint32_t)((order_key(v[e]) - lo) >> sh);
+}
+
+// The thread at the start of a run of equal 32-bit keys sorts the run's indices
+// by the full keys (insertion, stable).
+__global__ void k_fix_runs(const uint32_t* __restrict__ ks, const double* __restrict__ v, uint64_t ne, bool descending,
+                           uint32_t* __restrict__ os, unsigned long long* __restrict__ overflow) {
+    for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q + 1 < ne;
+         q += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t k = ks[q];
+        if (ks[q + 1] != k || (q > 0 && ks[q - 1] == k)) continue;
+        // how far the run goes, and whether it is in order as it stands
+        uint64_t end = q + 1;
+        unsigned long long last = order_key(v[os[q]]);
+        bool sorted = true;
+        for (; end < ne && ks[end] == k; ++end) {
+            const unsigned long long f = order_key(v[os[end]]);
+            sorted = sorted && (descending ? f <= last : f >= last);
+            last = f;
+            if (!sorted && end - q > kFixRun) break;
+        }
+        if (sorted) continue;
+        if (end - q > kFixRun) {
+            atomicAdd(overflow, 1ull);
+            continue;
+        }
+        for (uint64_t i = q + 1; i < end; ++i) {
+            const uint32_t x = os[i];
+            const unsigned long long f = order_key(v[x]);
+            uint64_t j = i;
+            for (; j > q; --j) {
+                const unsigned long long g = order_key(v[os[j - 1]]);
+                if (descending ? g >= f : g <= f) break;
+                os[j] = os[j - 1];
+            }
+            os[j] = x;
+        }
+    }
+}
+
+__global__ void k_gather_sorted(const double* __restrict__ v, const uint32_t* __restrict__ os, uint64_t ne,
+                                double* __restrict__ out) {
     for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < ne; q += (uint64_t)gridDim.x * blockDim.x)
-        head[q] = (q == 0 || keys[q] != keys[q - 1]) ? (uint32_t)q : 0u;
+        out[q] = v[os[q]];
+}
+
+// Sorted position p starts its run of equal values: p, else 0 (a max-scan then
+// gives every position the start of its run).  os: the values' places when
+// they are not sorted themselves.
+__global__ void k_run_heads(const double* __restrict__ keys, const uint32_t* __restrict__ os, uint64_t ne,
+                            uint32_t* __restrict__ head) {
+    for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < ne; q += (uint64_t)gridDim.x * blockDim.x) {
+        bool first = q == 0;
+        if (q) first = os ? keys[os[q]] != keys[os[q - 1]] : keys[q] != keys[q - 1];
+        head[q] = first ? (uint32_t)q : 0u;
+    }
 }
 
 // Ranks from the run starts: ascending sort -> the run's first rank ("min");
@@ -425,7 +574,21 @@ unsigned grid_for(mdet_ctx* ctx, uint64_t items, unsigned block) {
     return (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
 }
 
-// ranks of keys[0..ne) into rank (ascending "min" or, descending, "max")
+// ranks from sorted values (ks, or keys at os) into rank (ascending "min" or,
+// descending, "max")
+int ranks_of(mdet_ctx* ctx, const double* keys, const uint32_t* by, const uint32_t* os, uint64_t ne, bool descending,
+             uint32_t* head, uint32_t* start, uint32_t* rank, void* tmp, size_t tmpb) {
+    cudaStream_t s = ctx->stream;
+    k_run_heads<<<grid_for(ctx, ne, 256), 256, 0, s>>>(keys, by, ne, head);
+    MDET_LAUNCHED(ctx, "k_run_heads");
+    size_t tb = tmpb;
+    MDET_CUDA(ctx, cub::DeviceScan::InclusiveScan(tmp, tb, head, start, MaxOp(), (int)ne, s));
+    k_run_ranks<<<grid_for(ctx, ne, 256), 256, 0, s>>>(os, start, ne, descending, rank);
+    MDET_LAUNCHED(ctx, "k_run_ranks");
+    return MDET_OK;
+}
+
+// the same from a sort of the full keys
 int rank_runs(mdet_ctx* ctx, const double* keys, const uint32_t* idx, uint64_t ne, bool descending, double* ks,
               uint32_t* os, uint32_t* head, uint32_t* start, uint32_t* rank, void* tmp, size_t tmpb) {
     cudaStream_t s = ctx->stream;
@@ -434,13 +597,7 @@ int rank_runs(mdet_ctx* ctx, const double* keys, const uint32_t* idx, uint64_t n
         MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(tmp, tb, keys, ks, idx, os, (int)ne, 0, 64, s));
     else
         MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, keys, ks, idx, os, (int)ne, 0, 64, s));
-    k_run_heads<<<grid_for(ctx, ne, 256), 256, 0, s>>>(ks, ne, head);
-    MDET_LAUNCHED(ctx, "k_run_heads");
-    tb = tmpb;
-    MDET_CUDA(ctx, cub::DeviceScan::InclusiveScan(tmp, tb, head, start, MaxOp(), (int)ne, s));
-    k_run_ranks<<<grid_for(ctx, ne, 256), 256, 0, s>>>(os, start, ne, descending, rank);
-    MDET_LAUNCHED(ctx, "k_run_ranks");
-    return MDET_OK;
+    return ranks_of(ctx, ks, nullptr, os, ne, descending, head, start, rank, tmp, tmpb);
 }
 
 int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const double* stnf, uint64_t ne,
@@ -464,7 +621,11 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     uint32_t* rt = (uint32_t*)ctx_scratch(ctx, "abd.rt", ne * 4);
     uint32_t* rc = (uint32_t*)ctx_scratch(ctx, "abd.rc", ne * 4);
     double* distr = (double*)ctx_scratch(ctx, "abd.distr", ne * 8);
-    unsigned long long* bad = (unsigned long long*)ctx_scratch(ctx, "abd.bad", 8);
+    // [0] bad edges, [1] runs too long to fix, then the three key ranges
+    unsigned long long* bad = (unsigned long long*)ctx_scratch(ctx, "abd.bad", 16 + 3 * sizeof(KeyRange));
+    uint32_t* k32 = (uint32_t*)ctx_scratch(ctx, "abd.k32", ne * 12);
+    uint32_t* k32s = (uint32_t*)ctx_scratch(ctx, "abd.k32s", ne * 4);
+    if (!k32 || !k32s) return MDET_ERR_NOMEM;
     if (!raw || !nnz || !cor || !idx || !ks || !os || !head || !start || !rt || !rc || !distr || !bad)
         return MDET_ERR_NOMEM;
     size_t t1 = 0, t2 = 0, t3 = 0, t4 = 0;
@@ -472,10 +633,13 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(nullptr, t2, stnf, ks, idx, os, (int)ne, 0, 64, s));
     MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(nullptr, t3, cor, ks, idx, os, (int)ne, 0, 64, s));
     MDET_CUDA(ctx, cub::DeviceScan::InclusiveScan(nullptr, t4, head, start, MaxOp(), (int)ne, s));
-    const size_t tmpb = std::max(std::max(t1, t2), std::max(t3, t4));
+    size_t t5 = 0, t6 = 0;
+    MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(nullptr, t5, k32, k32s, idx, os, (int)ne, 0, 32, s));
+    MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(nullptr, t6, k32, k32s, idx, os, (int)ne, 0, 32, s));
+    const size_t tmpb = std::max(std::max(std::max(t1, t2), std::max(t3, t4)), std::max(t5, t6));
     void* tmp = ctx_scratch(ctx, "abd.cubtmp", tmpb);
     if (!tmp) return MDET_ERR_NOMEM;
-    MDET_CUDA(ctx, cudaMemsetAsync(bad, 0, 8, s));
+    MDET_CUDA(ctx, cudaMemsetAsync(bad, 0, 16 + 3 * sizeof(KeyRange), s));
 
     ScoreArgs p;
     p.from = from;
@@ -504,25 +668,58 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     ctx_timer_end(ctx, "k_abd_score");
     MDET_LAUNCHED(ctx, "k_abd_score");
 
-    // the abundance similarities in ascending order (partial_sort_copy)
-    ctx_timer_begin(ctx, "abd_ranks");
-    size_t tb = tmpb;
-    MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, tb, raw, distr, (int)ne, 0, 64, s));
-    MDET_TRY(rank_runs(ctx, stnf, idx, ne, false, ks, os, head, start, rt, tmp, tmpb));
-    if (corr) MDET_TRY(rank_runs(ctx, cor, idx, ne, true, ks, os, head, start, rc, tmp, tmpb));
-    ctx_timer_end(ctx, "abd_ranks");
-    ctx_timer_begin(ctx, "k_sscr");
-    k_sscr<<<grid_for(ctx, ne, 256), 256, 0, s>>>(raw, nnz, rt, rc, distr, ne, corr, out);
-    ctx_timer_end(ctx, "k_sscr");
-    MDET_LAUNCHED(ctx, "k_sscr");
-
-    unsigned long long nbad = 0;
-    MDET_CUDA(ctx, cudaMemcpyAsync(&nbad, bad, 8, cudaMemcpyDeviceToHost, s));
-    MDET_CUDA(ctx, cudaStreamSynchronize(s));
-    if (nbad)
+    // the abundance similarities in ascending order (partial_sort_copy), the
+    // ranks of sTNF and of the correlations, then the scores
+    const unsigned g = grid_for(ctx, ne, 256);
+    auto by_full_keys = [&]() -> int {
+        size_t tb = tmpb;
+        MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, tb, raw, distr, (int)ne, 0, 64, s));
+        MDET_TRY(rank_runs(ctx, stnf, idx, ne, false, ks, os, head, start, rt, tmp, tmpb));
+        if (corr) MDET_TRY(rank_runs(ctx, cor, idx, ne, true, ks, os, head, start, rc, tmp, tmpb));
+        return MDET_OK;
+    };
+    auto by_top_bits = [&]() -> int {
+        const RankArrays A{{raw, stnf, cor}, {k32, k32 + ne, k32 + 2 * ne}};
+        KeyRange* range = (KeyRange*)(bad + 2);
+        const dim3 g3(g, corr ? 3 : 2), gr(std::min<unsigned>(g, ctx->num_sms * 4), g3.y);
+        k_key_range<<<gr, 256, 0, s>>>(A, ne, range);
+        MDET_LAUNCHED(ctx, "k_key_range");
+        k_key32<<<g3, 256, 0, s>>>(A, ne, range);
+        MDET_LAUNCHED(ctx, "k_key32");
+        for (int k = 0; k < (corr ? 3 : 2); ++k) {
+            size_t tb = tmpb;
+            if (k == 2)
+                MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(tmp, tb, A.key[k], k32s, idx, os, (int)ne, 0,
+                                                                         32, s));
+            else
+                MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, A.key[k], k32s, idx, os, (int)ne, 0, 32, s));
+            k_fix_runs<<<g, 256, 0, s>>>(k32s, A.v[k], ne, k == 2, os, bad + 1);
+            MDET_LAUNCHED(ctx, "k_fix_runs");
+            if (k == 0) {
+                k_gather_sorted<<<g, 256, 0, s>>>(raw, os, ne, distr);
+                MDET_LAUNCHED(ctx, "k_gather_sorted");
+            } else {
+                MDET_TRY(ranks_of(ctx, A.v[k], os, os, ne, k == 2, head, start, k == 1 ? rt : rc, tmp, tmpb));
+            }
+        }
+        return MDET_OK;
+    };
+    unsigned long long h_bad[2] = {0, 0};
+    for (int full = 0; full < 2; ++full) {
+        ctx_timer_begin(ctx, "abd_ranks");
+        MDET_TRY(full ? by_full_keys() : by_top_bits());
+        ctx_timer_end(ctx, "abd_ranks");
+        ctx_timer_begin(ctx, "k_sscr");
+        k_sscr<<<g, 256, 0, s>>>(raw, nnz, rt, rc, distr, ne, corr, out);
+        ctx_timer_end(ctx, "k_sscr");
+        MDET_LAUNCHED(ctx, "k_sscr");
+        MDET_CUDA(ctx, cudaMemcpyAsync(h_bad, bad, 16, cudaMemcpyDeviceToHost, s));
+        MDET_CUDA(ctx, cudaStreamSynchronize(s));
+        if (!h_bad[1] || h_bad[0]) break;
+    }
+    if (h_bad[0])
         return ctx_fail(ctx, MDET_ERR_INVALID,
-                        "%llu edges have a contig index out of range or no sample with depth above min_cv",
-                        (unsigned long long)nbad);
+                        "%llu edges have a contig index out of range or no sample with depth above min_cv", h_bad[0]);
     return MDET_OK;
 }
 
