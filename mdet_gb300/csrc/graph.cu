@@ -37,12 +37,23 @@ struct PhaseTimer {
     }
 };
 
-__global__ void k_sample_sort_keys(const uint64_t* __restrict__ contigs, const uint32_t* __restrict__ inv, uint64_t m,
-                                   uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+// The sample goes by size whatever the prepared rows' order is, so that its
+// blocks' distance bounds stay tight.
+__global__ void k_sample_sort_keys(const uint64_t* __restrict__ contigs, const uint32_t* __restrict__ inv,
+                                   const double* __restrict__ ls, uint64_t m, uint32_t* __restrict__ keys,
+                                   uint32_t* __restrict__ vals) {
     uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (b >= m) return;
-    keys[b] = inv[contigs[b]];
+    const uint32_t f = __float_as_uint((float)ls[inv[contigs[b]]]);
+    keys[b] = (f & 0x80000000u) ? ~f : (f | 0x80000000u);
     vals[b] = (uint32_t)b;
+}
+
+// row_map[r]: prepared position of the sample's r-th contig by size
+__global__ void k_sample_rows_of(const uint64_t* __restrict__ contigs, const uint32_t* __restrict__ inv,
+                                 const uint32_t* __restrict__ order, uint64_t m, uint32_t* __restrict__ row_map) {
+    uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (r < m) row_map[r] = inv[contigs[order[r]]];
 }
 
 __global__ void k_sample_gather(const uint32_t* __restrict__ row_map, const uint32_t* __restrict__ order, uint64_t m,
@@ -196,7 +207,7 @@ int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const flo
                const DstarTable& tbl, const char* tag, uint2** cand_out, unsigned long long* ncand_out,
                const uint32_t* tiles, uint64_t nlist, const uint8_t* row_tbl, uint64_t tbl_stride, int bn,
                unsigned long long fixed_cap, unsigned long long** cnt_dev, const unsigned long long* rowoff,
-               const BSide* bside) {
+               const BSide* bside, uint64_t* kept) {
     cudaStream_t s = ctx->stream;
     if (bside && (mode == MDET_MODE_PLAIN || fixed_cap || tiles))
         return ctx_fail(ctx, MDET_ERR_INVALID, "a B-role subset needs a tensor-core form without a tile list");
@@ -227,6 +238,14 @@ int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const flo
         if (cnt_dev) *cnt_dev = cnt;
         return MDET_OK;
     }
+    // A preparation in bands: only the tiles that can hold a pair (the list's
+    // entries are 32-bit).  Up to kRowWaves contigs every CTA takes an equal run
+    // of the list (the rows stay in L2); beyond, the row tiles go out in waves, so
+    // that concurrent CTAs sweep the same B tiles.
+    constexpr uint64_t kRowWaves = 200000;
+    const bool prune = !rect && !bside && !tiles && g.prange && mode != MDET_MODE_PLAIN &&
+                       (uint64_t)(g.n / 128 + 1) * (g.n / 128 + 1) < (1ull << 32) && ctx->forced_shape != 256128;
+    TileList tl{};
     // remembered capacity (bytes of the candidate buffer) from earlier calls
     size_t guess = ((size_t)256 * (bside ? bside->nb : (rect ? na : g.n)) + (1u << 20)) * sizeof(uint2);
     DevBuf& cb = ctx->bufs[std::string(tag) + ".cand"];
@@ -243,6 +262,13 @@ int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const flo
                 MDET_TRY(filter_simt(ctx, A, rect ? na : g.n, rect ? ameta32 : g.meta32, g.x32, g.n, g.meta32, !rect,
                                      tbl, out, tiles, nlist, row_tbl, tbl_stride));
                 ctx->last_tile_n = 128128;
+            } else if (prune) {
+                MDET_TRY(kept_tiles(ctx, g, tbl, tf32 ? 128 : w, &tl));
+                const unsigned long long* ro = g.n > kRowWaves ? tl.rowoff : nullptr;
+                MDET_TRY(filter_tc(ctx, tf32 ? (const void*)g.ta : g.xa, g.nsq, g.n, g.meta,
+                                   tf32 ? (const void*)g.tb : g.xb, g.n, g.meta, true, tbl, out, tl.list, ~0ull,
+                                   nullptr, 0, tf32 ? kShapeTf32 : w, ro, tl.total));
+                ctx->last_tile_n = tf32 ? 128128 : 128 * 1000 + w;
             } else if (tf32) {
                 MDET_TRY(filter_tc(ctx, g.ta, g.nsq, g.n, g.meta, g.tb, g.n, g.meta, true, tbl, out, tiles, nlist,
                                    row_tbl, tbl_stride, kShapeTf32, rowoff));
@@ -263,9 +289,10 @@ int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const flo
             MDET_TRY(run(bn ? bn : 256));
         else
             MDET_TRY(tc_autotune(ctx, bside ? tc_shape_key(true, false, g.n, bside->nb)
-                                            : tc_shape_key(rect, false, rect ? na : g.n, g.n),
-                                 run));
+                                            : tc_shape_key(rect, prune, rect ? na : g.n, g.n),
+                                 run, prune));
         unsigned long long found = 0;
+        if (prune && kept) MDET_CUDA(ctx, cudaMemcpyAsync(kept, tl.total, 8, cudaMemcpyDeviceToHost, s));
         MDET_CUDA(ctx, cudaMemcpyAsync(&found, cnt, 8, cudaMemcpyDeviceToHost, s));
         MDET_CUDA(ctx, cudaStreamSynchronize(s));
         if (found <= cap) {
@@ -337,7 +364,7 @@ int graph_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n
     if (mode == MDET_MODE_LEARNED) return graph_learned(ctx, d_tnf, d_ls, n, cutoff, max_edges, st, g, total);
     PhaseTimer tm(ctx->stream);
     tm.mark();
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, tc_kind(mode), &g));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, tc_kind(mode), &g, nullptr, !in_bands(n, mode)));
     MDET_TRY(abd_gate(ctx, g));
     const double L = logit(cutoff);
     DstarTable tbl;
@@ -345,7 +372,9 @@ int graph_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n
     tm.mark();
     uint2* cand = nullptr;
     unsigned long long ncand = 0;
-    MDET_TRY(run_filter(ctx, mode, g, false, nullptr, nullptr, nullptr, 0, nullptr, nullptr, tbl, "g", &cand, &ncand));
+    uint64_t kept = ~0ull;
+    MDET_TRY(run_filter(ctx, mode, g, false, nullptr, nullptr, nullptr, 0, nullptr, nullptr, tbl, "g", &cand, &ncand,
+                        nullptr, 0, nullptr, 0, 0, 0, nullptr, nullptr, nullptr, &kept));
     tm.mark();
     Edge* edges = nullptr;
     unsigned long long ne = 0;
@@ -357,10 +386,11 @@ int graph_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n
     if (st) {
         st->n_candidates = ncand;
         st->n_above_cutoff = ne;
-        // 128 x 256 tiles of the triangular schedule
+        // tiles of the triangular schedule: 128 x 128 where the kept tiles are, else 128 x 256
         const uint64_t ta = (n + 127) / 128, tb = (n + 255) / 256, h = ta >> 1;
         st->tiles_total = ta * tb - ((ta & 1) ? h * h : (h ? h * (h - 1) : 0));
-        st->tiles_computed = st->tiles_total;
+        if (kept != ~0ull && ctx->last_tile_n == 128128) st->tiles_total = ta * (ta + 1) / 2;
+        st->tiles_computed = kept != ~0ull ? kept : st->tiles_total;
         st->ms_prep = tm.ms(0, 1);
         st->ms_filter = tm.ms(1, 2);
         st->ms_exact = tm.ms(2, 3);
@@ -399,7 +429,7 @@ int graph_shard_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint
     if (max_edges > 512) return ctx_fail(ctx, MDET_ERR_INVALID, "row shards need max_edges <= 512");
     PhaseTimer tm(ctx->stream);
     tm.mark();
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, tc_kind(mode), &g));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, tc_kind(mode), &g, nullptr, true));
     MDET_TRY(abd_gate(ctx, g));
     const uint64_t blocks = (n + 255) / 256;
     const uint32_t s0 = (uint32_t)std::min<uint64_t>(n, blocks * shard / nshards * 256);
@@ -476,14 +506,16 @@ int maxprob_core(mdet_ctx* ctx, const GraphPrep& g, const uint64_t* d_contigs, u
     BlockMeta* ameta32 = (BlockMeta*)ctx_scratch(ctx, "mp.meta32", nblk * sizeof(BlockMeta));
     BlockMeta* ameta = (BlockMeta*)ctx_scratch(ctx, "mp.meta", nblk * sizeof(BlockMeta));
     if (!keys || !keys2 || !vals || !order || !slot_of || !a32 || !als || !ameta32 || !ameta) return MDET_ERR_NOMEM;
-    k_sample_sort_keys<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(d_contigs, g.inv, m, keys, vals);
+    k_sample_sort_keys<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(d_contigs, g.inv, g.ls, m, keys, vals);
     MDET_LAUNCHED(ctx, "k_sample_sort_keys");
     size_t tb = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys2, vals, order, (int)m, 0, 32, s);
     void* tmp = ctx_scratch(ctx, "mp.cubtmp", tb);
     if (!tmp) return MDET_ERR_NOMEM;
     MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, vals, order, (int)m, 0, 32, s));
-    const uint32_t* row_map = keys2;  // sorted positions of the sample, ascending
+    uint32_t* row_map = keys;  // prepared positions of the sample, by size
+    k_sample_rows_of<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(d_contigs, g.inv, order, m, row_map);
+    MDET_LAUNCHED(ctx, "k_sample_rows_of");
     k_sample_gather<<<(unsigned)m, 64, 0, s>>>(row_map, order, m, g.x32, g.ls, a32, als, slot_of);
     MDET_LAUNCHED(ctx, "k_sample_gather");
     const double L = floor_prob > 0 ? logit(floor_prob) : -INFINITY;
@@ -674,7 +706,7 @@ int mdet_tnf_pair_scores_dev(mdet_ctx* ctx, const float* d_tnf, const double* d_
     if (!d_tnf || !d_log_size || !d_pairs || (!d_dist && !d_prob)) return ctx_fail(ctx, MDET_ERR_INVALID, "null pointer");
     if (n < 1 || n >= (1ull << 31)) return ctx_fail(ctx, MDET_ERR_INVALID, "bad contig count");
     GraphPrep g;
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, false, &g));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, false, &g, nullptr, true));
     MDET_TRY(pair_scores(ctx, g, d_pairs, m, d_dist, d_prob));
     MDET_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return check_flag(ctx);
@@ -696,7 +728,7 @@ int mdet_tnf_max_prob_dev(mdet_ctx* ctx, const float* d_tnf, const double* d_log
     // TF32 is asked for.
     if (mode == MDET_MODE_TF32) mode = MDET_MODE_BF16;
     GraphPrep g;
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, mode != MDET_MODE_PLAIN, &g));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, mode != MDET_MODE_PLAIN, &g, nullptr, true));
     MDET_TRY(maxprob_core(ctx, g, d_contigs, m, mode, floor_prob, d_out));
     return check_flag(ctx);
 }
@@ -739,7 +771,7 @@ int mdet_tnf_ptnf_search_dev(mdet_ctx* ctx, const float* d_tnf, const double* d_
     // maxima are exact whatever the filter form; see mdet_tnf_max_prob_dev)
     if (mode == MDET_MODE_TF32) mode = MDET_MODE_BF16;
     GraphPrep g;
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, mode != MDET_MODE_PLAIN, &g));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, mode != MDET_MODE_PLAIN, &g, nullptr, !in_bands(n, mode)));
     std::vector<uint64_t> idx(n);
     // sparse shuffle state: open addressing over positions (key ~0: empty)
     std::vector<uint64_t> mkey, mval;

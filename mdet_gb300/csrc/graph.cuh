@@ -115,6 +115,7 @@ struct GraphPrep {
     BlockMeta* meta32;               // per 128-row block (no rounding term)
     float* mu;                       // column means [136] (of every set)
     double lrange[2];                // log-size range of a preparation in size order
+    float2* prange;                  // per 128-row block: range of the GC projections (null: not in bands)
     const uint8_t* low = nullptr;    // abundance gate: sorted position has no depth above 1 (null: no gate)
 };
 
@@ -129,11 +130,28 @@ inline int tc_kind(int mode) {
     return mode == MDET_MODE_PLAIN ? kTcNone : (mode == MDET_MODE_TF32 ? kTcTf32 : kTcBf16);
 }
 
-// Prepares the contigs in ascending log-size order, or in `order` (original
-// index per position, device) when given.  tck: the reduced-precision rows
+// Prepares the contigs in bands of ascending log size and by GC projection
+// within a band, in ascending log-size order (by_size), or in `order`
+// (original index per position, device) when given.  tck: the reduced-precision rows
 // to make (kTcNone, kTcBf16, kTcTf32; a bool true means kTcBf16).
 int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, int tck, GraphPrep* out,
-                const uint32_t* order = nullptr);
+                const uint32_t* order = nullptr, bool by_size = false);
+// Whether a graph (and the cutoff search before it, which shares the
+// preparation) takes the order in bands: the tensor-core forms, from 8,192
+// contigs on.  At 8,192 the list leaves out 31 % of 2,080 tiles, as much time as
+// making it takes (two passes of k_tile_keep and a scan, 15 us); at 20,000 52 %
+// (TF32 filter 206 -> 111 us), at 1,000,000 69 % (104 -> 45 ms).  The plain form
+// evaluates every pair.
+inline bool in_bands(uint64_t n, int mode) { return mode != MDET_MODE_PLAIN && n >= 8192; }
+// The tiles (row-major, I * tiles_b + J) of the triangular schedule with column
+// tiles of bn that can hold a pair within tbl's bound; entries of row tile I
+// are [rowoff[I], rowoff[I + 1]), all counts on the device.
+struct TileList {
+    const uint32_t* list;
+    const unsigned long long* rowoff;
+    const unsigned long long* total;
+};
+int kept_tiles(mdet_ctx* ctx, const GraphPrep& g, const DstarTable& tbl, int bn, TileList* out);
 // One contig set of a preparation: n contigs whose prepared rows start at
 // `base` (a multiple of 256).
 struct PrepSeg {
@@ -194,12 +212,14 @@ int filter_simt(mdet_ctx* ctx, const float* a, uint32_t na, const BlockMeta* ame
 // to evaluate (column tiles of bn); null evaluates the whole schedule.
 // rowoff (with a list): entries of row tile I are [rowoff[I], rowoff[I+1]),
 // and row tiles are taken in the waves of the full schedule.
+// nlist_dev (with a list): its length on the device (nlist is then a bound).
 // bn: tile shape: 256 = 128 x 256 tiles (one CTA per SM), 128 = 128 x 128
 // (two per SM), kShapeTall = 256 x 128 with four B stages (no tile lists).
 int filter_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, const BlockMeta* ameta,
               const void* b, uint32_t nb, const BlockMeta* bmeta, bool triangular, const DstarTable& tbl,
               CandBuf out, const uint32_t* tiles = nullptr, uint64_t nlist = 0, const uint8_t* row_tbl = nullptr,
-              uint64_t tbl_stride = 0, int bn = 256, const unsigned long long* rowoff = nullptr);
+              uint64_t tbl_stride = 0, int bn = 256, const unsigned long long* rowoff = nullptr,
+              const unsigned long long* nlist_dev = nullptr);
 // Cutoff of one 256-row block of a batch: logit(cutoff) in float-float and
 // whether the second model is needed (logit(cutoff) < ln 9, decided in FP64).
 struct BlkCut {
@@ -242,13 +262,14 @@ struct BSide {
     uint32_t nb;
     const BlockMeta* meta;
 };
+// kept: with a preparation in bands, the tiles evaluated (unchanged when all were).
 int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const float* a32, const uint16_t* ab,
                const float* ansq, uint32_t na, const BlockMeta* ameta, const BlockMeta* ameta32,
                const DstarTable& tbl, const char* tag, uint2** cand_out, unsigned long long* ncand_out,
                const uint32_t* tiles = nullptr, uint64_t nlist = 0, const uint8_t* row_tbl = nullptr,
                uint64_t tbl_stride = 0, int bn = 0, unsigned long long fixed_cap = 0,
                unsigned long long** cnt_dev = nullptr, const unsigned long long* rowoff = nullptr,
-               const BSide* bside = nullptr);
+               const BSide* bside = nullptr, uint64_t* kept = nullptr);
 // Tile-shape autotuner: run(bn) performs one filter pass with column tiles
 // of bn.  The first pass of a shape class times bn = 256 and bn = 128 and
 // keeps the faster (the later pass's output stands); later passes use it.

@@ -88,6 +88,7 @@ struct TcArgs {
     uint32_t jnum, jden;  // the first column tile of row tile I is I * jnum / jden (BM / 128, BN / 128)
     const uint32_t* tiles;  // optional list of tiles (I * tb + J, row-major); null: full schedule
     uint64_t nlist;
+    const unsigned long long* nlist_dev;  // optional: the list's length
     const unsigned long long* rowoff;  // optional: list entries of row tile I are [rowoff[I], rowoff[I+1])
     const uint8_t* row_tbl;  // optional table index per row tile (tables tbl_stride floats apart)
     uint64_t tbl_stride;
@@ -369,6 +370,7 @@ template <int BM, int BN, int NST, int EB>
 __global__ void __launch_bounds__(Shape<BM, BN, NST, EB>::kThreads, Shape<BM, BN, NST, EB>::kCtasPerSm)
     k_filter_tc(const __grid_constant__ CUtensorMap tmA128, const __grid_constant__ CUtensorMap tmA32,
                 const __grid_constant__ CUtensorMap tmB128, const __grid_constant__ CUtensorMap tmB32, TcArgs p) {
+    if (p.nlist_dev) p.nlist = *p.nlist_dev;
     using S = Shape<BM, BN, NST, EB>;
     using E = typename S::E;
     extern __shared__ unsigned char smem_raw[];
@@ -581,33 +583,54 @@ __global__ void __launch_bounds__(Shape<BM, BN, NST, EB>::kThreads, Shape<BM, BN
                 // the hits are in registers: release the accumulator before emitting
                 tc_fence_before();
                 mbar_arrive(&ctl.acc_empty[s]);
-                while (mask) {
-                    const int k = __ffsll((long long)mask) - 1;
-                    mask &= mask - 1;
-                    const uint32_t col = gc0 + k;
-                    if (col < p.nb && row < p.na && (!diag || col > row)) {
-                        uint32_t slot = atomicAdd(qc, 1u);
-                        if (slot < (uint32_t)kQueue) {
-                            q[slot] = make_uint2(row, col);
-                        } else {
-                            unsigned long long pos = atomicAdd(p.out.count, 1ull);
-                            if (pos < p.out.cap) p.out.cand[pos] = make_uint2(row, col);
+                // rows and columns past the set, and the lower triangle of a
+                // diagonal tile
+                if (row >= p.na) mask = 0;
+                if (c.J * BN + BN > p.nb) {  // uniform: the last column tile
+                    const uint32_t left = p.nb > gc0 ? p.nb - gc0 : 0u;
+                    if (left < 64) mask &= (1ull << left) - 1ull;
+                }
+                if (diag && row >= gc0) mask &= row - gc0 >= 63 ? 0ull : ~0ull << (row - gc0 + 1);
+                const uint32_t mine = __popcll(mask);
+                const uint32_t T = __reduce_add_sync(0xffffffffu, mine);
+                if (T) {
+                    uint32_t cnt = *(volatile uint32_t*)qc;  // below kQueue / 2
+                    if (T > kQueue / 2) {
+                        // a dense chunk (rows of one genome against each other hold
+                        // thousands of pairs): straight to the list, one reservation
+                        // for the warp, each lane's hits after those of the lanes
+                        // before it
+                        uint32_t at = mine;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint32_t u = __shfl_up_sync(0xffffffffu, at, o);
+                            if (lane >= (uint32_t)o) at += u;
+                        }
+                        unsigned long long base = 0;
+                        if (lane == 0) base = atomicAdd(p.out.count, (unsigned long long)T);
+                        base = __shfl_sync(0xffffffffu, base, 0) + (at - mine);
+                        for (; mask; mask &= mask - 1, ++base)
+                            if (base < p.out.cap)
+                                p.out.cand[base] = make_uint2(row, gc0 + __ffsll((long long)mask) - 1);
+                    } else {
+                        for (; mask; mask &= mask - 1) {
+                            const uint32_t slot = atomicAdd(qc, 1u);  // fits: both are at most half
+                            q[slot] = make_uint2(row, gc0 + __ffsll((long long)mask) - 1);
+                        }
+                        // flush this warp's queue when it is half full
+                        __syncwarp();
+                        cnt += T;
+                        if (cnt >= kQueue / 2) {
+                            unsigned long long base = 0;
+                            if (lane == 0) base = atomicAdd(p.out.count, (unsigned long long)cnt);
+                            base = __shfl_sync(0xffffffffu, base, 0);
+                            for (uint32_t i = lane; i < cnt; i += 32)
+                                if (base + i < p.out.cap) p.out.cand[base + i] = q[i];
+                            __syncwarp();
+                            if (lane == 0) *(volatile uint32_t*)qc = 0;
+                            __syncwarp();
                         }
                     }
-                }
-                // flush this warp's queue when it is half full
-                __syncwarp();
-                uint32_t cnt = *(volatile uint32_t*)qc;
-                if (cnt >= kQueue / 2) {
-                    cnt = cnt < (uint32_t)kQueue ? cnt : (uint32_t)kQueue;
-                    unsigned long long base = 0;
-                    if (lane == 0) base = atomicAdd(p.out.count, (unsigned long long)cnt);
-                    base = __shfl_sync(0xffffffffu, base, 0);
-                    for (uint32_t i = lane; i < cnt; i += 32)
-                        if (base + i < p.out.cap) p.out.cand[base + i] = q[i];
-                    __syncwarp();
-                    if (lane == 0) *(volatile uint32_t*)qc = 0;
-                    __syncwarp();
                 }
             }
             // final flush
@@ -645,7 +668,7 @@ template <int BM, int BN, int NST, int EB>
 int launch_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, const BlockMeta* ameta,
               const void* b, uint32_t nb, const BlockMeta* bmeta, bool triangular, const DstarTable& tbl,
               CandBuf out, const uint32_t* tiles, uint64_t nlist, const uint8_t* row_tbl, uint64_t tbl_stride,
-              const unsigned long long* rowoff) {
+              const unsigned long long* rowoff, const unsigned long long* nlist_dev) {
     using S = Shape<BM, BN, NST, EB>;
     using E = typename S::E;
     const uint64_t na_pad = (na + 255) / 256 * 256, nb_pad = (nb + 255) / 256 * 256;
@@ -682,6 +705,7 @@ int launch_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, con
     while ((uint64_t)p.ta * p.segs < 2ull * ctas && p.segs < p.tb) ++p.segs;
     p.tiles = tiles;
     p.nlist = nlist;
+    p.nlist_dev = tiles ? nlist_dev : nullptr;
     p.rowoff = tiles ? rowoff : nullptr;
     p.row_tbl = row_tbl;
     p.tbl_stride = tbl_stride;
@@ -701,21 +725,21 @@ int launch_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, con
 int filter_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, const BlockMeta* ameta,
               const void* b, uint32_t nb, const BlockMeta* bmeta, bool triangular, const DstarTable& tbl,
               CandBuf out, const uint32_t* tiles, uint64_t nlist, const uint8_t* row_tbl, uint64_t tbl_stride,
-              int bn, const unsigned long long* rowoff) {
+              int bn, const unsigned long long* rowoff, const unsigned long long* nlist_dev) {
     if (na == 0 || nb == 0) return MDET_OK;
     if (bn == kShapeTf32)
         return launch_tc<128, 128, 2, 4>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
-                                         row_tbl, tbl_stride, rowoff);
+                                         row_tbl, tbl_stride, rowoff, nlist_dev);
     if (bn == 128)
         return launch_tc<128, 128, 2, 2>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
-                                         row_tbl, tbl_stride, rowoff);
+                                         row_tbl, tbl_stride, rowoff, nlist_dev);
     if (bn == kShapeTall) {
         if (tiles) return ctx_fail(ctx, MDET_ERR_INVALID, "tile lists use 128-row tiles");
         return launch_tc<256, 128, 4, 2>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
-                                         row_tbl, tbl_stride, rowoff);
+                                         row_tbl, tbl_stride, rowoff, nlist_dev);
     }
     return launch_tc<128, 256, 2, 2>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
-                                     row_tbl, tbl_stride, rowoff);
+                                     row_tbl, tbl_stride, rowoff, nlist_dev);
 }
 
 static PFN_cuTensorMapEncodeTiled_v12000 get_encode(mdet_ctx* ctx) {

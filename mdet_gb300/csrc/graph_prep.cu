@@ -1,8 +1,10 @@
 // graph_prep.cu -- per-call preparation of the pairwise stage.
 //
 // Contigs are put in ascending log-size order (stable, by original index on
-// ties) so that every tile of the pairwise schedule covers a narrow range of
-// sizes; the size-dependent distance threshold d*(x, y) of the MetaBAT2
+// ties), or, for a whole graph, in narrow bands of log size and by their GC
+// projection within a band (k_band_keys), so that every tile of the pairwise
+// schedule covers a narrow range of sizes and, in the second form, of the
+// projection; the size-dependent distance threshold d*(x, y) of the MetaBAT2
 // model (cuda/Cuda2.cu:199-240 solved for d) is then nearly constant over a
 // tile and one conservative bound per tile filters its pairs.  This file
 // builds: the permutation, sorted FP32 rows and log sizes, the per-contig
@@ -59,6 +61,19 @@ __global__ void k_keys(PrepSet v, uint64_t rows, unsigned long long* __restrict_
     vals[i] = (uint32_t)i;
 }
 
+// Order of a whole graph: bands of log size, `inv_h` per unit, and within a
+// band the GC projection in 16 bits.  Any order gives the same graph; this one
+// makes most tiles provably empty (k_tile_keep).
+__global__ void k_band_keys(const double* __restrict__ ls, const float* __restrict__ proj, uint64_t n, float inv_h,
+                            uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float band = fminf(fmaxf(floorf((float)ls[i] * inv_h), 0.f), 65535.f);  // NaN: band 0
+    const float p = fminf(fmaxf((proj[i] + 1.f) * 32767.5f, 0.f), 65535.f);
+    keys[i] = (uint32_t)band << 16 | (uint32_t)p;
+    vals[i] = (uint32_t)i;
+}
+
 // The segment index of every value, the key of the second (stable) sort.
 __global__ void k_seg_keys(PrepSet v, uint64_t rows, const uint32_t* __restrict__ vals, uint32_t* __restrict__ keys) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -66,8 +81,27 @@ __global__ void k_seg_keys(PrepSet v, uint64_t rows, const uint32_t* __restrict_
 }
 
 constexpr int kCols4 = MDET_NTNF / 4;  // 34
-constexpr int kScanGroups = 8;
-constexpr int kScanThreads = (kCols4 * kScanGroups + 31) / 32 * 32;  // whole warps
+constexpr int kScanWarps = 8;
+
+// The GC direction: the unit vector v whose entry is proportional to a
+// tetranucleotide's G and C bases less two.  |v . (a - b)| <= ||a - b|| for
+// every pair, and GC content is what TNF rows differ in most.
+struct GcVector {
+    float v[MDET_NTNF];
+};
+GcVector gc_vector() {
+    GcVector g;
+    double norm = 0;
+    for (int k = 0; k < MDET_NTNF; ++k) {
+        int gc = -2;  // C and G are the odd codes
+        for (int b = 0; b < 4; ++b) gc += (tn_tables().col_fw[k] >> (2 * b)) & 1;
+        g.v[k] = (float)gc;
+        norm += gc * gc;
+    }
+    const double scale = (1.0 - 1e-6) / sqrt(norm);  // rounding leaves the norm below 1
+    for (int k = 0; k < MDET_NTNF; ++k) g.v[k] = (float)(g.v[k] * scale);
+    return g;
+}
 
 // What k_scan finds over a single set: a hash of the contents, and the
 // smallest (complemented, so that zeros start both) and largest size key.
@@ -76,19 +110,21 @@ struct ScanStat {
     unsigned long long pad;
 };
 
-// One pass over the rows in their original order, rpb rows per block, thread
-// (row group, float4 column): column sums, and with stat the content hash --
-// per 16 bytes one 64 x 64 -> 128-bit product of the words, each offset by
-// its position, folded and added up -- and the log sizes' range.  The sums
-// run in float-float (250,000 contigs: 163 us for the FP64 adds of a separate
-// pass and 79 us for a separate hash; 62 us here, 136 MB); the last block of a
+// One pass over the rows in their original order, rpb rows per block, a warp
+// per row (four columns a lane, the last eight on lanes 0 to 7): column sums,
+// with stat the content hash -- per 16 bytes one 64 x 64 -> 128-bit product of
+// the words, each offset by its position, folded and added up -- and the log
+// sizes' range, and with proj the row's GC projection.  The sums run in
+// float-float (250,000 contigs: 163 us for the FP64 adds of a separate pass
+// and 79 us for a separate hash; 66 us here without projections, 76 us with, 136 MB); the last block of a
 // segment turns them into means.  rpb is 256, the size of a segment's blocks,
 // or 64 up to 65,536 rows, where 256 would leave SMs without a block (1,500
 // contigs: 22 us with 256, 10 us with 64).
-__global__ void __launch_bounds__(kScanThreads) k_scan(PrepSet v, uint32_t rpb, double* __restrict__ sums,
-                                                       uint32_t* __restrict__ done, float* __restrict__ mu,
-                                                       ScanStat* __restrict__ stat) {
-    __shared__ ff part[kScanGroups][MDET_NTNF];
+__global__ void __launch_bounds__(kScanWarps * 32) k_scan(PrepSet v, uint32_t rpb, double* __restrict__ sums,
+                                                          uint32_t* __restrict__ done, float* __restrict__ mu,
+                                                          ScanStat* __restrict__ stat, float* __restrict__ proj,
+                                                          const __grid_constant__ GcVector gc) {
+    __shared__ ff part[kScanWarps][MDET_NTNF];
     __shared__ bool last;
     PrepSeg seg;
     const uint64_t pos0 = (uint64_t)blockIdx.x * rpb;
@@ -96,32 +132,55 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PrepSet v, uint32_t rpb, 
     const uint32_t r0 = (uint32_t)(pos0 - seg.base);
     if (r0 >= seg.n) return;  // block-uniform
     const uint32_t rows = min(rpb, seg.n - r0);
-    const uint32_t t = threadIdx.x, c = t % kCols4, grp = t / kCols4;
+    const uint32_t t = threadIdx.x, w = t >> 5, lane = t & 31;
     const bool al = ((uintptr_t)seg.tnf & 15) == 0;
-    const float* src = seg.tnf + (uint64_t)r0 * MDET_NTNF + 4 * c;
-    ff acc[4];
+    float g[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    if (proj) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = ff_make(0.f, 0.f);
+        for (int j = 0; j < 4; ++j) g[j] = gc.v[4 * lane + j];
+        if (lane < 8) g[4] = gc.v[128 + lane];
+    }
+    ff acc[5];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) acc[j] = ff_make(0.f, 0.f);
     unsigned long long h = 0;
 #pragma unroll 4
-    for (uint32_t r = grp; r < (grp < kScanGroups ? rows : 0u); r += kScanGroups) {
-        const float4 x = load4(src + (uint64_t)r * MDET_NTNF, al);
+    for (uint32_t r = w; r < rows; r += kScanWarps) {
+        const float* row = seg.tnf + (uint64_t)(r0 + r) * MDET_NTNF;
+        const float4 x = load4(row + 4 * lane, al);
+        const float y = lane < 8 ? __ldg(row + 128 + lane) : 0.f;
+        const float e[5] = {x.x, x.y, x.z, x.w, y};
         if (sums) {
-            const float e[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < 5; ++j) {
                 const ff s2 = two_sum(acc[j].hi, e[j]);
                 acc[j].hi = s2.hi;
                 acc[j].lo = __fadd_rn(acc[j].lo, s2.lo);
             }
         }
         if (stat) {
-            const unsigned long long pos = ((uint64_t)(r0 + r) * kCols4 + c + 1) * 0x9E3779B97F4A7C15ull;
+            const unsigned long long pos = ((uint64_t)(r0 + r) * 32 + lane + 1) * 0x9E3779B97F4A7C15ull;
             const unsigned long long a =
                 ((unsigned long long)__float_as_uint(x.y) << 32 | __float_as_uint(x.x)) + pos;
             const unsigned long long b =
                 ((unsigned long long)__float_as_uint(x.w) << 32 | __float_as_uint(x.z)) ^ (pos + 0xBF58476D1CE4E5B9ull);
             h += (a * b) ^ __umul64hi(a, b) ^ (a + (b << 1));
+            const unsigned long long c = (pos ^ __float_as_uint(y)) * 0x94D049BB133111EBull;
+            h += c ^ (c >> 29);
+        }
+        if (proj) {
+            float d = __fmul_rn(e[0], g[0]);
+#pragma unroll
+            for (int j = 1; j < 5; ++j) d = __fmaf_rn(e[j], g[j], d);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            // the rounding bound of tile_kept needs entries of a unit row; any
+            // other row (or a NaN) keeps all its tiles
+            bool unit = true;
+#pragma unroll
+            for (int j = 0; j < 5; ++j) unit = unit && fabsf(e[j]) <= 1.0625f;
+            unit = __all_sync(0xffffffffu, unit);
+            if (lane == 0) proj[r0 + r] = unit ? d : __int_as_float(0x7fc00000);
         }
     }
     if (stat) {
@@ -143,7 +202,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PrepSet v, uint32_t rpb, 
             lo = lo > l2 ? lo : l2;
             hi = hi > h2 ? hi : h2;
         }
-        if ((t & 31) == 0) {
+        if (lane == 0) {
             atomicAdd(&stat->hash, h);
             if (hi | lo) {
                 atomicMax(&stat->min_inv, lo);
@@ -153,12 +212,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(PrepSet v, uint32_t rpb, 
     }
     if (!sums) return;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (grp < kScanGroups) part[grp][4 * c + j] = acc[j];
+    for (int j = 0; j < 4; ++j) part[w][4 * lane + j] = acc[j];
+    if (lane < 8) part[w][128 + lane] = acc[4];
     __syncthreads();
     if (t < MDET_NTNF) {
         ff a = part[0][t];
-        for (int q = 1; q < kScanGroups; ++q) a = ff_add(a, part[q][t]);
+        for (int q = 1; q < kScanWarps; ++q) a = ff_add(a, part[q][t]);
         atomicAdd(&sums[(uint64_t)k * MDET_NTNF + t], ff_to_double(a));
     }
     __threadfence();
@@ -345,7 +404,9 @@ __global__ void __launch_bounds__(256) k_rows(PrepSet v, uint64_t rows, uint32_t
 // its rows one dependent load after another: 24 us at 1,500 contigs and 39 us
 // at 250,000, 4.3 and 6.7 us so).
 __global__ void k_meta(PrepSet v, uint64_t nblk, const double* __restrict__ ls_s, const float* __restrict__ err,
-                       const float* __restrict__ nrm, BlockMeta* __restrict__ meta, BlockMeta* __restrict__ meta32) {
+                       const float* __restrict__ nrm, const float* __restrict__ proj,
+                       const uint32_t* __restrict__ perm, BlockMeta* __restrict__ meta, BlockMeta* __restrict__ meta32,
+                       float2* __restrict__ prange) {
     const uint64_t b = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31;
     if (b >= nblk) return;
@@ -354,6 +415,8 @@ __global__ void k_meta(PrepSet v, uint64_t nblk, const double* __restrict__ ls_s
     const uint64_t s0 = b * MDET_BLK, end = (uint64_t)seg.base + seg.n;
     BlockMeta m;
     m.emax = m.nmax = 0.f;
+    // the block's range of GC projections (one set only); empty for padding
+    float plo = __int_as_float(0x7f800000), phi = -plo;
     if (s0 >= end) {
         m.lo = m.hi = (float)ls_s[end - 1];
     } else {
@@ -368,9 +431,16 @@ __global__ void k_meta(PrepSet v, uint64_t nblk, const double* __restrict__ ls_s
                 e = fmaxf(e, err[s]);
                 nm = fmaxf(nm, nrm[s]);
             }
+            if (prange) {
+                const float p = proj[perm[s]], inf = __int_as_float(0x7f800000);
+                plo = fminf(plo, p == p ? p : -inf);
+                phi = fmaxf(phi, p == p ? p : inf);
+            }
         }
 #pragma unroll
         for (int d = 16; d; d >>= 1) {
+            plo = fminf(plo, __shfl_xor_sync(0xffffffffu, plo, d));
+            phi = fmaxf(phi, __shfl_xor_sync(0xffffffffu, phi, d));
             lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, d));
             hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, d));
             e = fmaxf(e, __shfl_xor_sync(0xffffffffu, e, d));
@@ -382,6 +452,7 @@ __global__ void k_meta(PrepSet v, uint64_t nblk, const double* __restrict__ ls_s
         m.nmax = nm;
     }
     if (lane) return;
+    if (prange) prange[b] = make_float2(plo, phi);
     if (meta) meta[b] = m;
     m.emax = 0.f;
     m.nmax = 0.f;
@@ -627,6 +698,7 @@ int prep_alloc(mdet_ctx* ctx, const char* tag, uint64_t rows, int tck, uint32_t 
     g->ls = (double*)ctx_scratch(ctx, (t + ".ls").c_str(), rows * 8);
     g->parts = (PartsFF*)ctx_scratch(ctx, (t + ".parts").c_str(), rows * sizeof(PartsFF));
     g->meta32 = (BlockMeta*)ctx_scratch(ctx, (t + ".meta32").c_str(), nblk * sizeof(BlockMeta));
+    g->prange = nullptr;
     g->mu = (float*)ctx_scratch(ctx, (t + ".mu").c_str(), (uint64_t)sets * MDET_NTNF * 4);
     g->xa = g->xb = nullptr;
     g->ta = g->tb = nullptr;
@@ -659,7 +731,9 @@ struct ScanBuf {
     uint32_t* done;
 };
 
-static int scan_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, bool stat, float* mu, ScanBuf* out) {
+static int scan_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, bool stat, float* mu, float* proj,
+                     ScanBuf* out) {
+    static const GcVector gc = gc_vector();
     const uint64_t nsum = (uint64_t)set.count * MDET_NTNF;
     const size_t bytes = sizeof(ScanStat) + nsum * 8 + set.count * 4ull;
     unsigned char* p = (unsigned char*)ctx_scratch(ctx, "pre.scan", bytes);
@@ -669,15 +743,24 @@ static int scan_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, 
     out->done = (uint32_t*)(out->sums + nsum);
     MDET_CUDA(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
     const uint32_t rpb = rows <= 65536 ? 64 : 256;
-    k_scan<<<(unsigned)(rows / rpb), kScanThreads, 0, ctx->stream>>>(
-        set, rpb, tck != kTcNone ? out->sums : nullptr, out->done, mu, stat ? out->stat : nullptr);
+    k_scan<<<(unsigned)(rows / rpb), kScanWarps * 32, 0, ctx->stream>>>(
+        set, rpb, tck != kTcNone ? out->sums : nullptr, out->done, mu, stat ? out->stat : nullptr, proj, gc);
     MDET_LAUNCHED(ctx, "k_scan");
     return MDET_OK;
 }
 
-// Everything after the scan: the order, the rows, the metadata.
+// Width of the log-size bands of a whole graph's order.  Within a band the
+// blocks are narrow in the GC projection, so wider bands (more blocks in each)
+// leave more tiles empty but loosen the tiles' distance bound, by 0.9 % of d*
+// at 0.1 and 2 % at 0.2: at 131,000 contigs 39, 54, 60 and 63 % of the tiles are
+// empty at widths 0.02, 0.05, 0.1 and 0.2, at 32,000 8, 28, 42 and 52 %.
+static float band_inv_width(uint64_t n) { return n > 500000 ? 20.f : n > 65536 ? 10.f : 5.f; }
+
+// Everything after the scan: the order, the rows, the metadata.  With proj (one
+// set) the order is by size bands and GC projection, else by size or the
+// caller's.
 static int prep_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, const GraphPrep& g,
-                     const uint32_t* order) {
+                     const uint32_t* order, const float* proj) {
     cudaStream_t s = ctx->stream;
     const uint64_t nblk = rows / MDET_BLK;
     // one set: its n contigs are sorted; several: every row, padding included
@@ -691,28 +774,39 @@ static int prep_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, 
         uint32_t* vals = (uint32_t*)ctx_scratch(ctx, "pre.vals", ns * 4);
         if (!keys || !keys2 || !vals) return MDET_ERR_NOMEM;
         const unsigned blocks = (unsigned)((ns + 255) / 256);
-        k_keys<<<blocks, 256, 0, s>>>(set, ns, keys, vals);
-        MDET_LAUNCHED(ctx, "k_keys");
-        // several sets: by size, then (stable) by set -- two sorts over all
-        // rows cost less than one per set
-        uint32_t* vals2 = set.segs ? (uint32_t*)ctx_scratch(ctx, "pre.vals2", ns * 4) : g.perm;
-        if (!vals2) return MDET_ERR_NOMEM;
-        size_t t1 = 0, t2 = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, t1, keys, keys2, vals, vals2, (int)ns, 0, 64, s);
-        int bits = 1;
-        uint32_t *k32 = (uint32_t*)keys, *k32b = (uint32_t*)keys2;
-        if (set.segs) {
-            while (bits < 32 && (set.count - 1) >> bits) ++bits;
-            cub::DeviceRadixSort::SortPairs(nullptr, t2, k32, k32b, vals2, g.perm, (int)ns, 0, bits, s);
-        }
-        size_t tb = t1 > t2 ? t1 : t2;
-        void* tmp = ctx_scratch(ctx, "pre.cubtmp", tb);
-        if (!tmp) return MDET_ERR_NOMEM;
-        MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, t1, keys, keys2, vals, vals2, (int)ns, 0, 64, s));
-        if (set.segs) {
-            k_seg_keys<<<blocks, 256, 0, s>>>(set, ns, vals2, k32);
-            MDET_LAUNCHED(ctx, "k_seg_keys");
-            MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, t2, k32, k32b, vals2, g.perm, (int)ns, 0, bits, s));
+        if (proj) {
+            uint32_t *k32 = (uint32_t*)keys, *k32b = (uint32_t*)keys2;
+            k_band_keys<<<blocks, 256, 0, s>>>(set.one.ls, proj, ns, band_inv_width(ns), k32, vals);
+            MDET_LAUNCHED(ctx, "k_band_keys");
+            size_t tb = 0;
+            cub::DeviceRadixSort::SortPairs(nullptr, tb, k32, k32b, vals, g.perm, (int)ns, 0, 32, s);
+            void* tmp = ctx_scratch(ctx, "pre.cubtmp", tb);
+            if (!tmp) return MDET_ERR_NOMEM;
+            MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, k32, k32b, vals, g.perm, (int)ns, 0, 32, s));
+        } else {
+            k_keys<<<blocks, 256, 0, s>>>(set, ns, keys, vals);
+            MDET_LAUNCHED(ctx, "k_keys");
+            // several sets: by size, then (stable) by set -- two sorts over all
+            // rows cost less than one per set
+            uint32_t* vals2 = set.segs ? (uint32_t*)ctx_scratch(ctx, "pre.vals2", ns * 4) : g.perm;
+            if (!vals2) return MDET_ERR_NOMEM;
+            size_t t1 = 0, t2 = 0;
+            cub::DeviceRadixSort::SortPairs(nullptr, t1, keys, keys2, vals, vals2, (int)ns, 0, 64, s);
+            int bits = 1;
+            uint32_t *k32 = (uint32_t*)keys, *k32b = (uint32_t*)keys2;
+            if (set.segs) {
+                while (bits < 32 && (set.count - 1) >> bits) ++bits;
+                cub::DeviceRadixSort::SortPairs(nullptr, t2, k32, k32b, vals2, g.perm, (int)ns, 0, bits, s);
+            }
+            size_t tb = t1 > t2 ? t1 : t2;
+            void* tmp = ctx_scratch(ctx, "pre.cubtmp", tb);
+            if (!tmp) return MDET_ERR_NOMEM;
+            MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, t1, keys, keys2, vals, vals2, (int)ns, 0, 64, s));
+            if (set.segs) {
+                k_seg_keys<<<blocks, 256, 0, s>>>(set, ns, vals2, k32);
+                MDET_LAUNCHED(ctx, "k_seg_keys");
+                MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, t2, k32, k32b, vals2, g.perm, (int)ns, 0, bits, s));
+            }
         }
     }
     RowsOut out{g.perm, g.inv, g.x32, g.ls, g.parts, g.xa, g.xb, g.ta, g.tb, g.nsq, nullptr, nullptr, g.mu};
@@ -729,23 +823,24 @@ static int prep_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, 
     else
         k_rows<kTcNone><<<grid, 256, 0, s>>>(set, rows, pblocks, out, model_split());
     MDET_LAUNCHED(ctx, "k_rows");
-    k_meta<<<(unsigned)((nblk * 32 + 255) / 256), 256, 0, s>>>(set, nblk, g.ls, out.err, out.nrm,
-                                                             tck != kTcNone ? g.meta : nullptr, g.meta32);
+    k_meta<<<(unsigned)((nblk * 32 + 255) / 256), 256, 0, s>>>(set, nblk, g.ls, out.err, out.nrm, proj, g.perm,
+                                                             tck != kTcNone ? g.meta : nullptr, g.meta32, g.prange);
     MDET_LAUNCHED(ctx, "k_meta");
     return MDET_OK;
 }
 
 int prep_set(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, const GraphPrep& g) {
     ScanBuf sb;
-    MDET_TRY(scan_rows(ctx, set, rows, tck, false, g.mu, &sb));
-    return prep_rows(ctx, set, rows, tck, g, nullptr);
+    MDET_TRY(scan_rows(ctx, set, rows, tck, false, g.mu, nullptr, &sb));
+    return prep_rows(ctx, set, rows, tck, g, nullptr, nullptr);
 }
 
-// Rows sorted by size (or in the caller's order).  A preparation of the very
+// Rows in bands of size (by_size: strictly by size; or in the caller's order).
+// A preparation of the very
 // same inputs that is still in place (same pointers and contents, no count
 // since) is used as it is: the search and the graph of one assembly share it.
 int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, int tck, GraphPrep* g,
-                const uint32_t* order) {
+                const uint32_t* order, bool by_size) {
     g->n = (uint32_t)n;
     g->npad = (uint32_t)((n + 255) / 256 * 256);
     MDET_TRY(prep_alloc(ctx, "pre", g->npad, tck, 1, g));
@@ -754,11 +849,17 @@ int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t 
     ScanBuf sb;
     if (order) {
         c.valid = false;
-        MDET_TRY(scan_rows(ctx, set, g->npad, tck, false, g->mu, &sb));
-        return prep_rows(ctx, set, g->npad, tck, *g, order);
+        MDET_TRY(scan_rows(ctx, set, g->npad, tck, false, g->mu, nullptr, &sb));
+        return prep_rows(ctx, set, g->npad, tck, *g, order, nullptr);
+    }
+    float* proj = nullptr;
+    if (!by_size) {
+        proj = (float*)ctx_scratch(ctx, "pre.proj", n * 4);
+        g->prange = (float2*)ctx_scratch(ctx, "pre.prange", (uint64_t)g->npad / MDET_BLK * sizeof(float2));
+        if (!proj || !g->prange) return MDET_ERR_NOMEM;
     }
     // the scan writes the means, so a preparation it confirms keeps equal ones
-    MDET_TRY(scan_rows(ctx, set, g->npad, tck, true, g->mu, &sb));
+    MDET_TRY(scan_rows(ctx, set, g->npad, tck, true, g->mu, proj, &sb));
     ScanStat st;
     MDET_CUDA(ctx, cudaMemcpyAsync(&st, sb.stat, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
     MDET_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -767,12 +868,13 @@ int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t 
     // a preparation with other reduced-precision rows (or none) is remade:
     // nsq and the block metadata describe the rows last made
     if (c.valid && c.tnf == d_tnf && c.ls == d_ls && c.n == n && (c.tck == tck || tck == kTcNone) &&
-        c.hash == st.hash && c.x32 == g->x32 && (tck == kTcNone || (c.xa == g->xa && c.ta == g->ta)) &&
+        c.by_size == by_size && c.hash == st.hash && c.x32 == g->x32 && (tck == kTcNone || (c.xa == g->xa && c.ta == g->ta)) &&
         c.gen == ctx->scratch_gen)
         return MDET_OK;
     c.valid = false;
-    MDET_TRY(prep_rows(ctx, set, g->npad, tck, *g, nullptr));
+    MDET_TRY(prep_rows(ctx, set, g->npad, tck, *g, nullptr, proj));
     c.valid = true;
+    c.by_size = by_size;
     c.tnf = d_tnf;
     c.ls = d_ls;
     c.n = n;
@@ -846,5 +948,80 @@ int build_dstar_table(mdet_ctx* ctx, const double* d_ls, uint64_t n, double logi
     t.L = logit_cut;
     t.lmin = lmin;
     t.lmax = lmax;
+    return MDET_OK;
+}
+
+// ---- tiles that can hold a pair ----
+// A pair of rows a, b has |v . (a - b)| <= ||a - b|| for the unit vector v, so a
+// tile whose blocks' ranges of v . x lie further apart than its distance bound
+// holds no pair within the bound.  (1M contigs in bands: two thirds of the
+// tiles, which the filter then never loads.)
+namespace {
+
+template <int W>  // 128-row blocks per column tile
+__device__ __forceinline__ bool tile_kept(const BlockMeta* __restrict__ meta, const float2* __restrict__ pr,
+                                          const DstarTable& tbl, uint32_t I, uint32_t J, uint32_t nblk) {
+    const uint32_t b0 = W * J, b1 = min(W * J + W - 1, nblk - 1);
+    const BlockMeta ma = meta[I], m0 = meta[b0], m1 = meta[b1];
+    const float2 pa = pr[I], p0 = pr[b0], p1 = pr[b1];
+    const float gap = fmaxf(fminf(p0.x, p1.x) - pa.y, pa.x - fmaxf(p0.y, p1.y));
+    // a projection is ten roundings of partial sums below 9.3 (entries up to
+    // 1.0625, the direction's add up to 8.7): 6e-6 off at most, a difference twice that
+    const float R = tile_dstar(tbl, ma.lo, ma.hi, fminf(m0.lo, m1.lo), fmaxf(m0.hi, m1.hi)) * (1.f + 2e-5f) + 2e-5f;
+    return !(gap > R);
+}
+
+// Warp per row tile I: how many of its column tiles are kept, or (list) which,
+// in order.
+template <int W>
+__global__ void __launch_bounds__(256) k_tile_keep(const BlockMeta* __restrict__ meta, const float2* __restrict__ pr,
+                                                   DstarTable tbl, uint32_t ta, uint32_t tb, uint32_t nblk,
+                                                   unsigned long long* __restrict__ cnt,
+                                                   const unsigned long long* __restrict__ off,
+                                                   uint32_t* __restrict__ list) {
+    const uint32_t I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (I >= ta) {
+        if (I == ta && lane == 0 && !list) cnt[ta] = 0;  // the scan's last entry is then the total
+        return;
+    }
+    unsigned long long at = list ? off[I] : 0ull;
+    uint32_t c = 0;
+    for (uint32_t j = I / W; j < tb; j += 32) {
+        const uint32_t J = j + lane;
+        const bool keep = J < tb && tile_kept<W>(meta, pr, tbl, I, J, nblk);
+        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+        if (list && keep) list[at + __popc(bal & ((1u << lane) - 1u))] = I * tb + J;
+        at += __popc(bal);
+        c += __popc(bal);
+    }
+    if (!list && lane == 0) cnt[I] = c;
+}
+
+}  // namespace
+
+int kept_tiles(mdet_ctx* ctx, const GraphPrep& g, const DstarTable& tbl, int bn, TileList* out) {
+    cudaStream_t s = ctx->stream;
+    const uint32_t nblk = g.npad / MDET_BLK, ta = (g.n + 127) / 128, tb = (g.n + bn - 1) / bn;
+    const uint64_t most = (uint64_t)ta * tb / 2 + 2ull * ta + tb;  // the triangle, diagonal tiles included
+    unsigned long long* cnt = (unsigned long long*)ctx_scratch(ctx, "tl.cnt", ((uint64_t)ta + 1) * 8);
+    unsigned long long* off = (unsigned long long*)ctx_scratch(ctx, "tl.off", ((uint64_t)ta + 1) * 8);
+    uint32_t* list = (uint32_t*)ctx_scratch(ctx, "tl.list", most * 4);
+    size_t tmpb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tmpb, cnt, off, (int)ta + 1, s);
+    void* tmp = ctx_scratch(ctx, "tl.cubtmp", tmpb);
+    if (!cnt || !off || !list || !tmp) return MDET_ERR_NOMEM;
+    const BlockMeta* meta = g.meta ? g.meta : g.meta32;
+    const unsigned blocks = (unsigned)(((uint64_t)(ta + 1) * 32 + 255) / 256);
+    for (int fill = 0; fill < 2; ++fill) {
+        if (bn == 256)
+            k_tile_keep<2><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, cnt, off, fill ? list : nullptr);
+        else
+            k_tile_keep<1><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, cnt, off, fill ? list : nullptr);
+        MDET_LAUNCHED(ctx, "k_tile_keep");
+        if (!fill) MDET_CUDA(ctx, cub::DeviceScan::ExclusiveSum(tmp, tmpb, cnt, off, (int)ta + 1, s));
+    }
+    out->list = list;
+    out->rowoff = off;
+    out->total = off + ta;
     return MDET_OK;
 }
