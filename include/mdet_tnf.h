@@ -64,10 +64,9 @@ const char* mdet_version(void);
 /* Tile-shape autotuner (on by default): the first call of each shape class
  * times the tensor-core filter's tile shapes -- 128 x 256 (one CTA per SM),
  * 128 x 128 (two per SM), 256 x 128 with four B stages (one per SM) -- and
- * the exact stage's blocks per SM, and keeps the fastest for the context.
- * mode 1: tune; 0: fixed 128 x 256 tiles and 8 blocks per SM; 128256,
- * 128128 or 256128: force that filter tile (tile lists fall back to 128 x 256
- * for 256128). */
+ * keeps the fastest for the context.  mode 1: tune; 0: fixed 128 x 256 tiles;
+ * 128256, 128128 or 256128: force that filter tile (tile lists fall back to
+ * 128 x 256 for 256128). */
 int mdet_ctx_set_autotune(mdet_ctx* ctx, int mode);
 
 /* Kernel timing: when enabled, the main kernels (k_count, k_filter_tc,

@@ -61,10 +61,8 @@ struct mdet_ctx {
     // tile-shape autotuner of the tensor-core filter: chosen column-tile
     // width per shape class, whether to tune, and the width of the last launch
     std::map<uint64_t, int> tc_shape;
-    std::map<uint64_t, int> exact_shape;  // blocks per SM of the exact stage
     bool autotune = true;
     int forced_shape = 0;  // tile-shape code forced by mdet_ctx_set_autotune (0: none)
-    int forced_exact = 0;  // exact-stage blocks per SM forced while a pass is captured (0: none)
     int last_tile_n = 0;
     // CUDA-graph capture of repeated batched passes
     bool graph_capture = true;

@@ -30,6 +30,40 @@ __device__ __forceinline__ void two_sum_acc(float& s, float& c, float t) {
     c = __fadd_rn(c, err);
 }
 
+// Two FP32 values in one 64-bit register pair: one instruction per operation on
+// both, each rounded as by itself.
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    return make_float2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
+}
+
+// Squares, each rounded by itself: a packed product may be contracted with the
+// addition that follows it, which would drop the term's rounding.
+__device__ __forceinline__ f32x2 square2(f32x2 a) {
+    const float2 v = unpack2(a);
+    return (f32x2)__float_as_uint(__fmul_rn(v.y, v.y)) << 32 | __float_as_uint(__fmul_rn(v.x, v.x));
+}
+
+// two_sum_acc on both halves
+__device__ __forceinline__ void two_sum_acc2(f32x2& s, f32x2& c, f32x2 t) {
+    const f32x2 sum = add2(s, t);
+    const f32x2 bp = sub2(sum, s);
+    const f32x2 err = add2(sub2(s, sub2(sum, bp)), sub2(t, bp));
+    s = sum;
+    c = add2(c, err);
+}
+
 // d in the reference's terms float((a_k-b_k)^2) (cuda/Cuda2.cu:194-196).
 // The reference adds them in FP64; FP64 throughput is scarce on this part, so
 // two FP32 chains with error-free TwoSum compensation carry the sum instead

@@ -319,12 +319,7 @@ bool record(mdet_ctx* ctx, const mdet_assembly* as, const Layout& L, int mode, B
         return false;
     if (upload_sides(ctx, as, L, d) != MDET_OK) return false;
     if (build_list(ctx, L, d, shape ? shape : 128, &np->nlist) != MDET_OK) return false;
-    int exact = 8;
-    auto ex = ctx->exact_shape.find(tc_shape_key(false, false, np->ncand, L.N));
-    if (ex != ctx->exact_shape.end()) exact = ex->second;
-    const int saved_exact = ctx->forced_exact;
     const bool saved_timing = ctx->timing;
-    ctx->forced_exact = exact;
     ctx->timing = false;
     int rc = MDET_OK;
     cudaGraph_t graph = nullptr;
@@ -354,7 +349,6 @@ bool record(mdet_ctx* ctx, const mdet_assembly* as, const Layout& L, int mode, B
         }
     }
     if (graph) cudaGraphDestroy(graph);
-    ctx->forced_exact = saved_exact;
     ctx->timing = saved_timing;
     if (rc != MDET_OK || !np->exec) return false;
     np->scratch_gen = ctx->scratch_gen;

@@ -42,8 +42,9 @@ struct ExactArgs {
 // Squared distances of 32 candidates per warp: candidate base + L belongs to
 // lane L.  Eight lanes share one candidate at a time, so each row is read in
 // coalesced 128-byte runs (lane k of the group takes float4 columns k, k+8,
-// ...); partial sums keep their rounding errors (TwoSum) through the group
-// reduction.  Returns the owner lane's (sum, error) pair and its rows.
+// k+16 and k+24 and column 128+k); partial sums keep their rounding errors
+// (TwoSum) through the group reduction.  Returns the owner lane's (sum, error)
+// pair and its rows.
 __device__ __forceinline__ ff warp_dist2(const uint2* __restrict__ cand, unsigned long long ncand,
                                          unsigned long long base, const uint32_t* __restrict__ row_map,
                                          const float* __restrict__ x32, uint32_t lane, uint32_t& si, uint32_t& sj,
@@ -69,21 +70,23 @@ __device__ __forceinline__ ff warp_dist2(const uint2* __restrict__ cand, unsigne
         const uint32_t b = __shfl_sync(0xffffffffu, sj, from);
         float s = 0.f, c = 0.f;
         if (k < ncand) {
-            const float4* ra = reinterpret_cast<const float4*>(x32 + (uint64_t)a * MDET_NTNF);
-            const float4* rb = reinterpret_cast<const float4*>(x32 + (uint64_t)b * MDET_NTNF);
+            const float* ra = x32 + (uint64_t)a * MDET_NTNF;
+            const float* rb = x32 + (uint64_t)b * MDET_NTNF;
+            f32x2 s2 = 0, c2 = 0;  // two chains, {0, 0}
 #pragma unroll
-            for (uint32_t q = 0; q < 5; ++q) {
-                const uint32_t col = sub + 8 * q;
-                if (col < MDET_NTNF / 4) {
-                    const float4 x = __ldg(ra + col), y = __ldg(rb + col);
-                    const float d0 = __fsub_rn(x.x, y.x), d1 = __fsub_rn(x.y, y.y);
-                    const float d2 = __fsub_rn(x.z, y.z), d3 = __fsub_rn(x.w, y.w);
-                    two_sum_acc(s, c, __fmul_rn(d0, d0));
-                    two_sum_acc(s, c, __fmul_rn(d1, d1));
-                    two_sum_acc(s, c, __fmul_rn(d2, d2));
-                    two_sum_acc(s, c, __fmul_rn(d3, d3));
-                }
+            for (uint32_t q = 0; q < 4; ++q) {
+                const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(ra) + sub + 8 * q);
+                const ulonglong2 y = __ldg(reinterpret_cast<const ulonglong2*>(rb) + sub + 8 * q);
+                const f32x2 d0 = sub2(x.x, y.x), d1 = sub2(x.y, y.y);
+                two_sum_acc2(s2, c2, square2(d0));
+                two_sum_acc2(s2, c2, square2(d1));
             }
+            const float d = __fsub_rn(__ldg(ra + 128 + sub), __ldg(rb + 128 + sub));
+            const float2 sv = unpack2(s2), cv = unpack2(c2);
+            const ff t = two_sum(sv.x, sv.y);
+            s = t.hi;
+            c = __fadd_rn(__fadd_rn(cv.x, cv.y), t.lo);
+            two_sum_acc(s, c, __fmul_rn(d, d));
         }
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) {
@@ -105,18 +108,25 @@ __device__ __forceinline__ ff warp_dist2(const uint2* __restrict__ cand, unsigne
     return quick_two_sum(ms, mc);
 }
 
-__global__ void __launch_bounds__(256) k_exact_graph(ExactArgs p) {
-    __shared__ uint32_t wcount[8];
-    __shared__ unsigned long long bbase;
+constexpr uint32_t kEdgeQueue = 96;
+
+// Bound by the row reads: from DRAM at a million contigs, by instruction issue
+// where the rows fit L2.  The kernel may take 80 registers (three blocks an
+// SM), so that a round's ten row loads are in flight at once (1,000,000 contigs:
+// 21.4 ms in 40 registers, 17.3 in 68); a warp collects its edges in shared
+// memory and reserves list slots 65 to 96 at a time, without a barrier.  20,000
+// contigs (2.85 M candidates): 281 us with 40 registers, six blocks and a
+// block-wide reservation, 243 us with packed arithmetic, 209 us here;
+// 1,000,000: 19.6 -> 17.3 ms.
+__global__ void __launch_bounds__(256, 3) k_exact_graph(ExactArgs p) {
+    __shared__ Edge queue[8][kEdgeQueue];
     if (p.ncand_dev) p.ncand = min(*p.ncand_dev, p.ncand);
     const bool model2 = p.L < kLn9;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    // the block takes 256 candidates per round (32 per warp), so every warp
-    // runs the same number of rounds and the block reserves its edge slots
-    // with one global atomic per round
-    for (unsigned long long bb = (unsigned long long)blockIdx.x * 256; bb < p.ncand;
-         bb += (unsigned long long)gridDim.x * 256) {
-        const unsigned long long base = bb + 32ull * w;
+    Edge* q = queue[w];
+    uint32_t held = 0;  // edges in the warp's queue
+    const unsigned long long step = gridDim.x * 256ull;
+    for (unsigned long long base = blockIdx.x * 256ull + 32ull * w; base < p.ncand; base += step) {
         uint32_t si, sj;
         const ff d2 = warp_dist2(p.cand, p.ncand, base, nullptr, p.x32, lane, si, sj);
         bool edge = false;
@@ -137,30 +147,30 @@ __global__ void __launch_bounds__(256) k_exact_graph(ExactArgs p) {
             }
         }
         const uint32_t bal = __ballot_sync(0xffffffffu, edge);
-        if (lane == 0) wcount[w] = __popc(bal);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t t = 0;
-            for (int k = 0; k < 8; ++k) t += wcount[k];
-            bbase = t ? atomicAdd(p.nedges, (unsigned long long)t) : 0ull;
-        }
-        __syncthreads();
-        uint32_t before = 0;
-        for (uint32_t k = 0; k < w; ++k) before += wcount[k];
         if (edge) {
             Edge e;
             e.i = si;
             e.j = sj;
             e.sim = sim;
-            p.edges[bbase + before + __popc(bal & ((1u << lane) - 1u))] = e;
+            q[held + __popc(bal & ((1u << lane) - 1u))] = e;
             atomicAdd(&p.deg[si], 1u);
             atomicAdd(&p.deg[sj], 1u);
         }
-        __syncthreads();  // wcount and bbase are rewritten next round
+        held += __popc(bal);
+        // flush when another 32 may not fit, and after the warp's last candidates
+        if (held > kEdgeQueue - 32 || (base + step >= p.ncand && held)) {
+            __syncwarp();
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(p.nedges, (unsigned long long)held);
+            at = __shfl_sync(0xffffffffu, at, 0);
+            for (uint32_t k = lane; k < held; k += 32) p.edges[at + k] = q[k];
+            held = 0;
+            __syncwarp();
+        }
     }
 }
 
-__global__ void __launch_bounds__(256) k_exact_maxprob(ExactArgs p) {
+__global__ void __launch_bounds__(256, 3) k_exact_maxprob(ExactArgs p) {
     const uint32_t lane = threadIdx.x & 31;
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x / 32);
     for (unsigned long long base = ((unsigned long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) * 32;
@@ -670,32 +680,14 @@ int exact_graph(mdet_ctx* ctx, const GraphPrep& g, const uint2* cand, unsigned l
         p.edges = edges;
         p.nedges = cnt;
         p.deg = deg;
-        // a block takes 256 candidates per round; blocks per SM (how many
-        // candidates are in flight, hence how far apart in the list the rows
-        // read at one time lie) is tuned once per shape class
-        const unsigned long long blocks = (ncand + 255) / 256;
-        auto run = [&](int per_sm) -> int {
-            MDET_CUDA(ctx, cudaMemsetAsync(cnt, 0, 8, s));
-            MDET_CUDA(ctx, cudaMemsetAsync(deg, 0, (uint64_t)g.n * 4, s));
-            const unsigned long long cap = (unsigned long long)ctx->num_sms * per_sm;
-            ctx_timer_begin(ctx, "k_exact_graph");
-            k_exact_graph<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(p);
-            ctx_timer_end(ctx, "k_exact_graph");
-            MDET_LAUNCHED(ctx, "k_exact_graph");
-            return MDET_OK;
-        };
-        if (ctx->forced_exact) {
-            MDET_TRY(run(ctx->forced_exact));
-        } else {
-            // candidates: as many blocks per SM as fit, half that, and 2
-            int fit = 0;
-            MDET_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_exact_graph, 256, 0));
-            fit = fit < 2 ? 2 : fit;
-            std::vector<int> cands = {fit};
-            if (fit / 2 > 2) cands.push_back(fit / 2);
-            if (fit > 2) cands.push_back(2);
-            MDET_TRY(launch_autotune(ctx, ctx->exact_shape, tc_shape_key(false, false, ncand, g.n), cands, run));
-        }
+        // up to eight waves of the three blocks that fit an SM, for a short tail
+        // (1,000,000 contigs: 4 blocks an SM 21.6 ms, 6 17.5, 24 17.4; 20,000
+        // contigs: 229, 214, 208 us)
+        const unsigned long long blocks = (ncand + 255) / 256, cap = (unsigned long long)ctx->num_sms * 24;
+        ctx_timer_begin(ctx, "k_exact_graph");
+        k_exact_graph<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(p);
+        ctx_timer_end(ctx, "k_exact_graph");
+        MDET_LAUNCHED(ctx, "k_exact_graph");
     }
     *edges_out = edges;
     *deg_out = deg;
