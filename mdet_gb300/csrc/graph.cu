@@ -240,8 +240,9 @@ int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const flo
     }
     // A preparation in bands: only the tiles that can hold a pair (the list's
     // entries are 32-bit).  Up to kRowWaves contigs every CTA takes an equal run
-    // of the list (the rows stay in L2); beyond, the row tiles go out in waves, so
-    // that concurrent CTAs sweep the same B tiles.
+    // of the list (the rows stay in L2); beyond, the row tiles go out in waves by GC
+    // projection, so that concurrent CTAs sweep the same B tiles and their pairs
+    // share rows.
     constexpr uint64_t kRowWaves = 200000;
     const bool prune = !rect && !bside && !tiles && g.prange && mode != MDET_MODE_PLAIN &&
                        (uint64_t)(g.n / 128 + 1) * (g.n / 128 + 1) < (1ull << 32) && ctx->forced_shape != 256128;
@@ -263,11 +264,12 @@ int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const flo
                                      tbl, out, tiles, nlist, row_tbl, tbl_stride));
                 ctx->last_tile_n = 128128;
             } else if (prune) {
-                MDET_TRY(kept_tiles(ctx, g, tbl, tf32 ? 128 : w, &tl));
-                const unsigned long long* ro = g.n > kRowWaves ? tl.rowoff : nullptr;
+                const uint32_t wave = g.n > kRowWaves ? filter_tc_ctas(ctx, tf32 ? kShapeTf32 : w) : 0u;
+                MDET_TRY(kept_tiles(ctx, g, tbl, tf32 ? 128 : w, wave, &tl));
+                const unsigned long long* ro = wave ? tl.rowoff : nullptr;
                 MDET_TRY(filter_tc(ctx, tf32 ? (const void*)g.ta : g.xa, g.nsq, g.n, g.meta,
                                    tf32 ? (const void*)g.tb : g.xb, g.n, g.meta, true, tbl, out, tl.list, ~0ull,
-                                   nullptr, 0, tf32 ? kShapeTf32 : w, ro, tl.total));
+                                   nullptr, 0, tf32 ? kShapeTf32 : w, ro, tl.total, tl.row_order));
                 ctx->last_tile_n = tf32 ? 128128 : 128 * 1000 + w;
             } else if (tf32) {
                 MDET_TRY(filter_tc(ctx, g.ta, g.nsq, g.n, g.meta, g.tb, g.n, g.meta, true, tbl, out, tiles, nlist,

@@ -90,6 +90,7 @@ struct TcArgs {
     uint64_t nlist;
     const unsigned long long* nlist_dev;  // optional: the list's length
     const unsigned long long* rowoff;  // optional: list entries of row tile I are [rowoff[I], rowoff[I+1])
+    const uint32_t* row_order;  // optional (with rowoff): the row tiles in the order of the waves
     const uint8_t* row_tbl;  // optional table index per row tile (tables tbl_stride floats apart)
     uint64_t tbl_stride;
     int triangular;
@@ -299,14 +300,16 @@ __device__ __forceinline__ void list_decode(const TcArgs& p, Cursor& k) {
 // Wave-ordered list: row tiles in the waves of the full schedule, each row
 // tile's listed column tiles in order (so concurrent CTAs sweep the same B
 // tiles, as in the full schedule).  Moves to the first non-empty row tile
-// from wave k.w on.
+// from wave k.w on.  p.row_order, when given, names the tiles of the waves: row
+// tiles that list the same column tiles.
 __device__ __forceinline__ void list_next_row(const TcArgs& p, Cursor& k, uint32_t c, uint32_t G) {
     while (true) {
-        const uint32_t I = unit_of_wave(k.w, c, G);
+        uint32_t I = unit_of_wave(k.w, c, G);
         if (I >= p.ta) {
             k.valid = false;
             return;
         }
+        if (p.row_order) I = p.row_order[I];
         k.li = p.rowoff[I];
         k.lend = p.rowoff[I + 1];
         if (k.li < k.lend) {
@@ -668,7 +671,7 @@ template <int BM, int BN, int NST, int EB>
 int launch_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, const BlockMeta* ameta,
               const void* b, uint32_t nb, const BlockMeta* bmeta, bool triangular, const DstarTable& tbl,
               CandBuf out, const uint32_t* tiles, uint64_t nlist, const uint8_t* row_tbl, uint64_t tbl_stride,
-              const unsigned long long* rowoff, const unsigned long long* nlist_dev) {
+              const unsigned long long* rowoff, const unsigned long long* nlist_dev, const uint32_t* row_order) {
     using S = Shape<BM, BN, NST, EB>;
     using E = typename S::E;
     const uint64_t na_pad = (na + 255) / 256 * 256, nb_pad = (nb + 255) / 256 * 256;
@@ -707,6 +710,7 @@ int launch_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, con
     p.nlist = nlist;
     p.nlist_dev = tiles ? nlist_dev : nullptr;
     p.rowoff = tiles ? rowoff : nullptr;
+    p.row_order = p.rowoff ? row_order : nullptr;
     p.row_tbl = row_tbl;
     p.tbl_stride = tbl_stride;
     unsigned grid =
@@ -722,24 +726,28 @@ int launch_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, con
 
 }  // namespace
 
+uint32_t filter_tc_ctas(mdet_ctx* ctx, int bn) {
+    return (uint32_t)ctx->num_sms * (bn == 128 ? Shape<128, 128, 2, 2>::kCtasPerSm : 1);
+}
+
 int filter_tc(mdet_ctx* ctx, const void* a, const float* a_nsq, uint32_t na, const BlockMeta* ameta,
               const void* b, uint32_t nb, const BlockMeta* bmeta, bool triangular, const DstarTable& tbl,
               CandBuf out, const uint32_t* tiles, uint64_t nlist, const uint8_t* row_tbl, uint64_t tbl_stride,
-              int bn, const unsigned long long* rowoff, const unsigned long long* nlist_dev) {
+              int bn, const unsigned long long* rowoff, const unsigned long long* nlist_dev, const uint32_t* row_order) {
     if (na == 0 || nb == 0) return MDET_OK;
     if (bn == kShapeTf32)
         return launch_tc<128, 128, 2, 4>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
-                                         row_tbl, tbl_stride, rowoff, nlist_dev);
+                                         row_tbl, tbl_stride, rowoff, nlist_dev, row_order);
     if (bn == 128)
         return launch_tc<128, 128, 2, 2>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
-                                         row_tbl, tbl_stride, rowoff, nlist_dev);
+                                         row_tbl, tbl_stride, rowoff, nlist_dev, row_order);
     if (bn == kShapeTall) {
         if (tiles) return ctx_fail(ctx, MDET_ERR_INVALID, "tile lists use 128-row tiles");
         return launch_tc<256, 128, 4, 2>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
-                                         row_tbl, tbl_stride, rowoff, nlist_dev);
+                                         row_tbl, tbl_stride, rowoff, nlist_dev, row_order);
     }
     return launch_tc<128, 256, 2, 2>(ctx, a, a_nsq, na, ameta, b, nb, bmeta, triangular, tbl, out, tiles, nlist,
-                                     row_tbl, tbl_stride, rowoff, nlist_dev);
+                                     row_tbl, tbl_stride, rowoff, nlist_dev, row_order);
 }
 
 static PFN_cuTensorMapEncodeTiled_v12000 get_encode(mdet_ctx* ctx) {

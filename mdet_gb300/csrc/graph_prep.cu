@@ -978,7 +978,7 @@ __global__ void __launch_bounds__(256) k_tile_keep(const BlockMeta* __restrict__
                                                    DstarTable tbl, uint32_t ta, uint32_t tb, uint32_t nblk,
                                                    unsigned long long* __restrict__ cnt,
                                                    const unsigned long long* __restrict__ off,
-                                                   uint32_t* __restrict__ list) {
+                                                   uint32_t* __restrict__ list, uint32_t* __restrict__ mid) {
     const uint32_t I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (I >= ta) {
         if (I == ta && lane == 0 && !list) cnt[ta] = 0;  // the scan's last entry is then the total
@@ -994,12 +994,29 @@ __global__ void __launch_bounds__(256) k_tile_keep(const BlockMeta* __restrict__
         at += __popc(bal);
         c += __popc(bal);
     }
-    if (!list && lane == 0) cnt[I] = c;
+    if (!list && lane == 0) {
+        cnt[I] = c;
+        if (mid) {  // sorts like the middle of the tile's projections
+            const uint32_t f = __float_as_uint(pr[I].x + pr[I].y);
+            mid[I] = (f & 0x80000000u) ? ~f : (f | 0x80000000u);
+            mid[ta + I] = I;
+        }
+    }
+}
+
+// Key of the row tile at every position of the order by projection: its group
+// of `group` tiles, within the group the longest list first.
+__global__ void k_wave_keys(const uint32_t* __restrict__ by_mid, const unsigned long long* __restrict__ cnt,
+                            uint32_t ta, uint32_t group, uint32_t* __restrict__ keys) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= ta) return;
+    const unsigned long long c = cnt[by_mid[r]];
+    keys[r] = (r / group) << 18 | (0x3ffffu - (uint32_t)(c < 0x3ffffull ? c : 0x3ffffull));
 }
 
 }  // namespace
 
-int kept_tiles(mdet_ctx* ctx, const GraphPrep& g, const DstarTable& tbl, int bn, TileList* out) {
+int kept_tiles(mdet_ctx* ctx, const GraphPrep& g, const DstarTable& tbl, int bn, uint32_t wave, TileList* out) {
     cudaStream_t s = ctx->stream;
     const uint32_t nblk = g.npad / MDET_BLK, ta = (g.n + 127) / 128, tb = (g.n + bn - 1) / bn;
     const uint64_t most = (uint64_t)ta * tb / 2 + 2ull * ta + tb;  // the triangle, diagonal tiles included
@@ -1010,18 +1027,36 @@ int kept_tiles(mdet_ctx* ctx, const GraphPrep& g, const DstarTable& tbl, int bn,
     cub::DeviceScan::ExclusiveSum(nullptr, tmpb, cnt, off, (int)ta + 1, s);
     void* tmp = ctx_scratch(ctx, "tl.cubtmp", tmpb);
     if (!cnt || !off || !list || !tmp) return MDET_ERR_NOMEM;
+    uint32_t* mid = nullptr;  // five arrays of ta: keys, tiles, their sorted copies, the order
+    if (wave && !(mid = (uint32_t*)ctx_scratch(ctx, "tl.mid", 5ull * ta * 4))) return MDET_ERR_NOMEM;
     const BlockMeta* meta = g.meta ? g.meta : g.meta32;
     const unsigned blocks = (unsigned)(((uint64_t)(ta + 1) * 32 + 255) / 256);
     for (int fill = 0; fill < 2; ++fill) {
         if (bn == 256)
-            k_tile_keep<2><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, cnt, off, fill ? list : nullptr);
+            k_tile_keep<2><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, cnt, off, fill ? list : nullptr,
+                                                  mid);
         else
-            k_tile_keep<1><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, cnt, off, fill ? list : nullptr);
+            k_tile_keep<1><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, cnt, off, fill ? list : nullptr,
+                                                  mid);
         MDET_LAUNCHED(ctx, "k_tile_keep");
         if (!fill) MDET_CUDA(ctx, cub::DeviceScan::ExclusiveSum(tmp, tmpb, cnt, off, (int)ta + 1, s));
     }
     out->list = list;
     out->rowoff = off;
     out->total = off + ta;
+    out->row_order = nullptr;
+    if (wave) {
+        uint32_t *keys = mid, *vals = mid + ta, *keys2 = mid + 2ull * ta, *vals2 = mid + 3ull * ta;
+        uint32_t* order = mid + 4ull * ta;
+        size_t sb = 0;
+        cub::DeviceRadixSort::SortPairs(nullptr, sb, keys, keys2, vals, vals2, (int)ta, 0, 32, s);
+        void* stmp = ctx_scratch(ctx, "tl.sorttmp", sb);
+        if (!stmp) return MDET_ERR_NOMEM;
+        MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(stmp, sb, keys, keys2, vals, vals2, (int)ta, 0, 32, s));
+        k_wave_keys<<<(ta + 255) / 256, 256, 0, s>>>(vals2, cnt, ta, kWaveGroup * wave, keys);
+        MDET_LAUNCHED(ctx, "k_wave_keys");
+        MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(stmp, sb, keys, keys2, vals2, order, (int)ta, 0, 32, s));
+        out->row_order = order;
+    }
     return MDET_OK;
 }
