@@ -350,6 +350,8 @@ __global__ void __launch_bounds__(1024) k_topk_big(const uint32_t* __restrict__ 
 }
 
 // ---- selection top-k: warp per contig --------------------------------------
+// topk_regs holds rows of up to 512 entries in registers; topk_any takes the rest:
+//
 // A row's kept set is its max_edges best entries under (sim descending, ocol
 // ascending).  Ordered as the 96-bit key (bits of sim, ~ocol) -- sim is a
 // positive double, so its bits order like its value -- the kept set is every
@@ -441,7 +443,7 @@ __device__ __forceinline__ void sort_out(const unsigned long long* __restrict__ 
 }
 
 constexpr int kSelWarps = 4;
-constexpr uint32_t kSelCap = 896;  // entries staged in shared memory per warp (46 KB per block)
+constexpr uint32_t kRowRegs = 512;  // entries of a row held in registers, 16 a lane
 
 __device__ __forceinline__ uint32_t sel_digit(unsigned long long hi, uint32_t lo, int p) {
     return p < 8 ? (uint32_t)(hi >> (56 - 8 * p)) & 255u : (lo >> (24 - 8 * (p - 8))) & 255u;
@@ -456,131 +458,307 @@ __device__ __forceinline__ bool sel_match(unsigned long long hi, uint32_t lo, un
     return p == 8 || (lo >> (32 - 8 * (p - 8))) == (P_lo >> (32 - 8 * (p - 8)));
 }
 
+// The highest bin of a 256-bin histogram at which the count from the top
+// reaches `need` (>= 1, at most the total), the count above it and its own.
+__device__ __forceinline__ void sel_bin(const uint32_t* __restrict__ hist, uint32_t lane, uint32_t need, uint32_t& bin,
+                                        uint32_t& above, uint32_t& count) {
+    // lane L owns bins [8L, 8L + 8); count the bins above each lane's
+    const uint4 b0 = *reinterpret_cast<const uint4*>(hist + 8 * lane);
+    const uint4 b1 = *reinterpret_cast<const uint4*>(hist + 8 * lane + 4);
+    const uint32_t b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    uint32_t own = 0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) own += b[t];
+    uint32_t suf = own;  // inclusive sum over lanes >= lane
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_down_sync(0xffffffffu, suf, o);
+        if (lane + o < 32) suf += v;
+    }
+    uint32_t at = suf - own;
+    int found = -1;
+    uint32_t cnt = 0;
+    if (at < need && need <= suf) {
+#pragma unroll
+        for (int t = 7; t >= 0; --t) {
+            if (found < 0 && at + b[t] >= need) {
+                found = (int)(lane * 8 + t);
+                cnt = b[t];
+            }
+            if (found < 0) at += b[t];
+        }
+    }
+    const uint32_t who = __ffs(__ballot_sync(0xffffffffu, found >= 0)) - 1;
+    bin = (uint32_t)__shfl_sync(0xffffffffu, found, who);
+    above = __shfl_sync(0xffffffffu, at, who);
+    count = __shfl_sync(0xffffffffu, cnt, who);
+}
+
+__device__ __forceinline__ void sel_clear(uint32_t* __restrict__ hist, uint32_t lane) {
+    *reinterpret_cast<uint4*>(hist + 8 * lane) = make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(hist + 8 * lane + 4) = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+}
+
+// A row of any length and with any scores: the entries are read from memory in
+// every pass, keys are the full 96 bits.
 template <int EMAX>
-__global__ void __launch_bounds__(kSelWarps * 32) k_topk_sel(const unsigned long long* __restrict__ rowptr,
+__device__ __noinline__ uint32_t topk_any(uint32_t cnt, uint32_t orow, uint32_t max_edges, Ent* __restrict__ row,
+                                          unsigned long long* __restrict__ key, uint32_t* __restrict__ col,
+                                          uint32_t* __restrict__ hist, uint32_t lane) {
+    // threshold key (P_hi, P_lo): kept iff key >= it
+    unsigned long long P_hi = 0;
+    uint32_t P_lo = 0;
+    if (cnt > max_edges) {
+        uint32_t need = max_edges;
+        for (int p = 0; p < 12; ++p) {
+            sel_clear(hist, lane);
+            for (uint32_t i = lane; i < cnt; i += 32) {
+                const Ent x = row[i];
+                const unsigned long long hi = (unsigned long long)__double_as_longlong(x.sim);
+                const uint32_t lo = ~x.ocol;
+                if (sel_match(hi, lo, P_hi, P_lo, p)) atomicAdd(&hist[sel_digit(hi, lo, p)], 1u);
+            }
+            __syncwarp();
+            uint32_t bin, above, count;
+            sel_bin(hist, lane, need, bin, above, count);
+            __syncwarp();
+            need -= above;
+            if (p < 8)
+                P_hi |= (unsigned long long)bin << (56 - 8 * p);
+            else
+                P_lo |= bin << (24 - 8 * (p - 8));
+            if (count == need) break;
+        }
+    }
+    // compact the kept entries with ocol > orow
+    uint32_t m = 0;
+    for (uint32_t base = 0; base < cnt; base += 32) {
+        const uint32_t i = base + lane;
+        unsigned long long hi = 0;
+        uint32_t c = 0;
+        bool take = false;
+        if (i < cnt) {
+            const Ent x = row[i];
+            hi = (unsigned long long)__double_as_longlong(x.sim);
+            c = x.ocol;
+            const uint32_t lo = ~c;
+            take = c > orow && (hi > P_hi || (hi == P_hi && lo >= P_lo));
+        }
+        const uint32_t bal = __ballot_sync(0xffffffffu, take);
+        const uint32_t q = m + __popc(bal & ((1u << lane) - 1u));
+        if (take && q < max_edges) {
+            key[q] = hi;
+            col[q] = c;
+        }
+        m += __popc(bal);
+    }
+    __syncwarp();
+    m = min(m, max_edges);
+    if (m <= 64)
+        sort_out<2>(key, col, m, lane, row);
+    else if (m <= 128)
+        sort_out<4>(key, col, m, lane, row);
+    else
+        sort_out<EMAX>(key, col, m, lane, row);
+    return m;
+}
+
+// Exchange of two values, the larger first when `up`.
+__device__ __forceinline__ void order2(unsigned long long& a, unsigned long long& b, bool up) {
+    const bool sw = (b > a) == up;
+    const unsigned long long t = sw ? b : a;
+    b = sw ? a : b;
+    a = t;
+}
+
+// Sorts 32 * E distinct values (zeros may repeat) in shared memory, largest
+// first: value i in lane i / E, slot i % E, so that strides below E stay in
+// the lane.
+template <int E>
+__device__ __forceinline__ void sort_desc(unsigned long long* __restrict__ v, uint32_t m, uint32_t lane) {
+    unsigned long long x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const uint32_t i = (uint32_t)e * 32u + lane;
+        x[e] = i < m ? v[i] : 0ull;
+    }
+    __syncwarp();
+    // every lane's slots, alternate lanes in opposite order
+#pragma unroll
+    for (int k = 2; k <= E; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if (!(e & j)) order2(x[e], x[e | j], k == E ? (lane & 1) == 0 : (e & k) == 0);
+    // merges of 2, 4, .. 32 lanes
+#pragma unroll 1
+    for (uint32_t k = 2; k <= 32; k <<= 1) {
+        const bool up = (lane & k) == 0;
+#pragma unroll 1
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            const bool large = ((lane & j) == 0) == up;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const unsigned long long o = __shfl_xor_sync(0xffffffffu, x[e], (int)j);
+                x[e] = (o > x[e]) == large ? o : x[e];
+            }
+        }
+#pragma unroll
+        for (int j = E >> 1; j > 0; j >>= 1)
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if (!(e & j)) order2(x[e], x[e | j], up);
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[lane * E + e] = x[e];
+    __syncwarp();
+}
+
+// A row of at most 32 * R entries in registers.  A value is the score's bits
+// above the row's smallest, plus one (53 bits), then the entry's slot (10) and
+// whether the row emits it (1): distinct, and ordered like the scores.  Returns
+// the number of edges, or ~0 where this form does not do: scores that span 53
+// bits, or equal scores whose order the columns decide.
+template <int R, int EMAX>
+__device__ __forceinline__ uint32_t topk_regs(uint32_t cnt, uint32_t orow, uint32_t max_edges, Ent* __restrict__ row,
+                                              unsigned long long* __restrict__ buf, uint32_t* __restrict__ col,
+                                              uint32_t* __restrict__ hist, uint32_t lane) {
+    unsigned long long x[R];
+    uint32_t emit = 0;
+    unsigned long long lo = ~0ull, hi = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = (uint32_t)r * 32u + lane;
+        x[r] = 0;
+        if (i < cnt) {
+            const Ent t = row[i];
+            x[r] = (unsigned long long)__double_as_longlong(t.sim);
+            col[i] = t.ocol;
+            emit |= (uint32_t)(t.ocol > orow) << r;
+            lo = x[r] < lo ? x[r] : lo;
+            hi = x[r] > hi ? x[r] : hi;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long l2 = __shfl_xor_sync(0xffffffffu, lo, o), h2 = __shfl_xor_sync(0xffffffffu, hi, o);
+        lo = l2 < lo ? l2 : lo;
+        hi = h2 > hi ? h2 : hi;
+    }
+    if (hi - lo >= (1ull << 53) - 2) return ~0u;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t i = (uint32_t)r * 32u + lane;
+        if (i < cnt) x[r] = (x[r] - lo + 1) << 11 | i << 1 | (emit >> r & 1u);
+    }
+    // the max_edges-th largest value: histograms of 8 bits from the top of the
+    // row's range down, until the bin has at most 32 values
+    unsigned long long T = 1;
+    if (cnt > max_edges) {
+        uint32_t need = max_edges;
+        int shift = 64 - __clzll((long long)((hi - lo + 2) << 11)) - 8;  // at least 5
+        int width = 8;
+        unsigned long long pre = 0;
+        uint32_t count;
+        while (true) {
+            sel_clear(hist, lane);
+            const uint32_t mask = (1u << width) - 1u;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (x[r] && (x[r] >> shift) >> width == pre) atomicAdd(&hist[(uint32_t)(x[r] >> shift) & mask], 1u);
+            __syncwarp();
+            uint32_t bin, above;
+            sel_bin(hist, lane, need, bin, above, count);
+            __syncwarp();
+            need -= above;
+            pre = pre << width | bin;
+            if (count <= 32 || shift == 0) break;
+            width = shift < 8 ? shift : 8;
+            shift -= width;
+        }
+        // the bin's values, one a lane; the need-th largest of them
+        uint32_t c = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool in = x[r] && x[r] >> shift == pre;
+            const uint32_t bal = __ballot_sync(0xffffffffu, in);
+            if (in) buf[c + __popc(bal & ((1u << lane) - 1u))] = x[r];
+            c += __popc(bal);
+        }
+        __syncwarp();
+        const unsigned long long mine = lane < c ? buf[lane] : 0ull;
+        uint32_t rank = 0;
+        for (uint32_t k = 0; k < c; ++k) rank += buf[k] > mine;
+        __syncwarp();
+        T = __shfl_sync(0xffffffffu, mine, __ffs(__ballot_sync(0xffffffffu, lane < c && rank + 1 == need)) - 1);
+        // an entry left out with the score of the last one kept
+        bool tie = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) tie |= x[r] < T && x[r] >> 11 == T >> 11;
+        if (__any_sync(0xffffffffu, tie)) return ~0u;
+    }
+    uint32_t m = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const bool take = x[r] >= T && (x[r] & 1);
+        const uint32_t bal = __ballot_sync(0xffffffffu, take);
+        if (take) buf[m + __popc(bal & ((1u << lane) - 1u))] = x[r];
+        m += __popc(bal);
+    }
+    __syncwarp();
+    if (m <= 32)
+        sort_desc<1>(buf, m, lane);
+    else if (m <= 64)
+        sort_desc<2>(buf, m, lane);
+    else if (m <= 128)
+        sort_desc<4>(buf, m, lane);
+    else if (EMAX == 8 || m <= 256)
+        sort_desc<8>(buf, m, lane);
+    else
+        sort_desc<EMAX>(buf, m, lane);
+    bool tie = false;
+    for (uint32_t i = lane; i + 1 < m; i += 32) tie |= buf[i] >> 11 == buf[i + 1] >> 11;
+    if (__any_sync(0xffffffffu, tie)) return ~0u;
+    for (uint32_t i = lane; i < m; i += 32) {
+        const unsigned long long v = buf[i];
+        Ent e;
+        e.sim = __longlong_as_double((long long)((v >> 11) - 1 + lo));
+        e.ocol = col[(uint32_t)(v >> 1) & 1023u];
+        e.pad = 0;
+        row[i] = e;
+    }
+    return m;
+}
+
+// Bound by instruction issue (the entries are read once): a row of up to 512
+// entries stays in registers as one 64-bit value per entry, about 2,000
+// instructions a row where 96-bit keys staged in shared memory took 5,250 at
+// 15 % occupancy (48 assemblies of 400 to 6,000: 1,098 -> 613 us; 1,500 contigs,
+// limit 200: 27 -> 16 us).  Seven blocks an SM need 72 registers, the most that
+// spill nothing; the form for limits above 256 would spill at more than four.
+template <int EMAX>
+__global__ void __launch_bounds__(kSelWarps * 32, EMAX == 8 ? 7 : 4) k_topk_sel(const unsigned long long* __restrict__ rowptr,
                                                              const uint32_t* __restrict__ deg,
                                                              const uint32_t* __restrict__ perm, uint32_t n,
                                                              uint32_t max_edges_all, const uint32_t* __restrict__ blk_K,
                                                              Ent* __restrict__ list, uint32_t* __restrict__ out_cnt) {
-    __shared__ unsigned long long s_key[kSelWarps][kSelCap];
-    __shared__ uint32_t s_col[kSelWarps][kSelCap];
-    __shared__ uint32_t s_hist[kSelWarps][256];
+    __shared__ unsigned long long s_buf[kSelWarps][32 * EMAX];
+    __shared__ uint32_t s_col[kSelWarps][kRowRegs];
+    __shared__ __align__(16) uint32_t s_hist[kSelWarps][256];
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned long long* key = s_key[w];
-    uint32_t* col = s_col[w];
-    uint32_t* hist = s_hist[w];
     for (uint32_t sp = blockIdx.x * kSelWarps + w; sp < n; sp += gridDim.x * kSelWarps) {
         const uint32_t cnt = deg[sp], orow = perm[sp];
         const uint32_t max_edges = blk_K ? blk_K[sp >> 8] : max_edges_all;
         Ent* row = list + rowptr[sp];
-        const bool staged = cnt <= kSelCap;
-        if (staged)
-            for (uint32_t i = lane; i < cnt; i += 32) {
-                const Ent x = row[i];
-                key[i] = (unsigned long long)__double_as_longlong(x.sim);
-                col[i] = x.ocol;
-            }
+        uint32_t m = cnt ? ~0u : 0u;
+        if (cnt && cnt <= 256)
+            m = topk_regs<8, EMAX>(cnt, orow, max_edges, row, s_buf[w], s_col[w], s_hist[w], lane);
+        else if (cnt && cnt <= kRowRegs)
+            m = topk_regs<16, EMAX>(cnt, orow, max_edges, row, s_buf[w], s_col[w], s_hist[w], lane);
         __syncwarp();
-        // threshold key (P_hi, P_lo): kept iff key >= it
-        unsigned long long P_hi = 0;
-        uint32_t P_lo = 0;
-        if (cnt > max_edges) {
-            uint32_t need = max_edges;
-            for (int p = 0; p < 12; ++p) {
-#pragma unroll
-                for (int t = 0; t < 8; ++t) hist[lane * 8 + t] = 0;
-                __syncwarp();
-                for (uint32_t i = lane; i < cnt; i += 32) {
-                    unsigned long long hi;
-                    uint32_t c;
-                    if (staged) {
-                        hi = key[i];
-                        c = col[i];
-                    } else {
-                        const Ent x = row[i];
-                        hi = (unsigned long long)__double_as_longlong(x.sim);
-                        c = x.ocol;
-                    }
-                    const uint32_t lo = ~c;
-                    if (sel_match(hi, lo, P_hi, P_lo, p)) atomicAdd(&hist[sel_digit(hi, lo, p)], 1u);
-                }
-                __syncwarp();
-                // lane L owns bins [8L, 8L + 8); count the bins above each lane's
-                uint32_t b[8], own = 0;
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    b[t] = hist[lane * 8 + t];
-                    own += b[t];
-                }
-                uint32_t suf = own;  // inclusive sum over lanes >= lane
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t v = __shfl_down_sync(0xffffffffu, suf, o);
-                    if (lane + o < 32) suf += v;
-                }
-                uint32_t above = suf - own;
-                int bin = -1;
-                uint32_t bin_above = 0, bin_cnt = 0;
-                if (above < need && need <= suf) {
-#pragma unroll
-                    for (int t = 7; t >= 0; --t) {
-                        if (bin < 0 && above + b[t] >= need) {
-                            bin = (int)(lane * 8 + t);
-                            bin_above = above;
-                            bin_cnt = b[t];
-                        }
-                        if (bin < 0) above += b[t];
-                    }
-                }
-                const uint32_t who = __ffs(__ballot_sync(0xffffffffu, bin >= 0)) - 1;
-                bin = __shfl_sync(0xffffffffu, bin, who);
-                bin_above = __shfl_sync(0xffffffffu, bin_above, who);
-                bin_cnt = __shfl_sync(0xffffffffu, bin_cnt, who);
-                need -= bin_above;
-                if (p < 8)
-                    P_hi |= (unsigned long long)bin << (56 - 8 * p);
-                else
-                    P_lo |= (uint32_t)bin << (24 - 8 * (p - 8));
-                if (bin_cnt == need) break;
-            }
-        }
-        // compact the kept entries with ocol > orow to the front of the buffer
-        uint32_t m = 0;
-        const uint32_t cap = max_edges;
-        for (uint32_t base = 0; base < cnt; base += 32) {
-            const uint32_t i = base + lane;
-            unsigned long long hi = 0;
-            uint32_t c = 0;
-            bool take = false;
-            if (i < cnt) {
-                if (staged) {
-                    hi = key[i];
-                    c = col[i];
-                } else {
-                    const Ent x = row[i];
-                    hi = (unsigned long long)__double_as_longlong(x.sim);
-                    c = x.ocol;
-                }
-                const uint32_t lo = ~c;
-                take = c > orow && (hi > P_hi || (hi == P_hi && lo >= P_lo));
-            }
-            const uint32_t bal = __ballot_sync(0xffffffffu, take);
-            __syncwarp();  // every lane has read its entry before any slot is rewritten
-            const uint32_t q = m + __popc(bal & ((1u << lane) - 1u));
-            if (take && q < cap) {
-                key[q] = hi;
-                col[q] = c;
-            }
-            m += __popc(bal);
-            __syncwarp();
-        }
-        m = min(m, cap);
-        if (m <= 64)
-            sort_out<2>(key, col, m, lane, row);
-        else if (m <= 128)
-            sort_out<4>(key, col, m, lane, row);
-        else
-            sort_out<EMAX>(key, col, m, lane, row);
+        if (m == ~0u) m = topk_any<EMAX>(cnt, orow, max_edges, row, s_buf[w], s_col[w], s_hist[w], lane);
         if (lane == 0) out_cnt[orow] = m;
         __syncwarp();
     }
