@@ -350,8 +350,6 @@ __global__ void __launch_bounds__(1024) k_topk_big(const uint32_t* __restrict__ 
 }
 
 // ---- selection top-k: warp per contig --------------------------------------
-// topk_regs holds rows of up to 512 entries in registers; topk_any takes the rest:
-//
 // A row's kept set is its max_edges best entries under (sim descending, ocol
 // ascending).  Ordered as the 96-bit key (bits of sim, ~ocol) -- sim is a
 // positive double, so its bits order like its value -- the kept set is every
@@ -443,7 +441,7 @@ __device__ __forceinline__ void sort_out(const unsigned long long* __restrict__ 
 }
 
 constexpr int kSelWarps = 4;
-constexpr uint32_t kRowRegs = 512;  // entries of a row held in registers, 16 a lane
+constexpr uint32_t kRowCap = 512;  // entries of a row staged in shared memory (28 KB a block)
 
 __device__ __forceinline__ uint32_t sel_digit(unsigned long long hi, uint32_t lo, int p) {
     return p < 8 ? (uint32_t)(hi >> (56 - 8 * p)) & 255u : (lo >> (24 - 8 * (p - 8))) & 255u;
@@ -616,60 +614,51 @@ __device__ __forceinline__ void sort_desc(unsigned long long* __restrict__ v, ui
     __syncwarp();
 }
 
-// A row of at most 32 * R entries in registers.  A value is the score's bits
-// above the row's smallest, plus one (53 bits), then the entry's slot (10) and
-// whether the row emits it (1): distinct, and ordered like the scores.  Returns
-// the number of edges, or ~0 where this form does not do: scores that span 53
-// bits, or equal scores whose order the columns decide.
-template <int R, int EMAX>
-__device__ __forceinline__ uint32_t topk_regs(uint32_t cnt, uint32_t orow, uint32_t max_edges, Ent* __restrict__ row,
-                                              unsigned long long* __restrict__ buf, uint32_t* __restrict__ col,
-                                              uint32_t* __restrict__ hist, uint32_t lane) {
-    unsigned long long x[R];
-    uint32_t emit = 0;
+// A row of at most kRowCap entries.  A value is the score's bits above the
+// row's smallest, plus one (53 bits), then the entry's slot (10) and whether the
+// row emits it (1): distinct, and ordered like the scores.  Returns the number
+// of edges, or ~0 where this form does not do: scores that span 53 bits, or
+// equal scores whose order the columns decide.
+template <int EMAX>
+__device__ __forceinline__ uint32_t topk_row(uint32_t cnt, uint32_t orow, uint32_t max_edges, Ent* __restrict__ row,
+                                             unsigned long long* __restrict__ x, uint32_t* __restrict__ col,
+                                             uint32_t* __restrict__ hist, uint32_t lane) {
     unsigned long long lo = ~0ull, hi = 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const uint32_t i = (uint32_t)r * 32u + lane;
-        x[r] = 0;
-        if (i < cnt) {
-            const Ent t = row[i];
-            x[r] = (unsigned long long)__double_as_longlong(t.sim);
-            col[i] = t.ocol;
-            emit |= (uint32_t)(t.ocol > orow) << r;
-            lo = x[r] < lo ? x[r] : lo;
-            hi = x[r] > hi ? x[r] : hi;
-        }
+#pragma unroll 4
+    for (uint32_t i = lane; i < cnt; i += 32) {
+        const Ent t = row[i];
+        const unsigned long long v = (unsigned long long)__double_as_longlong(t.sim);
+        x[i] = v;
+        col[i] = t.ocol;
+        lo = v < lo ? v : lo;
+        hi = v > hi ? v : hi;
     }
-#pragma unroll
+#pragma unroll 1
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long l2 = __shfl_xor_sync(0xffffffffu, lo, o), h2 = __shfl_xor_sync(0xffffffffu, hi, o);
         lo = l2 < lo ? l2 : lo;
         hi = h2 > hi ? h2 : hi;
     }
     if (hi - lo >= (1ull << 53) - 2) return ~0u;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const uint32_t i = (uint32_t)r * 32u + lane;
-        if (i < cnt) x[r] = (x[r] - lo + 1) << 11 | i << 1 | (emit >> r & 1u);
-    }
     // the max_edges-th largest value: histograms of 8 bits from the top of the
     // row's range down, until the bin has at most 32 values
+    const bool select = cnt > max_edges;
+    int shift = 64 - __clzll((long long)((hi - lo + 2) << 11)) - 8;  // at least 5
+    if (select) sel_clear(hist, lane);
+#pragma unroll 2
+    for (uint32_t i = lane; i < cnt; i += 32) {
+        const unsigned long long v = (x[i] - lo + 1) << 11 | i << 1 | (col[i] > orow ? 1u : 0u);
+        x[i] = v;
+        if (select) atomicAdd(&hist[(uint32_t)(v >> shift)], 1u);
+    }
     unsigned long long T = 1;
-    if (cnt > max_edges) {
-        uint32_t need = max_edges;
-        int shift = 64 - __clzll((long long)((hi - lo + 2) << 11)) - 8;  // at least 5
-        int width = 8;
+    if (select) {
+        uint32_t need = max_edges, bin, above, count;
         unsigned long long pre = 0;
-        uint32_t count;
+        int width = 8;
+#pragma unroll 1
         while (true) {
-            sel_clear(hist, lane);
-            const uint32_t mask = (1u << width) - 1u;
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (x[r] && (x[r] >> shift) >> width == pre) atomicAdd(&hist[(uint32_t)(x[r] >> shift) & mask], 1u);
             __syncwarp();
-            uint32_t bin, above;
             sel_bin(hist, lane, need, bin, above, count);
             __syncwarp();
             need -= above;
@@ -677,52 +666,57 @@ __device__ __forceinline__ uint32_t topk_regs(uint32_t cnt, uint32_t orow, uint3
             if (count <= 32 || shift == 0) break;
             width = shift < 8 ? shift : 8;
             shift -= width;
+            sel_clear(hist, lane);
+            for (uint32_t i = lane; i < cnt; i += 32) {
+                const unsigned long long v = x[i] >> shift;
+                if (v >> width == pre) atomicAdd(&hist[(uint32_t)v & ((1u << width) - 1u)], 1u);
+            }
         }
-        // the bin's values, one a lane; the need-th largest of them
+        // the bin's values, one a lane (in the histogram's place); the need-th largest
+        unsigned long long* few = reinterpret_cast<unsigned long long*>(hist);
         uint32_t c = 0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const bool in = x[r] && x[r] >> shift == pre;
+        for (uint32_t base = 0; base < cnt; base += 32) {
+            const unsigned long long v = base + lane < cnt ? x[base + lane] : 0ull;
+            const bool in = v && v >> shift == pre;
             const uint32_t bal = __ballot_sync(0xffffffffu, in);
-            if (in) buf[c + __popc(bal & ((1u << lane) - 1u))] = x[r];
+            if (in) few[c + __popc(bal & ((1u << lane) - 1u))] = v;
             c += __popc(bal);
         }
         __syncwarp();
-        const unsigned long long mine = lane < c ? buf[lane] : 0ull;
+        const unsigned long long mine = lane < c ? few[lane] : 0ull;
         uint32_t rank = 0;
-        for (uint32_t k = 0; k < c; ++k) rank += buf[k] > mine;
-        __syncwarp();
+#pragma unroll 1
+        for (uint32_t k = 0; k < c; ++k) rank += few[k] > mine;
         T = __shfl_sync(0xffffffffu, mine, __ffs(__ballot_sync(0xffffffffu, lane < c && rank + 1 == need)) - 1);
-        // an entry left out with the score of the last one kept
-        bool tie = false;
-#pragma unroll
-        for (int r = 0; r < R; ++r) tie |= x[r] < T && x[r] >> 11 == T >> 11;
-        if (__any_sync(0xffffffffu, tie)) return ~0u;
     }
+    // the values to emit to the front; an entry left out with the score of the
+    // last one kept is a tie
     uint32_t m = 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const bool take = x[r] >= T && (x[r] & 1);
-        const uint32_t bal = __ballot_sync(0xffffffffu, take);
-        if (take) buf[m + __popc(bal & ((1u << lane) - 1u))] = x[r];
+    bool tie = false;
+    __syncwarp();
+    for (uint32_t base = 0; base < cnt; base += 32) {
+        const unsigned long long v = base + lane < cnt ? x[base + lane] : 0ull;
+        const bool take = v >= T && (v & 1);
+        tie |= v && v < T && v >> 11 == T >> 11;
+        const uint32_t bal = __ballot_sync(0xffffffffu, take);  // every lane has read its value
+        if (take) x[m + __popc(bal & ((1u << lane) - 1u))] = v;
         m += __popc(bal);
     }
+    if (__any_sync(0xffffffffu, tie)) return ~0u;
     __syncwarp();
-    if (m <= 32)
-        sort_desc<1>(buf, m, lane);
-    else if (m <= 64)
-        sort_desc<2>(buf, m, lane);
+    if (m <= 64)
+        sort_desc<2>(x, m, lane);
     else if (m <= 128)
-        sort_desc<4>(buf, m, lane);
+        sort_desc<4>(x, m, lane);
     else if (EMAX == 8 || m <= 256)
-        sort_desc<8>(buf, m, lane);
+        sort_desc<8>(x, m, lane);
     else
-        sort_desc<EMAX>(buf, m, lane);
-    bool tie = false;
-    for (uint32_t i = lane; i + 1 < m; i += 32) tie |= buf[i] >> 11 == buf[i + 1] >> 11;
+        sort_desc<EMAX>(x, m, lane);
+    tie = false;
+    for (uint32_t i = lane; i + 1 < m; i += 32) tie |= x[i] >> 11 == x[i + 1] >> 11;
     if (__any_sync(0xffffffffu, tie)) return ~0u;
     for (uint32_t i = lane; i < m; i += 32) {
-        const unsigned long long v = buf[i];
+        const unsigned long long v = x[i];
         Ent e;
         e.sim = __longlong_as_double((long long)((v >> 11) - 1 + lo));
         e.ocol = col[(uint32_t)(v >> 1) & 1023u];
@@ -732,20 +726,21 @@ __device__ __forceinline__ uint32_t topk_regs(uint32_t cnt, uint32_t orow, uint3
     return m;
 }
 
-// Bound by instruction issue (the entries are read once): a row of up to 512
-// entries stays in registers as one 64-bit value per entry, about 2,000
-// instructions a row where 96-bit keys staged in shared memory took 5,250 at
-// 15 % occupancy (48 assemblies of 400 to 6,000: 1,098 -> 613 us; 1,500 contigs,
-// limit 200: 27 -> 16 us).  Seven blocks an SM need 72 registers, the most that
-// spill nothing; the form for limits above 256 would spill at more than four.
+// Bound by issue (the entries are read once, about 2,000 instructions a row): one
+// 64-bit value per entry, staged in shared memory so that the passes are short
+// loops.  Held in registers, the unrolled passes outgrew the instruction cache:
+// 48 assemblies of 400 to 6,000 contigs 613 us, 1,000,000 contigs 10.0 ms, with
+// this form 324 us and 5.9 ms (96-bit keys and twelve digit passes: 1,098 us and
+// 9.9 ms).  Seven blocks fit an SM's shared memory; 72 registers for them beat
+// 113 at four blocks (382 us, 6.8 ms).
 template <int EMAX>
 __global__ void __launch_bounds__(kSelWarps * 32, EMAX == 8 ? 7 : 4) k_topk_sel(const unsigned long long* __restrict__ rowptr,
                                                              const uint32_t* __restrict__ deg,
                                                              const uint32_t* __restrict__ perm, uint32_t n,
                                                              uint32_t max_edges_all, const uint32_t* __restrict__ blk_K,
                                                              Ent* __restrict__ list, uint32_t* __restrict__ out_cnt) {
-    __shared__ unsigned long long s_buf[kSelWarps][32 * EMAX];
-    __shared__ uint32_t s_col[kSelWarps][kRowRegs];
+    __shared__ unsigned long long s_x[kSelWarps][kRowCap];
+    __shared__ uint32_t s_col[kSelWarps][kRowCap];
     __shared__ __align__(16) uint32_t s_hist[kSelWarps][256];
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (uint32_t sp = blockIdx.x * kSelWarps + w; sp < n; sp += gridDim.x * kSelWarps) {
@@ -753,12 +748,10 @@ __global__ void __launch_bounds__(kSelWarps * 32, EMAX == 8 ? 7 : 4) k_topk_sel(
         const uint32_t max_edges = blk_K ? blk_K[sp >> 8] : max_edges_all;
         Ent* row = list + rowptr[sp];
         uint32_t m = cnt ? ~0u : 0u;
-        if (cnt && cnt <= 256)
-            m = topk_regs<8, EMAX>(cnt, orow, max_edges, row, s_buf[w], s_col[w], s_hist[w], lane);
-        else if (cnt && cnt <= kRowRegs)
-            m = topk_regs<16, EMAX>(cnt, orow, max_edges, row, s_buf[w], s_col[w], s_hist[w], lane);
+        if (cnt && cnt <= kRowCap)
+            m = topk_row<EMAX>(cnt, orow, max_edges, row, s_x[w], s_col[w], s_hist[w], lane);
         __syncwarp();
-        if (m == ~0u) m = topk_any<EMAX>(cnt, orow, max_edges, row, s_buf[w], s_col[w], s_hist[w], lane);
+        if (m == ~0u) m = topk_any<EMAX>(cnt, orow, max_edges, row, s_x[w], s_col[w], s_hist[w], lane);
         if (lane == 0) out_cnt[orow] = m;
         __syncwarp();
     }
