@@ -451,7 +451,6 @@ __device__ __forceinline__ void lp_enqueue(uint32_t w, uint32_t deg, uint32_t* n
     const uint32_t lane = threadIdx.x & 31, all = __activemask();
     const uint32_t most = __reduce_max_sync(all, deg);
     const uint32_t small = __ballot_sync(all, deg <= kWarpCap), big = all & ~small;
-    if (lane == __ffs(all) - 1) atomicMax(&info->maxall, most);
     if (deg <= kWarpCap) {
         uint32_t at = 0;
         if (lane == __ffs(small) - 1) at = atomicAdd(&info->nsmall, (unsigned)__popc(small));
@@ -499,9 +498,16 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_levels(LevelArgs A) {
     const uint32_t g0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const uint32_t gmask = 0xFFu << (threadIdx.x & 24);
     unsigned int target = 0;
+    // the largest degree: one atomic a block (one per joining contig and level
+    // was half of the atomics on a level's counters)
+    __shared__ uint32_t bmax;
+    if (threadIdx.x == 0) bmax = 0;
+    __syncthreads();
+    uint32_t most = 0;
     for (uint32_t pu = g0; pu < A.norder; pu += ng) {
         const uint32_t u = A.order[pu];
         const uint32_t s = A.inc_off[u], d = A.inc_off[u + 1] - s;
+        most = max(most, d);
         uint32_t c = 0;
         for (uint32_t j = sub; j < d; j += 8) c += A.pos_of[A.oth[s + j]] < pu;
 #pragma unroll
@@ -511,6 +517,11 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_levels(LevelArgs A) {
             if (c == 0) lp_enqueue(u, d, A.lvl, A.lvls, A.info, A.slot_of);
         }
     }
+    __syncwarp();
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0) atomicMax(&bmax, most);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(&A.info[0].maxall, bmax);
     uint32_t off = 0, soff = 0, done = 0, L = 0, maxdeg = 0, maxall = 0, maxbig = 0;
     for (;; ++L) {
         if (!grid_barrier(A.bar, target, A.flag)) return;
@@ -1039,13 +1050,13 @@ int lp_impl(mdet_ctx* ctx, const uint64_t* d_from, const uint64_t* d_to, const d
     S.ea = (uint32_t*)ctx_scratch(ctx, "lp.ea", ne1 * 4);
     S.eb = (uint32_t*)ctx_scratch(ctx, "lp.eb", ne1 * 4);
     S.lw = (double*)ctx_scratch(ctx, "lp.lw", ne1 * 8);
-    // edges traversed per pass: a stretch starts with about as many as n
-    // contigs need and takes four times as many each time it goes on (the first
+    // edges traversed per pass: a stretch starts with about n (n / 4 meant two
+    // passes a stretch: 8.0 -> 7.4 ms at 1,000,000 contigs) and takes four times as many each time it goes on (the first
     // stretches end within the first edges; passes of 4M edges from the start
     // took 1.0 of 6.5 ms at 60,000 contigs and 2.9M edges)
     const uint64_t kChunk = std::min<uint64_t>(ne1, 1ull << 22);
     uint64_t chunk0 = 1ull << 16;
-    while (chunk0 < n / 4 && chunk0 < kChunk) chunk0 <<= 1;
+    while (chunk0 < n && chunk0 < kChunk) chunk0 <<= 1;
     uint8_t* slot = (uint8_t*)ctx_scratch(ctx, "lp.slot", 2 * kChunk);
     uint32_t* ssel = (uint32_t*)ctx_scratch(ctx, "lp.ssel", 2 * kChunk * 4);
     uint32_t* sel = (uint32_t*)ctx_scratch(ctx, "lp.sel", kChunk * 4);
