@@ -426,7 +426,10 @@ __global__ void k_abd_score(ScoreArgs p) {
 // keys afterwards (k_fix_runs).  Runs longer than kFixRun whose full keys
 // differ -- values crowded within 2^-32 of the range -- raise a flag, and the call
 // sorts the full keys instead.  (3.8M edges: 1,093 us for the three full sorts
-// and their ranks, 898 us so.)
+// and their ranks, 898 us so.)  More edges crowd the runs: 90,000 contigs (limit 100)
+// 1,904 -> 1,622 us, 200,000 3,689 -> 3,767, 400,000 7,667 -> 9,584, and 80M edges
+// overflow, so beyond kTopBitsMost the full keys are sorted at once.
+constexpr uint64_t kTopBitsMost = 1ull << 23;
 constexpr uint32_t kFixRun = 48;
 
 struct KeyRange {
@@ -705,7 +708,7 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
         return MDET_OK;
     };
     unsigned long long h_bad[2] = {0, 0};
-    for (int full = 0; full < 2; ++full) {
+    for (int full = ne > kTopBitsMost; full < 2; ++full) {
         ctx_timer_begin(ctx, "abd_ranks");
         MDET_TRY(full ? by_full_keys() : by_top_bits());
         ctx_timer_end(ctx, "abd_ranks");
