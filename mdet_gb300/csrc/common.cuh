@@ -71,7 +71,7 @@ struct mdet_ctx {
     uint64_t graph_replays = 0;
     void* batch_plan = nullptr;
     void (*batch_plan_free)(void*) = nullptr;
-    // The last size-sorted preparation ("pre" buffers): which inputs it was
+    // The last single-set preparation ("pre" buffers): which inputs it was
     // made from (pointers, n, BF16 part, a hash of their contents) and which
     // buffers hold it.  Counting invalidates it (new TNF rows).
     struct PrepCache {

@@ -13,7 +13,7 @@ constexpr int kShapeTf32 = 2128;  // filter_tc shape code of 128 x 128 TF32 tile
 #define MDET_TBL_LEVELS 9 // sparse-table levels (2^8 = 256)
 #define MDET_BLK 128      // rows per metadata block
 
-// Per 128-row block of the length-sorted order.
+// Per 128-row block of the prepared order.
 struct BlockMeta {
     float lo, hi;  // log10 size range
     float emax;    // max rounding error ||x~ - x|| of the block's reduced-precision rows

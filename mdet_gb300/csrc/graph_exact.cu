@@ -354,11 +354,11 @@ __global__ void __launch_bounds__(1024) k_topk_big(const uint32_t* __restrict__ 
 // ascending).  Ordered as the 96-bit key (bits of sim, ~ocol) -- sim is a
 // positive double, so its bits order like its value -- the kept set is every
 // entry whose key is >= the max_edges-th largest key, found by a radix
-// select (8-bit digits, most significant first, stopping as soon as the
-// digit's bin holds exactly the entries still needed).  Only kept entries
-// with ocol above the row's own index are emitted, so only those are sorted
-// (bitonic network in registers: entry i of a chunk of 32*E in lane i % 32,
-// slot i / 32) and written to the front of the row.
+// select (8-bit digits, most significant first).  Only kept entries with ocol
+// above the row's own index are emitted, so only those are sorted (bitonic
+// network in registers) and written to the front of the row.  topk_row does
+// this on 64-bit values, where a row's scores differ; topk_any, on the full
+// keys, takes any row.
 
 // Keys are the bit patterns of positive doubles, which order like the
 // values, so every comparison is an integer one (FP64 is slow on this part).
