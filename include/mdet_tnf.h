@@ -310,7 +310,7 @@ int mdet_ctx_set_abundance(mdet_ctx* ctx, const double* abd, const double* abd_v
  * depth correlations, and so their ranks, are the reference's FP64 values
  * bit for bit; the similarities and the final sSCR are within 1e-12
  * (absolute or relative) of an FP64 evaluation (float-float normal CDFs,
- * crossing points and powers). */
+ * crossing points and powers).  sscr may be stnf (in place). */
 int mdet_edges_sscr(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const double* stnf,
                     uint64_t n_edges, double min_cv, uint32_t min_sample, double* sscr);
 int mdet_edges_sscr_dev(mdet_ctx* ctx, const uint64_t* d_from, const uint64_t* d_to,

@@ -424,8 +424,8 @@ __global__ void k_abd_score(ScoreArgs p) {
 // top 32 bits of the keys' offsets from their minimum (four passes over 8
 // bytes); the few runs of equal 32-bit keys are put in order by their full
 // keys afterwards (k_fix_runs).  Runs longer than kFixRun whose full keys
-// differ -- values crowded within 2^-32 of the range -- raise a flag, and the call
-// sorts the full keys instead.  (3.8M edges: 1,093 us for the three full sorts
+// differ -- values crowded within 2^-32 of the range -- raise a flag, and those
+// values are sorted by their full keys instead, before any score is written.  (3.8M edges: 1,093 us for the three full sorts
 // and their ranks, 898 us so.)  More edges crowd the runs: 90,000 contigs (limit 100)
 // 1,904 -> 1,622 us, 200,000 3,689 -> 3,767, 400,000 7,667 -> 9,584, and 80M edges
 // overflow, so beyond kTopBitsMost the full keys are sorted at once.
@@ -556,9 +556,13 @@ __global__ void k_run_ranks(const uint32_t* __restrict__ order, const uint32_t* 
 // good to ~1e-14, so sSCR is within ~1e-13 relative of the reference's FP64
 // pows (the values lie in [1e-6, 1]: every similarity term is at least
 // 1e-6).  The three FP64 pows cost ~250 FP64 operations an edge.
+// overflow: with any of the three counts set the ranks do not stand, and
+// nothing is written: out may be the sTNF values, which are then ranked again.
 __global__ void k_sscr(const double* __restrict__ raw, const uint32_t* __restrict__ nnz,
                        const uint32_t* __restrict__ rt, const uint32_t* __restrict__ rc,
-                       const double* __restrict__ distr, uint64_t ne, bool corr, double* __restrict__ out) {
+                       const double* __restrict__ distr, uint64_t ne, bool corr,
+                       const unsigned long long* __restrict__ overflow, double* __restrict__ out) {
+    if (overflow && (overflow[0] | overflow[1] | overflow[2])) return;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < ne; e += (uint64_t)gridDim.x * blockDim.x) {
         const ff t = ff_from_double(distr[rt[e] - 1]);
         const ff w = ff_recip(ff_make((float)(1 + nnz[e]), 0.f));
@@ -624,8 +628,9 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     uint32_t* rt = (uint32_t*)ctx_scratch(ctx, "abd.rt", ne * 4);
     uint32_t* rc = (uint32_t*)ctx_scratch(ctx, "abd.rc", ne * 4);
     double* distr = (double*)ctx_scratch(ctx, "abd.distr", ne * 8);
-    // [0] bad edges, [1] runs too long to fix, then the three key ranges
-    unsigned long long* bad = (unsigned long long*)ctx_scratch(ctx, "abd.bad", 16 + 3 * sizeof(KeyRange));
+    // [0] bad edges, [1 ..] runs too long to fix in each array of values, [4 ..] the key ranges
+    const size_t bad_bytes = 32 + 3 * sizeof(KeyRange);
+    unsigned long long* bad = (unsigned long long*)ctx_scratch(ctx, "abd.bad", bad_bytes);
     uint32_t* k32 = (uint32_t*)ctx_scratch(ctx, "abd.k32", ne * 12);
     uint32_t* k32s = (uint32_t*)ctx_scratch(ctx, "abd.k32s", ne * 4);
     if (!k32 || !k32s) return MDET_ERR_NOMEM;
@@ -642,7 +647,7 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     const size_t tmpb = std::max(std::max(std::max(t1, t2), std::max(t3, t4)), std::max(t5, t6));
     void* tmp = ctx_scratch(ctx, "abd.cubtmp", tmpb);
     if (!tmp) return MDET_ERR_NOMEM;
-    MDET_CUDA(ctx, cudaMemsetAsync(bad, 0, 16 + 3 * sizeof(KeyRange), s));
+    MDET_CUDA(ctx, cudaMemsetAsync(bad, 0, bad_bytes, s));
 
     ScoreArgs p;
     p.from = from;
@@ -674,29 +679,34 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     // the abundance similarities in ascending order (partial_sort_copy), the
     // ranks of sTNF and of the correlations, then the scores
     const unsigned g = grid_for(ctx, ne, 256);
-    auto by_full_keys = [&]() -> int {
+    const int arrays = corr ? 3 : 2;
+    // array k of the values by its full keys
+    auto by_full_keys = [&](int k) -> int {
         size_t tb = tmpb;
-        MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, tb, raw, distr, (int)ne, 0, 64, s));
-        MDET_TRY(rank_runs(ctx, stnf, idx, ne, false, ks, os, head, start, rt, tmp, tmpb));
-        if (corr) MDET_TRY(rank_runs(ctx, cor, idx, ne, true, ks, os, head, start, rc, tmp, tmpb));
+        if (k == 0)
+            MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, tb, raw, distr, (int)ne, 0, 64, s));
+        else if (k == 1)
+            MDET_TRY(rank_runs(ctx, stnf, idx, ne, false, ks, os, head, start, rt, tmp, tmpb));
+        else
+            MDET_TRY(rank_runs(ctx, cor, idx, ne, true, ks, os, head, start, rc, tmp, tmpb));
         return MDET_OK;
     };
     auto by_top_bits = [&]() -> int {
         const RankArrays A{{raw, stnf, cor}, {k32, k32 + ne, k32 + 2 * ne}};
-        KeyRange* range = (KeyRange*)(bad + 2);
-        const dim3 g3(g, corr ? 3 : 2), gr(std::min<unsigned>(g, ctx->num_sms * 4), g3.y);
+        KeyRange* range = (KeyRange*)(bad + 4);
+        const dim3 g3(g, arrays), gr(std::min<unsigned>(g, ctx->num_sms * 4), arrays);
         k_key_range<<<gr, 256, 0, s>>>(A, ne, range);
         MDET_LAUNCHED(ctx, "k_key_range");
         k_key32<<<g3, 256, 0, s>>>(A, ne, range);
         MDET_LAUNCHED(ctx, "k_key32");
-        for (int k = 0; k < (corr ? 3 : 2); ++k) {
+        for (int k = 0; k < arrays; ++k) {
             size_t tb = tmpb;
             if (k == 2)
                 MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(tmp, tb, A.key[k], k32s, idx, os, (int)ne, 0,
                                                                          32, s));
             else
                 MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, A.key[k], k32s, idx, os, (int)ne, 0, 32, s));
-            k_fix_runs<<<g, 256, 0, s>>>(k32s, A.v[k], ne, k == 2, os, bad + 1);
+            k_fix_runs<<<g, 256, 0, s>>>(k32s, A.v[k], ne, k == 2, os, bad + 1 + k);
             MDET_LAUNCHED(ctx, "k_fix_runs");
             if (k == 0) {
                 k_gather_sorted<<<g, 256, 0, s>>>(raw, os, ne, distr);
@@ -707,18 +717,26 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
         }
         return MDET_OK;
     };
-    unsigned long long h_bad[2] = {0, 0};
-    for (int full = ne > kTopBitsMost; full < 2; ++full) {
-        ctx_timer_begin(ctx, "abd_ranks");
-        MDET_TRY(full ? by_full_keys() : by_top_bits());
-        ctx_timer_end(ctx, "abd_ranks");
+    const bool top_bits = ne <= kTopBitsMost;
+    unsigned long long h_bad[4] = {0, 0, 0, 0};
+    ctx_timer_begin(ctx, "abd_ranks");
+    if (top_bits)
+        MDET_TRY(by_top_bits());
+    else
+        for (int k = 0; k < arrays; ++k) MDET_TRY(by_full_keys(k));
+    ctx_timer_end(ctx, "abd_ranks");
+    for (bool again = false;; again = true) {
         ctx_timer_begin(ctx, "k_sscr");
-        k_sscr<<<g, 256, 0, s>>>(raw, nnz, rt, rc, distr, ne, corr, out);
+        k_sscr<<<g, 256, 0, s>>>(raw, nnz, rt, rc, distr, ne, corr, top_bits && !again ? bad + 1 : nullptr, out);
         ctx_timer_end(ctx, "k_sscr");
         MDET_LAUNCHED(ctx, "k_sscr");
-        MDET_CUDA(ctx, cudaMemcpyAsync(h_bad, bad, 16, cudaMemcpyDeviceToHost, s));
+        MDET_CUDA(ctx, cudaMemcpyAsync(h_bad, bad, 32, cudaMemcpyDeviceToHost, s));
         MDET_CUDA(ctx, cudaStreamSynchronize(s));
-        if (!h_bad[1] || h_bad[0]) break;
+        if (again || h_bad[0] || !(h_bad[1] | h_bad[2] | h_bad[3])) break;
+        ctx_timer_begin(ctx, "abd_ranks_full");
+        for (int k = 0; k < arrays; ++k)
+            if (h_bad[1 + k]) MDET_TRY(by_full_keys(k));
+        ctx_timer_end(ctx, "abd_ranks_full");
     }
     if (h_bad[0])
         return ctx_fail(ctx, MDET_ERR_INVALID,
