@@ -598,6 +598,7 @@ __global__ void __launch_bounds__(Shape<BM, BN, NST, EB>::kThreads, Shape<BM, BN
                 const uint32_t T = __reduce_add_sync(0xffffffffu, mine);
                 if (T) {
                     uint32_t cnt = *(volatile uint32_t*)qc;  // below kQueue / 2
+                    __syncwarp();  // every lane has the count before any lane appends
                     if (T > kQueue / 2) {
                         // a dense chunk (rows of one genome against each other hold
                         // thousands of pairs): straight to the list, one reservation
