@@ -349,6 +349,13 @@ struct ScoreArgs {
     unsigned long long* bad;  // edges with an index out of range or no covered sample
 };
 
+// The ends of a sample's similarity, 1 - min(max(d, 1e-6), 1 - 1e-6) as FP64
+// forms them, and in float-float (the upper one needs all 53 bits, so the
+// values that reach an end take the FP64 one).
+constexpr double kSimMin = 1. - (1. - 1e-6), kSimMax = 1. - 1e-6;
+constexpr float kSimMinHi = (float)kSimMin, kSimMinLo = (float)(kSimMin - (double)kSimMinHi);
+constexpr float kSimMaxHi = (float)kSimMax, kSimMaxLo = (float)(kSimMax - (double)kSimMaxHi);
+
 // cal_abd_dist of one sample by the FP64 path: its similarity 1 - d.
 __device__ __noinline__ double abd_sim64(const ScoreArgs& p, uint64_t i1, uint64_t i2, ff f1, ff f2,
                                          const float* tab) {
@@ -387,8 +394,7 @@ __global__ void k_abd_score(ScoreArgs p) {
         // the cross sum of the Pearson correlation (cal_abd_corr), from the
         // rows' own deviations
         double sxy = 0.;
-        // 1 - min(max(d, 1e-6), 1 - 1e-6) at its ends, as FP64 forms them
-        const ff lo = ff_make(0x1.0c6f7ap-20f, 0x1.7p-49f), hi = ff_make(0x1.ffffdep-1f, 0x1.c842fap-27f);
+        const ff lo = ff_make(kSimMinHi, kSimMinLo), hi = ff_make(kSimMaxHi, kSimMaxLo);
         for (uint32_t i = 0; i < p.nabd; ++i) {
             const Rec a = load_rec(q1 + i), b = load_rec(q2 + i);
             // cal_abd_dist for sample i
@@ -401,9 +407,7 @@ __global__ void k_abd_score(ScoreArgs p) {
                 ff s = hi;
                 if (!same_mean(a, b)) s = abd_sim_ff(a, b, tab);
                 if (s.hi >= 0.f) {
-                    if (ff_gt(lo, s)) s = lo;
-                    if (ff_gt(s, hi)) s = hi;
-                    sum += ff_to_double(s);
+                    sum += !ff_gt(s, lo) ? kSimMin : !ff_gt(hi, s) ? kSimMax : ff_to_double(s);
                 } else {
                     sum += abd_sim64(p, r1 * p.nabd + i, r2 * p.nabd + i, a.isd, b.isd, tab);
                 }
