@@ -491,25 +491,39 @@ __global__ void k_key32(RankArrays A, uint64_t ne, const KeyRange* __restrict__ 
         A.key[blockIdx.y][e] = (uint32_t)((order_key(v[e]) - lo) >> sh);
 }
 
-// The thread at the start of a run of equal 32-bit keys sorts the run's indices
-// by the full keys (insertion, stable).
-__global__ void k_fix_runs(const uint32_t* __restrict__ ks, const double* __restrict__ v, uint64_t ne, bool descending,
-                           uint32_t* __restrict__ os, unsigned long long* __restrict__ overflow) {
-    for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q + 1 < ne;
+// Runs of equal 32-bit keys that are not in order by their full keys: the thread
+// at a position whose full key belongs before its predecessor's marks the run's
+// start.  Every position is looked at by a thread of its own, so a long run that
+// is in order (equal values: pairs at a similarity's end, say) costs no more
+// than others; a walk is at most kFixRun long.
+__global__ void k_mark_runs(const uint32_t* __restrict__ ks, const double* __restrict__ v,
+                            const uint32_t* __restrict__ os, uint64_t ne, bool descending, uint8_t* __restrict__ mark,
+                            unsigned long long* __restrict__ overflow) {
+    for (uint64_t q = 1 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < ne;
          q += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t k = ks[q];
-        if (ks[q + 1] != k || (q > 0 && ks[q - 1] == k)) continue;
-        // how far the run goes, and whether it is in order as it stands
+        if (ks[q - 1] != k) continue;
+        const unsigned long long a = order_key(v[os[q - 1]]), b = order_key(v[os[q]]);
+        if (descending ? b <= a : b >= a) continue;
+        uint64_t first = q - 1;
+        while (first > 0 && q - first < kFixRun && ks[first - 1] == k) --first;
+        if (first > 0 && ks[first - 1] == k)
+            atomicAdd(overflow, 1ull);
+        else
+            mark[first] = 1;
+    }
+}
+
+// The thread at the start of a marked run sorts the run's indices by the full
+// keys (insertion, stable).
+__global__ void k_fix_runs(const uint32_t* __restrict__ ks, const double* __restrict__ v,
+                           const uint8_t* __restrict__ mark, uint64_t ne, bool descending, uint32_t* __restrict__ os,
+                           unsigned long long* __restrict__ overflow) {
+    for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < ne; q += (uint64_t)gridDim.x * blockDim.x) {
+        if (!mark[q]) continue;
+        const uint32_t k = ks[q];
         uint64_t end = q + 1;
-        unsigned long long last = order_key(v[os[q]]);
-        bool sorted = true;
-        for (; end < ne && ks[end] == k; ++end) {
-            const unsigned long long f = order_key(v[os[end]]);
-            sorted = sorted && (descending ? f <= last : f >= last);
-            last = f;
-            if (!sorted && end - q > kFixRun) break;
-        }
-        if (sorted) continue;
+        while (end < ne && end - q <= kFixRun && ks[end] == k) ++end;
         if (end - q > kFixRun) {
             atomicAdd(overflow, 1ull);
             continue;
@@ -637,7 +651,8 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     unsigned long long* bad = (unsigned long long*)ctx_scratch(ctx, "abd.bad", bad_bytes);
     uint32_t* k32 = (uint32_t*)ctx_scratch(ctx, "abd.k32", ne * 12);
     uint32_t* k32s = (uint32_t*)ctx_scratch(ctx, "abd.k32s", ne * 4);
-    if (!k32 || !k32s) return MDET_ERR_NOMEM;
+    uint8_t* mark = (uint8_t*)ctx_scratch(ctx, "abd.mark", ne);
+    if (!k32 || !k32s || !mark) return MDET_ERR_NOMEM;
     if (!raw || !nnz || !cor || !idx || !ks || !os || !head || !start || !rt || !rc || !distr || !bad)
         return MDET_ERR_NOMEM;
     size_t t1 = 0, t2 = 0, t3 = 0, t4 = 0;
@@ -710,7 +725,10 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
                                                                          32, s));
             else
                 MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tb, A.key[k], k32s, idx, os, (int)ne, 0, 32, s));
-            k_fix_runs<<<g, 256, 0, s>>>(k32s, A.v[k], ne, k == 2, os, bad + 1 + k);
+            MDET_CUDA(ctx, cudaMemsetAsync(mark, 0, ne, s));
+            k_mark_runs<<<g, 256, 0, s>>>(k32s, A.v[k], os, ne, k == 2, mark, bad + 1 + k);
+            MDET_LAUNCHED(ctx, "k_mark_runs");
+            k_fix_runs<<<g, 256, 0, s>>>(k32s, A.v[k], mark, ne, k == 2, os, bad + 1 + k);
             MDET_LAUNCHED(ctx, "k_fix_runs");
             if (k == 0) {
                 k_gather_sorted<<<g, 256, 0, s>>>(raw, os, ne, distr);
