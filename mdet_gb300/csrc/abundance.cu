@@ -424,29 +424,50 @@ __global__ void k_abd_score(ScoreArgs p) {
 
 // ---- ranks by 32-bit sorts -------------------------------------------------
 // A radix sort of FP64 keys with indices takes eight passes over 12 bytes an
-// edge.  The values of one call span a narrow range, so the sorts run on the
-// top 32 bits of the keys' offsets from their minimum (four passes over 8
-// bytes); the few runs of equal 32-bit keys are put in order by their full
-// keys afterwards (k_fix_runs).  Runs longer than kFixRun whose full keys
-// differ -- values crowded within 2^-32 of the range -- raise a flag, and those
-// values are sorted by their full keys instead, before any score is written.  (3.8M edges: 1,093 us for the three full sorts
-// and their ranks, 898 us so.)  More edges crowd the runs: 90,000 contigs (limit 100)
-// 1,904 -> 1,622 us, 200,000 3,689 -> 3,767, 400,000 7,667 -> 9,584, and 80M edges
-// overflow, so beyond kTopBitsMost the full keys are sorted at once.
-constexpr uint64_t kTopBitsMost = 1ull << 23;
+// edge; the sorts here run on a 32-bit key that is monotone in the value (four
+// passes over 8 bytes), and runs of equal 32-bit keys that are out of order by
+// their full keys are put in order afterwards (k_mark_runs, k_fix_runs).
+//
+// The similarities and sTNF are positive and span a few octaves: their key is
+// the top 32 bits of the bit pattern's offset from the smallest (k_key_range;
+// NaN is set aside, so that it does not stretch the range).  Correlations change
+// sign and crowd at both ends -- two contigs of a genome, few samples -- so
+// their key is the bit pattern of 1 - |c| to either side of the middle, with 25
+// bits of every octave of the distance from +-1 (corr_key).  (A restatement of
+// 60,000 contigs' 3.8M edges: 19 % of the correlations in runs, the longest 6 to 7
+// long at 3 to 10 samples; by the pattern's offset from the smallest, 63 bits wide over
+// both signs, 78 % and 71 to 16,877.)  Runs out of order and longer than kFixRun
+// raise a flag, and those values are sorted by their full keys instead, before any
+// score is written.  Two samples' correlations are +-1 but for the last
+// bits, two runs of half the edges: they go by their full keys at once.
+//
+// The ranks by either route, 10 samples: 3.8M edges 1,186 us by the full keys and
+// 969 by these, 7.2M 1,920 and 1,612, 16M 3,693 and 3,505, 32M 7,667 and 8,375 (more
+// edges crowd the runs), 80M 20.7 and 26.5 ms; so up to 2^24 edges.
+constexpr uint64_t kTopBitsMost = 1ull << 24;
 constexpr uint32_t kFixRun = 48;
 
 struct KeyRange {
     unsigned long long min_inv, max;  // of the order keys; min complemented, so that zeros start both
 };
 
-// The order of the radix sort: negative values reversed, -0 as 0.
+// The order of the radix sort: negative values reversed, -0 as 0; NaN lies
+// beyond the infinities, on its sign's side.
 __device__ __forceinline__ unsigned long long order_key(double v) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v == 0. ? 0. : v);
     return (b & 0x8000000000000000ull) ? ~b : (b | 0x8000000000000000ull);
 }
 
-struct RankArrays {  // blockIdx.y: which
+// Correlation to 32 bits, monotone: 1 - |c| is in [2^-53, 1] or not positive.
+__device__ __forceinline__ uint32_t corr_key(double c) {
+    if (c != c) return __double2hiint(c) < 0 ? 0u : ~0u;
+    const long long base = (1023ll - 54) << 52, one = 1023ll << 52;
+    const long long t = __double_as_longlong(1. - fabs(c));  // negative when |c| rounds above 1
+    const uint32_t k = (uint32_t)((one - (t > base ? t : base)) >> 27);  // below 2^31: 54 octaves of 25 bits
+    return c >= 0. ? 0x80000000u + k : 0x7fffffffu - k;
+}
+
+struct RankArrays {  // blockIdx.y: which; the last one holds the correlations
     const double* v[3];
     uint32_t* key[3];
 };
@@ -455,7 +476,9 @@ __global__ void __launch_bounds__(256) k_key_range(RankArrays A, uint64_t ne, Ke
     const double* v = A.v[blockIdx.y];
     unsigned long long lo = 0, hi = 0;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < ne; e += (uint64_t)gridDim.x * blockDim.x) {
-        const unsigned long long k = order_key(v[e]);
+        const double x = v[e];
+        if (x != x) continue;
+        const unsigned long long k = order_key(x);
         lo = lo > ~k ? lo : ~k;
         hi = hi > k ? hi : k;
     }
@@ -485,10 +508,20 @@ __global__ void __launch_bounds__(256) k_key_range(RankArrays A, uint64_t ne, Ke
 
 __global__ void k_key32(RankArrays A, uint64_t ne, const KeyRange* __restrict__ r) {
     const double* v = A.v[blockIdx.y];
+    uint32_t* key = A.key[blockIdx.y];
+    const uint64_t e0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    if (blockIdx.y == 2) {
+        for (uint64_t e = e0; e < ne; e += step) key[e] = corr_key(v[e]);
+        return;
+    }
     const unsigned long long lo = ~r[blockIdx.y].min_inv, span = r[blockIdx.y].max - lo;
     const int sh = max(0, 32 - __clzll((long long)span));
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < ne; e += (uint64_t)gridDim.x * blockDim.x)
-        A.key[blockIdx.y][e] = (uint32_t)((order_key(v[e]) - lo) >> sh);
+    for (uint64_t e = e0; e < ne; e += step) {
+        const double x = v[e];
+        // 0 and ~0 are the NaNs'
+        const unsigned long long k = (order_key(x) - lo) >> sh;
+        key[e] = x != x ? (__double2hiint(x) < 0 ? 0u : ~0u) : 1u + (uint32_t)(k < 0xfffffffdull ? k : 0xfffffffdull);
+    }
 }
 
 // Runs of equal 32-bit keys that are not in order by their full keys: the thread
@@ -713,12 +746,16 @@ int sscr_core(mdet_ctx* ctx, const uint64_t* from, const uint64_t* to, const dou
     auto by_top_bits = [&]() -> int {
         const RankArrays A{{raw, stnf, cor}, {k32, k32 + ne, k32 + 2 * ne}};
         KeyRange* range = (KeyRange*)(bad + 4);
-        const dim3 g3(g, arrays), gr(std::min<unsigned>(g, ctx->num_sms * 4), arrays);
+        const dim3 g3(g, arrays), gr(std::min<unsigned>(g, ctx->num_sms * 4), 2);
         k_key_range<<<gr, 256, 0, s>>>(A, ne, range);
         MDET_LAUNCHED(ctx, "k_key_range");
         k_key32<<<g3, 256, 0, s>>>(A, ne, range);
         MDET_LAUNCHED(ctx, "k_key32");
         for (int k = 0; k < arrays; ++k) {
+            if (k == 2 && p.nabd == 2) {
+                MDET_TRY(by_full_keys(k));
+                continue;
+            }
             size_t tb = tmpb;
             if (k == 2)
                 MDET_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(tmp, tb, A.key[k], k32s, idx, os, (int)ne, 0,
