@@ -20,7 +20,9 @@
 // among the contig's neighbours earlier in the order, found by Kahn peeling):
 // the contigs of a level side by side, the levels in turn -- the same result
 // as the sequential sweep.  The peeling and all sweeps of a run are one
-// cooperative launch each, with a bounded grid barrier between levels.  A
+// cooperative launch each, with a bounded grid barrier between levels (lp_wait.h);
+// a run with a contig of more than 1,024 edges is swept by a launch per level
+// instead, so that no block waits for it.  A
 // block sorts its contig's (neighbour label, edge
 // position) keys (bitonic sort in shared memory, or in a global slice for
 // contigs with more than 1,024 edges), folds each label's log(1 - score) in
@@ -45,6 +47,9 @@
 #include "common.cuh"
 #include "lp_math.h"
 #include "lp_umap.h"
+#include "lp_wait.h"
+
+static_assert(lpw::kSpin == MDET_SPIN_CYCLES, "one bound for every wait");
 
 int check_flag(mdet_ctx* ctx);
 
@@ -125,10 +130,12 @@ __device__ bool visit(const LpArgs& P, uint32_t v, uint32_t lab, Tally& T) {
 }
 
 // A barrier over all blocks of a cooperative launch: every block adds one to
-// *bar, whose target grows by the grid's size each time.  The wait is bounded;
-// a block whose wait runs out raises the context's flag, and every block's
-// loops end at their next barrier.  False then.
-__device__ bool grid_barrier(unsigned int* bar, unsigned int& target, int* flag) {
+// *bar, whose target grows by the grid's size each time.  The wait is bounded by
+// budget() cycles (lp_wait.h; asked for by a block that has waited a while); a
+// block whose wait runs out raises the context's flag, and every block's loops
+// end at their next barrier.  False then.
+template <class Budget>
+__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int& target, int* flag, Budget budget) {
     __shared__ bool ok;
     target += gridDim.x;
     __syncthreads();
@@ -139,7 +146,7 @@ __device__ bool grid_barrier(unsigned int* bar, unsigned int& target, int* flag)
         const long long t0 = clock64();
         for (uint32_t poll = 1; (int)(*(volatile unsigned int*)bar - target) < 0; ++poll) {
             if (poll & 255u) continue;  // the flag and the clock now and then
-            const bool late = (unsigned long long)(clock64() - t0) > MDET_SPIN_CYCLES;
+            const bool late = (unsigned long long)(clock64() - t0) > budget();
             if (late) atomicOr(flag, MDET_FLAG_TIMEOUT);
             if (late || *(volatile int*)flag) {
                 good = false;
@@ -432,17 +439,32 @@ __device__ void lp_node_warp(const LpArgs& P, const WarpNode& N, WarpWs& W, Tall
 
 // ---- dependency levels of the order --------------------------------------
 
-__global__ void k_lp_pos(const uint32_t* __restrict__ order, uint32_t norder, uint32_t* __restrict__ pos_of) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < norder) pos_of[order[i]] = i;
-}
-
 // a level's contigs: those with at most kWarpCap edges (a warp each) and the
 // others (a block each; maxdeg and the global slices are theirs); off and
 // soff: where the level starts in the block and warp lists
 struct LevelInfo {
     unsigned int count, maxdeg, nbig, nsmall, maxall, off, soff, pad;
 };
+
+// Every contig's place in the order, and the largest degree (info->maxall).
+__global__ void __launch_bounds__(256) k_lp_pos(const uint32_t* __restrict__ order, uint32_t norder,
+                                                const uint32_t* __restrict__ deg, uint32_t* __restrict__ pos_of,
+                                                LevelInfo* info) {
+    __shared__ uint32_t most;
+    if (threadIdx.x == 0) most = 0;
+    __syncthreads();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t d = 0;
+    if (i < norder) {
+        const uint32_t v = order[i];
+        pos_of[v] = i;
+        d = deg[v];
+    }
+    d = __reduce_max_sync(0xffffffffu, d);
+    if ((threadIdx.x & 31) == 0) atomicMax(&most, d);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(&info->maxall, most);
+}
 
 // Contig w joins the next level.  The lanes that enqueue together share one
 // atomic per counter.
@@ -481,6 +503,7 @@ struct LevelArgs {
     uint32_t lcap;         // entries of info
     uint32_t* slot_of;
     LevelInfo* sum;        // over all levels: count = contigs levelled, nsmall = levels, the maxima
+    unsigned long long incidences;  // all of them (2 per edge)
     unsigned int* bar;
     int* flag;
 };
@@ -498,16 +521,10 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_levels(LevelArgs A) {
     const uint32_t g0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const uint32_t gmask = 0xFFu << (threadIdx.x & 24);
     unsigned int target = 0;
-    // the largest degree: one atomic a block (one per joining contig and level
-    // was half of the atomics on a level's counters)
-    __shared__ uint32_t bmax;
-    if (threadIdx.x == 0) bmax = 0;
-    __syncthreads();
-    uint32_t most = 0;
+    const uint32_t maxall = A.info[0].maxall;
     for (uint32_t pu = g0; pu < A.norder; pu += ng) {
         const uint32_t u = A.order[pu];
         const uint32_t s = A.inc_off[u], d = A.inc_off[u + 1] - s;
-        most = max(most, d);
         uint32_t c = 0;
         for (uint32_t j = sub; j < d; j += 8) c += A.pos_of[A.oth[s + j]] < pu;
 #pragma unroll
@@ -517,20 +534,19 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_levels(LevelArgs A) {
             if (c == 0) lp_enqueue(u, d, A.lvl, A.lvls, A.info, A.slot_of);
         }
     }
-    __syncwarp();
-    most = __reduce_max_sync(0xffffffffu, most);
-    if ((threadIdx.x & 31) == 0) atomicMax(&bmax, most);
-    __syncthreads();
-    if (threadIdx.x == 0) atomicMax(&A.info[0].maxall, bmax);
-    uint32_t off = 0, soff = 0, done = 0, L = 0, maxdeg = 0, maxall = 0, maxbig = 0;
+    uint32_t off = 0, soff = 0, done = 0, L = 0, maxdeg = 0, maxbig = 0;
+    uint32_t at_work = A.norder, longest = maxall;  // contigs of the step before the barrier, their largest degree
     for (;; ++L) {
-        if (!grid_barrier(A.bar, target, A.flag)) return;
+        if (!grid_barrier(A.bar, target, A.flag,
+                          [&] { return lpw::level_budget(at_work, ng, 8, longest, A.incidences); }))
+            return;
         if (L + 1 >= A.lcap) break;
         const uint32_t count = __ldcg(&A.info[L].count), nsmall = __ldcg(&A.info[L].nsmall);
         if (count + nsmall == 0) break;
         maxdeg = max(maxdeg, __ldcg(&A.info[L].maxdeg));
-        maxall = max(maxall, __ldcg(&A.info[L].maxall));
         maxbig = max(maxbig, __ldcg(&A.info[L].nbig));
+        at_work = count + nsmall;
+        longest = max(maxdeg, kWarpCap);
         done += count + nsmall;
         const uint32_t noff = off + count, nsoff = soff + nsmall;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -613,7 +629,10 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_sweeps(LpArgs P, const uint
                     T.moved = T.entries = 0;
                 }
             }
-            if (!grid_barrier(bar, target, flag)) return;
+            if (!grid_barrier(bar, target, flag, [&] {
+                    return lpw::sweep_budget(count, kGroups * gridDim.x, info[L].maxdeg, nsmall, nw, kWarpCap);
+                }))
+                return;
         }
         ++sweeps;
         if (threadIdx.x == 0) {
@@ -627,7 +646,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_sweeps(LpArgs P, const uint
         const unsigned long long moved = s_cnt[0] - before, err = s_cnt[1];
         before = s_cnt[0];
         // every block has read the counters before any goes on to change them
-        if (!grid_barrier(bar, target, flag)) return;
+        if (!grid_barrier(bar, target, flag, [] { return lpw::kSpin; })) return;
         if (err && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(P.counters + 2, err);
         if (err) break;
         if (moved < low) {
@@ -639,6 +658,28 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_sweeps(LpArgs P, const uint
         if (moved == 0) break;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) out[0] = sweeps;
+}
+
+// One level of a sweep as a launch of its own: block b < count evaluates the
+// level's b-th block contig, the others eight warp contigs each.
+__global__ void __launch_bounds__(kThreads) k_lp_level(LpArgs P, const uint32_t* __restrict__ lvl, uint32_t count,
+                                                       const uint32_t* __restrict__ lvls, uint32_t nsmall) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ BlockWs bws;
+    __shared__ Tally T;
+    if (threadIdx.x == 0) T.moved = T.entries = 0;
+    __syncthreads();
+    if (blockIdx.x < count) {
+        lp_node_block(P, lvl[blockIdx.x], smem, bws, T);
+    } else {
+        const uint32_t w = threadIdx.x >> 5, i = (blockIdx.x - count) * (kThreads / 32) + w;
+        lp_node_warp(P, lp_load(P, lvls, i, nsmall), reinterpret_cast<WarpWs*>(smem)[w], T);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (T.moved) atomicAdd(P.counters, (unsigned long long)T.moved);
+        if (T.entries) atomicAdd(P.counters + 1, (unsigned long long)T.entries);
+    }
 }
 
 // ---- the traversal ----------------------------------------------------------
@@ -853,6 +894,39 @@ int launch_grid(mdet_ctx* ctx, K kernel, size_t smem, const char* what, void** a
     return MDET_OK;
 }
 
+// The sweeps of a call as a launch per level, with the decisions of k_lp_sweeps
+// on the host.  hc: pinned, five counters as lp_call reads them.
+int sweeps_by_level(mdet_ctx* ctx, const LpArgs& P, const uint32_t* lvl, const uint32_t* lvls,
+                    const std::vector<LevelInfo>& info, unsigned long long* hc) {
+    cudaStream_t s = ctx->stream;
+    MDET_CUDA(ctx, cudaFuncSetAttribute(k_lp_level, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)ws_bytes(kSmallCap)));
+    unsigned long long before = 0, low = INT_MAX, attempt = 0, sweeps = 0;
+    while (true) {
+        for (const LevelInfo& h : info) {
+            const uint32_t wblocks = (h.nsmall + kThreads / 32 - 1) / (kThreads / 32);
+            size_t dyn = wblocks ? (kThreads / 32) * sizeof(WarpWs) : 0;
+            if (h.count) dyn = std::max(dyn, ws_bytes(std::min<uint32_t>(pow2_at_least(h.maxdeg), kSmallCap)));
+            k_lp_level<<<h.count + wblocks, kThreads, dyn, s>>>(P, lvl + h.off, h.count, lvls + h.soff, h.nsmall);
+            MDET_LAUNCHED(ctx, "k_lp_level");
+        }
+        MDET_CUDA(ctx, cudaMemcpyAsync(hc, P.counters, 32, cudaMemcpyDeviceToHost, s));
+        MDET_CUDA(ctx, cudaStreamSynchronize(s));
+        hc[4] = ++sweeps;
+        if (hc[1] * 4 > (P.vt_mask + 1) * 3) hc[2] |= kErrTable;
+        if (hc[2]) return MDET_OK;
+        const unsigned long long moved = hc[0] - before;
+        before = hc[0];
+        if (moved < low) {
+            low = moved;
+            attempt = 0;
+        } else if (++attempt >= 10) {
+            return MDET_OK;
+        }
+        if (moved == 0) return MDET_OK;
+    }
+}
+
 // One propagation call over the traversal graph (m2 edges) and order.
 int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
     cudaStream_t s = ctx->stream;
@@ -897,17 +971,17 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
     // dependency levels: per level, the warp contigs (lvls) and the block
     // contigs (lvl), each list's levels stored one after another
     MDET_CUDA(ctx, cudaMemsetAsync(pos_of, 0xFF, n * 4, s));
-    k_lp_pos<<<grid_for(no), 256, 0, s>>>(S.order, (uint32_t)no, pos_of);
-    MDET_LAUNCHED(ctx, "k_lp_pos");
     const uint64_t lcap = no + 2;
     LevelInfo* info = (LevelInfo*)ctx_scratch(ctx, "lp.info", (lcap + 2) * sizeof(LevelInfo));
     if (!info) return MDET_ERR_NOMEM;
     MDET_CUDA(ctx, cudaMemsetAsync(info, 0, (lcap + 2) * sizeof(LevelInfo), s));
+    k_lp_pos<<<grid_for(no), 256, 0, s>>>(S.order, (uint32_t)no, deg, pos_of, info);
+    MDET_LAUNCHED(ctx, "k_lp_pos");
     unsigned int* bar = (unsigned int*)(info + lcap + 1);  // barrier counters: levels, sweeps
     LevelInfo* dsum = info + lcap;
     {
         LevelArgs A{S.order, (uint32_t)no, pos_of, inc_off, oth, deg, pred, lvl, lvls, info, (uint32_t)lcap, slot_of, dsum,
-                    bar, ctx->d_flag};
+                    2 * m, bar, ctx->d_flag};
         void* args[] = {&A};
         MDET_TRY(launch_grid(ctx, k_lp_levels, 0, "k_lp_levels", args));
     }
@@ -925,6 +999,15 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
     st->levels_max = std::max<uint64_t>(st->levels_max, nlevels);
     st->degree_max = std::max<uint64_t>(st->degree_max, maxall);
     maxdeg = std::max(maxdeg, kWarpCap);
+    // A contig sorted in global memory (more than kSmallCap edges) can hold its
+    // level for as long as its edges take, millions of them for seconds: no block
+    // is to wait for it inside a kernel.
+    const bool by_level = maxdeg > kSmallCap;
+    std::vector<LevelInfo> levels(by_level ? nlevels : 0);
+    if (by_level) {
+        MDET_CUDA(ctx, cudaMemcpyAsync(levels.data(), info, nlevels * sizeof(LevelInfo), cudaMemcpyDeviceToHost, s));
+        MDET_CUDA(ctx, cudaStreamSynchronize(s));
+    }
     // the CDF's log-factorials up to the largest label count
     // (one thread sums the table in order; it is rebuilt only when a run
     // needs a longer one)
@@ -984,7 +1067,9 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
         unsigned int* sbar = bar + 1 + attempt_table;
         unsigned long long* dsweeps = S.cnt + 4;
         MDET_CUDA(ctx, cudaMemsetAsync(dsweeps, 0, 8, s));
-        {
+        if (by_level) {
+            MDET_TRY(sweeps_by_level(ctx, P, lvl, lvls, levels, hc));
+        } else {
             const uint32_t *a_lvl = lvl, *a_lvls = lvls;
             const LevelInfo* a_info = info;
             uint32_t a_n = nlevels;
@@ -994,8 +1079,10 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
             MDET_TRY(launch_grid(ctx, k_lp_sweeps, kGroups * dyn, "k_lp_sweeps", args));
         }
         ctx_timer_end(ctx, "lp_sweep");
-        MDET_CUDA(ctx, cudaMemcpyAsync(hc, S.cnt, 40, cudaMemcpyDeviceToHost, s));
-        MDET_CUDA(ctx, cudaStreamSynchronize(s));
+        if (!by_level) {
+            MDET_CUDA(ctx, cudaMemcpyAsync(hc, S.cnt, 40, cudaMemcpyDeviceToHost, s));
+            MDET_CUDA(ctx, cudaStreamSynchronize(s));
+        }
         const uint64_t sweeps = hc[4];
         if (sweeps == 0) {  // a barrier's wait ran out
             MDET_TRY(check_flag(ctx));
