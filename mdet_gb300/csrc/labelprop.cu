@@ -508,24 +508,62 @@ struct LevelArgs {
     int* flag;
 };
 
+// Level step of one contig by W lanes (this one is `sub`): its later neighbours
+// have one earlier neighbour less, and those with none left join the next level.
+// Four neighbours a lane at a time, their reads and atomics side by side: the
+// step is a chain of dependent accesses of half a microsecond each.
+template <int W>
+__device__ __forceinline__ void lp_release(const LevelArgs& A, uint32_t u, uint32_t sub, uint32_t* next,
+                                           uint32_t* next_small, LevelInfo* info) {
+    const uint32_t pu = A.pos_of[u], s = A.inc_off[u], d = A.inc_off[u + 1] - s;
+    for (uint32_t j = sub; j < d; j += 4 * W) {
+        uint32_t o[4], dego[4], left[4];
+        bool later[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o[k] = j + k * W < d ? A.oth[s + j + k * W] : u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            later[k] = A.pos_of[o[k]] > pu;
+            dego[k] = A.deg[o[k]];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) left[k] = later[k] ? atomicSub(A.pred + o[k], 1u) : 0u;
+#pragma unroll 1
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t l = k == 0 ? left[0] : k == 1 ? left[1] : k == 2 ? left[2] : left[3];
+            const uint32_t w = k == 0 ? o[0] : k == 1 ? o[1] : k == 2 ? o[2] : o[3];
+            const uint32_t dw = k == 0 ? dego[0] : k == 1 ? dego[1] : k == 2 ? dego[2] : dego[3];
+            if (l == 1u) lp_enqueue(w, dw, next, next_small, info, A.slot_of);
+        }
+    }
+}
+
 // The dependency levels of the order, one cooperative launch: the earlier
 // neighbours of each contig are counted (those with none form level 0), then
-// Kahn steps until a level is empty, a grid barrier after each -- eight lanes
-// per contig, and a contig whose last earlier neighbour is in level L joins
-// level L + 1.  (60,000 contigs, 10 runs: 176 launches of 6.1 us, queued
-// sixteen at a time past the last level, became 10 of these.)
+// Kahn steps until a level is empty, a grid barrier after each -- a warp per
+// contig of more than 32 edges, eight lanes for the others, and a contig whose
+// last earlier neighbour is in level L joins level L + 1.  (60,000 contigs of up
+// to 13 edges, 10 runs: 176 launches of 6.1 us, queued sixteen at a time past the
+// last level, became 10 of these.  A graph of 50,000 contigs, up to 187 edges
+// each and 62 levels: 6.7 ms with launches, 11.5 ms with eight lanes for
+// every contig, 6.6 ms so.)
 __global__ void __launch_bounds__(kCoopThreads) k_lp_levels(LevelArgs A) {
     // groups of eight lanes: most contigs have few edges, and the chain of
     // dependent loads wants as many contigs in flight as there are lanes for
     const uint32_t sub = threadIdx.x & 7, ng = gridDim.x * (blockDim.x >> 3);
     const uint32_t g0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const uint32_t gmask = 0xFFu << (threadIdx.x & 24);
+    // warps count from the last block, so that a narrow level's two kinds of
+    // contigs are on different SMs
+    const uint32_t nw = gridDim.x * (blockDim.x >> 5);
+    const uint32_t w0 = (gridDim.x - 1 - blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     unsigned int target = 0;
     const uint32_t maxall = A.info[0].maxall;
     for (uint32_t pu = g0; pu < A.norder; pu += ng) {
         const uint32_t u = A.order[pu];
         const uint32_t s = A.inc_off[u], d = A.inc_off[u + 1] - s;
         uint32_t c = 0;
+#pragma unroll 4
         for (uint32_t j = sub; j < d; j += 8) c += A.pos_of[A.oth[s + j]] < pu;
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(gmask, c, o);
@@ -535,34 +573,31 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_levels(LevelArgs A) {
         }
     }
     uint32_t off = 0, soff = 0, done = 0, L = 0, maxdeg = 0, maxbig = 0;
-    uint32_t at_work = A.norder, longest = maxall;  // contigs of the step before the barrier, their largest degree
+    uint32_t warps = 0, groups = A.norder, longest = maxall;  // contigs of the step before the barrier, largest degree
     for (;; ++L) {
-        if (!grid_barrier(A.bar, target, A.flag,
-                          [&] { return lpw::level_budget(at_work, ng, 8, longest, A.incidences); }))
+        if (!grid_barrier(A.bar, target, A.flag, [&] {
+                return lpw::level_budget(warps, nw, 32, longest, A.incidences) +
+                       lpw::level_budget(groups, ng, 8, L ? kWarpCap : longest, A.incidences);
+            }))
             return;
         if (L + 1 >= A.lcap) break;
         const uint32_t count = __ldcg(&A.info[L].count), nsmall = __ldcg(&A.info[L].nsmall);
         if (count + nsmall == 0) break;
         maxdeg = max(maxdeg, __ldcg(&A.info[L].maxdeg));
         maxbig = max(maxbig, __ldcg(&A.info[L].nbig));
-        at_work = count + nsmall;
-        longest = max(maxdeg, kWarpCap);
+        warps = count;
+        groups = nsmall;
+        longest = maxdeg;
         done += count + nsmall;
         const uint32_t noff = off + count, nsoff = soff + nsmall;
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             A.info[L].off = off;
             A.info[L].soff = soff;
         }
-        for (uint32_t wid = g0; wid < count + nsmall; wid += ng) {
-            const uint32_t u = wid < count ? __ldcg(A.lvl + off + wid) : __ldcg(A.lvls + soff + wid - count);
-            const uint32_t pu = A.pos_of[u];
-            const uint32_t s = A.inc_off[u], d = A.inc_off[u + 1] - s;
-            for (uint32_t j = sub; j < d; j += 8) {
-                const uint32_t o = A.oth[s + j], dego = A.deg[o];
-                if (A.pos_of[o] > pu && atomicSub(A.pred + o, 1u) == 1u)
-                    lp_enqueue(o, dego, A.lvl + noff, A.lvls + nsoff, A.info + L + 1, A.slot_of);
-            }
-        }
+        for (uint32_t i = w0; i < count; i += nw)
+            lp_release<32>(A, __ldcg(A.lvl + off + i), threadIdx.x & 31, A.lvl + noff, A.lvls + nsoff, A.info + L + 1);
+        for (uint32_t i = g0; i < nsmall; i += ng)
+            lp_release<8>(A, __ldcg(A.lvls + soff + i), sub, A.lvl + noff, A.lvls + nsoff, A.info + L + 1);
         off = noff;
         soff = nsoff;
     }
