@@ -20,22 +20,23 @@
 // among the contig's neighbours earlier in the order, found by Kahn peeling):
 // the contigs of a level side by side, the levels in turn -- the same result
 // as the sequential sweep.  The peeling and all sweeps of a run are one
-// cooperative launch each, with a bounded grid barrier between levels (lp_wait.h);
-// a run with a contig of more than 1,024 edges is swept by a launch per level
-// instead, so that no block waits for it.  A
-// block sorts its contig's (neighbour label, edge
-// position) keys (bitonic sort in shared memory, or in a global slice for
-// contigs with more than 1,024 edges), folds each label's log(1 - score) in
-// edge order (the reference's summation order), evaluates the CDF
-// (lp_math.h, bit-identical to the host checker) and breaks exact ties by the
-// reference map's iteration order (lp_umap.h); contigs with at most 32 edges
-// take a warp each, the keys sorted across its lanes.  A contig none of whose
-// neighbours changed label since its last evaluation is skipped: the same
-// label would win and its update would change nothing -- across runs too:
-// a run's first sweep evaluates the contigs with new edges, those frozen in
-// the previous run, and those whose neighbours changed since.  The visited (contig, label)
-// pairs of a call live in an open-addressing table; a call that overfills it
-// is re-run from its starting labels with a larger table.
+// cooperative launch each, with a bounded grid barrier between levels
+// (lp_wait.h); a run with a contig of more than 1,024 edges, or whose levels are
+// wide in contigs of more than 32, is swept by a launch per level instead.
+//
+// A group of threads sorts its contig's (neighbour label, edge position) keys
+// (bitonic sort in shared memory, or in a global slice for contigs with more
+// than 1,024 edges), folds each label's log(1 - score) in edge order (the
+// reference's summation order), evaluates the CDF (lp_math.h, bit-identical to
+// the host checker) and breaks exact ties by the reference map's iteration
+// order (lp_umap.h); contigs with at most 32 edges take a warp each, the keys
+// sorted across its lanes.  A contig none of whose neighbours changed label
+// since its last evaluation is skipped: the same label would win and its update
+// would change nothing -- across runs too: a run's first sweep evaluates the
+// contigs with new edges, those frozen in the previous run, and those whose
+// neighbours changed since.  The visited (contig, label) pairs of a call live in
+// an open-addressing table; a call that overfills it is re-run from its starting
+// labels with a larger table.
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 
@@ -162,8 +163,23 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int& ta
     return r;
 }
 
+// A contig's evaluation runs in the cooperative kernel, where labels and flags
+// change while it runs (they are read past the L1 cache) and a group is a part of
+// the block, or in a launch of its level alone (kLaunch), where what it reads does
+// not change and the group is the block.  A barrier named by the thread's
+// group counts as all sixteen of a block, which limits the blocks an SM holds.
+template <bool kLaunch, class T>
+__device__ __forceinline__ T changing(const T* p) {
+    return kLaunch ? *p : __ldcg(p);
+}
+
 // Barrier of the kThreads threads of this thread's group.
+template <bool kLaunch>
 __device__ __forceinline__ void group_sync() {
+    if (kLaunch) {
+        __syncthreads();
+        return;
+    }
     asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / kThreads), "n"(kThreads) : "memory");
 }
 
@@ -175,8 +191,8 @@ struct BlockWs {
     uint32_t ties, best, changed;
 };
 
-// One contig's sweep step by a group of kThreads threads.  Labels and flags change while
-// the sweep kernel runs, so they are read past the L1 cache.
+// One contig's sweep step by a group of kThreads threads.
+template <bool kLaunch>
 __device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, BlockWs& B, Tally& T) {
     double* red_v = B.red_v;
     uint32_t* red_c = B.red_c;
@@ -186,8 +202,8 @@ __device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, 
     const uint32_t d = P.inc_off[v + 1] - s;
     // no neighbour changed since the last evaluation: the same label wins
     // and the update is a no-op
-    if (d == 0 || !__ldcg(P.dirty + v)) return;
-    group_sync();  // the group's previous contig is done with the shared arrays
+    if (d == 0 || !changing<kLaunch>(P.dirty + v)) return;
+    group_sync<kLaunch>();  // the group's previous contig is done with the shared arrays
     const uint32_t N = pow2_at_least(d);
     unsigned char* base = smem;
     if (N > kSmallCap) {
@@ -211,14 +227,14 @@ __device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, 
     for (uint32_t j = t; j < N; j += kThreads) {
         if (j < d) {
             const uint32_t o = P.oth[s + j];
-            sk[j] = ((unsigned long long)__ldcg(P.mem + o) << 32) | j;
+            sk[j] = ((unsigned long long)changing<kLaunch>(P.mem + o) << 32) | j;
             w[j] = P.ilw[s + j];
         } else {
             sk[j] = ~0ull;
         }
         fidx[j] = -1;
     }
-    group_sync();
+    group_sync<kLaunch>();
     // bitonic sort, ascending
     for (uint32_t k = 2; k <= N; k <<= 1) {
         for (uint32_t jj = k >> 1; jj > 0; jj >>= 1) {
@@ -233,7 +249,7 @@ __device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, 
                     }
                 }
             }
-            group_sync();
+            group_sync<kLaunch>();
         }
     }
     // each label's run: the Fisher-combined CDF of its edges, folded in edge
@@ -258,31 +274,31 @@ __device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, 
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
     if ((t & 31) == 0) red_v[t >> 5] = vmax;
-    group_sync();
+    group_sync<kLaunch>();
     if (t == 0) {
         double m = red_v[0];
         for (int i = 1; i < kThreads / 32; ++i) m = fmax(m, red_v[i]);
         s_vmax = m;
     }
-    group_sync();
+    group_sync<kLaunch>();
     const double top = s_vmax;
     uint32_t ties = 0;
     for (uint32_t p = t; p < d; p += kThreads) ties += val[p] == top;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ties += __shfl_xor_sync(0xffffffffu, ties, o);
     if ((t & 31) == 0) red_c[t >> 5] = ties;
-    group_sync();
+    group_sync<kLaunch>();
     if (t == 0) {
         uint32_t nt = 0;
         for (int i = 0; i < kThreads / 32; ++i) nt += red_c[i];
         s_ties = nt;
     }
-    group_sync();
+    group_sync<kLaunch>();
     if (s_ties == 1) {
         for (uint32_t p = t; p < d; p += kThreads)
             if (val[p] == top) s_best = (uint32_t)(sk[p] >> 32);
     }
-    group_sync();
+    group_sync<kLaunch>();
     if (t == 0) {
         P.dirty[v] = 0;
         if (s_ties > 1) {
@@ -304,7 +320,7 @@ __device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, 
         }
         const uint32_t b = s_best;
         s_changed = 0;
-        if (__ldcg(P.mem + v) != b && !__ldcg(P.stuck + v)) {
+        if (changing<kLaunch>(P.mem + v) != b && !changing<kLaunch>(P.stuck + v)) {
             P.mem[v] = b;
             s_changed = 1;
             if (visit(P, v, b, T))
@@ -313,7 +329,7 @@ __device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, 
                 P.stuck[v] = 1;
         }
     }
-    group_sync();
+    group_sync<kLaunch>();
     if (s_changed)
         for (uint32_t j = t; j < d; j += kThreads) {
             P.dirty[P.oth[s + j]] = 1;
@@ -354,15 +370,16 @@ __device__ __forceinline__ WarpNode lp_load(const LpArgs& P, const uint32_t* __r
     return N;
 }
 
+template <bool kLaunch>
 __device__ void lp_node_warp(const LpArgs& P, const WarpNode& N, WarpWs& W, Tally& T) {
     const uint32_t lane = threadIdx.x & 31, v = N.v, d = N.d, o = N.o;
     if (d == 0) return;
     // all that changes between sweeps, loaded side by side: only this warp
     // writes its contig's label and frozen flag
-    const uint32_t other = lane < d ? __ldcg(P.mem + o) : 0u;
-    const uint32_t mine = __ldcg(P.mem + v);
-    const uint8_t frozen = __ldcg(P.stuck + v);
-    if (!__ldcg(P.dirty + v)) return;  // as in the block form
+    const uint32_t other = lane < d ? changing<kLaunch>(P.mem + o) : 0u;
+    const uint32_t mine = changing<kLaunch>(P.mem + v);
+    const uint8_t frozen = changing<kLaunch>(P.stuck + v);
+    if (!changing<kLaunch>(P.dirty + v)) return;  // as in the block form
     __syncwarp();
     unsigned long long key = ~0ull;
     if (lane < d) {
@@ -502,7 +519,7 @@ struct LevelArgs {
     LevelInfo* info;
     uint32_t lcap;         // entries of info
     uint32_t* slot_of;
-    LevelInfo* sum;        // over all levels: count = contigs levelled, nsmall = levels, the maxima
+    LevelInfo* sum;        // over all levels: count = contigs levelled, off = block contigs, nsmall = levels, the maxima
     unsigned long long incidences;  // all of them (2 per edge)
     unsigned int* bar;
     int* flag;
@@ -608,6 +625,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_levels(LevelArgs A) {
         r.maxdeg = maxdeg;
         r.maxall = maxall;
         r.nbig = maxbig;
+        r.off = off;
         *A.sum = r;
     }
 }
@@ -647,11 +665,11 @@ __global__ void __launch_bounds__(kCoopThreads) k_lp_sweeps(LpArgs P, const uint
         for (uint32_t L = 0; L < nlevels; ++L) {
             const uint32_t off = info[L].off, soff = info[L].soff, count = info[L].count, nsmall = info[L].nsmall;
             for (uint32_t i = grp * gridDim.x + blockIdx.x; i < count; i += kGroups * gridDim.x)
-                lp_node_block(P, lvl[off + i], smem + grp * group_bytes, bws[grp], T);
+                lp_node_block<false>(P, lvl[off + i], smem + grp * group_bytes, bws[grp], T);
             for (uint32_t i = w0; i < nsmall; i += nw) {
                 const WarpNode cur = next;
                 next = lp_load(P, lvls + soff, i + nw, nsmall);
-                lp_node_warp(P, cur, W, T);
+                lp_node_warp<false>(P, cur, W, T);
             }
             // the next level's first contig, in flight across the barrier
             const uint32_t Ln = L + 1 < nlevels ? L + 1 : 0;
@@ -705,10 +723,10 @@ __global__ void __launch_bounds__(kThreads) k_lp_level(LpArgs P, const uint32_t*
     if (threadIdx.x == 0) T.moved = T.entries = 0;
     __syncthreads();
     if (blockIdx.x < count) {
-        lp_node_block(P, lvl[blockIdx.x], smem, bws, T);
+        lp_node_block<true>(P, lvl[blockIdx.x], smem, bws, T);
     } else {
         const uint32_t w = threadIdx.x >> 5, i = (blockIdx.x - count) * (kThreads / 32) + w;
-        lp_node_warp(P, lp_load(P, lvls, i, nsmall), reinterpret_cast<WarpWs*>(smem)[w], T);
+        lp_node_warp<true>(P, lp_load(P, lvls, i, nsmall), reinterpret_cast<WarpWs*>(smem)[w], T);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1034,10 +1052,18 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
     st->levels_max = std::max<uint64_t>(st->levels_max, nlevels);
     st->degree_max = std::max<uint64_t>(st->degree_max, maxall);
     maxdeg = std::max(maxdeg, kWarpCap);
-    // A contig sorted in global memory (more than kSmallCap edges) can hold its
-    // level for as long as its edges take, millions of them for seconds: no block
-    // is to wait for it inside a kernel.
-    const bool by_level = maxdeg > kSmallCap;
+    // A launch per level instead of the cooperative sweeps
+    // - for a contig sorted in global memory (more than kSmallCap edges): it can hold
+    //   its level for as long as its edges take, millions of them for seconds, and
+    //   no block is to wait for it inside a kernel;
+    // - where levels are wide in block contigs, more than a third of the groups of the
+    //   cooperative kernel on average: it holds 32 warps an SM and deals contigs out
+    //   evenly, launches hold 40 and take the next block as one ends.  (A run's
+    //   sweeps by block contigs a level, cooperative and launched: 120 of them 2.36
+    //   and 2.51 ms, 187 2.77 and 2.73, 243 3.21 and 3.12, 480 4.41 and 3.94, 940 8.85
+    //   and 7.39.  Warp contigs alone, 50,000 a level: 9.5 and 11.4 ms in ten runs.)
+    const uint64_t nblock = hsum->off;
+    const bool by_level = maxdeg > kSmallCap || nblock * 3 > (uint64_t)nlevels * kGroups * ctx->num_sms;
     std::vector<LevelInfo> levels(by_level ? nlevels : 0);
     if (by_level) {
         MDET_CUDA(ctx, cudaMemcpyAsync(levels.data(), info, nlevels * sizeof(LevelInfo), cudaMemcpyDeviceToHost, s));
