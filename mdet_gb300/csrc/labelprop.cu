@@ -1198,10 +1198,13 @@ int lp_impl(mdet_ctx* ctx, const uint64_t* d_from, const uint64_t* d_to, const d
     S.ea = (uint32_t*)ctx_scratch(ctx, "lp.ea", ne1 * 4);
     S.eb = (uint32_t*)ctx_scratch(ctx, "lp.eb", ne1 * 4);
     S.lw = (double*)ctx_scratch(ctx, "lp.lw", ne1 * 8);
-    // edges traversed per pass: a stretch starts with about n (n / 4 meant two
-    // passes a stretch: 8.0 -> 7.4 ms at 1,000,000 contigs) and takes four times as many each time it goes on (the first
-    // stretches end within the first edges; passes of 4M edges from the start
-    // took 1.0 of 6.5 ms at 60,000 contigs and 2.9M edges)
+    // edges traversed per pass: the first stretch starts with about n (n / 4 meant two
+    // passes a stretch: 8.0 -> 7.4 ms at 1,000,000 contigs), a later one with twice
+    // the edges of the stretch before it where those were more, and takes four times
+    // as many each time it goes on.  (Passes of 4M edges throughout took 1.0 of 6.5 ms at
+    // 60,000 contigs and 2.9M edges, whose stretches end within their first edges;
+    // stretches that all started with n edges, 3.8 of 39.3 ms at 200,000 contigs
+    // and 15.7M edges, whose stretches are long: 2.2 so.)
     const uint64_t kChunk = std::min<uint64_t>(ne1, 1ull << 22);
     uint64_t chunk0 = 1ull << 16;
     while (chunk0 < n && chunk0 < kChunk) chunk0 <<= 1;
@@ -1237,7 +1240,7 @@ int lp_impl(mdet_ctx* ctx, const uint64_t* d_from, const uint64_t* d_to, const d
     std::vector<double> sched;
     for (int i = 1; i <= 10; ++i) sched.push_back(max_p / 10 * i);
     size_t which = 0;
-    uint64_t pos = 0;
+    uint64_t pos = 0, stretch = 0;
     constexpr uint64_t kNone = ~0ull;
     // select the set flags of [0, cnt) into out; returns how many
     auto select = [&](const uint8_t* flags, uint64_t cnt, uint32_t* out, const char* tag) -> long long {
@@ -1267,7 +1270,7 @@ int lp_impl(mdet_ctx* ctx, const uint64_t* d_from, const uint64_t* d_to, const d
         uint64_t i_run = kNone;
         bool at_last = false, ended = false;
         // the stretch from pos, a chunk at a time, until the run position
-        uint64_t chunk = chunk0;
+        uint64_t chunk = std::max(chunk0, 2 * stretch);
         for (uint64_t p0 = pos;; chunk = std::min(4 * chunk, kChunk)) {
             const uint64_t p1 = std::min(ne, p0 + std::min(chunk, kChunk));
             unsigned long long h2[2] = {kNone, kNone};
@@ -1330,6 +1333,7 @@ int lp_impl(mdet_ctx* ctx, const uint64_t* d_from, const uint64_t* d_to, const d
                 MDET_LAUNCHED(ctx, "k_lp_append");
                 S.m2 += (uint64_t)ka;
             }
+            stretch = cend - pos;
             if (i_run != kNone || ended) break;
             p0 = end;
         }
