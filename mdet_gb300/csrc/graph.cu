@@ -149,7 +149,7 @@ __global__ void k_sample_meta(const uint32_t* __restrict__ row_map, uint64_t m, 
 
 double logit(double cutoff) { return log((1.0 / (1. - cutoff)) - 1.0); }
 
-uint64_t tc_shape_key(bool rect, bool list, uint64_t na, uint64_t nb) {
+uint64_t tc_shape_key(bool rect, bool list, uint64_t na, uint64_t nb, int kept) {
     auto lg = [](uint64_t v) {
         uint64_t b = 0;
         while (v > 1) {
@@ -158,7 +158,7 @@ uint64_t tc_shape_key(bool rect, bool list, uint64_t na, uint64_t nb) {
         }
         return b;
     };
-    return (rect ? 1ull : 0ull) | (list ? 2ull : 0ull) | (lg(na) << 2) | (lg(nb) << 10);
+    return (rect ? 1ull : 0ull) | (list ? 2ull : 0ull) | (lg(na) << 2) | (lg(nb) << 10) | (uint64_t)kept << 18;
 }
 
 int launch_autotune(mdet_ctx* ctx, std::map<uint64_t, int>& table, uint64_t key, const std::vector<int>& values,
@@ -291,7 +291,8 @@ int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const flo
             MDET_TRY(run(bn ? bn : 256));
         else
             MDET_TRY(tc_autotune(ctx, bside ? tc_shape_key(true, false, g.n, bside->nb)
-                                            : tc_shape_key(rect, prune, rect ? na : g.n, g.n),
+                                            : tc_shape_key(rect, prune, rect ? na : g.n, g.n,
+                                                           prune ? (g.n > kRowWaves ? 2 : 1) : 0),
                                  run, prune));
         unsigned long long found = 0;
         if (prune && kept) MDET_CUDA(ctx, cudaMemcpyAsync(kept, tl.total, 8, cudaMemcpyDeviceToHost, s));

@@ -290,7 +290,10 @@ int tc_autotune(mdet_ctx* ctx, uint64_t key, const std::function<int(int)>& run,
 // in `table`; later calls run the kept value.
 int launch_autotune(mdet_ctx* ctx, std::map<uint64_t, int>& table, uint64_t key, const std::vector<int>& values,
                     const std::function<int(int)>& run);
-uint64_t tc_shape_key(bool rect, bool list, uint64_t na, uint64_t nb);
+// Shape class of a filter pass.  kept: the list is that of a preparation in bands,
+// taken in equal runs (1) or in waves (2); another list (0) sweeps otherwise and
+// is a class of its own.
+uint64_t tc_shape_key(bool rect, bool list, uint64_t na, uint64_t nb, int kept = 0);
 int graph_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, double cutoff, uint32_t max_edges,
                int mode, mdet_graph_stats* st, GraphPrep& g, uint64_t* total);
 int graph_learned(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, double cutoff, uint32_t max_edges,
