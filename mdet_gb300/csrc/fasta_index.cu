@@ -16,15 +16,15 @@
 // the file).  A thread that sees a '>' settles whether it is the
 // first of its line from its own 16 bytes or, when the line began in an
 // earlier chunk, by walking back to the line's previous '\n' or '>'.  A block
-// takes a contiguous range of the file and leaves its starts in order, so one
+// takes a contiguous range of at most 384 KB and leaves its starts in order, so one
 // small launch (k_fa_compact) joins them; a file with more records in a range
-// than a block's queue holds is scanned again with the starts appended as
-// they come, and sorted.  Pass 2
-// (k_fa_records) gives each record a warp: it finds the name line's newline and
+// than a block's queue holds (records of less than 170 bytes) is scanned again
+// with the starts appended as they come, and sorted.  Pass 2 (k_fa_records) gives each record a warp: it finds the name line's newline and
 // first space with ballots over 32-byte windows, and the view's newlines are
 // the byte array's sum over its whole 64-byte blocks and a count over the bytes
 // at its two ends, so the sequence is not read again.  A scan of the
 // size-class flags places the records with size >= min_contig in file order.
+#include <algorithm>
 #include <cstring>
 
 #include <cub/cub.cuh>
@@ -81,10 +81,16 @@ __device__ __forceinline__ uint32_t flags16(uint32_t a, uint32_t b, uint32_t c, 
 // Record starts found by a block, in shared memory until the block ends: an
 // atomic on the file's one counter per record start was what the scan waited
 // for at 4 KB a record.
-constexpr uint32_t kQueue = 1536;
+// A range is at most kRange bytes (and the file's last 2 KB), so that records of 170
+// bytes and more, a raw assembly's shortest, never fill a queue: with a grid that did not
+// grow with the file, 4.3M records of 280 bytes took 5.8 ms for the second scan and
+// the sort, 3.2 so.
+constexpr uint32_t kQueue = 2304;
+constexpr uint64_t kRange = 384 * 1024;
 struct StartQueue {
-    uint64_t pos[kQueue];
+    uint32_t pos[kQueue];  // from the range's first byte
     uint32_t n;
+    uint64_t base;
 };
 
 // The '>' bytes of one 16-byte chunk at base: queues the record starts, or
@@ -103,7 +109,7 @@ __device__ __noinline__ void chunk_starts(const unsigned char* __restrict__ b, u
         if (!first) continue;
         if (sq) {
             const uint32_t slot = atomicAdd(&sq->n, 1u);
-            if (slot < kQueue) sq->pos[slot] = base + j;
+            if (slot < kQueue) sq->pos[slot] = (uint32_t)(base + j - sq->base);
         } else {
             const unsigned long long pos = atomicAdd(count, 1ull);
             if (pos < cap) starts[pos] = base + j;
@@ -119,26 +125,32 @@ __device__ __forceinline__ uint32_t chunk_newlines(const uint4& q, uint32_t& gt)
     return __dp4a(acc, 0x01010101u, 0u);
 }
 
+// First 2-KB tile of block k of a grid of g (k = g: past the last).
+__device__ __forceinline__ uint64_t range_tile(uint64_t ntile, uint32_t k, uint32_t g) { return ntile * k / g; }
+
 // A warp per 2 KB: lane l takes the 16-byte chunks l, l + 32, l + 64 and
 // l + 96, all four loads in flight.  The four chunk counts ride in one word's
 // bytes, so two shuffle-adds make the sums of all 32 64-byte blocks, a byte per
 // lane to write.
 //
-// kAppend false: the block's starts go to found[blockIdx.x * kQueue ..] in
-// order and their number (which may exceed the queue) to nfound[blockIdx.x].
+// kAppend false: the block's starts go to found[blockIdx.x * kQueue ..] in order,
+// from the first byte of its range on, and their number (which may exceed the queue) to nfound[blockIdx.x].
 // (0.93 GB, 220,000 records: 465 us with a global atomic per start, 179 us so.)
 template <bool kAppend>
 __global__ void __launch_bounds__(256) k_fa_scan(const unsigned char* __restrict__ b, uint64_t nbytes,
-                                                 uint8_t* __restrict__ nlc, uint64_t* __restrict__ found,
-                                                 uint32_t* __restrict__ nfound, uint64_t cap,
-                                                 unsigned long long* __restrict__ count) {
+                                                 uint8_t* __restrict__ nlc, uint32_t* __restrict__ found,
+                                                 uint32_t* __restrict__ nfound, uint64_t* __restrict__ starts,
+                                                 uint64_t cap, unsigned long long* __restrict__ count) {
     __shared__ StartQueue queue;
     StartQueue* sq = kAppend ? nullptr : &queue;
-    if (threadIdx.x == 0) queue.n = 0;
-    __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t ntile = nbytes / 2048;
-    const uint64_t t0 = ntile * blockIdx.x / gridDim.x, t1 = ntile * (blockIdx.x + 1) / gridDim.x;
+    const uint64_t t0 = range_tile(ntile, blockIdx.x, gridDim.x), t1 = range_tile(ntile, blockIdx.x + 1, gridDim.x);
+    if (threadIdx.x == 0) {
+        queue.n = 0;
+        queue.base = t0 * 2048;
+    }
+    __syncthreads();
     for (uint64_t tile = t0 + (threadIdx.x >> 5); tile < t1; tile += blockDim.x >> 5) {
         const uint4* p = reinterpret_cast<const uint4*>(b + tile * 2048) + lane;
         uint4 q[4];
@@ -155,7 +167,7 @@ __global__ void __launch_bounds__(256) k_fa_scan(const unsigned char* __restrict
             for (int u = 0; u < 4; ++u) {
                 const uint4 c = u == 0 ? q[0] : u == 1 ? q[1] : u == 2 ? q[2] : q[3];
                 if (u == 0 ? gt[0] : u == 1 ? gt[1] : u == 2 ? gt[2] : gt[3])
-                    chunk_starts(b, tile * 2048 + 16 * lane + 512 * u, c, sq, found, cap, count);
+                    chunk_starts(b, tile * 2048 + 16 * lane + 512 * u, c, sq, starts, cap, count);
             }
         }
     }
@@ -170,7 +182,7 @@ __global__ void __launch_bounds__(256) k_fa_scan(const unsigned char* __restrict
             const uint4 c = make_uint4(w[0], w[1], w[2], w[3]);
             uint32_t gt;
             nl += chunk_newlines(c, gt);
-            if (gt) chunk_starts(b, base, c, sq, found, cap, count);
+            if (gt) chunk_starts(b, base, c, sq, starts, cap, count);
         }
         if ((g + 1) * kBlk <= nbytes) nlc[g] = (uint8_t)nl;
     }
@@ -184,28 +196,36 @@ __global__ void __launch_bounds__(256) k_fa_scan(const unsigned char* __restrict
     }
     if (n > kQueue) return;
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {  // its place is how many lie before it
-        const uint64_t v = queue.pos[i];
+        const uint32_t v = queue.pos[i];
         uint32_t at = 0;
         for (uint32_t k = 0; k < n; ++k) at += queue.pos[k] < v;
         found[(uint64_t)blockIdx.x * kQueue + at] = v;
     }
 }
 
-// Joins the blocks' starts: block k's go after those of blocks 0 .. k - 1.
-__global__ void __launch_bounds__(256) k_fa_compact(const uint64_t* __restrict__ found,
+// Joins the blocks' starts: block k's go after those of blocks 0 .. k - 1, which
+// it counts unless `before` says how many they are.
+__global__ void __launch_bounds__(256) k_fa_compact(const uint32_t* __restrict__ found,
                                                     const uint32_t* __restrict__ nfound,
+                                                    const uint32_t* __restrict__ before, uint64_t nbytes,
                                                     uint64_t* __restrict__ starts) {
     __shared__ uint32_t part[8];
-    uint32_t before = 0;
-    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) before += nfound[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = before;
-    __syncthreads();
     uint64_t at = 0;
-    for (int w = 0; w < 8; ++w) at += part[w];
+    if (before) {
+        at = before[blockIdx.x];
+    } else {
+        uint32_t sum = 0;
+        for (uint32_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) sum += nfound[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        for (int w = 0; w < 8; ++w) at += part[w];
+    }
     const uint32_t n = nfound[blockIdx.x];
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) starts[at + i] = found[(uint64_t)blockIdx.x * kQueue + i];
+    const uint64_t base = range_tile(nbytes / 2048, blockIdx.x, gridDim.x) * 2048;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+        starts[at + i] = base + found[(uint64_t)blockIdx.x * kQueue + i];
 }
 
 // (0.93 GB, 220,000 records: k_fa_records 661 us while it read the whole views
@@ -341,15 +361,21 @@ int index_core(mdet_ctx* ctx, const char* d_bytes, uint64_t nbytes, uint64_t min
     unsigned long long* cnt = (unsigned long long*)ctx_scratch(ctx, "fa.cnt", 3 * 8);
     if (!cnt) return MDET_ERR_NOMEM;
     uint8_t* nlc = (uint8_t*)ctx_scratch(ctx, "fa.nlc", nbytes / kBlk + 4);
-    const unsigned sgrid = grid_for(ctx, nbytes / kBlk, 256);
-    uint64_t* found = (uint64_t*)ctx_scratch(ctx, "fa.found", (uint64_t)sgrid * kQueue * 8);
+    // sixteen blocks an SM, or as many as keep a range within kRange, in whole waves of
+    // eight an SM
+    unsigned sgrid = grid_for(ctx, nbytes / kBlk, 256);
+    if (nbytes / kRange + 1 > sgrid) {
+        const uint64_t wave = (uint64_t)ctx->num_sms * 8;
+        sgrid = (unsigned)((nbytes / kRange + wave) / wave * wave);
+    }
+    uint32_t* found = (uint32_t*)ctx_scratch(ctx, "fa.found", (uint64_t)sgrid * kQueue * 4);
     uint32_t* nfound = (uint32_t*)ctx_scratch(ctx, "fa.nfound", sgrid * 4ull);
     if (!nlc || !found || !nfound) return MDET_ERR_NOMEM;
     // pass 1: record starts, queued per block
     unsigned long long h_cnt[3] = {0, 0, 0};
     MDET_CUDA(ctx, cudaMemsetAsync(cnt, 0, 3 * 8, s));
     ctx_timer_begin(ctx, "k_fa_scan");
-    k_fa_scan<false><<<sgrid, 256, 0, s>>>(b, nbytes, nlc, found, nfound, 0, cnt);
+    k_fa_scan<false><<<sgrid, 256, 0, s>>>(b, nbytes, nlc, found, nfound, nullptr, 0, cnt);
     ctx_timer_end(ctx, "k_fa_scan");
     MDET_LAUNCHED(ctx, "k_fa_scan");
     MDET_CUDA(ctx, cudaMemcpyAsync(h_cnt, cnt, 16, cudaMemcpyDeviceToHost, s));
@@ -375,14 +401,25 @@ int index_core(mdet_ctx* ctx, const char* d_bytes, uint64_t nbytes, uint64_t min
     while (bits < 64 && (nbytes >> bits)) ++bits;
     if (!queued) MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(nullptr, t1, starts, sorted, (int)nr, 0, bits, s));
     MDET_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, t2, large, dst, (int)nr + 1, s));
-    void* tmp = ctx_scratch(ctx, "fa.cubtmp", t1 > t2 ? t1 : t2);
+    // each block's sum over the blocks before it, up to 3 GB; beyond, one scan
+    size_t t3 = 0;
+    uint32_t* before = nullptr;
+    if (queued && sgrid > 8192) {
+        before = (uint32_t*)ctx_scratch(ctx, "fa.before", sgrid * 4ull);
+        if (!before) return MDET_ERR_NOMEM;
+        MDET_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, t3, nfound, before, (int)sgrid, s));
+    }
+    void* tmp = ctx_scratch(ctx, "fa.cubtmp", std::max(std::max(t1, t2), t3));
     if (!tmp) return MDET_ERR_NOMEM;
     MDET_CUDA(ctx, cudaMemsetAsync(cnt, 0, 3 * 8, s));
     if (queued) {
-        k_fa_compact<<<sgrid, 256, 0, s>>>(found, nfound, sorted);
+        if (before) MDET_CUDA(ctx, cub::DeviceScan::ExclusiveSum(tmp, t3, nfound, before, (int)sgrid, s));
+        k_fa_compact<<<sgrid, 256, 0, s>>>(found, nfound, before, nbytes, sorted);
         MDET_LAUNCHED(ctx, "k_fa_compact");
     } else {
-        k_fa_scan<true><<<sgrid, 256, 0, s>>>(b, nbytes, nlc, starts, nullptr, nr, cnt);
+        ctx_timer_begin(ctx, "k_fa_scan_append");
+        k_fa_scan<true><<<sgrid, 256, 0, s>>>(b, nbytes, nlc, nullptr, nullptr, starts, nr, cnt);
+        ctx_timer_end(ctx, "k_fa_scan_append");
         MDET_LAUNCHED(ctx, "k_fa_scan");
         MDET_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, t1, starts, sorted, (int)nr, 0, bits, s));
     }
