@@ -357,8 +357,7 @@ __global__ void __launch_bounds__(1024) k_topk_big(const uint32_t* __restrict__ 
 // select (8-bit digits, most significant first).  Only kept entries with ocol
 // above the row's own index are emitted, so only those are sorted (bitonic
 // network in registers) and written to the front of the row.  topk_row does
-// this on 64-bit values, where a row's scores differ; topk_any, on the full
-// keys, takes any row.
+// this on 64-bit values; topk_any, on the full keys, takes any row.
 
 // Keys are the bit patterns of positive doubles, which order like the
 // values, so every comparison is an integer one (FP64 is slow on this part).
@@ -441,7 +440,6 @@ __device__ __forceinline__ void sort_out(const unsigned long long* __restrict__ 
 }
 
 constexpr int kSelWarps = 4;
-constexpr uint32_t kRowCap = 512;  // entries of a row staged in shared memory (28 KB a block)
 
 __device__ __forceinline__ uint32_t sel_digit(unsigned long long hi, uint32_t lo, int p) {
     return p < 8 ? (uint32_t)(hi >> (56 - 8 * p)) & 255u : (lo >> (24 - 8 * (p - 8))) & 255u;
@@ -614,22 +612,53 @@ __device__ __forceinline__ void sort_desc(unsigned long long* __restrict__ v, ui
     __syncwarp();
 }
 
-// A row of at most kRowCap entries.  A value is the score's bits above the
-// row's smallest, plus one (53 bits), then the entry's slot (10) and whether the
-// row emits it (1): distinct, and ordered like the scores.  Returns the number
-// of edges, or ~0 where this form does not do: scores that span 53 bits, or
-// equal scores whose order the columns decide.
+// The first m of the row's values, largest first (shared memory).
 template <int EMAX>
+__device__ __forceinline__ void sort_row(unsigned long long* __restrict__ x, uint32_t m, uint32_t lane) {
+    if (m <= 64)
+        sort_desc<2>(x, m, lane);
+    else if (m <= 128)
+        sort_desc<4>(x, m, lane);
+    else if (EMAX == 8 || m <= 256)
+        sort_desc<8>(x, m, lane);
+    else
+        sort_desc<EMAX>(x, m, lane);
+}
+
+// The same out of line: one copy for both sorts of a row where registers are short
+// (limits to 256: rows of 99 and 499 entries 74 and 174 us inline, 63 and 166 so; larger
+// limits 301 inline and 328 out of line at 499), and for the second sort.
+template <int EMAX>
+__device__ __noinline__ void sort_again(unsigned long long* __restrict__ x, uint32_t m, uint32_t lane) {
+    sort_row<EMAX>(x, m, lane);
+}
+
+// A row of at most 1,024 entries.  A value is the score's bits above the
+// row's smallest, plus one (53 bits), then the entry's slot (10) and whether the
+// row emits it (1): distinct, and ordered like the scores.  Equal scores go by
+// column: at the border of the kept set by a selection among them, and in the
+// emitted list by a second sort.  (40,000 contigs in genomes of 500, limit 200: 166 us,
+// and 233 to 424 with equal contigs in pairs or in groups of 5, 20, 40 or 500; 784 to
+// 1,270 where such rows went to topk_any.  Genomes of 800: 229 us, 625 by topk_any.)
+// Returns the number of edges, or ~0 where
+// this form does not do: scores that span 53 bits.
+// col: the entries' columns in shared memory, or (kStaged false) none; they are then
+// read from the row, which is written last.
+template <int EMAX, bool kStaged>
 __device__ __forceinline__ uint32_t topk_row(uint32_t cnt, uint32_t orow, uint32_t max_edges, Ent* __restrict__ row,
                                              unsigned long long* __restrict__ x, uint32_t* __restrict__ col,
                                              uint32_t* __restrict__ hist, uint32_t lane) {
+    auto column = [&](unsigned long long v) {
+        const uint32_t slot = (uint32_t)(v >> 1) & 1023u;
+        return kStaged ? col[slot] : row[slot].ocol;
+    };
     unsigned long long lo = ~0ull, hi = 0;
 #pragma unroll 4
     for (uint32_t i = lane; i < cnt; i += 32) {
         const Ent t = row[i];
         const unsigned long long v = (unsigned long long)__double_as_longlong(t.sim);
         x[i] = v;
-        col[i] = t.ocol;
+        if (kStaged) col[i] = t.ocol;
         lo = v < lo ? v : lo;
         hi = v > hi ? v : hi;
     }
@@ -643,11 +672,12 @@ __device__ __forceinline__ uint32_t topk_row(uint32_t cnt, uint32_t orow, uint32
     // the max_edges-th largest value: histograms of 8 bits from the top of the
     // row's range down, until the bin has at most 32 values
     const bool select = cnt > max_edges;
-    int shift = 64 - __clzll((long long)((hi - lo + 2) << 11)) - 8;  // at least 5
+    int shift = max(11, 64 - __clzll((long long)((hi - lo + 2) << 11)) - 8);  // score bits only
     if (select) sel_clear(hist, lane);
 #pragma unroll 2
     for (uint32_t i = lane; i < cnt; i += 32) {
-        const unsigned long long v = (x[i] - lo + 1) << 11 | i << 1 | (col[i] > orow ? 1u : 0u);
+        const uint32_t c = kStaged ? col[i] : row[i].ocol;
+        const unsigned long long v = (x[i] - lo + 1) << 11 | i << 1 | (c > orow ? 1u : 0u);
         x[i] = v;
         if (select) atomicAdd(&hist[(uint32_t)(v >> shift)], 1u);
     }
@@ -663,8 +693,8 @@ __device__ __forceinline__ uint32_t topk_row(uint32_t cnt, uint32_t orow, uint32
             __syncwarp();
             need -= above;
             pre = pre << width | bin;
-            if (count <= 32 || shift == 0) break;
-            width = shift < 8 ? shift : 8;
+            if (count <= 32 || shift == 11) break;
+            width = shift - 11 < 8 ? shift - 11 : 8;
             shift -= width;
             sel_clear(hist, lane);
             for (uint32_t i = lane; i < cnt; i += 32) {
@@ -672,59 +702,140 @@ __device__ __forceinline__ uint32_t topk_row(uint32_t cnt, uint32_t orow, uint32
                 if (v >> width == pre) atomicAdd(&hist[(uint32_t)v & ((1u << width) - 1u)], 1u);
             }
         }
-        // the bin's values, one a lane (in the histogram's place); the need-th largest
-        unsigned long long* few = reinterpret_cast<unsigned long long*>(hist);
-        uint32_t c = 0;
-        for (uint32_t base = 0; base < cnt; base += 32) {
-            const unsigned long long v = base + lane < cnt ? x[base + lane] : 0ull;
-            const bool in = v && v >> shift == pre;
-            const uint32_t bal = __ballot_sync(0xffffffffu, in);
-            if (in) few[c + __popc(bal & ((1u << lane) - 1u))] = v;
-            c += __popc(bal);
-        }
-        __syncwarp();
-        const unsigned long long mine = lane < c ? few[lane] : 0ull;
-        uint32_t rank = 0;
+        if (count > 32) {
+            // that many have the border's score: the `need` smallest columns of them, by
+            // histograms of the columns' complements; the others drop out
+            uint32_t kpre = 0;
+            int ks = 24;
 #pragma unroll 1
-        for (uint32_t k = 0; k < c; ++k) rank += few[k] > mine;
-        T = __shfl_sync(0xffffffffu, mine, __ffs(__ballot_sync(0xffffffffu, lane < c && rank + 1 == need)) - 1);
+            for (;; ks -= 8) {
+                sel_clear(hist, lane);
+                for (uint32_t i = lane; i < cnt; i += 32) {
+                    const unsigned long long v = x[i];
+                    const uint32_t key = v >> 11 == pre ? ~column(v) : 0u;
+                    if (v >> 11 == pre && (ks == 24 || key >> (ks + 8) == kpre)) atomicAdd(&hist[key >> ks & 255u], 1u);
+                }
+                __syncwarp();
+                sel_bin(hist, lane, need, bin, above, count);
+                __syncwarp();
+                need -= above;
+                kpre = kpre << 8 | bin;
+                if (count == need || ks == 0) break;
+            }
+            for (uint32_t i = lane; i < cnt; i += 32)
+                if (x[i] >> 11 == pre && ~column(x[i]) >> ks < kpre) x[i] = 0ull;
+            T = pre << 11;
+        } else {
+            // the bin's values, one a lane (in the histogram's place); the need-th largest
+            unsigned long long* few = reinterpret_cast<unsigned long long*>(hist);
+            uint32_t c = 0;
+            for (uint32_t base = 0; base < cnt; base += 32) {
+                const unsigned long long v = base + lane < cnt ? x[base + lane] : 0ull;
+                const bool in = v && v >> shift == pre;
+                const uint32_t bal = __ballot_sync(0xffffffffu, in);
+                if (in) few[c + __popc(bal & ((1u << lane) - 1u))] = v;
+                c += __popc(bal);
+            }
+            __syncwarp();
+            const unsigned long long mine = lane < c ? few[lane] : 0ull;
+            uint32_t rank = 0;
+#pragma unroll 1
+            for (uint32_t k = 0; k < c; ++k) rank += few[k] > mine;
+            T = __shfl_sync(0xffffffffu, mine, __ffs(__ballot_sync(0xffffffffu, lane < c && rank + 1 == need)) - 1);
+            // all values of T's score are in the bin; one left out makes the border a
+            // tie: of them as many as are kept go by the smallest columns
+            const bool eq = lane < c && mine >> 11 == T >> 11;
+            if (__any_sync(0xffffffffu, eq && mine < T)) {
+                const uint32_t all = __ballot_sync(0xffffffffu, eq);
+                const uint32_t keep = __popc(__ballot_sync(0xffffffffu, eq && mine >= T));
+                const uint32_t my = eq ? column(mine) : 0u;
+                uint32_t before = 0;
+#pragma unroll 1
+                for (uint32_t m = all; m; m &= m - 1) before += __shfl_sync(0xffffffffu, my, __ffs(m) - 1) < my;
+                if (eq && before >= keep) x[(uint32_t)(mine >> 1) & 1023u] = 0ull;
+                T = T >> 11 << 11;
+            }
+        }
     }
-    // the values to emit to the front; an entry left out with the score of the
-    // last one kept is a tie
+    // the values to emit to the front
     uint32_t m = 0;
-    bool tie = false;
     __syncwarp();
     for (uint32_t base = 0; base < cnt; base += 32) {
         const unsigned long long v = base + lane < cnt ? x[base + lane] : 0ull;
         const bool take = v >= T && (v & 1);
-        tie |= v && v < T && v >> 11 == T >> 11;
         const uint32_t bal = __ballot_sync(0xffffffffu, take);  // every lane has read its value
         if (take) x[m + __popc(bal & ((1u << lane) - 1u))] = v;
         m += __popc(bal);
     }
-    if (__any_sync(0xffffffffu, tie)) return ~0u;
     __syncwarp();
-    if (m <= 64)
-        sort_desc<2>(x, m, lane);
-    else if (m <= 128)
-        sort_desc<4>(x, m, lane);
-    else if (EMAX == 8 || m <= 256)
-        sort_desc<8>(x, m, lane);
+    if (EMAX == 8)
+        sort_again<EMAX>(x, m, lane);
     else
-        sort_desc<EMAX>(x, m, lane);
-    tie = false;
+        sort_row<EMAX>(x, m, lane);
+    bool tie = false;
     for (uint32_t i = lane; i + 1 < m; i += 32) tie |= x[i] >> 11 == x[i + 1] >> 11;
-    if (__any_sync(0xffffffffu, tie)) return ~0u;
-    for (uint32_t i = lane; i < m; i += 32) {
-        const unsigned long long v = x[i];
-        Ent e;
-        e.sim = __longlong_as_double((long long)((v >> 11) - 1 + lo));
-        e.ocol = col[(uint32_t)(v >> 1) & 1023u];
-        e.pad = 0;
-        row[i] = e;
+    if (__any_sync(0xffffffffu, tie)) {
+        // equal scores by column: the columns sorted behind their run's first place,
+        // in the values' upper half (a place keeps its score, so only columns move)
+        unsigned long long* y = x + 32 * EMAX;
+        uint32_t run = 0;  // where the run of the last value before this lane's starts
+        for (uint32_t base = 0; base < m; base += 32) {
+            const uint32_t i = base + lane;
+            const bool first = i < m && (i == 0 || x[i - 1] >> 11 != x[i] >> 11);
+            const uint32_t heads = __ballot_sync(0xffffffffu, first) & (0xffffffffu >> (31 - lane));
+            const uint32_t at = heads ? base + 31 - __clz(heads) : run;
+            if (i < m) y[i] = ~((unsigned long long)at << 32 | column(x[i]));
+            run = __shfl_sync(0xffffffffu, at, 31);
+        }
+        __syncwarp();
+        sort_again<EMAX>(y, m, lane);
+        for (uint32_t i = lane; i < m; i += 32) {
+            Ent e;
+            e.sim = __longlong_as_double((long long)((x[i] >> 11) - 1 + lo));
+            e.ocol = ~(uint32_t)y[i];
+            e.pad = 0;
+            row[i] = e;
+        }
+        return m;
+    }
+    if (kStaged) {
+        for (uint32_t i = lane; i < m; i += 32) {
+            const unsigned long long v = x[i];
+            Ent e;
+            e.sim = __longlong_as_double((long long)((v >> 11) - 1 + lo));
+            e.ocol = column(v);
+            e.pad = 0;
+            row[i] = e;
+        }
+    } else {
+        // the columns of all edges, kept beside the sorted values, before the row is written
+        uint32_t c[EMAX];
+#pragma unroll
+        for (int e = 0; e < EMAX; ++e) c[e] = e * 32 + lane < m ? column(x[e * 32 + lane]) : 0u;
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < EMAX; ++e) {
+            const uint32_t i = e * 32 + lane;
+            if (i >= m) break;
+            Ent t;
+            t.sim = __longlong_as_double((long long)((x[i] >> 11) - 1 + lo));
+            t.ocol = c[e];
+            t.pad = 0;
+            row[i] = t;
+        }
     }
     return m;
 }
+
+// Entries staged in shared memory per row, the columns beside them or (kLong) the
+// values alone: limits to 256 fit seven blocks an SM with 7 KB a warp, the larger ones
+// run four blocks, with room for every slot.
+template <int EMAX>
+struct RowCaps {
+    static constexpr uint32_t kShort = EMAX == 8 ? 512 : 1024, kLong = EMAX == 8 ? 880 : 1024;
+    static_assert(kShort >= 64 * EMAX, "the emitted values and the columns of equal ones");
+    static constexpr uint32_t kBytes = kShort * 12 > kLong * 8 ? kShort * 12 : kLong * 8;
+};
 
 // Bound by issue (the entries are read once, about 2,000 instructions a row): one
 // 64-bit value per entry, staged in shared memory so that the passes are short
@@ -734,24 +845,28 @@ __device__ __forceinline__ uint32_t topk_row(uint32_t cnt, uint32_t orow, uint32
 // 9.9 ms).  Seven blocks fit an SM's shared memory; 72 registers for them beat
 // 113 at four blocks (382 us, 6.8 ms).
 template <int EMAX>
-__global__ void __launch_bounds__(kSelWarps * 32, EMAX == 8 ? 7 : 4) k_topk_sel(const unsigned long long* __restrict__ rowptr,
-                                                             const uint32_t* __restrict__ deg,
-                                                             const uint32_t* __restrict__ perm, uint32_t n,
-                                                             uint32_t max_edges_all, const uint32_t* __restrict__ blk_K,
-                                                             Ent* __restrict__ list, uint32_t* __restrict__ out_cnt) {
-    __shared__ unsigned long long s_x[kSelWarps][kRowCap];
-    __shared__ uint32_t s_col[kSelWarps][kRowCap];
-    __shared__ __align__(16) uint32_t s_hist[kSelWarps][256];
+__global__ void __launch_bounds__(kSelWarps * 32, EMAX == 8 ? 7 : 4)
+    k_topk_sel(const unsigned long long* __restrict__ rowptr, const uint32_t* __restrict__ deg,
+               const uint32_t* __restrict__ perm, uint32_t n, uint32_t max_edges_all,
+               const uint32_t* __restrict__ blk_K, Ent* __restrict__ list, uint32_t* __restrict__ out_cnt) {
+    using C = RowCaps<EMAX>;
+    extern __shared__ __align__(16) unsigned char sel_smem[];
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* base = sel_smem + w * (C::kBytes + 1024);
+    uint32_t* hist = reinterpret_cast<uint32_t*>(base);
+    unsigned long long* x = reinterpret_cast<unsigned long long*>(base + 1024);
+    uint32_t* col = reinterpret_cast<uint32_t*>(base + 1024 + C::kShort * 8);
     for (uint32_t sp = blockIdx.x * kSelWarps + w; sp < n; sp += gridDim.x * kSelWarps) {
         const uint32_t cnt = deg[sp], orow = perm[sp];
         const uint32_t max_edges = blk_K ? blk_K[sp >> 8] : max_edges_all;
         Ent* row = list + rowptr[sp];
         uint32_t m = cnt ? ~0u : 0u;
-        if (cnt && cnt <= kRowCap)
-            m = topk_row<EMAX>(cnt, orow, max_edges, row, s_x[w], s_col[w], s_hist[w], lane);
+        if (cnt && cnt <= C::kShort)
+            m = topk_row<EMAX, true>(cnt, orow, max_edges, row, x, col, hist, lane);
+        else if (EMAX == 8 && cnt && cnt <= C::kLong)
+            m = topk_row<EMAX, false>(cnt, orow, max_edges, row, x, col, hist, lane);
         __syncwarp();
-        if (m == ~0u) m = topk_any<EMAX>(cnt, orow, max_edges, row, s_x[w], s_col[w], s_hist[w], lane);
+        if (m == ~0u) m = topk_any<EMAX>(cnt, orow, max_edges, row, x, col, hist, lane);
         if (lane == 0) out_cnt[orow] = m;
         __syncwarp();
     }
@@ -956,10 +1071,14 @@ int select_topk(mdet_ctx* ctx, const GraphPrep& g, const Edge* edges, unsigned l
         const unsigned blocks =
             (unsigned)std::min<uint64_t>(((uint64_t)n + kSelWarps - 1) / kSelWarps, (uint64_t)ctx->num_sms * 32);
         ctx_timer_begin(ctx, "k_topk_sel");
-        if (max_edges <= 256)
-            k_topk_sel<8><<<blocks, kSelWarps * 32, 0, s>>>(rowptr, deg, g.perm, n, max_edges, blk_K, list, out_cnt);
-        else
-            k_topk_sel<16><<<blocks, kSelWarps * 32, 0, s>>>(rowptr, deg, g.perm, n, max_edges, blk_K, list, out_cnt);
+        if (max_edges <= 256) {
+            constexpr size_t dyn = kSelWarps * (RowCaps<8>::kBytes + 1024);
+            k_topk_sel<8><<<blocks, kSelWarps * 32, dyn, s>>>(rowptr, deg, g.perm, n, max_edges, blk_K, list, out_cnt);
+        } else {
+            constexpr size_t dyn = kSelWarps * (RowCaps<16>::kBytes + 1024);
+            MDET_CUDA(ctx, cudaFuncSetAttribute(k_topk_sel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+            k_topk_sel<16><<<blocks, kSelWarps * 32, dyn, s>>>(rowptr, deg, g.perm, n, max_edges, blk_K, list, out_cnt);
+        }
         ctx_timer_end(ctx, "k_topk_sel");
         MDET_LAUNCHED(ctx, "k_topk_sel");
     } else {
