@@ -79,7 +79,7 @@ struct mdet_ctx {
         const void* tnf = nullptr;
         const void* ls = nullptr;
         uint64_t n = 0;
-        bool by_size = false;  // strictly by size, not in bands
+        bool by_size = false;  // in ascending size, not in bands
         int tck = 0;  // reduced-precision rows made (0 none, 1 BF16, 2 TF32)
         unsigned long long hash = 0;
         const void* x32 = nullptr;

@@ -367,7 +367,7 @@ int graph_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n
     if (mode == MDET_MODE_LEARNED) return graph_learned(ctx, d_tnf, d_ls, n, cutoff, max_edges, st, g, total);
     PhaseTimer tm(ctx->stream);
     tm.mark();
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, tc_kind(mode), &g, nullptr, !in_bands(n, mode)));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, tc_kind(mode), &g, nullptr, graph_order(n, mode)));
     MDET_TRY(abd_gate(ctx, g));
     const double L = logit(cutoff);
     DstarTable tbl;
@@ -432,7 +432,7 @@ int graph_shard_core(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint
     if (max_edges > 512) return ctx_fail(ctx, MDET_ERR_INVALID, "row shards need max_edges <= 512");
     PhaseTimer tm(ctx->stream);
     tm.mark();
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, tc_kind(mode), &g, nullptr, true));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, tc_kind(mode), &g, nullptr, PrepOrder::size));
     MDET_TRY(abd_gate(ctx, g));
     const uint64_t blocks = (n + 255) / 256;
     const uint32_t s0 = (uint32_t)std::min<uint64_t>(n, blocks * shard / nshards * 256);
@@ -709,7 +709,7 @@ int mdet_tnf_pair_scores_dev(mdet_ctx* ctx, const float* d_tnf, const double* d_
     if (!d_tnf || !d_log_size || !d_pairs || (!d_dist && !d_prob)) return ctx_fail(ctx, MDET_ERR_INVALID, "null pointer");
     if (n < 1 || n >= (1ull << 31)) return ctx_fail(ctx, MDET_ERR_INVALID, "bad contig count");
     GraphPrep g;
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, false, &g, nullptr, true));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, false, &g, nullptr, PrepOrder::any));
     MDET_TRY(pair_scores(ctx, g, d_pairs, m, d_dist, d_prob));
     MDET_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return check_flag(ctx);
@@ -731,7 +731,7 @@ int mdet_tnf_max_prob_dev(mdet_ctx* ctx, const float* d_tnf, const double* d_log
     // TF32 is asked for.
     if (mode == MDET_MODE_TF32) mode = MDET_MODE_BF16;
     GraphPrep g;
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, mode != MDET_MODE_PLAIN, &g, nullptr, true));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, mode != MDET_MODE_PLAIN, &g, nullptr, PrepOrder::size));
     MDET_TRY(maxprob_core(ctx, g, d_contigs, m, mode, floor_prob, d_out));
     return check_flag(ctx);
 }
@@ -774,7 +774,7 @@ int mdet_tnf_ptnf_search_dev(mdet_ctx* ctx, const float* d_tnf, const double* d_
     // maxima are exact whatever the filter form; see mdet_tnf_max_prob_dev)
     if (mode == MDET_MODE_TF32) mode = MDET_MODE_BF16;
     GraphPrep g;
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, mode != MDET_MODE_PLAIN, &g, nullptr, !in_bands(n, mode)));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_log_size, n, mode != MDET_MODE_PLAIN, &g, nullptr, graph_order(n, mode)));
     std::vector<uint64_t> idx(n);
     // sparse shuffle state: open addressing over positions (key ~0: empty)
     std::vector<uint64_t> mkey, mval;

@@ -131,18 +131,22 @@ inline int tc_kind(int mode) {
 }
 
 // Prepares the contigs in bands of ascending log size and by GC projection
-// within a band, in ascending log-size order (by_size), or in `order`
+// within a band, in ascending log-size order, in whichever of the two is in place
+// already (by size when neither is), or in `order`
 // (original index per position, device) when given.  tck: the reduced-precision rows
 // to make (kTcNone, kTcBf16, kTcTf32; a bool true means kTcBf16).
+enum class PrepOrder { bands, size, any };
 int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, int tck, GraphPrep* out,
-                const uint32_t* order = nullptr, bool by_size = false);
+                const uint32_t* order = nullptr, PrepOrder how = PrepOrder::bands);
 // Whether a graph (and the cutoff search before it, which shares the
 // preparation) takes the order in bands: the tensor-core forms, from 8,192
 // contigs on.  At 8,192 the list leaves out 31 % of 2,080 tiles, as much time as
 // making it takes (two passes of k_tile_keep and a scan, 15 us); at 20,000 52 %
 // (TF32 filter 206 -> 111 us), at 1,000,000 69 % (104 -> 45 ms).  The plain form
 // evaluates every pair.
-inline bool in_bands(uint64_t n, int mode) { return mode != MDET_MODE_PLAIN && n >= 8192; }
+inline PrepOrder graph_order(uint64_t n, int mode) {
+    return mode != MDET_MODE_PLAIN && n >= 8192 ? PrepOrder::bands : PrepOrder::size;
+}
 // The tiles (row-major, I * tiles_b + J) of the triangular schedule with column
 // tiles of bn that can hold a pair within tbl's bound; entries of row tile I
 // are [rowoff[I], rowoff[I + 1]), all counts on the device.

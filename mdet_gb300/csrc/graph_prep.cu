@@ -835,12 +835,12 @@ int prep_set(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, const Gr
     return prep_rows(ctx, set, rows, tck, g, nullptr, nullptr);
 }
 
-// Rows in bands of size (by_size: strictly by size; or in the caller's order).
-// A preparation of the very
-// same inputs that is still in place (same pointers and contents, no count
-// since) is used as it is: the search and the graph of one assembly share it.
+// Rows in bands of size, strictly by size, or in the caller's order.  A preparation
+// of the very same inputs that is still in place (same pointers and contents, no
+// count since) is used as it is: the search and the graph of one assembly share it,
+// and a call that takes any order (PrepOrder::any) leaves it there.
 int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, int tck, GraphPrep* g,
-                const uint32_t* order, bool by_size) {
+                const uint32_t* order, PrepOrder how) {
     g->n = (uint32_t)n;
     g->npad = (uint32_t)((n + 255) / 256 * 256);
     MDET_TRY(prep_alloc(ctx, "pre", g->npad, tck, 1, g));
@@ -852,6 +852,8 @@ int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t 
         MDET_TRY(scan_rows(ctx, set, g->npad, tck, false, g->mu, nullptr, &sb));
         return prep_rows(ctx, set, g->npad, tck, *g, order, nullptr);
     }
+    const bool by_size =
+        how == PrepOrder::any ? !(c.valid && c.tnf == d_tnf && c.ls == d_ls && c.n == n) || c.by_size : how == PrepOrder::size;
     float* proj = nullptr;
     if (!by_size) {
         proj = (float*)ctx_scratch(ctx, "pre.proj", n * 4);

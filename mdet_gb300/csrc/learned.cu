@@ -408,7 +408,7 @@ int mdet_mlp_train(mdet_ctx* ctx, mdet_mlp* m, const float* d_tnf, const double*
     memset(&r, 0, sizeof(r));
     GraphPrep g;
     const int mode = (ctx->cc_major == 10 && ctx->cc_minor == 3) ? MDET_MODE_BF16 : MDET_MODE_PLAIN;
-    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, mode != MDET_MODE_PLAIN, &g, nullptr, true));
+    MDET_TRY(prep_sorted(ctx, d_tnf, d_ls, n, mode != MDET_MODE_PLAIN, &g, nullptr, PrepOrder::size));
     uint2* cand = nullptr;
     uint64_t ncand = 0;
     MDET_TRY(graph_candidates(ctx, g, tp->label_cutoff, mode, &cand, &ncand));
