@@ -242,8 +242,10 @@ int run_filter(mdet_ctx* ctx, int mode, const GraphPrep& g, bool rect, const flo
     // entries are 32-bit).  Up to kRowWaves contigs every CTA takes an equal run
     // of the list (the rows stay in L2); beyond, the row tiles go out in waves by GC
     // projection, so that concurrent CTAs sweep the same B tiles and their pairs
-    // share rows.
-    constexpr uint64_t kRowWaves = 200000;
+    // share rows.  (Graph in us by runs and by waves: 100,000 contigs 2,756 and 2,965,
+    // 150,000 4,581 and 4,713, 200,000 6,789 and 6,613, 250,000 9,135 and 8,925, 400,000
+    // 18.4 and 17.1 ms.)
+    constexpr uint64_t kRowWaves = 180000;
     const bool prune = !rect && !bside && !tiles && g.prange && mode != MDET_MODE_PLAIN &&
                        (uint64_t)(g.n / 128 + 1) * (g.n / 128 + 1) < (1ull << 32) && ctx->forced_shape != 256128;
     TileList tl{};

@@ -118,8 +118,9 @@ struct ScanStat {
 // float-float (250,000 contigs: 163 us for the FP64 adds of a separate pass
 // and 79 us for a separate hash; 66 us here without projections, 76 us with, 136 MB); the last block of a
 // segment turns them into means.  rpb is 256, the size of a segment's blocks,
-// or 64 up to 65,536 rows, where 256 would leave SMs without a block (1,500
-// contigs: 22 us with 256, 10 us with 64).
+// or 64 up to 65,536 rows, where 256 would leave SMs without a block (us with 64
+// and 256: 1,500 contigs 10 and 22, 16,000 20 and 34, 65,000 38 and 40, 100,000 54 and
+// 45, 262,000 102 and 85).
 __global__ void __launch_bounds__(kScanWarps * 32) k_scan(PrepSet v, uint32_t rpb, double* __restrict__ sums,
                                                           uint32_t* __restrict__ done, float* __restrict__ mu,
                                                           ScanStat* __restrict__ stat, float* __restrict__ proj,
@@ -749,12 +750,13 @@ static int scan_rows(mdet_ctx* ctx, const PrepSet& set, uint64_t rows, int tck, 
     return MDET_OK;
 }
 
-// Width of the log-size bands of a whole graph's order.  Within a band the
-// blocks are narrow in the GC projection, so wider bands (more blocks in each)
-// leave more tiles empty but loosen the tiles' distance bound, by 0.9 % of d*
-// at 0.1 and 2 % at 0.2: at 131,000 contigs 39, 54, 60 and 63 % of the tiles are
-// empty at widths 0.02, 0.05, 0.1 and 0.2, at 32,000 8, 28, 42 and 52 %.
-static float band_inv_width(uint64_t n) { return n > 500000 ? 20.f : n > 65536 ? 10.f : 5.f; }
+// Bands of log size per unit in a whole graph's order.  Within a band the blocks
+// are narrow in the GC projection, so wider bands (more blocks in each) leave more
+// tiles empty but loosen the tiles' distance bound (more candidates to score).
+// The graph's time in us at 5, 10, 20 and 40 bands: 9,000 contigs 420, 408, 404, 400;
+// 30,000 876, 859, 870, 905; 100,000 2,966, 2,759, 2,790, 2,863; 250,000 8,971, 8,891,
+// 9,066, 9,362; 600,000 31.9, 31.0, 31.1, 32.2 ms; 1,000,000 74.1, 71.6, 70.9, 72.6.
+static float band_inv_width(uint64_t n) { return n > 700000 ? 20.f : 10.f; }
 
 // Everything after the scan: the order, the rows, the metadata.  With proj (one
 // set) the order is by size bands and GC projection, else by size or the
