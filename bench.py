@@ -249,8 +249,8 @@ def abundance_leg(ctx, a, d_tnf, d_ls, n, cutoff, d_from, d_to, d_st, cap, mode,
     leg = {"metric": "sTNF -> sSCR edge scoring throughput", "value": ne / call_s, "unit": "edges/s",
            "edges": int(ne), "samples": ABD_SAMPLES, "ms_per_call": call_s * 1e3,
            "k_abd_score_ms": score_ms / max(score_n, 1), "ranks_ms": parts_ms["abd_ranks"],
-           "k_sscr_ms": parts_ms["k_sscr"], "bound": "float-float crossing points and erfc per edge and sample (FP32 pipes), the CDF "
-                    "combination and the branch tests in FP64",
+           "k_sscr_ms": parts_ms["k_sscr"], "bound": "float-float crossing points and erfc per edge and sample (FP32 pipes), the "
+                    "correlation's cross sum in FP64",
            "gated_graph_ms": st["ms_total"], "data": "synthetic coverage (synth.abundance, seed 20240607)"}
     if run_cpu:
         from oracle import oracle

@@ -305,7 +305,7 @@ int graph_learned(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_
 // Candidate pairs (prepared positions) of the triangular pass at `cutoff`.
 int graph_candidates(mdet_ctx* ctx, const GraphPrep& g, double cutoff, int mode, uint2** cand, uint64_t* ncand);
 // A-role BF16 rows of a prepared set gathered for a rectangular pass
-// (row_map: ascending prepared positions on the device, m entries), padded
+// (row_map: prepared positions on the device, m entries in the pass's order), padded
 // to 256 rows, with their norms and block metadata.
 struct RowSet {
     uint16_t* ab;
