@@ -138,11 +138,13 @@ inline int tc_kind(int mode) {
 enum class PrepOrder { bands, size, any };
 int prep_sorted(mdet_ctx* ctx, const float* d_tnf, const double* d_ls, uint64_t n, int tck, GraphPrep* out,
                 const uint32_t* order = nullptr, PrepOrder how = PrepOrder::bands);
-// Whether a graph (and the cutoff search before it, which shares the
-// preparation) takes the order in bands: the tensor-core forms, from 8,192
-// contigs on.  At 8,192 the list leaves out 31 % of 2,080 tiles, as much time as
-// making it takes (two passes of k_tile_keep and a scan, 15 us); at 20,000 52 %
-// (TF32 filter 206 -> 111 us), at 1,000,000 69 % (104 -> 45 ms).  The plain form
+// The order of a graph (and of the cutoff search before it, which shares the
+// preparation): in bands for the tensor-core forms from 8,192 contigs on.  The tiles
+// that it leaves out pay for the projections and the list from there on in TF32 and
+// from 12,000 to 16,000 contigs on in BF16 (the graph in us in bands and by size, TF32
+// and BF16: 8,300 contigs 390 and 393, 398 and 377; 12,000 495 and 503, 483 and 486;
+// 16,000 587 and 612, 563 and 562; 20,011 671 and 729, 637 and 664; 100,000 3,318 and
+// 4,791, 2,756 and 3,515; BF16's filter at 1,000,000 43 and 104 ms).  The plain form
 // evaluates every pair.
 inline PrepOrder graph_order(uint64_t n, int mode) {
     return mode != MDET_MODE_PLAIN && n >= 8192 ? PrepOrder::bands : PrepOrder::size;

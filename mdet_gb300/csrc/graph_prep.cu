@@ -1008,6 +1008,39 @@ __global__ void __launch_bounds__(256) k_tile_keep(const BlockMeta* __restrict__
     }
 }
 
+// The list in one launch: warp per row tile, lane k keeps the ballot of the k-th 32
+// column tiles, and the row's entries go where the counter says, in no order of the
+// rows.  Up to 65,536 contigs (the graph in us with two passes and a scan, and so: 20,011
+// contigs 646 and 631, 50,000 1,322 and 1,311); larger sets want neighbouring row tiles in
+// turn (100,000: 2,759 and 2,850).
+constexpr uint32_t kListRows = 65536;
+template <int W>
+__global__ void __launch_bounds__(256) k_tile_list(const BlockMeta* __restrict__ meta, const float2* __restrict__ pr,
+                                                   DstarTable tbl, uint32_t ta, uint32_t tb, uint32_t nblk,
+                                                   unsigned long long* __restrict__ total,
+                                                   uint32_t* __restrict__ list) {
+    const uint32_t I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, j0 = I / W;
+    if (I >= ta) return;
+    uint32_t mine = 0;
+    for (uint32_t j = j0, k = 0; j < tb; j += 32, ++k) {
+        const uint32_t J = j + lane;
+        const bool keep = J < tb && tile_kept<W>(meta, pr, tbl, I, J, nblk);
+        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+        if (lane == k) mine = bal;
+    }
+    const uint32_t own = __popc(mine);
+    uint32_t upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= (uint32_t)o) upto += u;
+    }
+    unsigned long long at = 0;
+    if (lane == 31 && upto) at = atomicAdd(total, (unsigned long long)upto);
+    at = __shfl_sync(0xffffffffu, at, 31) + (upto - own);
+    for (; mine; mine &= mine - 1) list[at++] = I * tb + j0 + 32 * lane + __ffs(mine) - 1;
+}
+
 // Key of the row tile at every position of the order by projection: its group
 // of `group` tiles, within the group the longest list first.
 __global__ void k_wave_keys(const uint32_t* __restrict__ by_mid, const unsigned long long* __restrict__ cnt,
@@ -1035,6 +1068,16 @@ int kept_tiles(mdet_ctx* ctx, const GraphPrep& g, const DstarTable& tbl, int bn,
     if (wave && !(mid = (uint32_t*)ctx_scratch(ctx, "tl.mid", 5ull * ta * 4))) return MDET_ERR_NOMEM;
     const BlockMeta* meta = g.meta ? g.meta : g.meta32;
     const unsigned blocks = (unsigned)(((uint64_t)(ta + 1) * 32 + 255) / 256);
+    if (!wave && g.n <= kListRows) {  // at most 512 column tiles, 32 a lane
+        MDET_CUDA(ctx, cudaMemsetAsync(off + ta, 0, 8, s));
+        if (bn == 256)
+            k_tile_list<2><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, off + ta, list);
+        else
+            k_tile_list<1><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, off + ta, list);
+        MDET_LAUNCHED(ctx, "k_tile_list");
+        *out = TileList{list, nullptr, off + ta, nullptr};
+        return MDET_OK;
+    }
     for (int fill = 0; fill < 2; ++fill) {
         if (bn == 256)
             k_tile_keep<2><<<blocks, 256, 0, s>>>(meta, g.prange, tbl, ta, tb, nblk, cnt, off, fill ? list : nullptr,
