@@ -8,7 +8,7 @@
 // exact integers; TNF = float(c / sqrt(sum float(c*c))).
 //
 // GB300 layout: the sequence bytes sit in HBM exactly as the FASTA reader
-// left them (newlines included).  Work is cut into pieces of 2 to 64 KB of
+// left them (newlines included).  Work is cut into pieces of 4 to 64 KB of
 // one contig (by the size of the whole); each warp takes pieces from a global counter, and each lane
 // walks a contiguous 1/32 of the piece with its own rolling state
 // (16-byte loads, the next one in flight), warmed up on the bytes just
@@ -34,8 +34,12 @@ namespace {
 
 constexpr int kWarps = 8;
 constexpr uint64_t kPiece = 65536;  // most bytes per piece
-constexpr uint64_t kMinPiece = 2048;
-constexpr uint64_t kPlanContigs = 8192;  // most contigs of the one-block plan
+constexpr uint64_t kMinPiece = 8192, kTinyPiece = 4096;  // least bytes; of buffers below kTinyBytes
+constexpr uint64_t kTinyBytes = 4 << 20;
+// Most contigs and map entries of the one-block plan, which fills the map alone (the call in
+// us with the general plan and with this: 8,192 contigs of 100 KB, 58,000 entries, 638
+// and 631; of 600 KB, 158,000 entries, 3,202 and 3,229).
+constexpr uint64_t kPlanContigs = 8192, kPlanMap = 65536;
 constexpr uint32_t kPoison = 0xFF00u;
 
 struct FoldTables {
@@ -419,14 +423,17 @@ static cudaError_t count_phase2(const CountScratch& S, const unsigned char* d_by
     return count_launch(S, d_bytes, d_off, d_len, n, piece, nullptr, total, d_counts, d_tnf, flag, grid, s);
 }
 
-// Bytes per piece: 64 KB (a warp's fixed work per piece, the fold of its
-// histogram, is then under 1 %), halved while the buffer would give the
-// chip's warps less than two pieces each: a lane walks its share of a piece
-// alone, at about 35 ns a byte, so a small set is as slow as one piece.  (300
-// contigs, 2.5 MB: k_count 72 us with 64 KB, 20 us with 2 KB.)
+// Bytes per piece: 64 KB, halved while the buffer would give the chip's warps less
+// than two pieces each: a lane walks its share of a piece alone, at about 35 ns a byte,
+// so a small set is as slow as one piece.  Not below 8 KB (4 KB in buffers of less than
+// 4 MB): a contig in several pieces adds up its 136 counts by atomics.  (The call in us
+// with pieces of 64, 16, 8, 4 and 2 KB, log-normal lengths: 2.4 MB in 300 contigs 100, 62,
+// 56, 51, 54; 16 MB 113, 65, 63, 76, 74; 66 MB 154, 121, 115, 131, 157; 130 MB 218, 181, 182,
+// 195, 232; 238 MB 281, 254, 258, 290, 362; 482 MB 438, 414, 430, 494, 648.)
 static uint64_t piece_bytes(uint64_t nbytes, int grid) {
+    const uint64_t least = nbytes < kTinyBytes ? kTinyPiece : kMinPiece;
     uint64_t p = kPiece;
-    while (p > kMinPiece && nbytes / p < 2ull * grid * kWarps) p >>= 1;
+    while (p > least && nbytes / p < 2ull * grid * kWarps) p >>= 1;
     return p;
 }
 
@@ -483,7 +490,7 @@ static int count_impl(mdet_ctx* ctx, const char* d_bytes, uint64_t nbytes, const
     // A small set is planned by one block and counted without a host check in
     // between; views that overlap may need more pieces than the buffer's
     // bytes do, in which case the general path below counts them.
-    if (n <= kPlanContigs && cap < 0xFFFFFFFFull) {
+    if (n <= kPlanContigs && cap <= kPlanMap) {
         S.pmap = (uint32_t*)ctx_scratch(ctx, "cnt.pmap", cap * 4);
         if (!S.pmap) return MDET_ERR_NOMEM;
         unsigned long long* h = (unsigned long long*)ctx_pinned(ctx, 64);
