@@ -416,7 +416,8 @@ __global__ void k_abd_score(ScoreArgs p) {
             if (i > 0) sxy += a.dev * b.dev * __ldg(p.ratio + i - 1);
         }
         if (k == 0) atomicAdd(p.bad, 1ull);
-        p.raw[e] = sum / (double)k;
+        const double mean = sum / (double)k;
+        p.raw[e] = mean != mean ? __longlong_as_double(0x7ff8000000000000ll) : mean;  // a NaN sorts last, whatever its sign was on the way
         p.nnz[e] = k;
         if (p.corr) p.cor[e] = sxy / (__ldg(p.sx + r1) * __ldg(p.sx + r2));
     }
