@@ -26,7 +26,7 @@
 //
 // A group of threads sorts its contig's (neighbour label, edge position) keys
 // (bitonic sort in shared memory, or in a global slice for contigs with more
-// than 1,024 edges), folds each label's log(1 - score) in edge order (the
+// than 2,048 edges), folds each label's log(1 - score) in edge order (the
 // reference's summation order), evaluates the CDF (lp_math.h, bit-identical to
 // the host checker) and breaks exact ties by the reference map's iteration
 // order (lp_umap.h); contigs with at most 32 edges take a warp each, the keys
@@ -57,6 +57,7 @@ int check_flag(mdet_ctx* ctx);
 namespace {
 
 constexpr uint32_t kSmallCap = 1024;  // incident edges a group sorts in shared memory (four areas per SM)
+constexpr uint32_t kLaunchCap = 2048; // the same where the group is a block
 constexpr uint32_t kWarpCap = 32;     // incident edges a warp sorts in registers
 constexpr int kThreads = 256;         // threads that evaluate one block contig
 // The cooperative kernels run one block of 32 warps per SM, four groups of
@@ -206,7 +207,7 @@ __device__ void lp_node_block(const LpArgs& P, uint32_t v, unsigned char* smem, 
     group_sync<kLaunch>();  // the group's previous contig is done with the shared arrays
     const uint32_t N = pow2_at_least(d);
     unsigned char* base = smem;
-    if (N > kSmallCap) {
+    if (N > (kLaunch ? kLaunchCap : kSmallCap)) {
         const uint32_t slot = P.slot_of[v];
         if (slot >= P.big_slots) {
             if (threadIdx.x == 0) atomicOr(P.counters + 2, kErrSlots);
@@ -953,13 +954,13 @@ int sweeps_by_level(mdet_ctx* ctx, const LpArgs& P, const uint32_t* lvl, const u
                     const std::vector<LevelInfo>& info, unsigned long long* hc) {
     cudaStream_t s = ctx->stream;
     MDET_CUDA(ctx, cudaFuncSetAttribute(k_lp_level, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)ws_bytes(kSmallCap)));
+                                        (int)ws_bytes(kLaunchCap)));
     unsigned long long before = 0, low = INT_MAX, attempt = 0, sweeps = 0;
     while (true) {
         for (const LevelInfo& h : info) {
             const uint32_t wblocks = (h.nsmall + kThreads / 32 - 1) / (kThreads / 32);
             size_t dyn = wblocks ? (kThreads / 32) * sizeof(WarpWs) : 0;
-            if (h.count) dyn = std::max(dyn, ws_bytes(std::min<uint32_t>(pow2_at_least(h.maxdeg), kSmallCap)));
+            if (h.count) dyn = std::max(dyn, ws_bytes(std::min<uint32_t>(pow2_at_least(h.maxdeg), kLaunchCap)));
             k_lp_level<<<h.count + wblocks, kThreads, dyn, s>>>(P, lvl + h.off, h.count, lvls + h.soff, h.nsmall);
             MDET_LAUNCHED(ctx, "k_lp_level");
         }
@@ -1053,9 +1054,9 @@ int lp_call(mdet_ctx* ctx, LpState& S, mdet_lp_stats* st) {
     st->degree_max = std::max<uint64_t>(st->degree_max, maxall);
     maxdeg = std::max(maxdeg, kWarpCap);
     // A launch per level instead of the cooperative sweeps
-    // - for a contig sorted in global memory (more than kSmallCap edges): it can hold
-    //   its level for as long as its edges take, millions of them for seconds, and
-    //   no block is to wait for it inside a kernel;
+    // - for a contig of more than kSmallCap edges (sorted in global memory from
+    //   kLaunchCap on): it can hold its level for as long as its edges take, millions of
+    //   them for seconds, and no block is to wait for it inside a kernel;
     // - where levels are wide in block contigs, more than a third of the groups of the
     //   cooperative kernel on average: it holds 32 warps an SM and deals contigs out
     //   evenly, launches hold 40 and take the next block as one ends.  (A run's

@@ -1,5 +1,5 @@
-"""Label propagation with contigs of more edges than a group sorts in shared memory
-(1,024), which are swept by a launch per level: degrees around that limit, hubs with
+"""Label propagation with contigs of more edges than a group or a block sorts in shared memory
+(1,024; 2,048), which are swept by a launch per level: degrees around those limits, hubs with
 exact ties and with distinct scores, among chains and cliques."""
 import numpy as np
 import pytest
@@ -17,7 +17,7 @@ def _check(ctx, fr, to, sc, n, **kw):
     return st
 
 
-@pytest.mark.parametrize("degree", [1022, 1023, 1024, 1025, 2049, 40000])
+@pytest.mark.parametrize("degree", [1022, 1023, 1024, 1025, 2047, 2048, 2049, 2300, 40000])
 @pytest.mark.parametrize("scores", ["distinct", "ties"])
 def test_hub_among_cliques(gpu_ctx, degree, scores):
     rng = np.random.default_rng(degree)
