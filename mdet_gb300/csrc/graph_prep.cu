@@ -63,7 +63,7 @@ __global__ void k_keys(PrepSet v, uint64_t rows, unsigned long long* __restrict_
 
 // Order of a whole graph: bands of log size, `inv_h` per unit, and within a
 // band the GC projection in 16 bits.  Any order gives the same graph; this one
-// makes most tiles provably empty (k_tile_keep).
+// makes most tiles provably empty (tile_kept).
 __global__ void k_band_keys(const double* __restrict__ ls, const float* __restrict__ proj, uint64_t n, float inv_h,
                             uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
